@@ -207,3 +207,24 @@ def tolerance(case):
         return {"rel": 4e-5, "max": 1.5e-4}
     terms = case["k"] * (2 if case["kind"] == "complex" else 1)
     return {"rel": 1e-6, "max": 6e-6} if terms <= 4096 else {"rel": 2.5e-6, "max": 1.2e-5}
+
+
+def exact(case, seed):
+    """What run(prepare(case, seed)) returns, from FP64 products of the same operands."""
+    s = prepare(dict(case, kind="sgemm", values="normal", layouts="rrr", beta=0.0) if case["kind"] == "packed" else case,
+                seed)
+    kind = case["kind"]
+    if kind == "complex":
+        return s["a"].to(torch.complex128) @ s["b"].to(torch.complex128)
+    if kind == "host":
+        return (s["a"].to(DEVICE).double() @ s["b"].to(DEVICE).double()).cpu()
+    if kind == "pointers":  # column-major storage: c holds the transpose of a^T b
+        return torch.bmm(s["b"].double(), s["a"].double().transpose(1, 2))
+    if kind == "strided":
+        return torch.bmm(s["a"].double(), s["b"].double())
+    c = s["a"].double() @ s["b"].double()
+    if kind == "sgemm":
+        c *= case["alpha"]
+        if case["beta"] != 0.0:
+            c += case["beta"] * s["c"].double()
+    return c
