@@ -180,7 +180,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));  // generic pointer to the same place
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = (rank == 0);
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -279,92 +279,98 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
     }
   } else if (warp < 4) {
     setmaxnreg_dec<Cfg::REGS_CONTROL>();
-    if (lane == 0 && warp == 0) {
-      // ---------------------------------------------------------- TMA producer
-      uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0;
-      [[maybe_unused]] uint32_t pit = 0;
-      bool ok = true;
-      for (int tile = pair; tile < ntiles && ok; tile += npairs) {
-        const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
-        const int arow = tc.mt * 256 + static_cast<int>(rank) * 128, brow = tc.nt * 256 + static_cast<int>(rank) * 128;
-        for (int kb = 0; kb < p.nkb; ++kb) {
-          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 64)) {
-            ok = false;
-            break;
-          }
-          const uint32_t landed = smem_u32(&bar_landed[s]);
-          const uint32_t dst = smem_base + s * Cfg::STAGE;
-          mbar_arrive_expect_tx(landed, Cfg::STAGE);
-          if (tracing) trace_slot(p.trace, 8, pit++);
-          armed |= 1u << s;
-          armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-          if (p.a_k_contiguous) {
-            tma_load_3d(dst, &map_a, landed, kb * 32, arow, tc.b);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j) tma_load_3d(dst + j * 4096, &map_a, landed, arow + 32 * j, kb * 32, tc.b);
-          }
-          if (p.b_k_contiguous) {
-            tma_load_3d(dst + Cfg::STG_A, &map_b, landed, kb * 32, brow, tc.b);
-          } else {
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              tma_load_3d(dst + Cfg::STG_A + j * 4096, &map_b, landed, brow + 32 * j, kb * 32, tc.b);
-          }
-          if (++s == static_cast<uint32_t>(NST)) {
-            s = 0;
-            ph ^= 1;
-          }
-        }
-      }
-      if (!ok) {
-        raise_abort_pair(&abort_flag);
-        atomicCAS(p.status, 0, kErrProducerWait);
-        for (uint32_t q = 0; q < static_cast<uint32_t>(NST); ++q)
-          if (armed & (1u << q)) mbar_wait_plain(smem_u32(&bar_landed[q]), (armed_parity >> q) & 1);
-      }
-    } else if (lane == 0 && warp == 3) {
-      // ---------------------------------------------------------- relay: my half of the stage is converted
-      uint32_t s = 0, ph = 0;
-      bool ok = true;
-      for (int tile = pair; tile < ntiles && ok; tile += npairs) {
-        for (int kb = 0; kb < p.nkb; ++kb) {
-          if (!mbar_wait(smem_u32(&bar_conv[s]), ph, abortp, 32)) {
-            ok = false;
-            break;
-          }
-          mbar_arrive_cluster(map_to_cta(smem_u32(&bar_full[s]), 0));
-          if (++s == static_cast<uint32_t>(NST)) {
-            s = 0;
-            ph ^= 1;
+    if (warp == 0) {
+      if (elect_one()) {
+        // ---------------------------------------------------------- TMA producer
+        uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0;
+        [[maybe_unused]] uint32_t pit = 0;
+        bool ok = true;
+        for (int tile = pair; tile < ntiles && ok; tile += npairs) {
+          const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
+          const int arow = tc.mt * 256 + static_cast<int>(rank) * 128, brow = tc.nt * 256 + static_cast<int>(rank) * 128;
+          for (int kb = 0; kb < p.nkb; ++kb) {
+            if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 64)) {
+              ok = false;
+              break;
+            }
+            const uint32_t landed = smem_u32(&bar_landed[s]);
+            const uint32_t dst = smem_base + s * Cfg::STAGE;
+            mbar_arrive_expect_tx(landed, Cfg::STAGE);
+            if (tracing) trace_slot(p.trace, 8, pit++);
+            armed |= 1u << s;
+            armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
+            if (p.a_k_contiguous) {
+              tma_load_3d(dst, &map_a, landed, kb * 32, arow, tc.b);
+            } else {
+  #pragma unroll
+              for (int j = 0; j < 4; ++j) tma_load_3d(dst + j * 4096, &map_a, landed, arow + 32 * j, kb * 32, tc.b);
+            }
+            if (p.b_k_contiguous) {
+              tma_load_3d(dst + Cfg::STG_A, &map_b, landed, kb * 32, brow, tc.b);
+            } else {
+  #pragma unroll
+              for (int j = 0; j < 4; ++j)
+                tma_load_3d(dst + Cfg::STG_A + j * 4096, &map_b, landed, brow + 32 * j, kb * 32, tc.b);
+            }
+            if (++s == static_cast<uint32_t>(NST)) {
+              s = 0;
+              ph ^= 1;
+            }
           }
         }
+        if (!ok) {
+          raise_abort_pair(&abort_flag);
+          atomicCAS(p.status, 0, kErrProducerWait);
+          for (uint32_t q = 0; q < static_cast<uint32_t>(NST); ++q)
+            if (armed & (1u << q)) mbar_wait_plain(smem_u32(&bar_landed[q]), (armed_parity >> q) & 1);
+        }
       }
-      if (!ok) {
-        raise_abort_pair(&abort_flag);
-        atomicCAS(p.status, 0, kErrMmaWait);
+    } else if (warp == 3) {
+      if (elect_one()) {
+        // ---------------------------------------------------------- relay: my half of the stage is converted
+        uint32_t s = 0, ph = 0;
+        bool ok = true;
+        for (int tile = pair; tile < ntiles && ok; tile += npairs) {
+          for (int kb = 0; kb < p.nkb; ++kb) {
+            if (!mbar_wait(smem_u32(&bar_conv[s]), ph, abortp, 32)) {
+              ok = false;
+              break;
+            }
+            mbar_arrive_cluster(map_to_cta(smem_u32(&bar_full[s]), 0));
+            if (++s == static_cast<uint32_t>(NST)) {
+              s = 0;
+              ph ^= 1;
+            }
+          }
+        }
+        if (!ok) {
+          raise_abort_pair(&abort_flag);
+          atomicCAS(p.status, 0, kErrMmaWait);
+        }
       }
-    } else if (lane == 0 && leader && (warp == 1 || (kEc && warp == 2))) {
-      // ---------------------------------------------------------- leader: MMA issuers (tcec_gemm_roles.cuh)
-      OperandImage im;
-      im.dconst = umma_desc_kmajor_noswizzle(0, 128, Cfg::GROUP_BYTES);  // core matrices 128 B apart along K, groups 1 KB apart
-      im.base16 = (smem_base & 0x3ffff) >> 4;
-      im.stage16 = Cfg::STAGE >> 4;
-      im.a_lo16 = 512 >> 4;
-      im.b_hi16 = Cfg::STG_A >> 4;
-      im.b_lo16 = (Cfg::STG_A + 512) >> 4;
-      im.idesc = umma_idesc(0u, 256, BN);
-      const StridedTiles tiles{pair, npairs, ntiles};
-      const KWalk walk{p.nkb, p.promo};
-      const RingBarriers ring{bar_full, bar_empty};
-      if (warp == 1) {
-        if (!issue_main_products<false, true, NST>(tiles, walk, im, tmem_main, ring, &bar_main_full, &bar_main_free,
-                                                   abortp, p.debug_flags, tracing ? p.trace : nullptr))
-          mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[0]);
-      } else {
-        if (!issue_corr_products<false, true, NST>(tiles, walk, im, tmem_corr, ring, &bar_corr_full, &bar_corr_free,
-                                                   abortp, p.debug_flags, tracing ? p.trace : nullptr))
-          mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[1]);
+    } else if (leader && (warp == 1 || (kEc && warp == 2))) {
+      if (elect_one()) {
+        // ---------------------------------------------------------- leader: MMA issuers (tcec_gemm_roles.cuh)
+        OperandImage im;
+        im.dconst = umma_desc_kmajor_noswizzle(0, 128, Cfg::GROUP_BYTES);  // core matrices 128 B apart along K, groups 1 KB apart
+        im.base16 = (smem_base & 0x3ffff) >> 4;
+        im.stage16 = Cfg::STAGE >> 4;
+        im.a_lo16 = 512 >> 4;
+        im.b_hi16 = Cfg::STG_A >> 4;
+        im.b_lo16 = (Cfg::STG_A + 512) >> 4;
+        im.idesc = umma_idesc(0u, 256, BN);
+        const StridedTiles tiles{pair, npairs, ntiles};
+        const KWalk walk{p.nkb, p.promo};
+        const RingBarriers ring{bar_full, bar_empty};
+        if (warp == 1) {
+          if (!issue_main_products<false, true, NST>(tiles, walk, im, tmem_main, ring, &bar_main_full, &bar_main_free,
+                                                     abortp, p.debug_flags, tracing ? p.trace : nullptr))
+            mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[0]);
+        } else {
+          if (!issue_corr_products<false, true, NST>(tiles, walk, im, tmem_corr, ring, &bar_corr_full, &bar_corr_free,
+                                                     abortp, p.debug_flags, tracing ? p.trace : nullptr))
+            mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[1]);
+        }
       }
     }
   } else {

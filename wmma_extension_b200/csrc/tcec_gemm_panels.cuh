@@ -66,13 +66,21 @@ struct GemmPanelParams {
 
 enum : int { kErrProducerWait = 1, kErrMmaWait = 2, kErrEpilogueWait = 3, kErrOperandWait = 4 };
 
+// K blocks per ring stage.  With error correction a stage is one K block: six MMAs, 768 tensor cycles.  Without it a
+// K block is two MMAs, 256 cycles, which a wait and a commit per block do not leave enough slack for; two blocks
+// share a stage.  8192^3 fp16 without correction: one block 1114 us, two 1050, four 1059 (all with the issuing
+// threads entered through elect.sync; 1399 before both).
+constexpr int stage_blocks(bool ec) { return ec ? 1 : 2; }
+
 template <int BN, bool kTf32, bool kEc>
 struct GemmPanelCfg {
   static constexpr int BM = 128;
   static constexpr int NB = BN / 128;                  // 128-row B panels per tile
   static constexpr int NP = kEc ? 2 : 1;               // hi (+ lo)
-  static constexpr int A_BYTES = kPanelBytes * NP;
-  static constexpr int B_BYTES = kPanelBytes * NP * NB;
+  static constexpr int KBS = stage_blocks(kEc);
+  static constexpr int A_BLOCK = kPanelBytes * NP;     // one K block of A's 128 rows
+  static constexpr int A_BYTES = A_BLOCK * KBS;
+  static constexpr int B_BYTES = kPanelBytes * NP * NB * KBS;
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int NST_RAW = (208 * 1024) / STAGE_BYTES;
   static constexpr int NST = NST_RAW > 8 ? 8 : NST_RAW;
@@ -113,6 +121,34 @@ __device__ __forceinline__ TileCoord decode_tile(int tile, int tiles_m, int tile
   return t;
 }
 
+// One thread: arms `full` and issues the copies of one stage, K blocks kb .. kb + nblk - 1 of A's row block
+// at `pa` and of the NB row blocks of B (each nkb blocks long) at `pb`.
+template <class Cfg>
+__device__ __forceinline__ void load_panel_stage(uint32_t dst, const uint8_t* pa, const uint8_t* pb, int nkb, int kb,
+                                                 int nblk, uint32_t full) {
+  mbar_arrive_expect_tx(full, static_cast<uint32_t>(nblk) * (Cfg::STAGE_BYTES / Cfg::KBS));
+  bulk_load(dst, pa + static_cast<size_t>(kb) * Cfg::A_BLOCK, nblk * Cfg::A_BLOCK, full);
+  if constexpr (Cfg::NP == 2) {
+#pragma unroll
+    for (int h = 0; h < Cfg::NB; ++h) {
+      const uint8_t* src = pb + (static_cast<size_t>(h) * nkb + kb) * (kPanelBytes * 2);
+      bulk_load(dst + Cfg::A_BYTES + h * kPanelBytes, src, kPanelBytes, full);
+      bulk_load(dst + Cfg::A_BYTES + (Cfg::NB + h) * kPanelBytes, src + kPanelBytes, kPanelBytes, full);
+    }
+  } else if constexpr (Cfg::NB == 1) {
+    bulk_load(dst + Cfg::A_BYTES, pb + static_cast<size_t>(kb) * kPanelBytes, nblk * kPanelBytes, full);
+  } else {
+    // an MMA reads its 256 rows of B at one group stride: the two row blocks of a K block are neighbours
+#pragma unroll
+    for (int i = 0; i < Cfg::KBS; ++i)
+      if (i < nblk)
+#pragma unroll
+        for (int h = 0; h < Cfg::NB; ++h)
+          bulk_load(dst + Cfg::A_BYTES + (i * Cfg::NB + h) * kPanelBytes,
+                    pb + (static_cast<size_t>(h) * nkb + kb + i) * kPanelBytes, kPanelBytes, full);
+  }
+}
+
 template <int BN, bool kTf32, bool kEc>
 __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
     tcec_gemm_panels_kernel(const GemmPanelParams p) {
@@ -128,7 +164,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));  // generic pointer to the same place
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int ntiles = p.tiles_m * p.tiles_n * p.batch;
 
   if (threadIdx.x == 0) {
@@ -164,7 +200,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
     if constexpr (Cfg::REBALANCE) setmaxnreg_dec<Cfg::REGS_CONTROL>();
   if (warp == 0) {
     // ------------------------------------------------------------ producer
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t it = 0, s = 0, ph = 0;
       uint32_t armed = 0, armed_parity = 0;  // per stage: a copy was issued, and in which phase
       bool ok = true;
@@ -217,12 +253,12 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
         // The next tile is claimed late in this one (two ring fills before its end), so the claim
         // follows the CTA's actual progress, and early enough for the atomic's latency to hide.
         int next_tile = tile + static_cast<int>(gridDim.x);
-        const int claim_kb = p.nkb > 2 * NST ? p.nkb - 2 * NST : 0;
+        const int claim_kb = p.nkb > 2 * NST * Cfg::KBS ? (p.nkb / Cfg::KBS - 2 * NST) * Cfg::KBS : 0;
         const uint8_t* pa = p.panels_a + tc.b * p.panels_a_batch_stride +
-                            static_cast<size_t>(tc.mt) * p.nkb * Cfg::A_BYTES;
+                            static_cast<size_t>(tc.mt) * p.nkb * Cfg::A_BLOCK;
         const uint8_t* pb = p.panels_b + tc.b * p.panels_b_batch_stride +
                             static_cast<size_t>(tc.nt) * Cfg::NB * p.nkb * (kPanelBytes * Cfg::NP);
-        for (int kb = 0; kb < p.nkb; ++kb, ++it, s = (s + 1 == NST ? 0 : s + 1), ph ^= (s == 0)) {
+        for (int kb = 0; kb < p.nkb; kb += Cfg::KBS, ++it, s = (s + 1 == NST ? 0 : s + 1), ph ^= (s == 0)) {
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 128)) {
             ok = false;
             break;
@@ -236,18 +272,10 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
           }
           // injected stall (failure-path test): the first stage after the first ring fill is never filled
           if (dev_flag(p.debug_flags, 32) && it == static_cast<uint32_t>(NST)) continue;
-          mbar_arrive_expect_tx(full, Cfg::STAGE_BYTES);
+          const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, p.nkb - kb);  // K blocks in this stage
           armed |= 1u << s;
           armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-          bulk_load(dst, pa + static_cast<size_t>(kb) * Cfg::A_BYTES, Cfg::A_BYTES, full);
-#pragma unroll
-          for (int h = 0; h < Cfg::NB; ++h) {
-            const uint8_t* src = pb + (static_cast<size_t>(h) * p.nkb + kb) * (kPanelBytes * Cfg::NP);
-            bulk_load(dst + Cfg::A_BYTES + h * kPanelBytes, src, kPanelBytes, full);
-            if constexpr (kEc)
-              bulk_load(dst + Cfg::A_BYTES + (Cfg::NB + h) * kPanelBytes, src + kPanelBytes,
-                        kPanelBytes, full);
-          }
+          load_panel_stage<Cfg>(dst, pa, pb, p.nkb, kb, nblk, full);
         }
         tile = next_tile;
       }
@@ -261,7 +289,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
     }
   } else if (warp == 1 || warp == 2) {
     // ------------------------------------------------------------ MMA issuers (tcec_gemm_roles.cuh)
-    if (lane == 0 && (warp == 1 || kEc)) {
+    if ((warp == 1 || kEc) && elect_one()) {
       OperandImage im;
       im.dconst = umma_desc_kmajor_noswizzle(0, 128, 512);
       im.base16 = (smem_base & 0x3ffff) >> 4;
@@ -270,12 +298,14 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
       im.b_hi16 = Cfg::A_BYTES >> 4;
       im.b_lo16 = (Cfg::A_BYTES + Cfg::NB * kPanelBytes) >> 4;
       im.idesc = umma_idesc(kTf32 ? 2u : 0u, 128, BN);
+      im.a_block16 = Cfg::A_BLOCK >> 4;
+      im.b_block16 = (Cfg::B_BYTES / Cfg::KBS) >> 4;
       RingTiles tiles{tile_ring, bar_tile_full, bar_tile_empty};
       const KWalk walk{p.nkb, p.promo};
       const RingBarriers ring{bar_full, bar_empty};
       unsigned long long* trace = blockIdx.x == 0 ? p.trace : nullptr;
       if (warp == 1) {
-        if (!issue_main_products<kTf32, false, NST>(tiles, walk, im, tmem_main, ring, &bar_main_full, &bar_main_free,
+        if (!issue_main_products<kTf32, false, NST, Cfg::KBS>(tiles, walk, im, tmem_main, ring, &bar_main_full, &bar_main_free,
                                                     abortp, p.debug_flags, trace))
           mma_thread_gave_up<false>(&abort_flag, p.status, kErrMmaWait, &bar_drain[0]);
       } else {

@@ -35,8 +35,10 @@ namespace tcec_sm100 {
 template <bool kTf32, bool kEc>
 struct GemmPairCfg {
   static constexpr int NP = kEc ? 2 : 1;
-  static constexpr int A_BYTES = kPanelBytes * NP;   // this CTA's 128 rows of A: hi (+ lo)
-  static constexpr int B_BYTES = kPanelBytes * NP;   // this CTA's 128 of the tile's 256 N rows
+  static constexpr int KBS = stage_blocks(kEc);      // K blocks per stage
+  static constexpr int BLOCK = kPanelBytes * NP;     // one K block of 128 rows: hi (+ lo)
+  static constexpr int A_BYTES = BLOCK * KBS;        // this CTA's 128 rows of A
+  static constexpr int B_BYTES = BLOCK * KBS;        // this CTA's 128 of the tile's 256 N rows
   static constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
   static constexpr int NST_RAW = (200 * 1024) / STAGE_BYTES;
   static constexpr int NST = NST_RAW > 8 ? 8 : NST_RAW;
@@ -68,7 +70,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
   const bool leader = (rank == 0);
   const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
@@ -108,6 +110,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   im.b_hi16 = Cfg::A_BYTES >> 4;
   im.b_lo16 = (Cfg::A_BYTES + kPanelBytes) >> 4;
   im.idesc = umma_idesc(kTf32 ? 2u : 0u, 256, BN);
+  im.a_block16 = im.b_block16 = Cfg::BLOCK >> 4;
   const StridedTiles tiles{pair, npairs, ntiles};
   const KWalk walk{p.nkb, p.promo};
   const RingBarriers ring{bar_full, bar_empty};
@@ -116,18 +119,18 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     setmaxnreg_dec<Cfg::REGS_CONTROL>();
     if (warp == 0) {
       // ---------------------------------------------------------- producer (each CTA, own panels)
-      if (lane == 0) {
+      if (elect_one()) {
         uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0, it = 0;
         bool ok = true;
         for (int tile = pair; tile < ntiles && ok; tile += npairs) {
           const TileCoord tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
           const uint8_t* pa = p.panels_a + tc.b * p.panels_a_batch_stride +
-                              static_cast<size_t>(tc.mt * 2 + rank) * p.nkb * Cfg::A_BYTES;
+                              static_cast<size_t>(tc.mt * 2 + rank) * p.nkb * Cfg::BLOCK;
           // whole tile: this CTA's 128-row panel of the tile's two; half: its 64 rows of the half's one panel
           const int nblock = tc.nt * 2 + (BN == 256 ? static_cast<int>(rank) : tile % HALVES);
           const uint8_t* pb = p.panels_b + tc.b * p.panels_b_batch_stride +
-                              static_cast<size_t>(nblock) * p.nkb * Cfg::B_BYTES + (BN == 256 ? 0u : rank * B_PIECE);
-          for (int kb = 0; kb < p.nkb; ++kb, ++it) {
+                              static_cast<size_t>(nblock) * p.nkb * Cfg::BLOCK + (BN == 256 ? 0u : rank * B_PIECE);
+          for (int kb = 0; kb < p.nkb; kb += Cfg::KBS, ++it) {
             if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 128)) {
               ok = false;
               break;
@@ -142,17 +145,22 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             }
             const uint32_t full = smem_u32(&bar_full[s]);
             const uint32_t dst = smem_base + s * Cfg::STAGE_BYTES;
-            mbar_arrive_expect_tx(full, Cfg::A_BYTES + Cfg::NP * B_PIECE);
+            const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, p.nkb - kb);  // K blocks in this stage
+            mbar_arrive_expect_tx(full, static_cast<uint32_t>(nblk) * (Cfg::BLOCK + Cfg::NP * B_PIECE));
             armed |= 1u << s;
             armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-            bulk_load(dst, pa + static_cast<size_t>(kb) * Cfg::A_BYTES, Cfg::A_BYTES, full);
-            const uint8_t* srcb = pb + static_cast<size_t>(kb) * Cfg::B_BYTES;
+            bulk_load(dst, pa + static_cast<size_t>(kb) * Cfg::BLOCK, nblk * Cfg::BLOCK, full);
+            const uint8_t* srcb = pb + static_cast<size_t>(kb) * Cfg::BLOCK;
             if constexpr (BN == 256) {
-              bulk_load(dst + Cfg::A_BYTES, srcb, Cfg::B_BYTES, full);
+              bulk_load(dst + Cfg::A_BYTES, srcb, nblk * Cfg::BLOCK, full);
             } else {
 #pragma unroll
-              for (int h = 0; h < Cfg::NP; ++h)  // hi (+ lo): each image keeps its place in the stage
-                bulk_load(dst + Cfg::A_BYTES + h * kPanelBytes, srcb + h * kPanelBytes, B_PIECE, full);
+              for (int i = 0; i < Cfg::KBS; ++i)
+                if (i < nblk)
+#pragma unroll
+                  for (int h = 0; h < Cfg::NP; ++h)  // hi (+ lo): each image keeps its place in the stage
+                    bulk_load(dst + Cfg::A_BYTES + i * Cfg::BLOCK + h * kPanelBytes, srcb + i * Cfg::BLOCK + h * kPanelBytes,
+                              B_PIECE, full);
             }
             if (++s == static_cast<uint32_t>(NST)) {
               s = 0;
@@ -168,13 +176,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
         }
       }
     } else if (warp == 1) {
-      if (lane == 0) {
+      if (elect_one()) {
         if (!leader) {
           // -------------------------------------------------------- peer: relay "my stage landed"
           uint32_t s = 0, ph = 0, it = 0;
           bool ok = true;
           for (int tile = pair; tile < ntiles && ok; tile += npairs) {
-            for (int kb = 0; kb < p.nkb; ++kb, ++it) {
+            for (int kb = 0; kb < p.nkb; kb += Cfg::KBS, ++it) {
               if (!mbar_wait(smem_u32(&bar_full[s]), ph, abortp, 32)) {
                 ok = false;
                 break;
@@ -192,8 +200,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
           }
         } else {
           // -------------------------------------------------------- leader: main products
-          if (!issue_main_products<kTf32, true, NST>(tiles, walk, im, tmem_main, ring, &bar_main_full,
-                                                                    &bar_main_free, abortp, p.debug_flags,
+          if (!issue_main_products<kTf32, true, NST, Cfg::KBS>(tiles, walk, im, tmem_main, ring, &bar_main_full,
+                                                          &bar_main_free, abortp, p.debug_flags,
                                                                     blockIdx.x == 0 ? p.trace : nullptr))
             mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[0]);
         }
@@ -201,7 +209,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     } else if (warp == 2) {
       // ---------------------------------------------------------- leader: correction products
       if constexpr (kEc) {
-        if (lane == 0 && leader) {
+        if (leader && elect_one()) {
           if (!issue_corr_products<kTf32, true, NST>(tiles, walk, im, tmem_corr, ring, &bar_corr_full, &bar_corr_free,
                                                      abortp, p.debug_flags, blockIdx.x == 0 ? p.trace : nullptr))
             mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[1]);

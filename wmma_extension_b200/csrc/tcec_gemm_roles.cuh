@@ -21,6 +21,8 @@ struct OperandImage {
   uint32_t b_hi16;
   uint32_t b_lo16;
   uint32_t idesc;      // instruction descriptor (type, M, N)
+  uint32_t a_block16 = 0;  // distance between the K blocks that share a stage (0 with one block per stage)
+  uint32_t b_block16 = 0;
 };
 
 // How K is cut.
@@ -112,8 +114,9 @@ __device__ __forceinline__ void trace_slot(unsigned long long*, int, uint32_t) {
 // One thread: the main products of every tile of the walk.  Kept to a handful of integer
 // instructions per MMA: descriptors are a constant OR-ed with a 14-bit address field, ring
 // positions and the promotion interval are counters.  Returns false when a bounded wait ran out.
+// A stage holds kBlocks K blocks (the last one of a tile perhaps fewer).
 // Develop builds only: debug_flags bit 1 issues no MMAs.
-template <bool kTf32, bool kPair, int NST, class TileSource>
+template <bool kTf32, bool kPair, int NST, int kBlocks = 1, class TileSource>
 __device__ __forceinline__ bool issue_main_products(TileSource tiles, const KWalk& w, const OperandImage& im,
                                                     uint32_t tmem_main,
                                                     const RingBarriers& ring, uint64_t* bar_main_full,
@@ -125,28 +128,34 @@ __device__ __forceinline__ bool issue_main_products(TileSource tiles, const KWal
     if (tile == kNoMoreTiles) break;
     if (tile == kTileWaitFailed) return false;
     int left_in_chunk = 0;  // K blocks still to issue in the current chunk
-    for (int kb = 0; kb < w.nkb; ++kb, ++it) {
+    for (int kb0 = 0; kb0 < w.nkb; kb0 += kBlocks, ++it) {
       if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 32u)) return false;
       trace_slot(trace, 0, it);
-      const bool first_in_chunk = (left_in_chunk == 0);
-      if (first_in_chunk) {
-        const int rest = w.nkb - kb;
-        left_in_chunk = (w.promo && w.promo < rest) ? w.promo : rest;
-        // the epilogue has drained the previous chunk (hot poll: the tensor pipe waits on this)
-        if (!mbar_wait(smem_u32(bar_main_free), (chunk & 1) ^ 1, abortp, 0)) return false;
-        trace_slot(trace, 1, chunk);
-      }
-      tc_fence_after();
-      const uint32_t a16 = im.base16 + s * im.stage16;
-      if (!dev_flag(debug_flags, 2)) {
 #pragma unroll
-        for (uint32_t j = 0; j < 2; ++j)
-          umma_issue<kTf32, kPair>(tmem_main, im.dconst | (a16 + 16 * j), im.dconst | (a16 + im.b_hi16 + 16 * j),
-                                   im.idesc, (first_in_chunk && j == 0) ? 0u : 1u);
-      }
-      if (--left_in_chunk == 0) {
-        umma_commit_to<kPair>(smem_u32(bar_main_full));
-        ++chunk;
+      for (int i = 0; i < kBlocks; ++i) {
+        const int kb = kb0 + i;
+        if (i > 0 && kb >= w.nkb) break;
+        const bool first_in_chunk = (left_in_chunk == 0);
+        if (first_in_chunk) {
+          const int rest = w.nkb - kb;
+          left_in_chunk = (w.promo && w.promo < rest) ? w.promo : rest;
+          // the epilogue has drained the previous chunk (hot poll: the tensor pipe waits on this)
+          if (!mbar_wait(smem_u32(bar_main_free), (chunk & 1) ^ 1, abortp, 0)) return false;
+          trace_slot(trace, 1, chunk);
+        }
+        if (i == 0 || first_in_chunk) tc_fence_after();
+        const uint32_t a16 = im.base16 + s * im.stage16 + (kBlocks > 1 ? i * im.a_block16 : 0);
+        const uint32_t b16 = im.base16 + s * im.stage16 + im.b_hi16 + (kBlocks > 1 ? i * im.b_block16 : 0);
+        if (!dev_flag(debug_flags, 2)) {
+#pragma unroll
+          for (uint32_t j = 0; j < 2; ++j)
+            umma_issue<kTf32, kPair>(tmem_main, im.dconst | (a16 + 16 * j), im.dconst | (b16 + 16 * j), im.idesc,
+                                     (first_in_chunk && j == 0) ? 0u : 1u);
+        }
+        if (--left_in_chunk == 0) {
+          umma_commit_to<kPair>(smem_u32(bar_main_full));
+          ++chunk;
+        }
       }
       umma_commit_to<kPair>(smem_u32(&ring.empty[s]));
       trace_slot(trace, 5, it);
