@@ -286,6 +286,10 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                whenever the call allows it (fp16 policies, n > 128, 16-byte aligned operands
  *                with leading dimensions that are multiples of 4, no pointer arrays).
  *                Automatic picks it for batches with k <= 512, which are bound by DRAM traffic.
+ *   "direct_kernel" one launch that reads FP32 operands of any layout, alignment and batch form with
+ *                ordinary loads and splits them on the way into shared memory; bit-identical
+ *                results.  -1 (default) = for matrices with m, n <= 128; 0 = never; 1 = whenever
+ *                "path", "cta_pair" and "tile_n" are automatic.
  */
 int tcec_set_option(const char* name, int value);
 int tcec_get_option(const char* name, int* value);

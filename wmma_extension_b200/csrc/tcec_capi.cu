@@ -9,6 +9,7 @@
 #include <mutex>
 #include <utility>
 
+#include "tcec_gemm_direct.cuh"
 #include "tcec_gemm_fused.cuh"
 #include "tcec_gemm_panels.cuh"
 #include "tcec_gemm_panels_pair.cuh"
@@ -36,6 +37,23 @@ cudaError_t set_smem_attr() {
   return cudaFuncSetAttribute(tcec_gemm_panels_kernel<BN, T, E>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                               GemmPanelCfg<BN, T, E>::SMEM_BYTES);
+}
+
+template <bool T, bool E, bool AK, bool BK>
+cudaError_t set_direct_smem_attr() {
+  const cudaError_t e = cudaFuncSetAttribute(tcec_gemm_direct_kernel<T, E, AK, BK, 64>,
+                                             cudaFuncAttributeMaxDynamicSharedMemorySize, GemmDirectCfg<T, E>::SMEM_BYTES);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(tcec_gemm_direct_kernel<T, E, AK, BK, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              GemmDirectCfg<T, E>::SMEM_BYTES);
+}
+template <bool T, bool E>
+cudaError_t set_direct_smem_attrs() {
+  cudaError_t e = set_direct_smem_attr<T, E, false, false>();
+  if (e == cudaSuccess) e = set_direct_smem_attr<T, E, false, true>();
+  if (e == cudaSuccess) e = set_direct_smem_attr<T, E, true, false>();
+  if (e == cudaSuccess) e = set_direct_smem_attr<T, E, true, true>();
+  return e;
 }
 
 template <bool T, bool E>
@@ -72,6 +90,10 @@ int get_device_state(DeviceState** out) {
     TCEC_CUDA((set_pair_smem_attr<false, false>()));
     TCEC_CUDA((set_pair_smem_attr<true, true>()));
     TCEC_CUDA((set_pair_smem_attr<true, false>()));
+    TCEC_CUDA((set_direct_smem_attrs<false, true>()));
+    TCEC_CUDA((set_direct_smem_attrs<false, false>()));
+    TCEC_CUDA((set_direct_smem_attrs<true, true>()));
+    TCEC_CUDA((set_direct_smem_attrs<true, false>()));
     if (cudaMalloc(&st.status, sizeof(int)) != cudaSuccess) return TCEC_ERR_ALLOC;
     TCEC_CUDA(cudaMemset(st.status, 0, sizeof(int)));
     st.attrs_done = true;
@@ -492,6 +514,72 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
   return true;
 }
 
+// ---------------------------------------------------------------- direct path
+template <bool T, bool E, bool AK, bool BK>
+void launch_direct_as(const GemmDirectParams& dp, int grid, cudaStream_t stream) {
+  using Cfg = GemmDirectCfg<T, E>;
+  if (dp.slot == 128) tcec_gemm_direct_kernel<T, E, AK, BK, 64><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(dp);
+  else tcec_gemm_direct_kernel<T, E, AK, BK, 32><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(dp);
+}
+template <bool T, bool E>
+void launch_direct(const GemmDirectParams& dp, int grid, cudaStream_t stream) {
+  if (dp.a.k_contiguous && dp.b.k_contiguous) launch_direct_as<T, E, true, true>(dp, grid, stream);
+  else if (dp.a.k_contiguous) launch_direct_as<T, E, true, false>(dp, grid, stream);
+  else if (dp.b.k_contiguous) launch_direct_as<T, E, false, true>(dp, grid, stream);
+  else launch_direct_as<T, E, false, false>(dp, grid, stream);
+}
+
+// Launches the direct kernel if the call is one for it; returns false (nothing launched) otherwise.
+bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const float* a, const float* const* a_array,
+                long long lda, long long stride_a, const float* b, const float* const* b_array, long long ldb,
+                long long stride_b, float beta, float* c, float* const* c_array, long long ldc, long long stride_c,
+                int batch, int policy, const DeviceState* st, cudaStream_t stream, const Options& opt) {
+  // an option that asks for another kernel is obeyed
+  if (opt.direct_kernel == 0 || opt.path != 0 || opt.cta_pair != -1 || opt.tile_n != 0) return false;
+  // A matrix of at most one tile: nothing is read or split twice, and no panel is padded to 256 rows (16384 x 64^3:
+  // 1176 -> 175 us, 8192 x 70^3: 772 -> 395, 4096 x 128^3: 465 -> 197, 1000 x 100 x 100 x 400: 292 -> 137; one 32^3: 31 -> 23 with
+  // the host's part).  With more tiles per matrix each operand is loaded and split once per tile that uses it, and the loaders
+  // are what bounds the kernel: 1024 x 201^3 358 us either way, 256 x 512^3 474 against 236.
+  if (opt.direct_kernel == -1 && !(m <= 128 && n <= 128)) return false;
+  GemmDirectParams dp{};
+  dp.a = DirectOperand{a, a_array, lda, stride_a, m, la == TCEC_ROW_MAJOR};
+  dp.b = DirectOperand{b, b_array, ldb, stride_b, n, lb == TCEC_COL_MAJOR};
+  dp.M = m;
+  dp.N = n;
+  dp.K = k;
+  dp.batch = batch;
+  const int larger = m > n ? m : n;
+  dp.slot_log2 = batch == 1 || larger > 64 ? 7 : (larger > 32 ? 6 : 5);
+  dp.slot = 1 << dp.slot_log2;
+  dp.tiles_m = (m + 127) / 128;
+  dp.tiles_n = (n + 127) / 128;
+  const long long per_tile = 128 / dp.slot;
+  const long long ntiles = static_cast<long long>(dp.tiles_m) * dp.tiles_n * ((batch + per_tile - 1) / per_tile);
+  if (ntiles > 0x3fffffffll) return false;  // tile indices are 32-bit
+  // Few matrices of long K would leave most SMs idle and walk K one granule after the other: panels.
+  if (opt.direct_kernel == -1 && k > 1024 && ntiles < st->sm_count / 2) return false;
+  dp.ntiles = static_cast<int>(ntiles);
+  dp.promo = promote_blocks(k, policy, policy_tf32(policy) ? 16 : 32, opt);
+  dp.alpha = alpha;
+  dp.beta = beta;
+  dp.c = c;
+  dp.c_array = c_array;
+  dp.ldc = ldc;
+  dp.c_batch_stride = stride_c;
+  dp.c_col_major = (lc == TCEC_COL_MAJOR);
+  dp.status = st->status;
+  const int sms = st->sm_count - opt.reserve_sms > 1 ? st->sm_count - opt.reserve_sms : 1;
+  const int grid = dp.ntiles < sms ? dp.ntiles : sms;
+  if (policy_tf32(policy)) {
+    if (policy_ec(policy)) launch_direct<true, true>(dp, grid, stream);
+    else launch_direct<true, false>(dp, grid, stream);
+  } else {
+    if (policy_ec(policy)) launch_direct<false, true>(dp, grid, stream);
+    else launch_direct<false, false>(dp, grid, stream);
+  }
+  return true;
+}
+
 int scale_only(float beta, float* c, float* const* c_array, long long ldc, long long stride_c, int m,
                int n, int lc, int batch, cudaStream_t stream) {
   if (beta == 1.f) return TCEC_OK;
@@ -536,6 +624,11 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
   }
   if (k == 0 || alpha == 0.f) return scale_only(beta, c, c_array, ldc, stride_c, m, n, lc, batch, stream);
 
+  if (try_direct(la, lb, lc, m, n, k, alpha, a, a_array, lda, stride_a, b, b_array, ldb, stride_b, beta, c, c_array, ldc,
+                 stride_c, batch, policy, st, stream, opt)) {
+    TCEC_CUDA(cudaGetLastError());
+    return TCEC_OK;
+  }
   if (!a_array && !b_array && !c_array &&
       try_fused(la, lb, lc, m, n, k, alpha, a, lda, stride_a, b, ldb, stride_b, beta, c, ldc, stride_c, batch, policy,
                 st, stream, opt)) {
@@ -858,6 +951,7 @@ const OptionEntry kOptions[] = {
     {"cta_pair", &Options::cta_pair, -1, 1, any_value},
     {"half_tiles", &Options::half_tiles, 0, 1, any_value},
     {"path", &Options::path, 0, 2, any_value},
+    {"direct_kernel", &Options::direct_kernel, -1, 1, any_value},
     {"store_turn", &Options::store_turn, 0, 1, any_value},
     {"reserve_sms", &Options::reserve_sms, 0, 64, any_value},
     {"static_tiles", &Options::static_tiles, 0, 1, any_value},

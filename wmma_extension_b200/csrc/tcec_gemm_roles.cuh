@@ -210,6 +210,94 @@ __device__ __forceinline__ bool issue_corr_products(TileSource tiles, const KWal
   return true;
 }
 
+// The two issuing threads of the kernels whose tiles are at most 128 columns wide.  There TMEM holds both accumulators
+// twice: the main products of a promotion chunk run while the epilogue drains the chunk before, the correction
+// products of a tile while it folds the tile before.  Same products in the same order as above.
+struct DoubleImage {
+  uint64_t dconst;
+  uint32_t base16, stage16;
+  uint32_t a_lo16, b_hi16, b_lo16;  // inside a K block (A hi is at 0)
+  uint32_t kstep16;                 // from one MMA's K to the next
+  uint32_t a_block16, b_block16;    // between the K blocks of a stage
+};
+constexpr uint32_t kDoubleCols = 128;  // columns from one accumulator buffer to the other
+
+// `next_tile(idesc)` moves to the thread's next tile and gives its instruction descriptor; false = no more.
+template <bool kTf32, int NST, int kBlocks, class NextTile>
+__device__ __forceinline__ bool issue_main_double(NextTile next_tile, const KWalk& w, const DoubleImage& im, uint32_t tmem_main,
+                                                  const RingBarriers& ring, uint64_t* main_full, uint64_t* main_free,
+                                                  volatile uint32_t* abortp) {
+  uint32_t s = 0, ph = 0, chunk = 0, idesc = 0;
+  while (next_tile(idesc)) {
+    int left = 0;  // K blocks still to issue in the current chunk
+    for (int kb0 = 0; kb0 < w.nkb; kb0 += kBlocks) {
+      if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 20)) return false;
+#pragma unroll
+      for (int i = 0; i < kBlocks; ++i) {
+        const int kb = kb0 + i;
+        if (i > 0 && kb >= w.nkb) break;
+        const bool first = left == 0;
+        if (first) {
+          const int rest = w.nkb - kb;
+          left = (w.promo && w.promo < rest) ? w.promo : rest;
+          if (!mbar_wait(smem_u32(&main_free[chunk & 1]), ((chunk >> 1) & 1) ^ 1, abortp, 0)) return false;
+        }
+        if (i == 0 || first) tc_fence_after();
+        const uint32_t a16 = im.base16 + s * im.stage16 + i * im.a_block16;
+        const uint32_t b16 = im.base16 + s * im.stage16 + im.b_hi16 + i * im.b_block16;
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j)
+          umma_ss<kTf32>(tmem_main + (chunk & 1) * kDoubleCols, im.dconst | (a16 + j * im.kstep16),
+                         im.dconst | (b16 + j * im.kstep16), idesc, (first && j == 0) ? 0u : 1u);
+        if (--left == 0) {
+          umma_commit(smem_u32(&main_full[chunk & 1]));
+          ++chunk;
+        }
+      }
+      umma_commit(smem_u32(&ring.empty[s]));
+      if (++s == static_cast<uint32_t>(NST)) {
+        s = 0;
+        ph ^= 1;
+      }
+    }
+  }
+  return true;
+}
+template <bool kTf32, int NST, int kBlocks, class NextTile>
+__device__ __forceinline__ bool issue_corr_double(NextTile next_tile, const KWalk& w, const DoubleImage& im, uint32_t tmem_corr,
+                                                  const RingBarriers& ring, uint64_t* corr_full, uint64_t* corr_free,
+                                                  volatile uint32_t* abortp) {
+  uint32_t s = 0, ph = 0, tcount = 0, idesc = 0;
+  for (; next_tile(idesc); ++tcount) {
+    const uint32_t d = tmem_corr + (tcount & 1) * kDoubleCols;
+    if (!mbar_wait(smem_u32(&corr_free[tcount & 1]), ((tcount >> 1) & 1) ^ 1, abortp, 0)) return false;
+    for (int kb0 = 0; kb0 < w.nkb; kb0 += kBlocks) {
+      if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 20)) return false;
+      tc_fence_after();
+#pragma unroll
+      for (int i = 0; i < kBlocks; ++i) {
+        if (i > 0 && kb0 + i >= w.nkb) break;
+        const uint32_t a16 = im.base16 + s * im.stage16 + i * im.a_block16;
+        const uint32_t bh16 = im.base16 + s * im.stage16 + im.b_hi16 + i * im.b_block16, bl16 = bh16 + (im.b_lo16 - im.b_hi16);
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j)
+          umma_ss<kTf32>(d, im.dconst | (a16 + im.a_lo16 + j * im.kstep16), im.dconst | (bh16 + j * im.kstep16), idesc,
+                         (kb0 + i == 0 && j == 0) ? 0u : 1u);
+#pragma unroll
+        for (uint32_t j = 0; j < 2; ++j)
+          umma_ss<kTf32>(d, im.dconst | (a16 + j * im.kstep16), im.dconst | (bl16 + j * im.kstep16), idesc, 1u);
+      }
+      umma_commit(smem_u32(&ring.empty[s]));
+      if (++s == static_cast<uint32_t>(NST)) {
+        s = 0;
+        ph ^= 1;
+      }
+    }
+    umma_commit(smem_u32(&corr_full[tcount & 1]));
+  }
+  return true;
+}
+
 // An MMA thread whose wait ran out: raise the flags, then make sure nothing it issued still
 // writes TMEM when the CTA releases it.
 template <bool kPair>
@@ -331,6 +419,44 @@ __device__ __forceinline__ void fold_correction_narrow(float (&acc)[128], uint32
     for (int i = 0; i < 16; ++i) {
       acc[cc * 32 + i] = acc[cc * 32 + i] + __uint_as_float(v0[i]) * scale;
       acc[cc * 32 + 16 + i] = acc[cc * 32 + 16 + i] + __uint_as_float(v1[i]) * scale;
+    }
+  }
+}
+
+// The same two steps for tiles of at most 128 columns (NC = 32 or 64 per epilogue warp).
+template <int NC>
+__device__ __forceinline__ void promote_main_double(float (&acc)[NC], uint32_t taddr, bool first) {
+  if (first) {
+#pragma unroll
+    for (int c = 0; c < NC; c += 32) tmem_ld_32x32b_x32_f(taddr + c, &acc[c]);
+    tmem_ld_wait();
+  } else {
+#pragma unroll
+    for (int c = 0; c < NC; c += 32) {
+      uint32_t v0[16], v1[16];
+      tmem_ld_32x32b_x16(taddr + c, v0);
+      tmem_ld_32x32b_x16(taddr + c + 16, v1);
+      tmem_ld_wait();
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        acc[c + i] += __uint_as_float(v0[i]);
+        acc[c + 16 + i] += __uint_as_float(v1[i]);
+      }
+    }
+  }
+}
+template <int NC>
+__device__ __forceinline__ void fold_correction_double(float (&acc)[NC], uint32_t taddr, float scale) {
+#pragma unroll
+  for (int c = 0; c < NC; c += 32) {
+    uint32_t v0[16], v1[16];
+    tmem_ld_32x32b_x16(taddr + c, v0);
+    tmem_ld_32x32b_x16(taddr + c + 16, v1);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      acc[c + i] = acc[c + i] + __uint_as_float(v0[i]) * scale;
+      acc[c + 16 + i] = acc[c + 16 + i] + __uint_as_float(v1[i]) * scale;
     }
   }
 }
