@@ -12,6 +12,7 @@
 #include "tcec_gemm_direct.cuh"
 #include "tcec_gemm_fused.cuh"
 #include "tcec_gemm_panels.cuh"
+#include "tcec_gemm_panels_narrow.cuh"
 #include "tcec_gemm_panels_pair.cuh"
 #include "tcec_internal.h"
 #include "tcec_panels.cuh"
@@ -57,6 +58,19 @@ cudaError_t set_direct_smem_attrs() {
 }
 
 template <bool T, bool E>
+cudaError_t set_narrow_smem_attr() {
+  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<32, T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       GemmNarrowCfg<32, E>::SMEM_BYTES);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<64, T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             GemmNarrowCfg<64, E>::SMEM_BYTES);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<128, T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             GemmNarrowCfg<128, E>::SMEM_BYTES);
+  return e;
+}
+
+template <bool T, bool E>
 cudaError_t set_pair_smem_attr() {
   cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, GemmPairCfg<T, E>::SMEM_BYTES);
@@ -88,6 +102,10 @@ int get_device_state(DeviceState** out) {
                                    GemmFusedCfg<false>::SMEM_BYTES));
     TCEC_CUDA((set_pair_smem_attr<false, true>()));
     TCEC_CUDA((set_pair_smem_attr<false, false>()));
+    TCEC_CUDA((set_narrow_smem_attr<false, false>()));
+    TCEC_CUDA((set_narrow_smem_attr<false, true>()));
+    TCEC_CUDA((set_narrow_smem_attr<true, false>()));
+    TCEC_CUDA((set_narrow_smem_attr<true, true>()));
     TCEC_CUDA((set_pair_smem_attr<true, true>()));
     TCEC_CUDA((set_pair_smem_attr<true, false>()));
     TCEC_CUDA((set_direct_smem_attrs<false, true>()));
@@ -235,6 +253,51 @@ void launch_gemm(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
       <<<grid, Cfg::THREADS, gp.store_turn ? Cfg::SMEM_BYTES : Cfg::SMEM_BYTES_NO_TURN, stream>>>(gp);
 }
 
+// Width of the narrow tiles if they would finish the call sooner than 256-wide ones, else 0.  Cycles per K block of a
+// tile, fitted to what was measured: wide tiles pay their MMAs and, per promotion, about 1700 cycles in which the main
+// products wait (2048^3 on CTA pairs, a promotion every 2 blocks: 69 us; 4096^3, every 4: 83 us a tile); narrow ones take the
+// larger of their MMAs and their copies at 42 bytes per cycle and SM (2048^3 in 128-wide tiles: 62 us), and at least what
+// their epilogue takes.  Both sides at the sizes where the choice turns: 1000 x 777 x 1111 36 us wide, 25 with 64;
+// 1500^3 41 and 34 (128); 2048^3 69 and 63 (128); 1000 x 4096 x 4096 107 and 108; 4096^3 stays wide.
+int narrow_width(int m, int n, int batch, int promo, const Shape& s, int sms, bool pair) {
+  const long long tiles_m = (m + 127) / 128;
+  const int rows = m < 128 ? (m + 7) & ~7 : 128;
+  const long long wide_tiles =
+      pair ? static_cast<long long>((m + 255) / 256) * ((n + 255) / 256) * batch : tiles_m * ((n + s.tile_n - 1) / s.tile_n) * batch;
+  const int wide_slots = pair ? sms / 2 : sms;
+  // Beyond two rounds of wide tiles the last, partly empty one weighs little (256 x 512^3: 308 us wide, 324 with 128).
+  if (wide_tiles > 2 * wide_slots) return 0;
+  const bool ec = s.np == 2;
+  const double wide_block = (ec ? 768.0 : 300.0) + 1700.0 / (promo ? promo : s.nkb);
+  double best = ((wide_tiles + wide_slots - 1) / wide_slots) * (s.nkb * wide_block + 10000.0);
+  int width = 0;
+  const double mma[3] = {240.0, 288.0, 446.0};
+  for (int i = 0; i < 3; ++i) {
+    const int bn = 32 << i;
+    if (i > 0 && n <= bn / 2) break;
+    const long long tiles = tiles_m * ((n + bn - 1) / bn) * batch;
+    const double copy = (rows + bn) * 64.0 * s.np / 42.0, products = ec ? mma[i] : mma[i] / 3.0;
+    const double tile = s.nkb * (products > copy ? products : copy);
+    const double cost = ((tiles + sms - 1) / sms) * (tile > 6000.0 ? tile : 6000.0) + 4000.0;
+    if (cost < best) {
+      best = cost;
+      width = bn;
+    }
+  }
+  return width;
+}
+template <int BN, bool T, bool E>
+void launch_narrow(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
+  using Cfg = GemmNarrowCfg<BN, E>;
+  tcec_gemm_panels_narrow_kernel<BN, T, E><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(gp);
+}
+template <bool T, bool E>
+void launch_narrow_as(int width, const GemmPanelParams& gp, int grid, cudaStream_t stream) {
+  if (width == 32) launch_narrow<32, T, E>(gp, grid, stream);
+  else if (width == 64) launch_narrow<64, T, E>(gp, grid, stream);
+  else launch_narrow<128, T, E>(gp, grid, stream);
+}
+
 bool bad_layout(int l) { return l != TCEC_ROW_MAJOR && l != TCEC_COL_MAJOR; }
 
 static SplitParams split_params(bool k_contiguous, int rows, int k, const float* src, const float* const* src_array,
@@ -342,6 +405,22 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
   const double flops = 2.0 * m * static_cast<double>(n) * k * batch;
   const bool want_pair = !ex.force_one_sm && !ex.row_ready && !ex.sched &&
                          (opt.cta_pair == 1 || (opt.cta_pair == -1 && (!ec || flops <= 2.5e11)));
+  // Options that ask for one of the wide kernels, or for something only they do, are obeyed there.
+  if (!ex.force_one_sm && !ex.row_ready && !ex.sched && opt.cta_pair == -1 && opt.tile_n == 0 && opt.store_turn &&
+      !opt.static_tiles && !opt.debug_flags && opt.narrow_tiles != 0) {
+    const int width = opt.narrow_tiles > 0 ? opt.narrow_tiles
+                                           : narrow_width(m, n, batch, gp.promo, s, sms, want_pair && s.tile_n == 256 && m > 128);
+    const long long ntiles = static_cast<long long>(s.tiles_m) * ((n + width - 1) / (width ? width : 1)) * batch;
+    if (width && ntiles <= 0x3fffffffll) {
+      gp.tiles_n = (n + width - 1) / width;
+      const int grid = static_cast<int>(ntiles < sms ? ntiles : sms);
+      if (tf32 && ec) launch_narrow_as<true, true>(width, gp, grid, stream);
+      else if (tf32) launch_narrow_as<true, false>(width, gp, grid, stream);
+      else if (ec) launch_narrow_as<false, true>(width, gp, grid, stream);
+      else launch_narrow_as<false, false>(width, gp, grid, stream);
+      return TCEC_OK;
+    }
+  }
   if (want_pair && s.tile_n == 256 && m > 128) {
     // CTA pairs: 256 x 256 tiles, grid of up to sms/2 clusters of two CTAs
     gp.tiles_m = (m + 255) / 256;
@@ -556,7 +635,7 @@ bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const 
   const long long per_tile = 128 / dp.slot;
   const long long ntiles = static_cast<long long>(dp.tiles_m) * dp.tiles_n * ((batch + per_tile - 1) / per_tile);
   if (ntiles > 0x3fffffffll) return false;  // tile indices are 32-bit
-  // Few matrices of long K would leave most SMs idle and walk K one granule after the other: panels.
+  // Few matrices of long K would leave most SMs idle and walk K one granule after the other: panels, in narrow tiles.
   if (opt.direct_kernel == -1 && k > 1024 && ntiles < st->sm_count / 2) return false;
   dp.ntiles = static_cast<int>(ntiles);
   dp.promo = promote_blocks(k, policy, policy_tf32(policy) ? 16 : 32, opt);
@@ -944,6 +1023,7 @@ struct OptionEntry {
 };
 bool any_value(int) { return true; }
 bool tile_value(int v) { return v == 0 || v == 128 || v == 256; }
+bool narrow_value(int v) { return v <= 0 || v == 32 || v == 64 || v == 128; }
 bool panel_rows_value(int v) { return v % 256 == 0; }
 const OptionEntry kOptions[] = {
     {"promote_k", &Options::promote_k, -1, 0x7fffffff, any_value},
@@ -951,6 +1031,7 @@ const OptionEntry kOptions[] = {
     {"cta_pair", &Options::cta_pair, -1, 1, any_value},
     {"half_tiles", &Options::half_tiles, 0, 1, any_value},
     {"path", &Options::path, 0, 2, any_value},
+    {"narrow_tiles", &Options::narrow_tiles, -1, 128, narrow_value},
     {"direct_kernel", &Options::direct_kernel, -1, 1, any_value},
     {"store_turn", &Options::store_turn, 0, 1, any_value},
     {"reserve_sms", &Options::reserve_sms, 0, 64, any_value},
@@ -1091,6 +1172,10 @@ int static_device_state(StaticDevice** out) {
     TCEC_CUDA((set_pair_smem_attr<false, false>()));
     TCEC_CUDA((set_pair_smem_attr<true, false>()));
     TCEC_CUDA((set_pair_smem_attr<false, true>()));
+    TCEC_CUDA((set_narrow_smem_attr<false, false>()));
+    TCEC_CUDA((set_narrow_smem_attr<false, true>()));
+    TCEC_CUDA((set_narrow_smem_attr<true, false>()));
+    TCEC_CUDA((set_narrow_smem_attr<true, true>()));
     TCEC_CUDA((set_pair_smem_attr<true, true>()));
     sd.ready = true;
   }

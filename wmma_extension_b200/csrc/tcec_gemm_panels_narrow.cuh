@@ -1,0 +1,208 @@
+// The panel GEMM on narrow tiles (128 x BN, BN = 32, 64 or 128), one SM per tile, for calls whose 256-wide tiles are
+// too few to fill the GPU.
+//
+// Same panels, products, order and promotion interval as tcec_gemm_panels.cuh, so the same bits; K is not divided,
+// because the correction accumulates over all of it.  With 64 x 4096 x 4096 the wide kernel has 16 tiles for 148
+// SMs, this one 128.
+//
+// What bounds it: the copies.  A K block of a 128 x 32 tile brings 16 + 4 KB for 240 tensor cycles (an MMA with N = 32
+// takes 40 cycles, 64: 48, 128: 64), which is more than an SM takes in at 64 bytes per cycle; rows of A's panel that lie
+// beyond the matrix are therefore not copied (64 rows of A: 8 + 4 KB).  Up to 200 KB of copies are in flight.
+// Both accumulators exist twice in TMEM, so promotions, which a tile of long K has many of, cost no tensor time.
+#pragma once
+#include "tcec_gemm_panels.cuh"
+#include "tcec_gemm_roles.cuh"
+
+namespace tcec_sm100 {
+
+template <int BN, bool kEc>
+struct GemmNarrowCfg {
+  static constexpr int NP = kEc ? 2 : 1;
+  static constexpr int KBS = BN == 128 ? 1 : 2;          // K blocks per stage
+  static constexpr int A_BLOCK = kPanelBytes * NP;        // hi (lo) of 128 rows
+  static constexpr int B_IMAGE = BN * 64;                 // hi or lo of BN rows
+  static constexpr int B_BLOCK = B_IMAGE * NP;
+  static constexpr int STAGE_BYTES = KBS * (A_BLOCK + B_BLOCK);
+  static constexpr int NST_RAW = (200 * 1024) / STAGE_BYTES;
+  static constexpr int NST = NST_RAW > 8 ? 8 : NST_RAW;
+  static constexpr int EPI_WARPS = BN == 32 ? 4 : 8;
+  static constexpr int NC = BN == 128 ? 64 : 32;          // columns per epilogue warp
+  static constexpr int EPI_OFFSET = NST * STAGE_BYTES;
+  static constexpr int SMEM_BYTES = NST * STAGE_BYTES + EPI_WARPS * kEpiBufBytes + 1024;
+  static_assert(SMEM_BYTES <= 232448 - 512, "dynamic + static shared memory exceed an SM");
+  static constexpr int THREADS = 128 + 32 * EPI_WARPS;
+  static constexpr int TMEM_COLS = kEc ? 512 : 256;
+  static constexpr int GROUP_M = 16;
+};
+
+template <int BN, bool kTf32, bool kEc>
+__global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_panels_narrow_kernel(const GemmPanelParams p) {
+  using Cfg = GemmNarrowCfg<BN, kEc>;
+  constexpr int NST = Cfg::NST;
+  extern __shared__ uint8_t smem_raw[];
+  __shared__ uint64_t bar_full[NST], bar_empty[NST];
+  __shared__ uint64_t bar_main_full[2], bar_main_free[2], bar_corr_full[2], bar_corr_free[2], bar_drain[2];
+  __shared__ uint32_t tmem_base_s;
+  __shared__ uint32_t abort_flag;
+
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
+  const int warp = warp_index(), lane = threadIdx.x & 31;
+  const int ntiles = p.tiles_m * p.tiles_n * p.batch;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NST; ++s) {
+      mbar_init(smem_u32(&bar_full[s]), 1);
+      mbar_init(smem_u32(&bar_empty[s]), kEc ? 2 : 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(smem_u32(&bar_main_full[i]), 1);
+      mbar_init(smem_u32(&bar_main_free[i]), Cfg::EPI_WARPS);
+      mbar_init(smem_u32(&bar_corr_full[i]), 1);
+      mbar_init(smem_u32(&bar_corr_free[i]), Cfg::EPI_WARPS);
+      mbar_init(smem_u32(&bar_drain[i]), 1);
+    }
+    abort_flag = 0;
+    fence_mbar_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(smem_u32(&tmem_base_s), Cfg::TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_base_s;  // main buffers at +0 and +128, correction buffers at +256 and +384
+  volatile uint32_t* abortp = &abort_flag;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------ producer
+    if (elect_one()) {
+      uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0;
+      bool ok = true;
+      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+        const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
+        const uint8_t* pa = p.panels_a + tc.b * p.panels_a_batch_stride + static_cast<size_t>(tc.mt) * p.nkb * Cfg::A_BLOCK;
+        const int brow = tc.nt * BN;
+        const uint8_t* pb = p.panels_b + tc.b * p.panels_b_batch_stride +
+                            static_cast<size_t>(brow / 128) * p.nkb * (kPanelBytes * Cfg::NP) + (brow % 128) * 64;
+        const int rows = (min(128, p.M - tc.mt * 128) + 7) & ~7;  // of A's panel that the matrix has, in whole groups
+        for (int kb = 0; kb < p.nkb; kb += Cfg::KBS) {
+          if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 32)) {
+            ok = false;
+            break;
+          }
+          const uint32_t full = smem_u32(&bar_full[s]);
+          const uint32_t dst = smem_base + s * Cfg::STAGE_BYTES;
+          const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, p.nkb - kb);
+          mbar_arrive_expect_tx(full, nblk * Cfg::NP * (rows * 64 + Cfg::B_IMAGE));
+          armed |= 1u << s;
+          armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
+          const uint8_t* sa = pa + static_cast<size_t>(kb) * Cfg::A_BLOCK;
+          if (rows == 128) {
+            bulk_load(dst, sa, nblk * Cfg::A_BLOCK, full);
+          } else {
+            for (int i = 0; i < nblk * Cfg::NP; ++i) bulk_load(dst + i * kPanelBytes, sa + i * kPanelBytes, rows * 64, full);
+          }
+          const uint8_t* sb = pb + static_cast<size_t>(kb) * (kPanelBytes * Cfg::NP);
+          const uint32_t db = dst + Cfg::KBS * Cfg::A_BLOCK;
+          for (int i = 0; i < nblk * Cfg::NP; ++i) bulk_load(db + i * Cfg::B_IMAGE, sb + i * kPanelBytes, Cfg::B_IMAGE, full);
+          if (++s == static_cast<uint32_t>(NST)) {
+            s = 0;
+            ph ^= 1;
+          }
+        }
+      }
+      if (!ok) {
+        abort_flag = 1;
+        atomicCAS(p.status, 0, kErrProducerWait);
+        // let this thread's own copies land before the CTA gives up its shared memory
+        for (uint32_t q = 0; q < static_cast<uint32_t>(NST); ++q)
+          if (armed & (1u << q)) mbar_wait_plain(smem_u32(&bar_full[q]), (armed_parity >> q) & 1);
+      }
+    }
+  } else if (warp == 1 || warp == 2) {
+    // ------------------------------------------------------------ MMA issuers (tcec_gemm_roles.cuh)
+    if ((warp == 1 || kEc) && elect_one()) {
+      DoubleImage im;
+      im.dconst = umma_desc_kmajor_noswizzle(0, 128, 512);
+      im.base16 = (smem_base & 0x3ffff) >> 4;
+      im.stage16 = Cfg::STAGE_BYTES >> 4;
+      im.a_lo16 = kPanelBytes >> 4;
+      im.b_hi16 = (Cfg::KBS * Cfg::A_BLOCK) >> 4;
+      im.b_lo16 = im.b_hi16 + (Cfg::B_IMAGE >> 4);
+      im.kstep16 = 16;
+      im.a_block16 = Cfg::A_BLOCK >> 4;
+      im.b_block16 = Cfg::B_BLOCK >> 4;
+      int tile = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
+      auto next_tile = [&](uint32_t& idesc) {
+        tile += gridDim.x;
+        idesc = umma_idesc(kTf32 ? 2u : 0u, 128, BN);
+        return tile < ntiles;
+      };
+      const KWalk walk{p.nkb, p.promo};
+      const RingBarriers ring{bar_full, bar_empty};
+      const bool ok =
+          warp == 1 ? issue_main_double<kTf32, NST, Cfg::KBS>(next_tile, walk, im, tmem, ring, bar_main_full, bar_main_free, abortp)
+                    : issue_corr_double<kTf32, NST, Cfg::KBS>(next_tile, walk, im, tmem + 256, ring, bar_corr_full,
+                                                              bar_corr_free, abortp);
+      if (!ok) mma_thread_gave_up<false>(&abort_flag, p.status, kErrMmaWait, &bar_drain[warp - 1]);
+    }
+  } else if (warp >= 4) {
+    // ------------------------------------------------------------ epilogue
+    const int ew = warp - 4, q = warp & 3, col_in = (ew >> 2) * Cfg::NC;
+    const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + col_in;
+    const int nchunks = p.promo ? (p.nkb + p.promo - 1) / p.promo : 1;
+    uint32_t chunk = 0, tcount = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
+      const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
+      float acc[Cfg::NC];
+      for (int c = 0; c < nchunks; ++c, ++chunk) {
+        if (!mbar_wait_warp(smem_u32(&bar_main_full[chunk & 1]), (chunk >> 1) & 1, abortp, 64)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        promote_main_double(acc, taddr + (chunk & 1) * kDoubleCols, c == 0);
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_main_free[chunk & 1]));
+      }
+      if (!ok) break;
+      if constexpr (kEc) {
+        if (!mbar_wait_warp(smem_u32(&bar_corr_full[tcount & 1]), (tcount >> 1) & 1, abortp, 64)) {
+          ok = false;
+          break;
+        }
+        tc_fence_after();
+        fold_correction_double(acc, taddr + 256 + (tcount & 1) * kDoubleCols, kTf32 ? 1.0f : (1.0f / 2048.0f));
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(smem_u32(&bar_corr_free[tcount & 1]));
+      }
+      StoreTarget st;
+      st.cbase = p.c_array ? p.c_array[tc.b] : p.c + tc.b * p.c_batch_stride;
+      st.ldc = p.ldc;
+      st.M = p.M;
+      st.N = p.N;
+      st.col_major = p.c_col_major;
+      st.vec_ok = !p.c_col_major && (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(st.cbase) & 15) == 0);
+      st.alpha = p.alpha;
+      st.beta = p.beta;
+      const int row0 = tc.mt * 128 + q * 32, col0 = tc.nt * BN + col_in;
+      if (row0 < p.M && col0 < p.N)
+        store_warp_block(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
+    }
+    if (!ok) {
+      abort_flag = 1;
+      if (lane == 0) atomicCAS(p.status, 0, kErrEpilogueWait);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) tmem_dealloc(tmem, Cfg::TMEM_COLS);
+}
+
+}  // namespace tcec_sm100

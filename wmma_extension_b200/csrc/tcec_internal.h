@@ -31,6 +31,7 @@ struct Options {
   int cta_pair = -1;    // -1: CTA-pair kernel for the policies without error correction; 0: never; 1: whenever it applies
   int half_tiles = 1;   // CTA-pair kernel: calls with very few tiles run on 256 x 128 half tiles
   int path = 0;         // 0: chosen per call, 1: always operand panels, 2: FP32-tile kernel whenever it applies
+  int narrow_tiles = -1;   // panels: width of the narrow tiles (32, 64, 128) for calls with few tiles; -1: chosen per call; 0: never
   int direct_kernel = -1;  // -1: chosen per call from the sizes; 0: never; 1: whenever the other options allow it
   int comm_sms = 8;     // SMs the column-sharded step leaves to the broadcast (also the broadcast's CTA limit)
   int comm_panel_rows = 2048;  // rows of A per broadcast
