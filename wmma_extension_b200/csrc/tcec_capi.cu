@@ -301,8 +301,7 @@ void launch_narrow_as(int width, const GemmPanelParams& gp, int grid, cudaStream
 bool bad_layout(int l) { return l != TCEC_ROW_MAJOR && l != TCEC_COL_MAJOR; }
 
 static SplitParams split_params(bool k_contiguous, int rows, int k, const float* src, const float* const* src_array,
-                                long long ld, long long stride, uint8_t* panels, size_t panels_stride, int policy,
-                                const PackPart& part) {
+                                long long ld, long long stride, uint8_t* panels, size_t panels_stride, int policy) {
   const int kop = policy_tf32(policy) ? 16 : 32;
   SplitParams sp{};
   sp.src = src;
@@ -316,18 +315,13 @@ static SplitParams split_params(bool k_contiguous, int rows, int k, const float*
   sp.nkb = (k + kop - 1) / kop;
   sp.panels = panels;
   sp.panels_batch_stride = static_cast<long long>(panels_stride);
-  sp.mul = part.mul;
-  sp.elem_stride = part.elem_stride;
-  sp.kb_offset = part.kb_offset;
-  sp.nkb_out = part.nkb_out;
   return sp;
 }
 
 void pack_operand(bool k_contiguous, int rows, int k, const float* src, const float* const* src_array,
                   long long ld, long long stride, int batch, uint8_t* panels, size_t panels_stride,
-                  int policy, cudaStream_t stream, const PackPart& part) {
-  const SplitParams sp = split_params(k_contiguous, rows, k, src, src_array, ld, stride, panels, panels_stride, policy,
-                                      part);
+                  int policy, cudaStream_t stream) {
+  const SplitParams sp = split_params(k_contiguous, rows, k, src, src_array, ld, stride, panels, panels_stride, policy);
   if (policy_tf32(policy)) {
     if (policy_ec(policy)) launch_split<true, true>(sp, batch, stream);
     else launch_split<true, false>(sp, batch, stream);
@@ -342,9 +336,8 @@ void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a
                uint8_t* panels_a, size_t a_stride, bool b_k_contiguous, int n, const float* b, const float* const* b_array,
                long long ldb, long long stride_b, uint8_t* panels_b, size_t b_stride, int k, int batch, int policy,
                cudaStream_t stream) {
-  const PackPart plain;
-  const SplitParams pa = split_params(a_k_contiguous, m, k, a, a_array, lda, stride_a, panels_a, a_stride, policy, plain);
-  const SplitParams pb = split_params(b_k_contiguous, n, k, b, b_array, ldb, stride_b, panels_b, b_stride, policy, plain);
+  const SplitParams pa = split_params(a_k_contiguous, m, k, a, a_array, lda, stride_a, panels_a, a_stride, policy);
+  const SplitParams pb = split_params(b_k_contiguous, n, k, b, b_array, ldb, stride_b, panels_b, b_stride, policy);
   const unsigned long long na = static_cast<unsigned long long>(pa.nkb) * pa.row_blocks * batch;
   const unsigned long long nb = static_cast<unsigned long long>(pb.nkb) * pb.row_blocks * batch;
   if (na + nb > 0x7fffffffull) {  // beyond one grid: one launch (or several) per operand
@@ -740,19 +733,17 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
 }
 
 // ---------------------------------------------------------------- complex GEMM (four real products)
-// C = alpha * (Pr + i Pi) + beta * C on interleaved complex C; Pr, Pi are dense planar products.
-__global__ void cgemm_combine_kernel(const float* __restrict__ pr, const float* __restrict__ pi, float2* c,
-                                     long long ldc, int inner, int outer, float2 alpha, float2 beta,
-                                     int has_product) {
+// C = alpha * P + beta * C on interleaved complex C; P is the dense interleaved product (rows of `inner`).
+__global__ void cgemm_combine_kernel(const float2* __restrict__ prod, float2* c, long long ldc, int inner, int outer,
+                                     float2 alpha, float2 beta, int has_product) {
   for (int o = blockIdx.y; o < outer; o += gridDim.y)
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < inner; i += gridDim.x * blockDim.x) {
       float2* dst = c + static_cast<long long>(o) * ldc + i;
       float2 out = make_float2(0.f, 0.f);
       if (has_product) {
-        const long long q = static_cast<long long>(o) * inner + i;
-        const float xr = pr[q], xi = pi[q];
-        out.x = alpha.x * xr - alpha.y * xi;
-        out.y = alpha.x * xi + alpha.y * xr;
+        const float2 x = prod[static_cast<long long>(o) * inner + i];
+        out.x = alpha.x * x.x - alpha.y * x.y;
+        out.y = alpha.x * x.y + alpha.y * x.x;
       }
       if (beta.x != 0.f || beta.y != 0.f) {
         const float2 old = *dst;
@@ -765,10 +756,11 @@ __global__ void cgemm_combine_kernel(const float* __restrict__ pr, const float* 
 
 // The reference builds a complex product from four real TCEC products
 // (include/wmma_extension/tcec/complex.hpp:646-727): real = Ar Br + Ai (-Bi), imag = Ai Br + Ar Bi.
-// Here the two products of each part become ONE real GEMM over a K of twice the length:
-// [Ar | Ai] x [Br ; -Bi] and [Ar | Ai] x [Bi ; Br].  A is split once into a concatenated panel
-// set, B into two; both GEMMs run through the real kernel into planar scratch, and an
-// elementwise pass applies the complex alpha and beta into the interleaved C.
+// Here all four are ONE real GEMM of twice the N and K (tcec_panels.cuh: A' = A as it lies, re and im alternating along K;
+// B' = the 2 x 2 blocks [re -im; im re]), whose row-major result is interleaved complex C.  A column-major C is the
+// row-major transposed product of the swapped operands.  With real alpha and beta the GEMM writes C itself;
+// otherwise it writes a scratch product and an elementwise pass applies them.  2048^3: one split launch of both operands and
+// one GEMM launch instead of six and two, and no combining pass.
 int cgemm_impl(int la, int lb, int lc, int m, int n, int k, const float* alpha, const float* a, long long lda,
                const float* b, long long ldb, const float* beta, float* c, long long ldc, int policy,
                void* stream_v) {
@@ -797,57 +789,71 @@ int cgemm_impl(int la, int lb, int lc, int m, int n, int k, const float* alpha, 
   const dim3 cgrid((inner + 255) / 256, outer < 32768 ? outer : 32768);
   const float2 al = make_float2(alpha[0], alpha[1]), be = make_float2(beta[0], beta[1]);
   if (!has_product) {
-    cgemm_combine_kernel<<<cgrid, 256, 0, stream>>>(nullptr, nullptr, reinterpret_cast<float2*>(c), ldc, inner,
-                                                    outer, al, be, 0);
+    cgemm_combine_kernel<<<cgrid, 256, 0, stream>>>(nullptr, reinterpret_cast<float2*>(c), ldc, inner, outer, al, be, 0);
     TCEC_CUDA(cudaGetLastError());
     return TCEC_OK;
   }
   const int kop = policy_tf32(policy) ? 16 : 32;
-  const int nkb = (k + kop - 1) / kop;
-  const long long k2_ll = 2ll * nkb * kop;
-  if (k2_ll > 0x7fffffff) return TCEC_ERR_INVALID_ARGUMENT;
-  const int k2 = static_cast<int>(k2_ll);
-  const Shape s = plan(m, n, k2, policy, opt);
-  const size_t plane = ((static_cast<size_t>(m) * n * sizeof(float)) + 255) & ~static_cast<size_t>(255);
+  if (2ll * ((k + kop - 1) / kop) * kop > 0x7fffffff) return TCEC_ERR_INVALID_ARGUMENT;
+  if (inner > 0x3fffffff) return TCEC_ERR_ALLOC;  // its panels alone are beyond any device's memory
+  const int k2 = 2 * k, n2 = 2 * inner;
+  const Shape s = plan(outer, n2, k2, policy, opt);
+  const bool real_scalars = alpha[1] == 0.f && beta[1] == 0.f;
+  const size_t product = real_scalars ? 0 : static_cast<size_t>(outer) * n2 * sizeof(float);
+  const unsigned long long na = static_cast<unsigned long long>(s.nkb) * s.a_row_blocks;
+  const unsigned long long nb = static_cast<unsigned long long>(s.nkb) * s.b_row_blocks;
+  if (na + nb > 0x7fffffffull) return TCEC_ERR_ALLOC;  // 2^31 panels of 8 KB
   void* ws = nullptr;
   void* old = nullptr;
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    rc = get_workspace(st, stream, s.a_bytes + 2 * s.b_bytes + 2 * plane, &ws, &old);
+    rc = get_workspace(st, stream, s.a_bytes + s.b_bytes + product, &ws, &old);
   }
   const int rel = release_old_workspace(old, stream);
   if (rc != TCEC_OK) return rc;
   if (rel != TCEC_OK) return rel;
-  uint8_t* pa = static_cast<uint8_t*>(ws);
-  uint8_t* pbr = pa + s.a_bytes;
-  uint8_t* pbi = pbr + s.b_bytes;
-  float* prod_r = reinterpret_cast<float*>(pbi + s.b_bytes);
-  float* prod_i = reinterpret_cast<float*>(pbi + s.b_bytes + plane);
-  const bool a_kc = (la == TCEC_ROW_MAJOR), b_kc = (lb == TCEC_COL_MAJOR);
-  PackPart first, second;
-  first.elem_stride = second.elem_stride = 2;
-  first.nkb_out = second.nkb_out = 2 * nkb;
-  second.kb_offset = nkb;
-  // A' = [Ar | Ai]
-  pack_operand(a_kc, m, k, a, nullptr, 2 * lda, 0, 1, pa, 0, policy, stream, first);
-  pack_operand(a_kc, m, k, a + 1, nullptr, 2 * lda, 0, 1, pa, 0, policy, stream, second);
-  // B'r = [Br ; -Bi], B'i = [Bi ; Br]
-  pack_operand(b_kc, n, k, b, nullptr, 2 * ldb, 0, 1, pbr, 0, policy, stream, first);
-  PackPart neg = second;
-  neg.mul = -1.0f;
-  pack_operand(b_kc, n, k, b + 1, nullptr, 2 * ldb, 0, 1, pbr, 0, policy, stream, neg);
-  pack_operand(b_kc, n, k, b + 1, nullptr, 2 * ldb, 0, 1, pbi, 0, policy, stream, first);
-  pack_operand(b_kc, n, k, b, nullptr, 2 * ldb, 0, 1, pbi, 0, policy, stream, second);
+  uint8_t* panels_a = static_cast<uint8_t*>(ws);
+  uint8_t* panels_b = panels_a + s.a_bytes;
+  float* scratch = reinterpret_cast<float*>(panels_b + s.b_bytes);
+  const bool row = lc == TCEC_ROW_MAJOR;
+  // what multiplies from the left (rows = outer) and from the right (columns = inner)
+  ComplexSplitParams pa{}, pb{};
+  pa.src = row ? a : b;
+  pa.ld = row ? lda : ldb;
+  pa.k_contiguous = row ? la == TCEC_ROW_MAJOR : lb == TCEC_COL_MAJOR;
+  pa.rows = outer;
+  pa.row_blocks = s.a_row_blocks;
+  pa.panels = panels_a;
+  pb.src = row ? b : a;
+  pb.ld = row ? ldb : lda;
+  pb.k_contiguous = row ? lb == TCEC_COL_MAJOR : la == TCEC_ROW_MAJOR;
+  pb.rows = inner;
+  pb.doubled = 1;
+  pb.row_blocks = s.b_row_blocks;
+  pb.panels = panels_b;
+  pa.k = pb.k = k;
+  pa.nkb = pb.nkb = s.nkb;
+  const unsigned int grid = static_cast<unsigned int>(na + nb), first_b = static_cast<unsigned int>(na);
+  if (policy_tf32(policy)) {
+    if (policy_ec(policy)) tcec_split_complex_kernel<true, true><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+    else tcec_split_complex_kernel<true, false><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+  } else {
+    if (policy_ec(policy)) tcec_split_complex_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+    else tcec_split_complex_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+  }
   {
-    std::lock_guard<std::mutex> lock(g_mu);
-    rc = gemm_packed(s, m, n, k2, 1.0f, pa, 0, pbr, 0, 0.0f, prod_r, nullptr, inner, 0, lc, 1, policy, st, stream, opt);
-    if (rc == TCEC_OK)
-      rc = gemm_packed(s, m, n, k2, 1.0f, pa, 0, pbi, 0, 0.0f, prod_i, nullptr, inner, 0, lc, 1, policy, st, stream,
-                       opt);
+    std::lock_guard<std::mutex> lock(g_mu);  // the per-stream tile counters may be created here
+    if (real_scalars)
+      rc = gemm_packed(s, outer, n2, k2, alpha[0], panels_a, 0, panels_b, 0, beta[0], c, nullptr, 2 * ldc, 0,
+                       TCEC_ROW_MAJOR, 1, policy, st, stream, opt);
+    else
+      rc = gemm_packed(s, outer, n2, k2, 1.0f, panels_a, 0, panels_b, 0, 0.0f, scratch, nullptr, n2, 0, TCEC_ROW_MAJOR, 1,
+                       policy, st, stream, opt);
   }
   if (rc != TCEC_OK) return rc;
-  cgemm_combine_kernel<<<cgrid, 256, 0, stream>>>(prod_r, prod_i, reinterpret_cast<float2*>(c), ldc, inner,
-                                                  outer, al, be, 1);
+  if (!real_scalars)
+    cgemm_combine_kernel<<<cgrid, 256, 0, stream>>>(reinterpret_cast<const float2*>(scratch), reinterpret_cast<float2*>(c), ldc,
+                                                    inner, outer, al, be, 1);
   TCEC_CUDA(cudaGetLastError());
   return TCEC_OK;
 }

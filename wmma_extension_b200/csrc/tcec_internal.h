@@ -80,17 +80,8 @@ size_t packed_bytes(int rows, int k, int policy);
 Shape plan(int m, int n, int k, int policy, const Options& opt);
 
 // Split one operand (A: rows = m; B: rows = n) into panels on `stream`.
-// `part` describes an operand that is one half of a K-concatenated panel set built from
-// interleaved complex data: element stride 2, a sign, and where its k blocks go.
-struct PackPart {
-  int elem_stride = 1;
-  float mul = 1.0f;
-  int kb_offset = 0;
-  int nkb_out = 0;
-};
 void pack_operand(bool k_contiguous, int rows, int k, const float* src, const float* const* src_array, long long ld,
-                  long long stride, int batch, uint8_t* panels, size_t panels_stride, int policy, cudaStream_t stream,
-                  const PackPart& part = PackPart());
+                  long long stride, int batch, uint8_t* panels, size_t panels_stride, int policy, cudaStream_t stream);
 
 // What a launch of the packed GEMM may add to the plain call.
 struct LaunchExtras {

@@ -84,11 +84,6 @@ struct SplitParams {
   int nkb;                       // number of k blocks
   uint8_t* panels;               // output
   long long panels_batch_stride; // bytes
-  float mul;                     // value multiplied in before the split (1 for plain loads)
-  int elem_stride;               // floats between consecutive elements (0 or 1: dense; 2: one part of
-                                 // interleaved complex data, `src` pointing at that part)
-  int kb_offset;                 // first k block written (operands concatenated along K)
-  int nkb_out;                   // k blocks per row block in the destination (0: nkb)
 };
 
 // One CTA's work: the hi(+lo) panel of k block `kb`, row block `rb` of matrix `b`.
@@ -99,11 +94,9 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
   const float* __restrict__ src =
       p.src_array ? p.src_array[b] : p.src + static_cast<long long>(b) * p.batch_stride;
   uint8_t* out = p.panels + static_cast<long long>(b) * p.panels_batch_stride +
-                 (static_cast<size_t>(rb) * (p.nkb_out ? p.nkb_out : p.nkb) + p.kb_offset + kb) *
-                     (kEc ? 2 : 1) * kPanelBytes;
+                 (static_cast<size_t>(rb) * p.nkb + kb) * (kEc ? 2 : 1) * kPanelBytes;
   const int k0 = kb * KOP;
-  const int es = p.elem_stride > 1 ? p.elem_stride : 1;
-  const bool vec_ok = (es == 1) && (p.ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
+  const bool vec_ok = (p.ld % 4 == 0) && ((reinterpret_cast<uintptr_t>(src) & 15) == 0);
 #pragma unroll
   for (int it = 0; it < 2; ++it) {
     const int item = threadIdx.x + it * 256;  // 512 (row, chunk) items per panel
@@ -119,7 +112,7 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
     const int kk = k0 + c * KCH;
     float v[KCH];
     if (p.k_contiguous) {
-      const float* s = src + static_cast<long long>(row) * p.ld + static_cast<long long>(kk) * es;
+      const float* s = src + static_cast<long long>(row) * p.ld + kk;
       if (row < p.rows && kk + KCH <= p.k && vec_ok) {
 #pragma unroll
         for (int q = 0; q < KCH / 4; ++q) {
@@ -131,18 +124,14 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
         }
       } else {
 #pragma unroll
-        for (int q = 0; q < KCH; ++q) v[q] = (row < p.rows && kk + q < p.k) ? __ldg(s + q * es) : 0.f;
+        for (int q = 0; q < KCH; ++q) v[q] = (row < p.rows && kk + q < p.k) ? __ldg(s + q) : 0.f;
       }
     } else {
 #pragma unroll
       for (int q = 0; q < KCH; ++q)
         v[q] = (row < p.rows && kk + q < p.k)
-                   ? __ldg(src + static_cast<long long>(kk + q) * p.ld + static_cast<long long>(row) * es)
+                   ? __ldg(src + static_cast<long long>(kk + q) * p.ld + row)
                    : 0.f;
-    }
-    if (p.mul != 1.0f) {
-#pragma unroll
-      for (int q = 0; q < KCH; ++q) v[q] *= p.mul;
     }
     uint4 hi, lo;
     if constexpr (kTf32) {
@@ -154,6 +143,69 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
     *reinterpret_cast<uint4*>(out + off) = hi;
     if constexpr (kEc) *reinterpret_cast<uint4*>(out + kPanelBytes + off) = lo;
   }
+}
+
+// Split of one operand of a complex product into the panels of a real one of twice the K.  With K' = 2p + d and
+// rows (plain, for A) or doubled rows (for B)
+//   A'(i, 2p) = Re A(i, p),  A'(i, 2p + 1) = Im A(i, p)
+//   B'(2j, 2p) = Re B(p, j), B'(2j, 2p + 1) = -Im B(p, j);  B'(2j + 1, 2p) = Im B(p, j), B'(2j + 1, 2p + 1) = Re B(p, j)
+// column 2j of A' B' is the real part and column 2j + 1 the imaginary part of column j of A B: the real GEMM
+// writes interleaved C.  Every complex element is read once; a doubled operand writes it into two rows.
+struct ComplexSplitParams {
+  const float* src;   // interleaved; 8-byte alignment is used where it is there, not required
+  long long ld;       // complex elements
+  int rows, k;        // complex extents
+  int k_contiguous;   // element (r, p) at r*ld + p, else at p*ld + r
+  int doubled;
+  int row_blocks;     // of the panels, padded rows / 128
+  int nkb;            // K blocks of the panels
+  uint8_t* panels;
+};
+template <bool kTf32, bool kEc>
+__device__ __forceinline__ void split_complex_panel(const ComplexSplitParams& p, int kb, int rb) {
+  constexpr int PC = kTf32 ? 2 : 4;  // complex elements per 16-byte operand chunk
+  uint8_t* out = p.panels + (static_cast<size_t>(rb) * p.nkb + kb) * (kEc ? 2 : 1) * kPanelBytes;
+  const int R = p.doubled ? 64 : 128;  // complex rows of this panel
+  const bool pairs = (reinterpret_cast<uintptr_t>(p.src) & 7) == 0;
+  for (int item = threadIdx.x; item < R * 4; item += 256) {
+    const int r = p.k_contiguous ? item >> 2 : item % R, c = p.k_contiguous ? item & 3 : item / R;
+    const int row = rb * R + r, k0 = (kb * 4 + c) * PC;
+    const long long step = p.k_contiguous ? 1 : p.ld;
+    const float* q =
+        p.src + 2 * (p.k_contiguous ? static_cast<long long>(row) * p.ld + k0 : static_cast<long long>(k0) * p.ld + row);
+    float2 z[PC];
+#pragma unroll
+    for (int e = 0; e < PC; ++e) {
+      const float* x = q + 2 * e * step;
+      z[e] = make_float2(0.f, 0.f);
+      if (row < p.rows && k0 + e < p.k) z[e] = pairs ? __ldg(reinterpret_cast<const float2*>(x)) : make_float2(__ldg(x), __ldg(x + 1));
+    }
+    const int halves = p.doubled ? 2 : 1;
+    for (int h = 0; h < halves; ++h) {
+      const int orow = p.doubled ? 2 * r + h : r;
+      float v[2 * PC];
+#pragma unroll
+      for (int e = 0; e < PC; ++e) {
+        v[2 * e] = h ? z[e].y : z[e].x;
+        v[2 * e + 1] = h ? z[e].x : (p.doubled ? -z[e].y : z[e].y);
+      }
+      uint4 hi, lo;
+      if constexpr (kTf32) split4_tf32(v, hi, lo);
+      else split8_f16(v, hi, lo);
+      const int off = (orow >> 3) * 512 + c * 128 + (orow & 7) * 16;
+      *reinterpret_cast<uint4*>(out + off) = hi;
+      if constexpr (kEc) *reinterpret_cast<uint4*>(out + kPanelBytes + off) = lo;
+    }
+  }
+}
+// Both operands of a complex product: blocks below `panels_a` write A's panels.
+template <bool kTf32, bool kEc>
+__global__ void __launch_bounds__(256) tcec_split_complex_kernel(const ComplexSplitParams pa, const ComplexSplitParams pb,
+                                                                 unsigned int panels_a) {
+  const bool second = blockIdx.x >= panels_a;
+  const ComplexSplitParams& p = second ? pb : pa;
+  const unsigned int i = second ? blockIdx.x - panels_a : blockIdx.x;
+  split_complex_panel<kTf32, kEc>(p, i % p.nkb, i / p.nkb);
 }
 
 // grid = (nkb, row_blocks, batch), 256 threads: one CTA writes one hi(+lo) panel.
