@@ -336,8 +336,12 @@ void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a
                uint8_t* panels_a, size_t a_stride, bool b_k_contiguous, int n, const float* b, const float* const* b_array,
                long long ldb, long long stride_b, uint8_t* panels_b, size_t b_stride, int k, int batch, int policy,
                cudaStream_t stream) {
-  const SplitParams pa = split_params(a_k_contiguous, m, k, a, a_array, lda, stride_a, panels_a, a_stride, policy);
-  const SplitParams pb = split_params(b_k_contiguous, n, k, b, b_array, ldb, stride_b, panels_b, b_stride, policy);
+  SplitParams pa = split_params(a_k_contiguous, m, k, a, a_array, lda, stride_a, panels_a, a_stride, policy);
+  SplitParams pb = split_params(b_k_contiguous, n, k, b, b_array, ldb, stride_b, panels_b, b_stride, policy);
+  // These panels are the library's own and live for one call: the rows that pad them to 256 are not written.
+  pa.skip_padding = pb.skip_padding = 1;
+  pa.row_blocks = (m + 127) / 128;
+  pb.row_blocks = (n + 127) / 128;
   const unsigned long long na = static_cast<unsigned long long>(pa.nkb) * pa.row_blocks * batch;
   const unsigned long long nb = static_cast<unsigned long long>(pb.nkb) * pb.row_blocks * batch;
   if (na + nb > 0x7fffffffull) {  // beyond one grid: one launch (or several) per operand
@@ -1218,8 +1222,8 @@ int tcec_sgemm_static(int layout_a, int layout_b, int layout_c, int m, int n, in
   StaticDevice* sd = nullptr;
   const int rc = static_device_state(&sd);
   if (rc != TCEC_OK) return rc;
-  // Nothing in the array has to start at zero: the two split kernels below write every byte of
-  // every panel the GEMM reads (rows and K beyond the matrix are written as zeros), and the
+  // Nothing in the array has to start at zero: the split below writes every row of the matrices, with zeros for
+  // K beyond them; rows beyond them reach only elements of the product that are not stored; and the
   // status word is only ever raised, never relied on to be clear by the kernels.
   uint8_t* panels_a = sd->panels;
   uint8_t* panels_b = sd->panels + s.a_bytes;  // a_bytes is a multiple of 8192

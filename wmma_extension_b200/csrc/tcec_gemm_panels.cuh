@@ -121,11 +121,35 @@ __device__ __forceinline__ TileCoord decode_tile(int tile, int tiles_m, int tile
   return t;
 }
 
+// Rows of a 128-row panel block starting at `first` that a matrix of `rows` rows has, in whole groups of 8: what is
+// worth copying of it.  The others would only reach elements of the product that are not stored.
+__device__ __forceinline__ int panel_rows(int rows, int first) {
+  const int left = rows - first;
+  return left >= 128 ? 128 : (left > 0 ? (left + 7) & ~7 : 0);
+}
+// `images` consecutive panel images (hi, lo or K blocks of either), their first `rows` rows each.
+__device__ __forceinline__ void load_panel_rows(uint32_t dst, const uint8_t* src, int images, int rows, uint32_t full) {
+  if (rows == 0) return;
+  for (int i = 0; i < images; ++i) bulk_load(dst + i * kPanelBytes, src + i * kPanelBytes, rows * 64, full);
+}
+
 // One thread: arms `full` and issues the copies of one stage, K blocks kb .. kb + nblk - 1 of A's row block
 // at `pa` and of the NB row blocks of B (each nkb blocks long) at `pb`.
 template <class Cfg>
 __device__ __forceinline__ void load_panel_stage(uint32_t dst, const uint8_t* pa, const uint8_t* pb, int nkb, int kb,
-                                                 int nblk, uint32_t full) {
+                                                 int nblk, uint32_t full, int arows, int brows0, int brows1) {
+  if (arows + brows0 + (Cfg::NB == 2 ? brows1 : 128) < 384) {  // the matrix ends inside this tile
+    mbar_arrive_expect_tx(full, nblk * Cfg::NP * (arows + brows0 + (Cfg::NB == 2 ? brows1 : 0)) * 64);
+    load_panel_rows(dst, pa + static_cast<size_t>(kb) * Cfg::A_BLOCK, nblk * Cfg::NP, arows, full);
+#pragma unroll
+    for (int h = 0; h < Cfg::NB; ++h)
+      for (int i = 0; i < nblk; ++i)
+#pragma unroll
+        for (int lo = 0; lo < Cfg::NP; ++lo)
+          load_panel_rows(dst + Cfg::A_BYTES + ((i * Cfg::NP + lo) * Cfg::NB + h) * kPanelBytes,
+                          pb + ((static_cast<size_t>(h) * nkb + kb + i) * Cfg::NP + lo) * kPanelBytes, 1, h ? brows1 : brows0, full);
+    return;
+  }
   mbar_arrive_expect_tx(full, static_cast<uint32_t>(nblk) * (Cfg::STAGE_BYTES / Cfg::KBS));
   bulk_load(dst, pa + static_cast<size_t>(kb) * Cfg::A_BLOCK, nblk * Cfg::A_BLOCK, full);
   if constexpr (Cfg::NP == 2) {
@@ -258,6 +282,8 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
                             static_cast<size_t>(tc.mt) * p.nkb * Cfg::A_BLOCK;
         const uint8_t* pb = p.panels_b + tc.b * p.panels_b_batch_stride +
                             static_cast<size_t>(tc.nt) * Cfg::NB * p.nkb * (kPanelBytes * Cfg::NP);
+        const int arows = panel_rows(p.M, tc.mt * 128), brows0 = panel_rows(p.N, tc.nt * BN);
+        const int brows1 = panel_rows(p.N, tc.nt * BN + 128);
         for (int kb = 0; kb < p.nkb; kb += Cfg::KBS, ++it, s = (s + 1 == NST ? 0 : s + 1), ph ^= (s == 0)) {
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 128)) {
             ok = false;
@@ -275,7 +301,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
           const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, p.nkb - kb);  // K blocks in this stage
           armed |= 1u << s;
           armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-          load_panel_stage<Cfg>(dst, pa, pb, p.nkb, kb, nblk, full);
+          load_panel_stage<Cfg>(dst, pa, pb, p.nkb, kb, nblk, full, arows, brows0, brows1);
         }
         tile = next_tile;
       }

@@ -130,6 +130,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
           const int nblock = tc.nt * 2 + (BN == 256 ? static_cast<int>(rank) : tile % HALVES);
           const uint8_t* pb = p.panels_b + tc.b * p.panels_b_batch_stride +
                               static_cast<size_t>(nblock) * p.nkb * Cfg::BLOCK + (BN == 256 ? 0u : rank * B_PIECE);
+          const int arows = panel_rows(p.M, tc.mt * 256 + static_cast<int>(rank) * 128);
+          const int brows = BN == 256 ? panel_rows(p.N, nblock * 128) : 128;
           for (int kb = 0; kb < p.nkb; kb += Cfg::KBS, ++it) {
             if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 128)) {
               ok = false;
@@ -146,13 +148,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             const uint32_t full = smem_u32(&bar_full[s]);
             const uint32_t dst = smem_base + s * Cfg::STAGE_BYTES;
             const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, p.nkb - kb);  // K blocks in this stage
-            mbar_arrive_expect_tx(full, static_cast<uint32_t>(nblk) * (Cfg::BLOCK + Cfg::NP * B_PIECE));
+            mbar_arrive_expect_tx(full, static_cast<uint32_t>(nblk) * Cfg::NP * (arows * 64 + (BN == 256 ? brows * 64 : B_PIECE)));
             armed |= 1u << s;
             armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
-            bulk_load(dst, pa + static_cast<size_t>(kb) * Cfg::BLOCK, nblk * Cfg::BLOCK, full);
+            const uint8_t* srca = pa + static_cast<size_t>(kb) * Cfg::BLOCK;
+            if (arows == 128) bulk_load(dst, srca, nblk * Cfg::BLOCK, full);
+            else load_panel_rows(dst, srca, nblk * Cfg::NP, arows, full);
             const uint8_t* srcb = pb + static_cast<size_t>(kb) * Cfg::BLOCK;
             if constexpr (BN == 256) {
-              bulk_load(dst + Cfg::A_BYTES, srcb, nblk * Cfg::BLOCK, full);
+              if (brows == 128) bulk_load(dst + Cfg::A_BYTES, srcb, nblk * Cfg::BLOCK, full);
+              else load_panel_rows(dst + Cfg::A_BYTES, srcb, nblk * Cfg::NP, brows, full);
             } else {
 #pragma unroll
               for (int i = 0; i < Cfg::KBS; ++i)

@@ -84,6 +84,8 @@ struct SplitParams {
   int nkb;                       // number of k blocks
   uint8_t* panels;               // output
   long long panels_batch_stride; // bytes
+  int skip_padding;              // 1: rows beyond the matrix are left as they are (they only reach elements of the product
+                                 // that nobody stores); 0: they are written as zeros
 };
 
 // One CTA's work: the hi(+lo) panel of k block `kb`, row block `rb` of matrix `b`.
@@ -109,6 +111,7 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
       c = item >> 7;
     }
     const int row = rb * kPanelRows + r;
+    if (p.skip_padding && row >= p.rows) continue;
     const int kk = k0 + c * KCH;
     float v[KCH];
     if (p.k_contiguous) {
