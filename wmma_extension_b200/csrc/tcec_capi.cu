@@ -546,8 +546,10 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
                long long ldc, long long stride_c, int batch, int policy, const DeviceState* st,
                cudaStream_t stream, const Options& opt) {
   if (policy_tf32(policy) || !a || !b || !c || n <= 128) return false;
-  // Worth it only where the GEMM is bound by DRAM traffic, which the split pass doubles: short K.
-  const bool wanted = opt.path == 2 || (opt.path == 0 && batch > 1 && k <= 512);
+  // Worth it where the split pass, which doubles the DRAM traffic, costs more than conversion in every tile does: short
+  // K, and, up to where the promotion interval of the panel kernels grows, batches of longer K (panels against this,
+  // us: 64 x 400 x 400 x 1000 197 and 141, 32 x 1024^3 296 and 255, 32 x 1024 x 1024 x 2048 552 and 523).
+  const bool wanted = opt.path == 2 || (opt.path == 0 && batch > 1 && k <= 2048);
   if (!wanted) return false;
   if (!tma_addressable(a, lda, stride_a, batch) || !tma_addressable(b, ldb, stride_b, batch)) return false;
   const bool a_kc = (la == TCEC_ROW_MAJOR), b_kc = (lb == TCEC_COL_MAJOR);
