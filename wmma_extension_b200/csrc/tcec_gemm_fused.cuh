@@ -457,7 +457,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
       st.vec_ok = !p.c_col_major && (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(st.cbase) & 15) == 0);
       st.alpha = 1.0f;  // already applied
       st.beta = p.beta;
-      store_warp_block(acc, row0, col0, st,
+      store_warp_block<false>(acc, row0, col0, st,
                        reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * (Cfg::EPI_BYTES / Cfg::EPI_WARPS / 4), lane);
       if (etrace) trace_slot(p.trace, 7, 3 * tcount + 2);
     }

@@ -405,7 +405,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
       st.alpha = p.alpha;
       st.beta = p.beta;
       if (p.store_turn)
-        store_warp_block(acc, tc.mt * 128 + q * 32, col0, st,
+        store_warp_block<true>(acc, tc.mt * 128 + q * 32, col0, st,
                          reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
       else
         store_row_slice(acc, tc.mt * 128 + q * 32 + lane, col0, st);

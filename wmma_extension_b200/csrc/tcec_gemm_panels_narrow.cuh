@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
       st.beta = p.beta;
       const int row0 = tc.mt * 128 + q * 32, col0 = tc.nt * BN + col_in;
       if (row0 < p.M && col0 < p.N)
-        store_warp_block(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
+        store_warp_block<true>(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
     }
     if (!ok) {
       abort_flag = 1;

@@ -278,7 +278,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       st.vec_ok = vec_ok;
       st.alpha = p.alpha;
       st.beta = p.beta;
-      store_warp_block(acc, tc.mt * 256 + static_cast<int>(rank) * 128 + q * 32, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
+      store_warp_block<true>(acc, tc.mt * 256 + static_cast<int>(rank) * 128 + q * 32, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
     }
     if (!ok) {
       raise_abort_pair(&abort_flag);
