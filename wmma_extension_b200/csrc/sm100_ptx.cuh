@@ -117,6 +117,19 @@ __device__ __forceinline__ void tc_fence_after() {
 __device__ __forceinline__ void tma_prefetch_desc(const void* tmap) {
   asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
 }
+// Tensor maps in global memory: another base address for a map (generic proxy), and the fences that order such a change
+// before a use of the map by TMA on this GPU.
+__device__ __forceinline__ void tensormap_set_address(void* tmap, const void* base) {
+  asm volatile("tensormap.replace.tile.global_address.global.b1024.b64 [%0], %1;" ::"l"(
+                   __cvta_generic_to_global(tmap)), "l"(reinterpret_cast<uint64_t>(base))
+               : "memory");
+}
+__device__ __forceinline__ void tensormap_release() {
+  asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
+}
+__device__ __forceinline__ void tensormap_acquire(const void* tmap) {
+  asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(reinterpret_cast<uint64_t>(tmap)) : "memory");
+}
 // Tiled 3-D load (x fastest). Every CTA fetches its own tile.
 __device__ __forceinline__ void tma_load_3d(uint32_t dst, const void* tmap, uint32_t bar, int x,
                                             int y, int z) {

@@ -335,7 +335,7 @@ void pack_operand(bool k_contiguous, int rows, int k, const float* src, const fl
 void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a_array, long long lda, long long stride_a,
                uint8_t* panels_a, size_t a_stride, bool b_k_contiguous, int n, const float* b, const float* const* b_array,
                long long ldb, long long stride_b, uint8_t* panels_b, size_t b_stride, int k, int batch, int policy,
-               cudaStream_t stream) {
+               cudaStream_t stream, const int* only_if = nullptr, int sm_count = 0) {
   SplitParams pa = split_params(a_k_contiguous, m, k, a, a_array, lda, stride_a, panels_a, a_stride, policy);
   SplitParams pb = split_params(b_k_contiguous, n, k, b, b_array, ldb, stride_b, panels_b, b_stride, policy);
   // These panels are the library's own and live for one call: the rows that pad them to 256 are not written.
@@ -344,18 +344,19 @@ void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a
   pb.row_blocks = (n + 127) / 128;
   const unsigned long long na = static_cast<unsigned long long>(pa.nkb) * pa.row_blocks * batch;
   const unsigned long long nb = static_cast<unsigned long long>(pb.nkb) * pb.row_blocks * batch;
-  if (na + nb > 0x7fffffffull) {  // beyond one grid: one launch (or several) per operand
+  if (na + nb > 0x7fffffffull && !only_if) {  // beyond one grid: one launch (or several) per operand
     pack_operand(a_k_contiguous, m, k, a, a_array, lda, stride_a, batch, panels_a, a_stride, policy, stream);
     pack_operand(b_k_contiguous, n, k, b, b_array, ldb, stride_b, batch, panels_b, b_stride, policy, stream);
     return;
   }
-  const unsigned int grid = static_cast<unsigned int>(na + nb), first_b = static_cast<unsigned int>(na);
+  const unsigned int all = static_cast<unsigned int>(na + nb), first_b = static_cast<unsigned int>(na);
+  const unsigned int strided = static_cast<unsigned int>(8 * sm_count), grid = only_if && all > strided ? strided : all;
   if (policy_tf32(policy)) {
-    if (policy_ec(policy)) tcec_split_both_kernel<true, true><<<grid, 256, 0, stream>>>(pa, pb, first_b);
-    else tcec_split_both_kernel<true, false><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+    if (policy_ec(policy)) tcec_split_both_kernel<true, true><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
+    else tcec_split_both_kernel<true, false><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
   } else {
-    if (policy_ec(policy)) tcec_split_both_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b);
-    else tcec_split_both_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+    if (policy_ec(policy)) tcec_split_both_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
+    else tcec_split_both_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
   }
 }
 
@@ -389,6 +390,7 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
   gp.debug_flags = opt.debug_flags;
   gp.store_turn = opt.store_turn;
   gp.trace = opt.trace;
+  gp.only_if = ex.only_if;
   gp.row_ready = ex.row_ready;
   gp.ready_rows = ex.ready_rows;
   gp.ready_epoch = ex.ready_epoch;
@@ -540,25 +542,51 @@ bool tma_addressable(const float* base, long long ld, long long stride, int batc
          ld < (1ll << 36) && stride < (1ll << 36);
 }
 
+// Whether the FP32-tile kernel is the one for a call of this shape (its operands must be addressable as well).
+bool fused_wanted(int n, int k, int batch, int policy, const Options& opt) {
+  if (policy_tf32(policy) || n <= 128) return false;
+  // Worth it where the split pass, which doubles the DRAM traffic, costs more than conversion in every tile does: short
+  // K, and, up to where the promotion interval of the panel kernels grows, batches of longer K (panels against this,
+  // us: 64 x 400 x 400 x 1000 197 and 141, 32 x 1024^3 296 and 255, 32 x 1024 x 1024 x 2048 552 and 523).
+  return opt.path == 2 || (opt.path == 0 && batch > 1 && k <= 2048);
+}
+// What a call with pointer tables lends to the FP32-tile kernel: room for two maps per matrix, and the count of pointers
+// that TMA cannot address.
+struct TableMaps {
+  const float* const* a_array = nullptr;
+  const float* const* b_array = nullptr;
+  float* const* c_array = nullptr;
+  CUtensorMap* maps = nullptr;
+  int* bad = nullptr;
+};
+
 // Launches the FP32-tile kernel if the call qualifies; returns false (nothing launched) otherwise.
 bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const float* a, long long lda,
                long long stride_a, const float* b, long long ldb, long long stride_b, float beta, float* c,
                long long ldc, long long stride_c, int batch, int policy, const DeviceState* st,
-               cudaStream_t stream, const Options& opt) {
-  if (policy_tf32(policy) || !a || !b || !c || n <= 128) return false;
-  // Worth it where the split pass, which doubles the DRAM traffic, costs more than conversion in every tile does: short
-  // K, and, up to where the promotion interval of the panel kernels grows, batches of longer K (panels against this,
-  // us: 64 x 400 x 400 x 1000 197 and 141, 32 x 1024^3 296 and 255, 32 x 1024 x 1024 x 2048 552 and 523).
-  const bool wanted = opt.path == 2 || (opt.path == 0 && batch > 1 && k <= 2048);
-  if (!wanted) return false;
-  if (!tma_addressable(a, lda, stride_a, batch) || !tma_addressable(b, ldb, stride_b, batch)) return false;
+               cudaStream_t stream, const Options& opt, const TableMaps* table = nullptr) {
+  if (!fused_wanted(n, k, batch, policy, opt)) return false;
   const bool a_kc = (la == TCEC_ROW_MAJOR), b_kc = (lb == TCEC_COL_MAJOR);
   CUtensorMap map_a, map_b, map_c;
-  if (!encode_operand_map(&map_a, a, a_kc, m, k, lda, stride_a, batch, 128)) return false;
-  if (!encode_operand_map(&map_b, b, b_kc, n, k, ldb, stride_b, batch, 128)) return false;
-  // C goes out through tensor stores when nothing has to be read back and its rows are addressable.
-  const bool c_tma = lc == TCEC_ROW_MAJOR && beta == 0.f && tma_addressable(c, ldc, stride_c, batch) &&
-                     encode_c_map(&map_c, c, m, n, ldc, stride_c, batch);
+  bool c_tma = false;
+  if (table) {
+    // templates: every map takes its address from the table (the one given here only has to be aligned)
+    const float* any = reinterpret_cast<const float*>(table->maps);
+    if (!tma_addressable(any, lda, 0, 1) || !tma_addressable(any, ldb, 0, 1)) return false;
+    if (!encode_operand_map(&map_a, any, a_kc, m, k, lda, 0, 1, 128)) return false;
+    if (!encode_operand_map(&map_b, any, b_kc, n, k, ldb, 0, 1, 128)) return false;
+    cudaMemsetAsync(table->bad, 0, sizeof(int), stream);
+    tcec_table_maps_kernel<<<(batch + 127) / 128 < st->sm_count ? (batch + 127) / 128 : st->sm_count, 128, 0, stream>>>(
+        table->a_array, table->b_array, batch, map_a, map_b, table->maps, table->bad);
+  } else {
+    if (!a || !b || !c) return false;
+    if (!tma_addressable(a, lda, stride_a, batch) || !tma_addressable(b, ldb, stride_b, batch)) return false;
+    if (!encode_operand_map(&map_a, a, a_kc, m, k, lda, stride_a, batch, 128)) return false;
+    if (!encode_operand_map(&map_b, b, b_kc, n, k, ldb, stride_b, batch, 128)) return false;
+    // C goes out through tensor stores when nothing has to be read back and its rows are addressable.
+    c_tma = lc == TCEC_ROW_MAJOR && beta == 0.f && tma_addressable(c, ldc, stride_c, batch) &&
+            encode_c_map(&map_c, c, m, n, ldc, stride_c, batch);
+  }
   if (!c_tma) map_c = map_a;  // unused by the kernel
   GemmFusedParams fp{};
   fp.c_tma = c_tma ? 1 : 0;
@@ -575,6 +603,11 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
   fp.alpha = alpha;
   fp.beta = beta;
   fp.c = c;
+  if (table) {
+    fp.c_array = table->c_array;
+    fp.table_maps = table->maps;
+    fp.table_bad = table->bad;
+  }
   fp.ldc = ldc;
   fp.c_batch_stride = stride_c;
   fp.c_col_major = (lc == TCEC_COL_MAJOR);
@@ -714,24 +747,41 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
     return TCEC_OK;
   }
   const Shape s = plan(m, n, k, policy, opt);
+  // Pointer tables: whether TMA can address every matrix is known on the device only, so both ways are launched and one
+  // of them does nothing.
+  const size_t panel_bytes = (s.a_bytes + s.b_bytes) * batch;
+  const bool table_maps = a_array && b_array && c_array && lda % 4 == 0 && ldb % 4 == 0 && fused_wanted(n, k, batch, policy, opt);
   void* ws = nullptr;
   void* old = nullptr;
   int rc;
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    rc = get_workspace(st, stream, (s.a_bytes + s.b_bytes) * batch, &ws, &old);
+    rc = get_workspace(st, stream, panel_bytes + (table_maps ? 2 * sizeof(CUtensorMap) * static_cast<size_t>(batch) + 128 : 0), &ws,
+                       &old);
   }
   const int rel = release_old_workspace(old, stream);
   if (rc != TCEC_OK) return rc;
   if (rel != TCEC_OK) return rel;
   uint8_t* panels_a = static_cast<uint8_t*>(ws);
   uint8_t* panels_b = panels_a + s.a_bytes * batch;
+  LaunchExtras gate;
+  if (table_maps) {
+    TableMaps table;
+    table.a_array = a_array;
+    table.b_array = b_array;
+    table.c_array = c_array;
+    table.maps = reinterpret_cast<CUtensorMap*>(panels_a + panel_bytes);  // panels are 8 KB each: 128-byte aligned
+    table.bad = reinterpret_cast<int*>(table.maps + 2 * static_cast<size_t>(batch));
+    if (try_fused(la, lb, lc, m, n, k, alpha, nullptr, lda, 0, nullptr, ldb, 0, beta, nullptr, ldc, 0, batch, policy, st, stream,
+                  opt, &table))
+      gate.only_if = table.bad;
+  }
   pack_both(la == TCEC_ROW_MAJOR, m, a, a_array, lda, stride_a, panels_a, s.a_bytes, lb == TCEC_COL_MAJOR, n, b, b_array,
-            ldb, stride_b, panels_b, s.b_bytes, k, batch, policy, stream);
+            ldb, stride_b, panels_b, s.b_bytes, k, batch, policy, stream, gate.only_if, st->sm_count);
   {
     std::lock_guard<std::mutex> lock(g_mu);  // the per-stream tile counters may be created here
     rc = gemm_packed(s, m, n, k, alpha, panels_a, s.a_bytes, panels_b, s.b_bytes, beta, c, c_array, ldc, stride_c,
-                     lc, batch, policy, st, stream, opt);
+                     lc, batch, policy, st, stream, opt, &gate);
   }
   if (rc != TCEC_OK) return rc;
   TCEC_CUDA(cudaGetLastError());

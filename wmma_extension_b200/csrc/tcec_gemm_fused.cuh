@@ -56,7 +56,10 @@
 //   warps 12-19  converters (sixteen warps were measured no faster than eight: the conversion is
 //                bound by shared-memory bandwidth, not by issue slots)
 // fp16 policies only; operands must be TMA-addressable (16-byte aligned base, leading
-// dimension and batch stride multiples of 4 elements).
+// dimension and batch stride multiples of 4 elements).  Pointer tables: a small launch before this one
+// (tcec_table_maps_kernel) writes a tensor map per matrix and operand and counts pointers that TMA cannot address; if
+// there are any, this kernel does nothing and the operand-panel kernels, launched behind it, do the work; if there
+// are none, they do nothing.
 #pragma once
 #include <cuda.h>
 
@@ -79,6 +82,9 @@ struct GemmFusedParams {
   int c_tma;             // C is written with tensor stores through map_c (row-major, beta == 0)
   float alpha, beta;
   float* c;
+  float* const* c_array;
+  const CUtensorMap* table_maps;  // pointer tables: maps of A's matrices, then of B's; null: map_a and map_b
+  const int* table_bad;           // pointer tables: pointers that are not 16-byte aligned
   long long ldc, c_batch_stride;
   int c_col_major;
   int* status;
@@ -116,6 +122,32 @@ struct GemmFusedCfg {
   static constexpr int GROUP_M = 8;         // pair tiles are 256 rows tall
   static constexpr int kBoxBarrier0 = 1;    // hardware barriers 1..4: one per converter warp pair
 };
+
+// One thread per matrix: the maps of its two operands and the check of their alignment.  `bad` is zero before.
+__global__ void tcec_table_maps_kernel(const float* const* a_array, const float* const* b_array, int batch,
+                                       const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
+                                       CUtensorMap* maps, int* bad) {
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x) {
+    const float* pa = a_array[i];
+    const float* pb = b_array[i];
+    if (((reinterpret_cast<uintptr_t>(pa) | reinterpret_cast<uintptr_t>(pb)) & 15) != 0) {
+      atomicAdd(bad, 1);
+      continue;
+    }
+    const uint4* sa = reinterpret_cast<const uint4*>(&map_a);
+    const uint4* sb = reinterpret_cast<const uint4*>(&map_b);
+    uint4* da = reinterpret_cast<uint4*>(maps + i);
+    uint4* db = reinterpret_cast<uint4*>(maps + batch + i);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      da[j] = sa[j];
+      db[j] = sb[j];
+    }
+    tensormap_set_address(maps + i, pa);
+    tensormap_set_address(maps + batch + i, pb);
+    tensormap_release();
+  }
+}
 
 // U K-contiguous units, `stride` bytes apart: each is 8 rows x 32 k (1 KB).  Lane = (row r,
 // 8-float chunk c).  All units are read before any is written, so the loads overlap.
@@ -172,6 +204,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
                            const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c) {
   using Cfg = GemmFusedCfg<kEc>;
   constexpr int NST = Cfg::NST, BN = Cfg::BN;
+  if (p.table_bad && *p.table_bad != 0) return;  // every CTA of the launch, before anything is set up
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_landed[NST], bar_conv[NST], bar_full[NST], bar_empty[NST];
   __shared__ uint64_t bar_main_full, bar_main_free, bar_corr_full, bar_corr_free, bar_drain[2];
@@ -288,6 +321,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
         for (int tile = pair; tile < ntiles && ok; tile += npairs) {
           const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
           const int arow = tc.mt * 256 + static_cast<int>(rank) * 128, brow = tc.nt * 256 + static_cast<int>(rank) * 128;
+          const CUtensorMap* ma = &map_a;
+          const CUtensorMap* mb = &map_b;
+          int z = tc.b;
+          if (p.table_maps) {
+            ma = p.table_maps + tc.b;
+            mb = p.table_maps + p.batch + tc.b;
+            z = 0;
+            tensormap_acquire(ma);
+            tensormap_acquire(mb);
+          }
           for (int kb = 0; kb < p.nkb; ++kb) {
             if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 64)) {
               ok = false;
@@ -300,17 +343,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
             armed |= 1u << s;
             armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
             if (p.a_k_contiguous) {
-              tma_load_3d(dst, &map_a, landed, kb * 32, arow, tc.b);
+              tma_load_3d(dst, ma, landed, kb * 32, arow, z);
             } else {
   #pragma unroll
-              for (int j = 0; j < 4; ++j) tma_load_3d(dst + j * 4096, &map_a, landed, arow + 32 * j, kb * 32, tc.b);
+              for (int j = 0; j < 4; ++j) tma_load_3d(dst + j * 4096, ma, landed, arow + 32 * j, kb * 32, z);
             }
             if (p.b_k_contiguous) {
-              tma_load_3d(dst + Cfg::STG_A, &map_b, landed, kb * 32, brow, tc.b);
+              tma_load_3d(dst + Cfg::STG_A, mb, landed, kb * 32, brow, z);
             } else {
   #pragma unroll
               for (int j = 0; j < 4; ++j)
-                tma_load_3d(dst + Cfg::STG_A + j * 4096, &map_b, landed, brow + 32 * j, kb * 32, tc.b);
+                tma_load_3d(dst + Cfg::STG_A + j * 4096, mb, landed, brow + 32 * j, kb * 32, z);
             }
             if (++s == static_cast<uint32_t>(NST)) {
               s = 0;
@@ -449,7 +492,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
         continue;
       }
       StoreTarget st;
-      st.cbase = p.c + tc.b * p.c_batch_stride;
+      st.cbase = p.c_array ? p.c_array[tc.b] : p.c + tc.b * p.c_batch_stride;
       st.ldc = p.ldc;
       st.M = p.M;
       st.N = p.N;

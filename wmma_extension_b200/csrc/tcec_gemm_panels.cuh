@@ -56,6 +56,7 @@ struct GemmPanelParams {
   const unsigned int* row_ready;  // optional: one word per `ready_rows` rows of A; the producer loads a tile's
   int ready_rows;                 // operands only once the word of the tile's rows equals `ready_epoch` (A is
   unsigned int ready_epoch;       // arriving from another GPU while the kernel runs); the wait is bounded
+  const int* only_if;          // optional device word: zero = this launch does nothing (another kernel did the work)
   int tile_first, tile_count;  // CTA-pair kernel only: the pair tiles this launch covers
   int store_turn;          // 1: stores go through the per-warp shared-memory buffers (launched with
                            // SMEM_BYTES); 0: direct stores, launched with SMEM_BYTES_NO_TURN
@@ -178,6 +179,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
     tcec_gemm_panels_kernel(const GemmPanelParams p) {
   using Cfg = GemmPanelCfg<BN, kTf32, kEc>;
   constexpr int NST = Cfg::NST;
+  if (p.only_if && *p.only_if == 0) return;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[NST], bar_empty[NST];
   __shared__ uint64_t bar_main_full, bar_main_free, bar_corr_full, bar_corr_free, bar_drain[2];

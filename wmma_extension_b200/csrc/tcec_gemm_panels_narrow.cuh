@@ -39,6 +39,7 @@ template <int BN, bool kTf32, bool kEc>
 __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_panels_narrow_kernel(const GemmPanelParams p) {
   using Cfg = GemmNarrowCfg<BN, kEc>;
   constexpr int NST = Cfg::NST;
+  if (p.only_if && *p.only_if == 0) return;
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[NST], bar_empty[NST];
   __shared__ uint64_t bar_main_full[2], bar_main_free[2], bar_corr_full[2], bar_corr_free[2], bar_drain[2];

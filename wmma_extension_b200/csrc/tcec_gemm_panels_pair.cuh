@@ -59,6 +59,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   static_assert(BN == 256 || BN == 128, "whole or half-width pair tiles");
   using Cfg = GemmPairCfg<kTf32, kEc>;
   constexpr int NST = Cfg::NST;
+  if (p.only_if && *p.only_if == 0) return;
   constexpr int HALVES = 256 / BN;            // work items per pair tile
   constexpr int NC = BN / 2;                  // columns per epilogue warp
   constexpr int B_PIECE = kPanelBytes / HALVES;  // bytes of one B image (hi or lo) per CTA and K block
