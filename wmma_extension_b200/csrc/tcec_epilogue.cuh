@@ -94,8 +94,43 @@ constexpr int kEpiBufBytes = kEpiBufFloats * 4;      // 4224
 template <bool kWide, int NC>
 __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row0, int col0, const StoreTarget& t,
                                                  float* wbuf, int lane) {
+  // Old values of C a lane holds at once (beta != 0).  Read one before each store, every load waited for the store before it:
+  // 1000 x 777 x 1111 with a column-major C and beta 26.6 us, in groups 20.5.  The kernels with fewer registers left
+  // (kWide = false) stay with one: groups of 8 cost them 4096 x 128^3 195 -> 230 us without any beta.
+  constexpr int kGroup = 16;
   if (t.col_major) {
-    store_row_slice(acc, row0 + lane, col0, t);
+    // Consecutive lanes hold consecutive addresses; one pointer walks the columns (multiplying and comparing per column
+    // cost 256 x 512^3 by pointer tables 342 us instead of 289).
+    if (row0 + lane >= t.M) return;
+    float* dst = t.cbase + static_cast<long long>(col0) * t.ldc + row0 + lane;
+    if (t.beta == 0.f && col0 + NC <= t.N) {
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        *dst = __fmul_rn(t.alpha, acc[i]);
+        dst += t.ldc;
+      }
+      return;
+    }
+    if constexpr (!kWide) {
+      store_row_slice(acc, row0 + lane, col0, t);
+      return;
+    }
+#pragma unroll
+    for (int g = 0; g < NC; g += kGroup) {
+      const int left = t.N - col0 - g;
+      float old[kGroup];
+      float* q = dst;
+#pragma unroll
+      for (int i = 0; i < kGroup; ++i) {
+        old[i] = (t.beta != 0.f && i < left) ? *q : 0.f;
+        q += t.ldc;
+      }
+#pragma unroll
+      for (int i = 0; i < kGroup; ++i) {
+        if (i < left) *dst = t.beta != 0.f ? axpby(t.alpha, acc[g + i], t.beta, old[i]) : __fmul_rn(t.alpha, acc[g + i]);
+        dst += t.ldc;
+      }
+    }
     return;
   }
   if (kWide && t.vec_ok && t.beta == 0.f && col0 + NC <= t.N && t.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(t.cbase) & 31) == 0) {
@@ -117,31 +152,81 @@ __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row
 #pragma unroll
     for (int i = 0; i < 32; ++i) wbuf[lane * 33 + i] = acc[cc * 32 + i];
     __syncwarp();
+    if constexpr (kWide) {
+      // in groups of row slices, so that a group's old values of C (beta != 0) are on their way together
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int r = j * 4 + rsub;
-      const int row = row0 + r, col = col0 + cc * 32 + cv;
-      const float* src = wbuf + r * 33 + cv;
-      const float v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
-      if (row < t.M) {
-        float* dst = t.cbase + static_cast<long long>(row) * t.ldc + col;
-        if (t.vec_ok && col + 3 < t.N) {
-          float4 o;
-          if (t.beta != 0.f) {
-            const float4 old = *reinterpret_cast<const float4*>(dst);
-            o = make_float4(axpby(t.alpha, v0, t.beta, old.x), axpby(t.alpha, v1, t.beta, old.y),
-                            axpby(t.alpha, v2, t.beta, old.z), axpby(t.alpha, v3, t.beta, old.w));
-          } else {
-            o = make_float4(__fmul_rn(t.alpha, v0), __fmul_rn(t.alpha, v1), __fmul_rn(t.alpha, v2),
-                            __fmul_rn(t.alpha, v3));
+      for (int part = 0; part < 8; part += kGroup / 4) {
+        const int col = col0 + cc * 32 + cv;
+        const bool vec = t.vec_ok && col + 3 < t.N;
+        float4 old[kGroup / 4];
+#pragma unroll
+        for (int j = 0; j < kGroup / 4; ++j) {
+          old[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+          const int row = row0 + (part + j) * 4 + rsub;
+          if (t.beta != 0.f && row < t.M) {
+            const float* src = t.cbase + static_cast<long long>(row) * t.ldc + col;
+            if (vec) {
+              old[j] = *reinterpret_cast<const float4*>(src);
+            } else {
+              if (col < t.N) old[j].x = src[0];
+              if (col + 1 < t.N) old[j].y = src[1];
+              if (col + 2 < t.N) old[j].z = src[2];
+              if (col + 3 < t.N) old[j].w = src[3];
+            }
           }
-          *reinterpret_cast<float4*>(dst) = o;
-        } else {
-          const float v[4] = {v0, v1, v2, v3};
+        }
 #pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            if (col + e < t.N)
-              dst[e] = t.beta != 0.f ? axpby(t.alpha, v[e], t.beta, dst[e]) : __fmul_rn(t.alpha, v[e]);
+        for (int j = 0; j < kGroup / 4; ++j) {
+          const int r = (part + j) * 4 + rsub;
+          const int row = row0 + r;
+          const float* src = wbuf + r * 33 + cv;
+          const float v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
+          if (row < t.M) {
+            float* dst = t.cbase + static_cast<long long>(row) * t.ldc + col;
+            float4 o;
+            if (t.beta != 0.f)
+              o = make_float4(axpby(t.alpha, v0, t.beta, old[j].x), axpby(t.alpha, v1, t.beta, old[j].y),
+                              axpby(t.alpha, v2, t.beta, old[j].z), axpby(t.alpha, v3, t.beta, old[j].w));
+            else
+              o = make_float4(__fmul_rn(t.alpha, v0), __fmul_rn(t.alpha, v1), __fmul_rn(t.alpha, v2), __fmul_rn(t.alpha, v3));
+            if (vec) {
+              *reinterpret_cast<float4*>(dst) = o;
+            } else {
+              if (col < t.N) dst[0] = o.x;
+              if (col + 1 < t.N) dst[1] = o.y;
+              if (col + 2 < t.N) dst[2] = o.z;
+              if (col + 3 < t.N) dst[3] = o.w;
+            }
+          }
+        }
+      }
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = j * 4 + rsub;
+        const int row = row0 + r, col = col0 + cc * 32 + cv;
+        const float* src = wbuf + r * 33 + cv;
+        const float v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
+        if (row < t.M) {
+          float* dst = t.cbase + static_cast<long long>(row) * t.ldc + col;
+          if (t.vec_ok && col + 3 < t.N) {
+            float4 o;
+            if (t.beta != 0.f) {
+              const float4 old = *reinterpret_cast<const float4*>(dst);
+              o = make_float4(axpby(t.alpha, v0, t.beta, old.x), axpby(t.alpha, v1, t.beta, old.y),
+                              axpby(t.alpha, v2, t.beta, old.z), axpby(t.alpha, v3, t.beta, old.w));
+            } else {
+              o = make_float4(__fmul_rn(t.alpha, v0), __fmul_rn(t.alpha, v1), __fmul_rn(t.alpha, v2),
+                              __fmul_rn(t.alpha, v3));
+            }
+            *reinterpret_cast<float4*>(dst) = o;
+          } else {
+            const float v[4] = {v0, v1, v2, v3};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if (col + e < t.N)
+                dst[e] = t.beta != 0.f ? axpby(t.alpha, v[e], t.beta, dst[e]) : __fmul_rn(t.alpha, v[e]);
+            }
           }
         }
       }
