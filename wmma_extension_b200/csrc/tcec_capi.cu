@@ -647,6 +647,7 @@ bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const 
                 int batch, int policy, const DeviceState* st, cudaStream_t stream, const Options& opt) {
   // an option that asks for another kernel is obeyed
   if (opt.direct_kernel == 0 || opt.path != 0 || opt.cta_pair != -1 || opt.tile_n != 0) return false;
+  if (k > (1 << 30)) return false;  // granule offsets are 32-bit
   // A matrix of at most one tile: nothing is read or split twice, and no panel is padded to 256 rows (16384 x 64^3:
   // 1176 -> 175 us, 8192 x 70^3: 772 -> 395, 4096 x 128^3: 465 -> 197, 1000 x 100 x 100 x 400: 292 -> 137; one 32^3: 31 -> 23 with
   // the host's part).  With more tiles per matrix each operand is loaded and split once per tile that uses it, and the loaders

@@ -19,9 +19,8 @@
 //   warp 1      MMA main  - one thread issues the A_hi*B_hi products; owns TMEM
 //   warp 2      MMA corr  - one thread issues the A_lo*B_hi and A_hi*B_lo products
 //   warps 4..   epilogue  - tcgen05.ld, RN promotion, fold, alpha/beta, stores
-// (issuing an MMA, a commit or a barrier wait costs the issuing thread 50 to 200
-// cycles each, so a single thread cannot keep a 128-cycle MMA pipe fed with six
-// MMAs, a commit and a wait per k block; two threads can.)
+// (two issuing threads, so that the correction products run on while the main products wait for a
+// promotion; both are entered through elect.sync, see sm100_ptx.cuh)
 // All hand-offs are mbarriers; every wait is bounded and raises `status`.
 #pragma once
 #include "sm100_ptx.cuh"

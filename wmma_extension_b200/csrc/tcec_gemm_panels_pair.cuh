@@ -7,7 +7,7 @@
 // 48 KB instead of 72 KB of operands are read from shared memory, and the ring holds 6 stages
 // instead of 4.  Measured: a little faster than one SM per tile while the clocks are high
 // (4096^3), but it draws more power per product, so it is slower once the board sits at its
-// power cap (16384^3); the host library therefore keeps it behind an option.
+// power cap (16384^3); the host library chooses by the call's size.
 //
 // Pair protocol (rank 0 = leader, rank 1 = peer):
 //   full[s]   leader's barrier: its own copies' bytes + one remote arrive by the peer's relay
