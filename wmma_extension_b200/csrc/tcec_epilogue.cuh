@@ -113,22 +113,22 @@ __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row
     }
     if constexpr (!kWide) {
       store_row_slice(acc, row0 + lane, col0, t);
-      return;
-    }
+    } else {
 #pragma unroll
-    for (int g = 0; g < NC; g += kGroup) {
-      const int left = t.N - col0 - g;
-      float old[kGroup];
-      float* q = dst;
+      for (int g = 0; g < NC; g += kGroup) {
+        const int left = t.N - col0 - g;
+        float old[kGroup];
+        float* q = dst;
 #pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        old[i] = (t.beta != 0.f && i < left) ? *q : 0.f;
-        q += t.ldc;
-      }
+        for (int i = 0; i < kGroup; ++i) {
+          old[i] = (t.beta != 0.f && i < left) ? *q : 0.f;
+          q += t.ldc;
+        }
 #pragma unroll
-      for (int i = 0; i < kGroup; ++i) {
-        if (i < left) *dst = t.beta != 0.f ? axpby(t.alpha, acc[g + i], t.beta, old[i]) : __fmul_rn(t.alpha, acc[g + i]);
-        dst += t.ldc;
+        for (int i = 0; i < kGroup; ++i) {
+          if (i < left) *dst = t.beta != 0.f ? axpby(t.alpha, acc[g + i], t.beta, old[i]) : __fmul_rn(t.alpha, acc[g + i]);
+          dst += t.ldc;
+        }
       }
     }
     return;
