@@ -284,8 +284,9 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                (two kernels; the faster one whenever the tensor pipe is the limit); 2 = use
  *                the single kernel that TMA-loads FP32 tiles and splits them in registers
  *                whenever the call allows it (fp16 policies, n > 128, 16-byte aligned operands
- *                with leading dimensions that are multiples of 4, no pointer arrays).
- *                Automatic picks it for batches with k <= 2048.
+ *                with leading dimensions that are multiples of 4; pointer arrays too, where alignment is found
+ *                out on the device).  Automatic picks it for batches with k <= 2048 whose matrices are so many, and
+ *                so small, that the split would cost more than conversion in every tile.
  *   "narrow_tiles" -1 (default) = a call whose 256-wide tiles are too few to fill the GPU runs in tiles of
  *                128 x 32, 64 or 128 (64 x 4096 x 4096 on packed operands: 82 -> 35 us with the packing of A);
  *                0 = never; 32, 64, 128 = that width.  Only while "cta_pair" and "tile_n" are automatic,

@@ -1,0 +1,74 @@
+"""The rules that choose a kernel from sizes (csrc/tcec_dispatch.h), compiled for the host: each against what both sides were
+measured to take on a B200."""
+import ctypes
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+SMS = 148
+
+
+@pytest.fixture(scope="module")
+def rules(tmp_path_factory):
+    so = str(tmp_path_factory.mktemp("dispatch") / "dispatch.so")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-Wall", "-Werror", "-shared", "-fPIC", "-o", so,
+                    os.path.join(ROOT, "tests", "dispatch_harness.cpp")], check=True)
+    return ctypes.CDLL(so)
+
+
+def _promo(k, ec):
+    return 0 if not ec else 2 if k <= 2048 else 4 if k <= 4096 else 8  # K blocks of 32 per promotion
+
+
+# batch, m, n, k, with error correction, us on the FP32-tile kernel, us split and from panels (strided batches)
+FUSED_OR_PANELS = [
+    # large matrices: conversion in every tile costs more than one split
+    (2, 8192, 8192, 2048, 1, 1808, 1500), (2, 4096, 4096, 2048, 1, 437, 377), (4, 4096, 4096, 2048, 1, 886, 778),
+    (4, 4096, 4096, 1024, 1, 446, 411), (8, 2048, 2048, 512, 0, 91.5, 69.0),
+    # few tiles, where K runs serially in them, and three whose panels are slow all the same
+    (2, 1024, 1024, 512, 1, 22.3, 15.3), (2, 1024, 1024, 1024, 1, 37.2, 21.8), (2, 1024, 1024, 2048, 1, 69.4, 37.2),
+    (2, 256, 256, 256, 1, 14.6, 8.5), (2, 256, 256, 2048, 1, 73.8, 24.7), (16, 256, 256, 512, 1, 22.3, 14.4),
+    (16, 256, 256, 2048, 1, 72.8, 40.2), (8, 512, 512, 2048, 1, 66.6, 47.4), (2, 64, 4096, 1024, 1, 39.7, 25.5),
+    (2, 4096, 160, 2048, 1, 63.8, 47.6), (74, 36, 136, 1412, 0, 34.8, 48.3), (131, 16, 432, 356, 1, 51.2, 59.7),
+    (2, 2048, 2048, 256, 1, 24.8, 28.4),
+    # many matrices of a few tiles: the split is what costs
+    (8192, 256, 256, 256, 1, 1290, 2400), (128, 256, 256, 256, 1, 24.8, 46.2), (128, 256, 256, 2048, 1, 128, 270),
+    (1024, 160, 160, 160, 1, 75, 183), (1024, 160, 160, 1024, 1, 397, 853), (64, 400, 400, 1024, 1, 128, 174),
+    (64, 512, 512, 512, 1, 67.4, 101.5), (32, 1024, 1024, 512, 1, 117, 145), (32, 1024, 1024, 1024, 1, 220, 281),
+    (32, 1024, 1024, 2048, 1, 425, 488), (8, 1024, 1024, 1024, 1, 65.0, 73.9), (8, 1024, 1024, 256, 1, 23.5, 27.7),
+    (8, 2048, 2048, 256, 1, 64.9, 81.0), (4, 4096, 4096, 256, 1, 126, 157), (64, 512, 136, 2048, 1, 129, 210),
+    (16, 4096, 256, 1024, 1, 124, 191), (512, 64, 200, 300, 1, 75.5, 166), (64, 256, 256, 256, 0, 13.0, 19.1),
+]
+
+
+@pytest.mark.parametrize("case", FUSED_OR_PANELS, ids=lambda c: "x".join(map(str, c[:4])) + ("" if c[4] else "_no_ec"))
+def test_batches_take_the_side_that_was_measured_faster(rules, case):
+    batch, m, n, k, ec, fused_us, panels_us = case
+    got = rules.fused_pays_c(m, n, k, batch, _promo(k, ec), ec, SMS, 0)
+    assert bool(got) == (fused_us < panels_us)
+
+
+# the same by pointer tables: us with the maps written and the panels' launches idle, us split and from panels
+TABLES = [
+    (2, 256, 256, 256, 23.3, 8.1), (2, 512, 512, 512, 29.3, 10.1), (2, 1024, 1024, 1024, 41.2, 20.4),
+    (16, 256, 256, 128, 22.3, 8.8), (2, 4096, 4096, 512, 138.8, 126.5),
+    (256, 512, 512, 512, 245, 348), (256, 512, 512, 2048, 828, 1349), (1024, 160, 160, 160, 155, 183),
+    (4096, 132, 132, 132, 503, 638), (32, 1024, 1024, 2048, 406, 510),
+]
+
+
+@pytest.mark.parametrize("case", TABLES, ids=lambda c: "x".join(map(str, c[:4])))
+def test_pointer_tables_take_the_side_that_was_measured_faster(rules, case):
+    batch, m, n, k, fused_us, panels_us = case
+    assert bool(rules.fused_pays_c(m, n, k, batch, _promo(k, 1), 1, SMS, 2)) == (fused_us < panels_us)
+
+
+def test_the_choice_does_not_flip_back_with_more_matrices(rules):
+    """One and the same matrix size: once a batch is large enough for the FP32-tile kernel, larger ones stay there, apart from
+    the rounds in which a few more tiles start a new round."""
+    for m, n, k in ((256, 256, 256), (512, 300, 1000), (160, 160, 2048), (1024, 1024, 512)):
+        picks = [rules.fused_pays_c(m, n, k, 2 ** e, _promo(k, 1), 1, SMS, 0) for e in range(1, 16)]
+        first = picks.index(1)
+        assert all(picks[max(first, 8):]), (m, n, k, picks)

@@ -286,12 +286,11 @@ def test_fp32_tile_kernel_batched_and_fallback():
     b = rng.standard_normal((6, 256, 256)).astype(np.float32)
     tcec.set_option("path", 1)
     want = tcec.sgemm_strided_batched(_t(a), _t(b))
-    tcec.set_option("path", 0)  # automatic: short-K batches take the FP32-tile kernel
+    tcec.set_option("path", 2)
     got = tcec.sgemm_strided_batched(_t(a), _t(b))
     tcec.device_status()
     assert torch.equal(got, want)
     # operands the TMA cannot address (leading dimension not a multiple of 4) fall back to panels
-    tcec.set_option("path", 2)
     buf = torch.zeros(256, 259, device=DEV)
     buf[:, :256] = _t(a[0])
     odd = tcec.sgemm(buf[:, :256], _t(b[0]))

@@ -1,0 +1,57 @@
+"""Calls whose kernel is chosen from their sizes: the same bits on either side of a choice, and no workspace where none can be
+allocated."""
+import pytest
+import torch
+
+from wmma_extension_b200 import tcec
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.fixture(autouse=True)
+def _default_options():
+    yield
+    tcec.set_option("path", 0)
+
+
+def _rand(gen, *shape):
+    return torch.rand(shape, generator=gen, device=DEV).mul_(2).sub_(1)
+
+
+@pytest.mark.parametrize("batch,m,n,k", [
+    (2, 256, 256, 512), (2, 1024, 516, 1028),  # few tiles: from panels
+    (90, 256, 132, 96), (40, 300, 260, 1028),  # many: on the FP32-tile kernel
+])
+def test_strided_batches_have_the_bits_of_the_panel_path(batch, m, n, k):
+    gen = torch.Generator(device=DEV).manual_seed(batch + m)
+    a, b, c0 = _rand(gen, batch, m, k), _rand(gen, batch, k, n), _rand(gen, batch, n, m)
+    for transposed, alpha, beta in ((False, 1.0, 0.0), (True, -0.5, 0.75)):
+        out = []
+        for path in (1, 0):
+            tcec.set_option("path", path)
+            c = c0.clone()
+            tcec.sgemm_strided_batched(a, b, c.transpose(1, 2) if transposed else c.view(batch, m, n), alpha=alpha, beta=beta)
+            tcec.device_status()
+            out.append(c)
+        assert torch.equal(out[0], out[1]), (transposed, alpha, beta)
+
+
+@pytest.mark.parametrize("batch,m,n,k", [(2, 256, 256, 512)])
+def test_a_first_call_may_be_captured(batch, m, n, k):
+    """On a stream that has no workspace yet such a call, which would otherwise run from panels, takes the kernel without one."""
+    gen = torch.Generator(device=DEV).manual_seed(k)
+    a, b = _rand(gen, batch, m, k), _rand(gen, batch, k, n)
+    torch.cuda.synchronize()
+    tcec.destroy()  # no stream has a workspace
+    want = tcec.sgemm_strided_batched(a, b)  # the library's state exists again, and this stream's workspace
+    c = torch.zeros_like(want)
+    s = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        tcec.sgemm_strided_batched(a, b, c)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(c, want)
+    tcec.device_status()

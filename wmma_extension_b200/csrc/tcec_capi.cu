@@ -9,6 +9,7 @@
 #include <mutex>
 #include <utility>
 
+#include "tcec_dispatch.h"
 #include "tcec_gemm_direct.cuh"
 #include "tcec_gemm_fused.cuh"
 #include "tcec_gemm_panels.cuh"
@@ -138,6 +139,15 @@ int get_workspace(DeviceState* st, cudaStream_t stream, size_t bytes, void** out
   *out = w.ptr;
   return TCEC_OK;
 }
+// Whether a workspace of `bytes` would have to be allocated while the stream is being captured, which is not possible.
+static bool cannot_grow_workspace(DeviceState* st, cudaStream_t stream, size_t bytes) {
+  {
+    std::lock_guard<std::mutex> lock(g_mu);
+    if (st->ws[stream].bytes >= bytes) return false;
+  }
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  return cudaStreamIsCapturing(stream, &status) == cudaSuccess && status == cudaStreamCaptureStatusActive;
+}
 // Work queued on the stream may still read a replaced workspace: wait for it, then free.
 static int release_old_workspace(void* old, cudaStream_t stream) {
   if (!old) return TCEC_OK;
@@ -253,39 +263,6 @@ void launch_gemm(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
       <<<grid, Cfg::THREADS, gp.store_turn ? Cfg::SMEM_BYTES : Cfg::SMEM_BYTES_NO_TURN, stream>>>(gp);
 }
 
-// Width of the narrow tiles if they would finish the call sooner than 256-wide ones, else 0.  Cycles per K block of a
-// tile, fitted to what was measured: wide tiles pay their MMAs and, per promotion, about 1700 cycles in which the main
-// products wait (2048^3 on CTA pairs, a promotion every 2 blocks: 69 us; 4096^3, every 4: 83 us a tile); narrow ones take the
-// larger of their MMAs and their copies at 42 bytes per cycle and SM (2048^3 in 128-wide tiles: 62 us), and at least what
-// their epilogue takes.  Both sides at the sizes where the choice turns: 1000 x 777 x 1111 36 us wide, 25 with 64;
-// 1500^3 41 and 34 (128); 2048^3 69 and 63 (128); 1000 x 4096 x 4096 107 and 108; 4096^3 stays wide.
-int narrow_width(int m, int n, int batch, int promo, const Shape& s, int sms, bool pair) {
-  const long long tiles_m = (m + 127) / 128;
-  const int rows = m < 128 ? (m + 7) & ~7 : 128;
-  const long long wide_tiles =
-      pair ? static_cast<long long>((m + 255) / 256) * ((n + 255) / 256) * batch : tiles_m * ((n + s.tile_n - 1) / s.tile_n) * batch;
-  const int wide_slots = pair ? sms / 2 : sms;
-  // Beyond two rounds of wide tiles the last, partly empty one weighs little (256 x 512^3: 308 us wide, 324 with 128).
-  if (wide_tiles > 2 * wide_slots) return 0;
-  const bool ec = s.np == 2;
-  const double wide_block = (ec ? 768.0 : 300.0) + 1700.0 / (promo ? promo : s.nkb);
-  double best = ((wide_tiles + wide_slots - 1) / wide_slots) * (s.nkb * wide_block + 10000.0);
-  int width = 0;
-  const double mma[3] = {240.0, 288.0, 446.0};
-  for (int i = 0; i < 3; ++i) {
-    const int bn = 32 << i;
-    if (i > 0 && n <= bn / 2) break;
-    const long long tiles = tiles_m * ((n + bn - 1) / bn) * batch;
-    const double copy = (rows + bn) * 64.0 * s.np / 42.0, products = ec ? mma[i] : mma[i] / 3.0;
-    const double tile = s.nkb * (products > copy ? products : copy);
-    const double cost = ((tiles + sms - 1) / sms) * (tile > 6000.0 ? tile : 6000.0) + 4000.0;
-    if (cost < best) {
-      best = cost;
-      width = bn;
-    }
-  }
-  return width;
-}
 template <int BN, bool T, bool E>
 void launch_narrow(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
   using Cfg = GemmNarrowCfg<BN, E>;
@@ -397,18 +374,14 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
   const int reserve = ex.reserve_sms >= 0 ? ex.reserve_sms : opt.reserve_sms;
   const int sms = st->sm_count - reserve > 1 ? st->sm_count - reserve : 1;
   const bool tf32 = policy_tf32(policy), ec = policy_ec(policy);
-  // One product per K block makes the kernel wait on operands from L2, which a CTA pair halves
-  // for B: measured 10-15 % faster there.  With three products the pair is faster only while the
-  // clocks are high, i.e. for calls too short to reach the board's power cap (2048^3: +8 %,
-  // 4096^3: +2 %; 16384^3 back to back: -5 %), so the automatic choice takes it below ~5000^3.
-  const double flops = 2.0 * m * static_cast<double>(n) * k * batch;
   const bool want_pair = !ex.force_one_sm && !ex.row_ready && !ex.sched &&
-                         (opt.cta_pair == 1 || (opt.cta_pair == -1 && (!ec || flops <= 2.5e11)));
+                         (opt.cta_pair == 1 || (opt.cta_pair == -1 && pairs_pay(m, n, k, batch, ec)));
   // Options that ask for one of the wide kernels, or for something only they do, are obeyed there.
   if (!ex.force_one_sm && !ex.row_ready && !ex.sched && opt.cta_pair == -1 && opt.tile_n == 0 && opt.store_turn &&
       !opt.static_tiles && !opt.debug_flags && opt.narrow_tiles != 0) {
     const int width = opt.narrow_tiles > 0 ? opt.narrow_tiles
-                                           : narrow_width(m, n, batch, gp.promo, s, sms, want_pair && s.tile_n == 256 && m > 128);
+                                           : panel_choice(m, n, batch, s.nkb, gp.promo, ec, s.tile_n, sms,
+                                                          want_pair && s.tile_n == 256 && m > 128).width;
     const long long ntiles = static_cast<long long>(s.tiles_m) * ((n + width - 1) / (width ? width : 1)) * batch;
     if (width && ntiles <= 0x3fffffffll) {
       gp.tiles_n = (n + width - 1) / width;
@@ -543,12 +516,15 @@ bool tma_addressable(const float* base, long long ld, long long stride, int batc
 }
 
 // Whether the FP32-tile kernel is the one for a call of this shape (its operands must be addressable as well).
-bool fused_wanted(int n, int k, int batch, int policy, const Options& opt) {
+bool fused_wanted(int m, int n, int k, int batch, int policy, const DeviceState* st, const Options& opt,
+                  FusedStores stores) {
   if (policy_tf32(policy) || n <= 128) return false;
-  // Worth it where the split pass, which doubles the DRAM traffic, costs more than conversion in every tile does: short
-  // K, and, up to where the promotion interval of the panel kernels grows, batches of longer K (panels against this,
-  // us: 64 x 400 x 400 x 1000 197 and 141, 32 x 1024^3 296 and 255, 32 x 1024 x 1024 x 2048 552 and 523).
-  return opt.path == 2 || (opt.path == 0 && batch > 1 && k <= 2048);
+  if (opt.path == 2) return true;
+  if (opt.path != 0 || batch <= 1 || k > 2048) return false;
+  const bool ec = policy_ec(policy);
+  const int sms = st->sm_count - opt.reserve_sms > 1 ? st->sm_count - opt.reserve_sms : 1;
+  return fused_pays(m, n, k, batch, (k + 31) / 32, promote_blocks(k, policy, 32, opt), ec, sms,
+                    m > 128 && pairs_pay(m, n, k, batch, ec), stores);
 }
 // What a call with pointer tables lends to the FP32-tile kernel: room for two maps per matrix, and the count of pointers
 // that TMA cannot address.
@@ -565,7 +541,9 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
                long long stride_a, const float* b, long long ldb, long long stride_b, float beta, float* c,
                long long ldc, long long stride_c, int batch, int policy, const DeviceState* st,
                cudaStream_t stream, const Options& opt, const TableMaps* table = nullptr) {
-  if (!fused_wanted(n, k, batch, policy, opt)) return false;
+  const FusedStores stores =
+      table ? FusedStores::kTables : (lc == TCEC_ROW_MAJOR && beta == 0.f ? FusedStores::kTensor : FusedStores::kPlain);
+  if (!fused_wanted(m, n, k, batch, policy, st, opt, stores)) return false;
   const bool a_kc = (la == TCEC_ROW_MAJOR), b_kc = (lb == TCEC_COL_MAJOR);
   CUtensorMap map_a, map_b, map_c;
   bool c_tma = false;
@@ -748,10 +726,22 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
     return TCEC_OK;
   }
   const Shape s = plan(m, n, k, policy, opt);
+  // A call that is faster from panels, captured before its stream has the workspace for them: the kernel that needs none.
+  if (!a_array && !b_array && !c_array && batch > 1 && opt.path == 0 &&
+      cannot_grow_workspace(st, stream, (s.a_bytes + s.b_bytes) * batch)) {
+    Options whenever = opt;
+    whenever.path = 2;
+    if (try_fused(la, lb, lc, m, n, k, alpha, a, lda, stride_a, b, ldb, stride_b, beta, c, ldc, stride_c, batch, policy, st,
+                  stream, whenever)) {
+      TCEC_CUDA(cudaGetLastError());
+      return TCEC_OK;
+    }
+  }
   // Pointer tables: whether TMA can address every matrix is known on the device only, so both ways are launched and one
   // of them does nothing.
   const size_t panel_bytes = (s.a_bytes + s.b_bytes) * batch;
-  const bool table_maps = a_array && b_array && c_array && lda % 4 == 0 && ldb % 4 == 0 && fused_wanted(n, k, batch, policy, opt);
+  const bool table_maps = a_array && b_array && c_array && lda % 4 == 0 && ldb % 4 == 0 &&
+                          fused_wanted(m, n, k, batch, policy, st, opt, FusedStores::kTables);
   void* ws = nullptr;
   void* old = nullptr;
   int rc;

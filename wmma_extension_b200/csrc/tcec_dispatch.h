@@ -1,0 +1,105 @@
+// Which kernel a call runs on, as far as sizes decide it: plain C++ without CUDA, so that the rules can be checked
+// on any machine.  Costs are SM cycles at 1.92 GHz.
+#pragma once
+
+namespace tcec_host {
+
+inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
+
+// Whether the wide tiles of the panel GEMM go to CTA pairs.  One product per K block makes the kernel wait on operands from L2,
+// which a pair halves for B: measured 10-15 % faster there.  With three products the pair is faster only while the clocks are
+// high, i.e. for calls too short to reach the board's power cap (2048^3: +8 %, 4096^3: +2 %; 16384^3 back to back: -5 %), so
+// the automatic choice takes it below ~5000^3.
+inline bool pairs_pay(int m, int n, int k, int batch, bool ec) {
+  return !ec || 2.0 * m * static_cast<double>(n) * k * batch <= 2.5e11;
+}
+
+// The panel GEMM of a call: `width` of the narrow tiles if they would finish the call sooner than 256-wide ones, else 0,
+// and what the call is expected to take without its split.
+struct PanelChoice {
+  double cycles;
+  int width;
+};
+
+// Cycles per K block of a tile, fitted to what was measured: wide tiles pay their MMAs and, per promotion, about 1700 cycles in
+// which the main products wait (2048^3 on CTA pairs, a promotion every 2 blocks: 69 us; 4096^3, every 4: 83 us a tile); narrow
+// ones take the larger of their MMAs and their copies at 42 bytes per cycle and SM (2048^3 in 128-wide tiles: 62 us), and at
+// least what their epilogue takes.  Both sides at the sizes where the choice turns: 1000 x 777 x 1111 36 us wide, 25 with 64;
+// 1500^3 41 and 34 (128); 2048^3 69 and 63 (128); 1000 x 4096 x 4096 107 and 108; 4096^3 stays wide.
+// `promo`: K blocks per promotion, 0 = one at the end; `tile_n`: width of the one-SM kernel's tiles; `pair`: the wide
+// tiles would be 256 x 256 on CTA pairs.
+inline PanelChoice panel_choice(int m, int n, int batch, int nkb, int promo, bool ec, int tile_n, int sms, bool pair) {
+  const long long tiles_m = ceil_div(m, 128);
+  const int rows = m < 128 ? (m + 7) & ~7 : 128;
+  const long long wide_tiles = pair ? ceil_div(m, 256) * ceil_div(n, 256) * batch : tiles_m * ceil_div(n, tile_n) * batch;
+  const int wide_slots = pair ? (sms / 2 > 1 ? sms / 2 : 1) : sms;
+  const double rounds = static_cast<double>(ceil_div(wide_tiles, wide_slots));
+  PanelChoice c{0.0, 0};
+  // Beyond two rounds of wide tiles the last, partly empty one weighs little (256 x 512^3: 308 us wide, 324 with 128).
+  if (wide_tiles <= 2 * wide_slots) {
+    const double wide_block = (ec ? 768.0 : 300.0) + 1700.0 / (promo ? promo : nkb);
+    c.cycles = rounds * (nkb * wide_block + 10000.0);
+    const double mma[3] = {240.0, 288.0, 446.0};
+    double expected = c.cycles;
+    for (int i = 0; i < 3; ++i) {
+      const int bn = 32 << i;
+      if (i > 0 && n <= bn / 2) break;
+      const long long tiles = tiles_m * ceil_div(n, bn) * batch;
+      const double copy = (rows + bn) * 64.0 * (ec ? 2 : 1) / 42.0, products = ec ? mma[i] : mma[i] / 3.0;
+      const double tile = nkb * (products > copy ? products : copy);
+      const double in_a_row = static_cast<double>(ceil_div(tiles, sms)), cost = in_a_row * (tile > 6000.0 ? tile : 6000.0) + 4000.0;
+      if (cost < c.cycles) {
+        c.cycles = cost;
+        c.width = bn;
+        // tiles in a row wait for one another's epilogues (2 x 2048 x 2048 x 256, four rounds: 28 us with its split), and a K
+        // block takes 290 cycles at least (74 x 36 x 136 x 1412 without correction, three rounds: 48 us)
+        double all = tile > nkb * 290.0 ? tile : nkb * 290.0;
+        if (in_a_row > 1 && all < 10000.0) all = 10000.0;
+        expected = in_a_row * (all > 6000.0 ? all : 6000.0) + 4000.0;
+      }
+    }
+    c.cycles = expected;
+  }
+  // What wide tiles take in a row: on pairs a round adds 9400 cycles to its K blocks, on one SM 14000, and 28000 where a tile is
+  // mostly padding (55 x 120 x 3536 x 16 is six rounds and 77 us, 2 x 128 x 20000 x 2048 two and 229).
+  if (c.width == 0 && !pair) c.cycles = rounds * (nkb * (ec ? 1130.0 : 480.0) + (m > 128 ? 14000.0 : 28000.0));
+  else if (c.width == 0 && wide_tiles > 2 * wide_slots) c.cycles = rounds * (nkb * (ec ? 1150.0 : 255.0) + 9400.0);
+  return c;
+}
+
+// The split in front of the panel GEMM: a launch, and reading FP32 and writing the images at 2970 bytes per cycle.
+inline double split_cycles(int m, int n, int k, int batch, bool ec) {
+  return 7700.0 + (static_cast<double>(m) + n) * k * batch * (ec ? 8.0 : 6.0) / 2970.0;
+}
+
+// How C leaves the FP32-tile kernel: by tensor stores (row-major, beta = 0), by plain ones, or through pointer tables, which add
+// the launch that writes the tensor maps and the launches that then do nothing (16 x 256 x 256 x 128: 14 us strided, 22 by
+// tables).  Plain stores keep a tile for 18000 cycles at least (1024 x 160^3 by tables 155 us, 4096 x 132^3 503).
+enum class FusedStores { kTensor, kPlain, kTables };
+
+// The FP32-tile kernel (fp16 policies): rounds of 256 x 256 tiles on CTA pairs, each loading and converting its own
+// operands.
+inline double fused_cycles(int m, int n, int nkb, int batch, bool ec, int sms, FusedStores stores) {
+  const long long tiles = ceil_div(m, 256) * ceil_div(n, 256) * batch;
+  double tile = 3425.0 + nkb * (ec ? 1634.0 : 1043.0);
+  if (stores != FusedStores::kTensor && tile < 18000.0) tile = 18000.0;
+  return 12300.0 + (stores == FusedStores::kTables ? 15400.0 : 0.0) +
+         static_cast<double>(ceil_div(tiles, sms / 2 > 1 ? sms / 2 : 1)) * tile;
+}
+
+// Whether a batch (fp16 policy, n > 128, operands that TMA can address) is expected to take less time on the FP32-tile kernel
+// than split and multiplied from panels.  Conversion is repeated in every tile of a matrix and K runs serially in tiles
+// of 256 x 256, so large matrices and few of them are better off with panels; the split moves all operands through DRAM once
+// more, so many matrices of one or a few tiles are better off without.  On 321 shapes (2 to 1400 matrices of 16 to 8192, K
+// from 16 to 6000) the fit is within 12 % (this kernel) and 17 % (panels) rms, and the rule takes the slower side by more
+// than 5 % on 19 of them, against 85 with a bound on K alone.  Panels against this kernel, us:
+//   64 x 400 x 400 x 1000 171, 128    32 x 1024^3 281, 220    8 x 1024 x 1024 x 2048 137, 123    128 x 256^3 46, 25
+//   2 x 8192 x 8192 x 2048 1500, 1808    2 x 1024^3 22, 37    16 x 256 x 256 x 2048 40, 73    2 x 256 x 256 x 512 10, 23
+inline bool fused_pays(int m, int n, int k, int batch, int nkb, int promo, bool ec, int sms, bool pair,
+                       FusedStores stores) {
+  // about equal: this kernel, which needs no workspace
+  return fused_cycles(m, n, nkb, batch, ec, sms, stores) <
+         1.03 * (split_cycles(m, n, k, batch, ec) + panel_choice(m, n, batch, nkb, promo, ec, 256, sms, pair).cycles);
+}
+
+}  // namespace tcec_host
