@@ -31,6 +31,7 @@ def _matrices(gen, batch, rows, cols, layout, ld, offsets):
 @pytest.mark.parametrize("m,n,k,batch,offsets", [
     (130, 132, 36, 3, [0]), (256, 256, 64, 90, [0]), (512, 300, 160, 40, [0]), (37, 260, 500, 4, [0]), (300, 140, 1030, 3, [0]),
     (130, 132, 36, 5, [0, 0, 1]), (256, 256, 64, 90, [2]), (300, 140, 130, 5, [0, 3]),
+    (37, 132, 20, 801, [0, 0, 0, 2]),  # an odd number of panels, more than the split's CTAs draw at first
 ])
 def test_same_bits_as_the_panel_path(m, n, k, batch, offsets, policy):
     gen = torch.Generator(device=DEV).manual_seed(m + n + k)

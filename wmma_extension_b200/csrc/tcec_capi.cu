@@ -312,7 +312,7 @@ void pack_operand(bool k_contiguous, int rows, int k, const float* src, const fl
 void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a_array, long long lda, long long stride_a,
                uint8_t* panels_a, size_t a_stride, bool b_k_contiguous, int n, const float* b, const float* const* b_array,
                long long ldb, long long stride_b, uint8_t* panels_b, size_t b_stride, int k, int batch, int policy,
-               cudaStream_t stream, const int* only_if = nullptr, int sm_count = 0) {
+               cudaStream_t stream, unsigned int* gate = nullptr, int sm_count = 0) {
   SplitParams pa = split_params(a_k_contiguous, m, k, a, a_array, lda, stride_a, panels_a, a_stride, policy);
   SplitParams pb = split_params(b_k_contiguous, n, k, b, b_array, ldb, stride_b, panels_b, b_stride, policy);
   // These panels are the library's own and live for one call: the rows that pad them to 256 are not written.
@@ -321,19 +321,23 @@ void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a
   pb.row_blocks = (n + 127) / 128;
   const unsigned long long na = static_cast<unsigned long long>(pa.nkb) * pa.row_blocks * batch;
   const unsigned long long nb = static_cast<unsigned long long>(pb.nkb) * pb.row_blocks * batch;
-  if (na + nb > 0x7fffffffull && !only_if) {  // beyond one grid: one launch (or several) per operand
+  if (na + nb > 0x7fffffffull && !gate) {  // beyond one grid: one launch (or several) per operand
     pack_operand(a_k_contiguous, m, k, a, a_array, lda, stride_a, batch, panels_a, a_stride, policy, stream);
     pack_operand(b_k_contiguous, n, k, b, b_array, ldb, stride_b, batch, panels_b, b_stride, policy, stream);
     return;
   }
   const unsigned int all = static_cast<unsigned int>(na + nb), first_b = static_cast<unsigned int>(na);
-  const unsigned int strided = static_cast<unsigned int>(8 * sm_count), grid = only_if && all > strided ? strided : all;
-  if (policy_tf32(policy)) {
-    if (policy_ec(policy)) tcec_split_both_kernel<true, true><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
-    else tcec_split_both_kernel<true, false><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
+  if (gate) {  // fp16 policies only
+    const unsigned int most = static_cast<unsigned int>(8 * sm_count), claims = (all + kGatedPanels - 1) / kGatedPanels;
+    const unsigned int grid = claims < most ? claims : most;
+    if (policy_ec(policy)) tcec_split_both_gated_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, gate);
+    else tcec_split_both_gated_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, gate);
+  } else if (policy_tf32(policy)) {
+    if (policy_ec(policy)) tcec_split_both_kernel<true, true><<<all, 256, 0, stream>>>(pa, pb, first_b);
+    else tcec_split_both_kernel<true, false><<<all, 256, 0, stream>>>(pa, pb, first_b);
   } else {
-    if (policy_ec(policy)) tcec_split_both_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
-    else tcec_split_both_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, only_if);
+    if (policy_ec(policy)) tcec_split_both_kernel<false, true><<<all, 256, 0, stream>>>(pa, pb, first_b);
+    else tcec_split_both_kernel<false, false><<<all, 256, 0, stream>>>(pa, pb, first_b);
   }
 }
 
@@ -533,7 +537,7 @@ struct TableMaps {
   const float* const* b_array = nullptr;
   float* const* c_array = nullptr;
   CUtensorMap* maps = nullptr;
-  int* bad = nullptr;
+  unsigned int* bad = nullptr;  // followed by the counter from which a split behind this gate draws its panels
 };
 
 // Launches the FP32-tile kernel if the call qualifies; returns false (nothing launched) otherwise.
@@ -553,7 +557,7 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
     if (!tma_addressable(any, lda, 0, 1) || !tma_addressable(any, ldb, 0, 1)) return false;
     if (!encode_operand_map(&map_a, any, a_kc, m, k, lda, 0, 1, 128)) return false;
     if (!encode_operand_map(&map_b, any, b_kc, n, k, ldb, 0, 1, 128)) return false;
-    cudaMemsetAsync(table->bad, 0, sizeof(int), stream);
+    cudaMemsetAsync(table->bad, 0, 2 * sizeof(unsigned int), stream);
     tcec_table_maps_kernel<<<(batch + 127) / 128 < st->sm_count ? (batch + 127) / 128 : st->sm_count, 128, 0, stream>>>(
         table->a_array, table->b_array, batch, map_a, map_b, table->maps, table->bad);
   } else {
@@ -756,19 +760,20 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
   uint8_t* panels_a = static_cast<uint8_t*>(ws);
   uint8_t* panels_b = panels_a + s.a_bytes * batch;
   LaunchExtras gate;
+  unsigned int* gated = nullptr;
   if (table_maps) {
     TableMaps table;
     table.a_array = a_array;
     table.b_array = b_array;
     table.c_array = c_array;
     table.maps = reinterpret_cast<CUtensorMap*>(panels_a + panel_bytes);  // panels are 8 KB each: 128-byte aligned
-    table.bad = reinterpret_cast<int*>(table.maps + 2 * static_cast<size_t>(batch));
+    table.bad = reinterpret_cast<unsigned int*>(table.maps + 2 * static_cast<size_t>(batch));
     if (try_fused(la, lb, lc, m, n, k, alpha, nullptr, lda, 0, nullptr, ldb, 0, beta, nullptr, ldc, 0, batch, policy, st, stream,
                   opt, &table))
-      gate.only_if = table.bad;
+      gate.only_if = gated = table.bad;
   }
   pack_both(la == TCEC_ROW_MAJOR, m, a, a_array, lda, stride_a, panels_a, s.a_bytes, lb == TCEC_COL_MAJOR, n, b, b_array,
-            ldb, stride_b, panels_b, s.b_bytes, k, batch, policy, stream, gate.only_if, st->sm_count);
+            ldb, stride_b, panels_b, s.b_bytes, k, batch, policy, stream, gated, st->sm_count);
   {
     std::lock_guard<std::mutex> lock(g_mu);  // the per-stream tile counters may be created here
     rc = gemm_packed(s, m, n, k, alpha, panels_a, s.a_bytes, panels_b, s.b_bytes, beta, c, c_array, ldc, stride_c,

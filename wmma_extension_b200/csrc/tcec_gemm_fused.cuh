@@ -84,7 +84,7 @@ struct GemmFusedParams {
   float* c;
   float* const* c_array;
   const CUtensorMap* table_maps;  // pointer tables: maps of A's matrices, then of B's; null: map_a and map_b
-  const int* table_bad;           // pointer tables: pointers that are not 16-byte aligned
+  const unsigned int* table_bad;  // pointer tables: pointers that are not 16-byte aligned
   long long ldc, c_batch_stride;
   int c_col_major;
   int* status;
@@ -126,12 +126,12 @@ struct GemmFusedCfg {
 // One thread per matrix: the maps of its two operands and the check of their alignment.  `bad` is zero before.
 __global__ void tcec_table_maps_kernel(const float* const* a_array, const float* const* b_array, int batch,
                                        const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                                       CUtensorMap* maps, int* bad) {
+                                       CUtensorMap* maps, unsigned int* bad) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x) {
     const float* pa = a_array[i];
     const float* pb = b_array[i];
     if (((reinterpret_cast<uintptr_t>(pa) | reinterpret_cast<uintptr_t>(pb)) & 15) != 0) {
-      atomicAdd(bad, 1);
+      atomicAdd(bad, 1u);
       continue;
     }
     const uint4* sa = reinterpret_cast<const uint4*>(&map_a);

@@ -55,7 +55,7 @@ struct GemmPanelParams {
   const unsigned int* row_ready;  // optional: one word per `ready_rows` rows of A; the producer loads a tile's
   int ready_rows;                 // operands only once the word of the tile's rows equals `ready_epoch` (A is
   unsigned int ready_epoch;       // arriving from another GPU while the kernel runs); the wait is bounded
-  const int* only_if;          // optional device word: zero = this launch does nothing (another kernel did the work)
+  const unsigned int* only_if; // optional device word: zero = this launch does nothing (another kernel did the work)
   int tile_first, tile_count;  // CTA-pair kernel only: the pair tiles this launch covers
   int store_turn;          // 1: stores go through the per-warp shared-memory buffers (launched with
                            // SMEM_BYTES); 0: direct stores, launched with SMEM_BYTES_NO_TURN

@@ -93,7 +93,7 @@ struct LaunchExtras {
   unsigned int* sched = nullptr;           // tile counters shared by several launches (reset by the caller)
   int sched_base = 0;                      // with `sched`: tiles below this index belong to the first launch's CTAs
   int all_from_counter = 0;                // with `sched`: this launch's CTAs draw even their first tile
-  const int* only_if = nullptr;            // device word: zero = the launch does nothing
+  const unsigned int* only_if = nullptr;   // device word: zero = the launch does nothing
   int force_one_sm = 0;                    // never the CTA-pair kernel (it knows neither flags nor shared counters)
 };
 int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t* panels_a, size_t a_stride,

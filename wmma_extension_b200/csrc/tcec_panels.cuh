@@ -220,21 +220,41 @@ __global__ void __launch_bounds__(256) tcec_split_panels_kernel(const SplitParam
 // Both operands of a product in one launch (grid.x = panels of A + panels of B, all matrices of the
 // batch): one launch gap and one grid tail less than two launches, which is what a short call
 // notices (4096^3: 3 of 361 us; 1024^3: 3 of 30).
-// `only_if`: optional device word, zero = the launch does nothing; such launches take a small grid that strides over the
-// panels, so that doing nothing is short.
+template <bool kTf32, bool kEc>
+__device__ __forceinline__ void split_panel_of_both(const SplitParams& pa, const SplitParams& pb, unsigned int panels_a,
+                                                    unsigned int x) {
+  const bool second = x >= panels_a;
+  const SplitParams& p = second ? pb : pa;
+  unsigned int i = second ? x - panels_a : x;
+  const int kb = i % p.nkb;
+  i /= p.nkb;
+  const int rb = i % p.row_blocks;
+  split_one_panel<kTf32, kEc>(p, kb, rb, static_cast<int>(i / p.row_blocks));
+}
 template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_both_kernel(const SplitParams pa, const SplitParams pb,
-                                                              unsigned int panels_a, unsigned int panels,
-                                                              const int* only_if) {
-  if (only_if && *only_if == 0) return;
-  for (unsigned int x = blockIdx.x; x < panels; x += gridDim.x) {
-    const bool second = x >= panels_a;
-    const SplitParams& p = second ? pb : pa;
-    unsigned int i = second ? x - panels_a : x;
-    const int kb = i % p.nkb;
-    i /= p.nkb;
-    const int rb = i % p.row_blocks;
-    split_one_panel<kTf32, kEc>(p, kb, rb, static_cast<int>(i / p.row_blocks));
+                                                              unsigned int panels_a) {
+  split_panel_of_both<kTf32, kEc>(pa, pb, panels_a, blockIdx.x);
+}
+
+// The same behind a device word: gate[0] zero = the launch does nothing, for which its grid is small (eight CTAs per SM; a
+// CTA per panel would take 20 us to do nothing at 32768 panels).  CTAs draw their panels two at a time from gate[1], zero
+// before the launch: striding over them leaves SMs idle that were faster than others and spreads the accesses (4096 x
+// 132^3 by tables with one matrix unaligned: 748 us strided, 668 drawn, 640 with a CTA per panel).
+constexpr unsigned int kGatedPanels = 2;
+template <bool kTf32, bool kEc>
+__global__ void __launch_bounds__(256) tcec_split_both_gated_kernel(const SplitParams pa, const SplitParams pb,
+                                                                    unsigned int panels_a, unsigned int panels,
+                                                                    unsigned int* gate) {
+  if (*gate == 0) return;
+  __shared__ unsigned int next[2];
+  int turn = 0;
+  for (unsigned int x = blockIdx.x * kGatedPanels; x < panels; turn ^= 1) {
+    if (threadIdx.x == 0) next[turn] = (gridDim.x + atomicAdd(gate + 1, 1u)) * kGatedPanels;
+    for (const unsigned int last = min(panels, x + kGatedPanels); x < last; ++x)
+      split_panel_of_both<kTf32, kEc>(pa, pb, panels_a, x);
+    __syncthreads();
+    x = next[turn];
   }
 }
 
