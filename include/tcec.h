@@ -293,8 +293,9 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                "store_turn" is 1 and "static_tiles" 0.  Same results bit for bit.
  *   "direct_kernel" one launch that reads FP32 operands of any layout, alignment and batch form with
  *                ordinary loads and splits them on the way into shared memory; bit-identical
- *                results.  -1 (default) = for matrices with m, n <= 128; 0 = never; 1 = whenever
- *                "path", "cta_pair" and "tile_n" are automatic.
+ *                results.  -1 (default) = for matrices with m, n <= 128, unless they are few and their K long (one
+ *                128 x 128 x k beyond k = 192), which panels in narrow tiles spread over more SMs; 0 = never;
+ *                1 = whenever "path", "cta_pair" and "tile_n" are automatic.
  */
 int tcec_set_option(const char* name, int value);
 int tcec_get_option(const char* name, int* value);

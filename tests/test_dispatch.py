@@ -72,3 +72,28 @@ def test_the_choice_does_not_flip_back_with_more_matrices(rules):
         picks = [rules.fused_pays_c(m, n, k, 2 ** e, _promo(k, 1), 1, SMS, 0) for e in range(1, 16)]
         first = picks.index(1)
         assert all(picks[max(first, 8):]), (m, n, k, picks)
+
+
+# batch, m, n, k, K per block, us on the direct kernel, us from panels, each one call after another (a launch more costs the
+# panels up to 3 us there, which the times of longer calls, taken from graphs, have been given)
+DIRECT_OR_PANELS = [
+    (1, 32, 32, 32, 32, 10.2, 15.4), (1, 128, 128, 96, 32, 11.1, 15.4), (1, 128, 128, 192, 32, 13.4, 15.3),
+    (1, 128, 128, 384, 32, 18.5, 14.9), (1, 128, 128, 512, 32, 21.5, 13.3), (1, 128, 128, 1024, 32, 34.8, 16.4),
+    (1, 128, 128, 4096, 32, 110, 29.6), (1, 1, 128, 512, 32, 18.7, 12.3), (1, 16, 16, 1024, 32, 32.2, 16.3),
+    (8, 128, 128, 128, 32, 12.1, 14.2), (8, 128, 128, 512, 32, 21.4, 13.9), (32, 128, 128, 192, 32, 13.3, 13.8),
+    (32, 128, 128, 512, 32, 21.6, 17.4), (32, 128, 128, 1024, 32, 34.9, 24.6), (64, 128, 128, 512, 32, 22.3, 22.5),
+    (64, 128, 128, 1024, 32, 34.9, 38.8), (64, 128, 128, 2048, 32, 71.4, 65.2), (74, 128, 128, 4096, 32, 133, 146),
+    (100, 128, 128, 4096, 32, 136, 197), (100, 32, 32, 128, 32, 8.3, 11.3), (100, 32, 32, 1024, 32, 31.0, 26.0),
+    (100, 32, 32, 4096, 32, 126, 78), (200, 32, 32, 1024, 32, 31.1, 41.5), (200, 32, 32, 4096, 32, 128, 147),
+    (48, 64, 64, 1024, 32, 31.2, 22.3), (200, 64, 64, 4096, 32, 132, 213), (16384, 64, 64, 64, 32, 195, 1200),
+    (1, 128, 128, 64, 16, 11.3, 13.2), (1, 128, 128, 192, 16, 16.4, 13.6), (1, 128, 128, 1024, 16, 53.2, 19.5),
+    (32, 128, 128, 96, 16, 12.3, 13.7), (32, 128, 128, 512, 16, 30.7, 21.6), (64, 128, 128, 512, 16, 30.7, 31.7),
+    (64, 128, 128, 1024, 16, 53.5, 61.4), (64, 128, 128, 4096, 16, 207, 216), (48, 128, 128, 1024, 16, 52.2, 46.3),
+    (100, 32, 32, 1024, 16, 51.0, 40.8), (100, 64, 64, 1024, 16, 49.8, 51.5),
+]
+
+
+@pytest.mark.parametrize("case", DIRECT_OR_PANELS, ids=lambda c: "x".join(map(str, c[:4])) + ("_tf32" if c[4] == 16 else ""))
+def test_small_matrices_take_the_side_that_was_measured_faster(rules, case):
+    batch, m, n, k, kop, direct_us, panels_us = case
+    assert bool(rules.direct_pays_c(m, n, -(-k // kop), batch, kop == 16, SMS)) == (direct_us < panels_us)

@@ -37,7 +37,7 @@ def test_strided_batches_have_the_bits_of_the_panel_path(batch, m, n, k):
         assert torch.equal(out[0], out[1]), (transposed, alpha, beta)
 
 
-@pytest.mark.parametrize("batch,m,n,k", [(2, 256, 256, 512)])
+@pytest.mark.parametrize("batch,m,n,k", [(2, 256, 256, 512), (1, 100, 128, 700), (3, 128, 40, 3000)])
 def test_a_first_call_may_be_captured(batch, m, n, k):
     """On a stream that has no workspace yet such a call, which would otherwise run from panels, takes the kernel without one."""
     gen = torch.Generator(device=DEV).manual_seed(k)
@@ -55,3 +55,16 @@ def test_a_first_call_may_be_captured(batch, m, n, k):
     torch.cuda.synchronize()
     assert torch.equal(c, want)
     tcec.device_status()
+
+
+@pytest.mark.parametrize("policy", ["fp16_ec", "tf32_ec"])
+@pytest.mark.parametrize("batch,m,n,k", [(1, 128, 128, 192), (1, 128, 128, 193), (1, 33, 128, 1030), (30, 100, 64, 500), (120, 20, 40, 700)])
+def test_small_matrices_have_the_bits_of_the_panel_path(batch, m, n, k, policy):
+    gen = torch.Generator(device=DEV).manual_seed(batch + k)
+    a, b = _rand(gen, batch, m, k), _rand(gen, batch, k, n)
+    out = []
+    for path in (1, 0):
+        tcec.set_option("path", path)
+        out.append(tcec.sgemm_strided_batched(a, b, policy=policy))
+        tcec.device_status()
+    assert torch.equal(out[0], out[1])

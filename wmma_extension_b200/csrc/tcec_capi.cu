@@ -631,10 +631,13 @@ bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const 
   if (opt.direct_kernel == 0 || opt.path != 0 || opt.cta_pair != -1 || opt.tile_n != 0) return false;
   if (k > (1 << 30)) return false;  // granule offsets are 32-bit
   // A matrix of at most one tile: nothing is read or split twice, and no panel is padded to 256 rows (16384 x 64^3:
-  // 1176 -> 175 us, 8192 x 70^3: 772 -> 395, 4096 x 128^3: 465 -> 197, 1000 x 100 x 100 x 400: 292 -> 137; one 32^3: 31 -> 23 with
-  // the host's part).  With more tiles per matrix each operand is loaded and split once per tile that uses it, and the loaders
-  // are what bounds the kernel: 1024 x 201^3 358 us either way, 256 x 512^3 474 against 236.
-  if (opt.direct_kernel == -1 && !(m <= 128 && n <= 128)) return false;
+  // 1199 -> 195 us, 8192 x 70^3: 772 -> 395, 4096 x 128^3: 465 -> 197, 1000 x 100 x 100 x 400: 292 -> 137; one 32^3 through
+  // the Python binding: 21 -> 12).  With more tiles per matrix each operand is loaded and split once per tile that uses it, and
+  // the loaders are what bounds the kernel: 1024 x 201^3 358 us either way, 256 x 512^3 474 against 236.
+  const int kop = policy_tf32(policy) ? 16 : 32;
+  if (opt.direct_kernel == -1 &&
+      !(m <= 128 && n <= 128 && direct_pays(m, n, (k + kop - 1) / kop, batch, policy_tf32(policy), st->sm_count)))
+    return false;
   GemmDirectParams dp{};
   dp.a = DirectOperand{a, a_array, lda, stride_a, m, la == TCEC_ROW_MAJOR};
   dp.b = DirectOperand{b, b_array, ldb, stride_b, n, lb == TCEC_COL_MAJOR};
@@ -650,10 +653,8 @@ bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const 
   const long long per_tile = 128 / dp.slot;
   const long long ntiles = static_cast<long long>(dp.tiles_m) * dp.tiles_n * ((batch + per_tile - 1) / per_tile);
   if (ntiles > 0x3fffffffll) return false;  // tile indices are 32-bit
-  // Few matrices of long K would leave most SMs idle and walk K one granule after the other: panels, in narrow tiles.
-  if (opt.direct_kernel == -1 && k > 1024 && ntiles < st->sm_count / 2) return false;
   dp.ntiles = static_cast<int>(ntiles);
-  dp.promo = promote_blocks(k, policy, policy_tf32(policy) ? 16 : 32, opt);
+  dp.promo = promote_blocks(k, policy, kop, opt);
   dp.alpha = alpha;
   dp.beta = beta;
   dp.c = c;
@@ -730,13 +731,16 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
     return TCEC_OK;
   }
   const Shape s = plan(m, n, k, policy, opt);
-  // A call that is faster from panels, captured before its stream has the workspace for them: the kernel that needs none.
-  if (!a_array && !b_array && !c_array && batch > 1 && opt.path == 0 &&
-      cannot_grow_workspace(st, stream, (s.a_bytes + s.b_bytes) * batch)) {
+  // A call that is faster from panels, captured before its stream has the workspace for them: a kernel that needs none.
+  const bool one_tile = m <= 128 && n <= 128, strided = !a_array && !b_array && !c_array && batch > 1;
+  if (opt.path == 0 && (one_tile || strided) && cannot_grow_workspace(st, stream, (s.a_bytes + s.b_bytes) * batch)) {
     Options whenever = opt;
-    whenever.path = 2;
-    if (try_fused(la, lb, lc, m, n, k, alpha, a, lda, stride_a, b, ldb, stride_b, beta, c, ldc, stride_c, batch, policy, st,
-                  stream, whenever)) {
+    if (one_tile && opt.direct_kernel == -1) whenever.direct_kernel = 1;
+    if (!one_tile) whenever.path = 2;
+    if (one_tile ? try_direct(la, lb, lc, m, n, k, alpha, a, a_array, lda, stride_a, b, b_array, ldb, stride_b, beta, c, c_array,
+                              ldc, stride_c, batch, policy, st, stream, whenever)
+                 : try_fused(la, lb, lc, m, n, k, alpha, a, lda, stride_a, b, ldb, stride_b, beta, c, ldc, stride_c, batch,
+                             policy, st, stream, whenever)) {
       TCEC_CUDA(cudaGetLastError());
       return TCEC_OK;
     }

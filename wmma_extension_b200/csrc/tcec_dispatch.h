@@ -102,4 +102,17 @@ inline bool fused_pays(int m, int n, int k, int batch, int nkb, int promo, bool 
          1.03 * (split_cycles(m, n, k, batch, ec) + panel_choice(m, n, batch, nkb, promo, ec, 256, sms, pair).cycles);
 }
 
+// Whether matrices of at most one 128 x 128 tile go to the direct kernel.  It needs one launch instead of two and moves nothing
+// twice, but one CTA walks the K of its tile (0.8 us per 32 of K; tf32 1.4), where panels in narrow tiles give a matrix four
+// CTAs and every K block little more than 0.15 us.  Few matrices (weighed by their rows, of which the panels' split has as
+// much to do) of long K are therefore multiplied from panels.  One call after another, us, direct against panels:
+//   one 128 x 128 x K, K = 96: 11, 15   192: 13, 15   256: 15, 15   512: 22, 13   1024: 35, 16 (tf32 96: 12, 13   128: 14, 13)
+//   32 of them, K = 256: 14, 14   512: 22, 17   64 of them, K = 1024: 35, 39   2048: 71, 65   100, K = 4096: 136, 197
+//   100 x 32 x 32 x 1024: 31, 23   200: 31, 42
+// tf32 panels are twice the bytes: 64 x 128 x 128 x 1024 54, 61; 48 of them 52, 46
+inline bool direct_pays(int m, int n, int nkb, int batch, bool tf32, int sms) {
+  const double matrices = batch * (0.35 + 0.65 * (static_cast<double>(m) + n) / 256.0) * (tf32 ? 1.2 : 1.0), slots = sms / 2;
+  return nkb * (slots - matrices) <= 6.0 * slots;
+}
+
 }  // namespace tcec_host
