@@ -57,7 +57,10 @@ extern "C" {
  * kernel it stands for is bgemm_kernel (test/tcec/batch_gemm.cu:261-386), whose
  * fixed layout (A row-major, B col-major, C col-major) is one of the eight
  * layout combinations accepted here.  beta == 0 never reads C, as in the
- * reference epilogue (test/tcec/batch_gemm.cu:124-158).
+ * reference epilogue (test/tcec/batch_gemm.cu:124-158).  C may lie over A or B:
+ * the result is that of operands read before anything is written (likewise
+ * below, except that in a pointer-array batch C must not lie over an operand
+ * of another matrix, nor over its own with "direct_kernel" 1 beyond 128 x 128).
  */
 int tcec_sgemm(int layout_a, int layout_b, int layout_c, int m, int n, int k, float alpha,
                const float* a, long long lda, const float* b, long long ldb, float beta, float* c,

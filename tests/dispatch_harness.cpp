@@ -11,4 +11,12 @@ int fused_pays_c(int m, int n, int k, int batch, int promo, int ec, int sms, int
 int direct_pays_c(int m, int n, int nkb, int batch, int tf32, int sms) {
   return direct_pays(m, n, nkb, batch, tf32 != 0, sms);
 }
+int batch_overlap_c(const Extent* c, const Extent* x, int batch) {
+  const Overlap o = batch_overlap(*c, *x, batch);
+  return (o.own ? 1 : 0) | (o.across ? 2 : 0);
+}
+int matrices_may_overlap_c(const Extent* c, const Extent* x) {
+  return matrices_may_overlap(reinterpret_cast<unsigned long long>(c->base), c->ld, c->inner, c->outer,
+                              reinterpret_cast<unsigned long long>(x->base), x->ld, x->inner, x->outer);
+}
 }

@@ -2,6 +2,7 @@
 measured to take on a B200."""
 import ctypes
 import os
+import random
 import subprocess
 
 import pytest
@@ -97,3 +98,64 @@ DIRECT_OR_PANELS = [
 def test_small_matrices_take_the_side_that_was_measured_faster(rules, case):
     batch, m, n, k, kop, direct_us, panels_us = case
     assert bool(rules.direct_pays_c(m, n, -(-k // kop), batch, kop == 16, SMS)) == (direct_us < panels_us)
+
+
+# ---------------------------------------------------------------- results that lie over operands
+class Extent(ctypes.Structure):
+    _fields_ = [("base", ctypes.c_void_p), ("ld", ctypes.c_longlong), ("stride", ctypes.c_longlong), ("inner", ctypes.c_int),
+                ("outer", ctypes.c_int)]
+
+
+def _elements(e, i):
+    at = e.base // 4 + i * e.stride
+    return {at + r * e.ld + j for r in range(e.outer) for j in range(e.inner)}
+
+
+def _meet(c, x, batch):
+    cs, xs = [_elements(c, i) for i in range(batch)], [_elements(x, i) for i in range(batch)]
+    own = any(cs[i] & xs[i] for i in range(batch))
+    across = any(cs[i] & xs[j] for i in range(batch) for j in range(batch) if i != j)
+    return own, across
+
+
+def test_no_overlap_goes_unseen(rules):
+    """Every call whose result shares an element with an operand is seen, over random positions, leading dimensions and strides
+    (negative and zero ones too); calls that are told apart are apart."""
+    rng = random.Random(7)
+    told_apart = 0
+    for _ in range(20000):
+        batch = rng.choice([1, 1, 2, 3, 5])
+        inner, outer = rng.randrange(1, 5), rng.randrange(1, 4)
+        ld = inner + rng.choice([0, 0, 1, 3, 6])
+        span = (outer - 1) * ld + inner
+        x = Extent(4 * rng.randrange(400, 500), ld, rng.choice([0, span, span + 2, outer * ld, 2 * outer * ld, inner, -span, 7]),
+                   inner, outer)
+        if rng.random() < 0.6:
+            c = Extent(x.base + 4 * rng.randrange(-40, 40), ld, x.stride, rng.randrange(1, ld + 1), rng.randrange(1, 4))
+        else:
+            i2 = rng.randrange(1, 5)
+            c = Extent(x.base + 4 * rng.randrange(-40, 40), i2 + rng.randrange(0, 4), rng.choice([0, 3, 9, 20, -12]), i2,
+                       rng.randrange(1, 4))
+        own, across = _meet(c, x, batch)
+        got = rules.batch_overlap_c(ctypes.byref(c), ctypes.byref(x), batch)
+        assert (not own or got & 1) and (not across or got & 2), [(e.base, e.ld, e.stride, e.inner, e.outer) for e in (c, x)]
+        told_apart += got == 0
+        if batch == 1:
+            one = rules.matrices_may_overlap_c(ctypes.byref(c), ctypes.byref(x))
+            assert one or not own
+    assert told_apart > 4000
+
+
+@pytest.mark.parametrize("what,c,x,batch,want", [
+    ("apart", Extent(8192, 8, 64, 8, 8), Extent(4096, 8, 64, 8, 8), 16, 0),
+    ("in place", Extent(4096, 8, 64, 8, 8), Extent(4096, 8, 64, 8, 8), 16, 1),
+    ("in place, padded", Extent(4096, 10, 100, 8, 8), Extent(4096, 10, 100, 8, 8), 16, 1),
+    ("one matrix on", Extent(4096 + 256, 8, 64, 8, 8), Extent(4096, 8, 64, 8, 8), 16, 2),
+    ("alternating matrices", Extent(4096 + 256, 8, 128, 8, 8), Extent(4096, 8, 128, 8, 8), 16, 0),
+    ("column blocks of one matrix", Extent(4096 + 32, 24, 24 * 8, 8, 8), Extent(4096, 24, 24 * 8, 8, 8), 16, 0),
+    ("one operand for all, result over it", Extent(4096, 8, 64, 8, 8), Extent(4096, 8, 0, 8, 8), 16, 3),
+    ("single product in place", Extent(4096, 8, 0, 8, 8), Extent(4096, 8, 0, 8, 8), 1, 1),
+    ("strides near the end of 64 bits", Extent(4096, 8, 2 ** 61, 8, 8), Extent(2 ** 40, 8, -2 ** 61, 8, 8), 2 ** 30, 3),
+], ids=lambda v: v if isinstance(v, str) else "")
+def test_usual_forms_are_told_apart(rules, what, c, x, batch, want):
+    assert rules.batch_overlap_c(ctypes.byref(c), ctypes.byref(x), batch) == want

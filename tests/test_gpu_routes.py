@@ -68,3 +68,33 @@ def test_small_matrices_have_the_bits_of_the_panel_path(batch, m, n, k, policy):
         out.append(tcec.sgemm_strided_batched(a, b, policy=policy))
         tcec.device_status()
     assert torch.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("batch,mn", [(40, 300), (90, 256), (100, 64), (3, 100)])
+def test_results_over_their_operands(batch, mn):
+    """In place, and one matrix on (C_i over A_i+1): as if the operands had been read before anything is written."""
+    gen = torch.Generator(device=DEV).manual_seed(mn)
+    pool, w = _rand(gen, batch + 1, mn, mn), _rand(gen, batch, mn, mn)
+    want = tcec.sgemm_strided_batched(pool[:batch].clone(), w)
+    for shift in (0, 1):
+        x = pool.clone()
+        tcec.sgemm_strided_batched(x[:batch], w, x[shift:shift + batch])
+        assert torch.equal(x[shift:shift + batch], want), shift
+    x = pool.clone()
+    tcec.sgemm_batched(list(x[:batch]), list(w), list(x[:batch]))
+    assert torch.equal(x[:batch], want)
+    # B in place, C column-major
+    want_t = tcec.sgemm_strided_batched(w, pool[:batch].transpose(1, 2).clone())
+    x = pool[:batch].clone()
+    tcec.sgemm_strided_batched(w, x.transpose(1, 2), x.transpose(1, 2))
+    assert torch.equal(x.transpose(1, 2), want_t)
+    tcec.device_status()
+
+
+def test_a_single_product_in_place():
+    gen = torch.Generator(device=DEV).manual_seed(8)
+    for mn in (100, 700):
+        a, w = _rand(gen, mn, mn), _rand(gen, mn, mn)
+        want = tcec.sgemm(a, w)
+        assert torch.equal(tcec.sgemm(a, w, a), want)
+    tcec.device_status()

@@ -530,8 +530,8 @@ bool fused_wanted(int m, int n, int k, int batch, int policy, const DeviceState*
   return fused_pays(m, n, k, batch, (k + 31) / 32, promote_blocks(k, policy, 32, opt), ec, sms,
                     m > 128 && pairs_pay(m, n, k, batch, ec), stores);
 }
-// What a call with pointer tables lends to the FP32-tile kernel: room for two maps per matrix, and the count of pointers
-// that TMA cannot address.
+// What a call with pointer tables lends to the FP32-tile kernel: room for two maps per matrix, and the count of matrices that
+// it cannot take.
 struct TableMaps {
   const float* const* a_array = nullptr;
   const float* const* b_array = nullptr;
@@ -539,6 +539,20 @@ struct TableMaps {
   CUtensorMap* maps = nullptr;
   unsigned int* bad = nullptr;  // followed by the counter from which a split behind this gate draws its panels
 };
+
+// What C of a strided batch (or single call) shares with A or B.
+Overlap operand_overlap(int la, int lb, int lc, int m, int n, int k, const float* a, long long lda, long long stride_a,
+                        const float* b, long long ldb, long long stride_b, const float* c, long long ldc, long long stride_c,
+                        int batch) {
+  auto extent = [](const float* p, int layout, int rows, int cols, long long ld, long long stride) {
+    const bool row = layout == TCEC_ROW_MAJOR;
+    return Extent{p, ld, stride, row ? cols : rows, row ? rows : cols};
+  };
+  const Extent ec = extent(c, lc, m, n, ldc, stride_c);
+  const Overlap with_a = batch_overlap(ec, extent(a, la, m, k, lda, stride_a), batch);
+  const Overlap with_b = batch_overlap(ec, extent(b, lb, k, n, ldb, stride_b), batch);
+  return {with_a.own || with_b.own, with_a.across || with_b.across};
+}
 
 // Launches the FP32-tile kernel if the call qualifies; returns false (nothing launched) otherwise.
 bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const float* a, long long lda,
@@ -558,11 +572,18 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
     if (!encode_operand_map(&map_a, any, a_kc, m, k, lda, 0, 1, 128)) return false;
     if (!encode_operand_map(&map_b, any, b_kc, n, k, ldb, 0, 1, 128)) return false;
     cudaMemsetAsync(table->bad, 0, 2 * sizeof(unsigned int), stream);
+    const bool c_row = lc == TCEC_ROW_MAJOR, more_tiles = m > 256 || n > 256;
+    const TableShape shape{more_tiles ? table->c_array : nullptr, lda, ldb, ldc, a_kc ? k : m, a_kc ? m : k, b_kc ? k : n,
+                           b_kc ? n : k, c_row ? n : m, c_row ? m : n};
     tcec_table_maps_kernel<<<(batch + 127) / 128 < st->sm_count ? (batch + 127) / 128 : st->sm_count, 128, 0, stream>>>(
-        table->a_array, table->b_array, batch, map_a, map_b, table->maps, table->bad);
+        table->a_array, table->b_array, batch, map_a, map_b, table->maps, table->bad, shape);
   } else {
     if (!a || !b || !c) return false;
     if (!tma_addressable(a, lda, stride_a, batch) || !tma_addressable(b, ldb, stride_b, batch)) return false;
+    // Operands are read while results are written.  A C over A or B works from panels (both are split before), and here if it
+    // is over its own operands only and one tile holds the matrix.
+    const Overlap over = operand_overlap(la, lb, lc, m, n, k, a, lda, stride_a, b, ldb, stride_b, c, ldc, stride_c, batch);
+    if (over.across || (over.own && (m > 256 || n > 256))) return false;
     if (!encode_operand_map(&map_a, a, a_kc, m, k, lda, stride_a, batch, 128)) return false;
     if (!encode_operand_map(&map_b, b, b_kc, n, k, ldb, stride_b, batch, 128)) return false;
     // C goes out through tensor stores when nothing has to be read back and its rows are addressable.
@@ -638,6 +659,10 @@ bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const 
   if (opt.direct_kernel == -1 &&
       !(m <= 128 && n <= 128 && direct_pays(m, n, (k + kop - 1) / kop, batch, policy_tf32(policy), st->sm_count)))
     return false;
+  if (!a_array && !b_array && !c_array) {  // as in try_fused; a tile here is 128 x 128
+    const Overlap over = operand_overlap(la, lb, lc, m, n, k, a, lda, stride_a, b, ldb, stride_b, c, ldc, stride_c, batch);
+    if (over.across || (over.own && (m > 128 || n > 128))) return false;
+  }
   GemmDirectParams dp{};
   dp.a = DirectOperand{a, a_array, lda, stride_a, m, la == TCEC_ROW_MAJOR};
   dp.b = DirectOperand{b, b_array, ldb, stride_b, n, lb == TCEC_COL_MAJOR};

@@ -2,6 +2,12 @@
 // on any machine.  Costs are SM cycles at 1.92 GHz.
 #pragma once
 
+#ifdef __CUDACC__
+#define TCEC_HOST_DEVICE __host__ __device__
+#else
+#define TCEC_HOST_DEVICE
+#endif
+
 namespace tcec_host {
 
 inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
@@ -113,6 +119,63 @@ inline bool fused_pays(int m, int n, int k, int batch, int nkb, int promo, bool 
 inline bool direct_pays(int m, int n, int nkb, int batch, bool tf32, int sms) {
   const double matrices = batch * (0.35 + 0.65 * (static_cast<double>(m) + n) / 256.0) * (tf32 ? 1.2 : 1.0), slots = sms / 2;
   return nkb * (slots - matrices) <= 6.0 * slots;
+}
+
+// ---------------------------------------------------------------- results that lie over operands
+// Where the matrices of a call lie: `outer` runs of `inner` consecutive floats, `ld` apart, and matrix i `stride` floats behind
+// matrix 0.
+struct Extent {
+  const void* base;
+  long long ld, stride;
+  int inner, outer;
+};
+
+// Whether one matrix at `c` and one at `x` may share an element: not if their spans are apart, nor if they are column ranges
+// of rows of one length (blocks of one larger matrix).
+TCEC_HOST_DEVICE inline bool matrices_may_overlap(unsigned long long c, long long ldc, int c_inner, int c_outer,
+                                                  unsigned long long x, long long ldx, int x_inner, int x_outer) {
+  const unsigned long long c_span = 4ull * ((c_outer - 1) * ldc + c_inner), x_span = 4ull * ((x_outer - 1) * ldx + x_inner);
+  if (c >= x + x_span || x >= c + c_span) return false;
+  if (ldc == ldx && ldc > 0) {
+    const long long row = 4 * ldc;
+    long long d = static_cast<long long>(c - x) % row;  // columns of C begin d bytes behind those of X
+    if (d < 0) d += row;
+    if (d >= 4ll * x_inner && d + 4ll * c_inner <= row) return false;
+  }
+  return true;
+}
+
+// Which matrices of a batch a result may share elements with: those of the same index, those of another one.
+struct Overlap {
+  bool own, across;
+};
+inline Overlap batch_overlap(const Extent& c, const Extent& x, int batch) {
+  typedef __int128 wide;  // strides are the caller's and may be anything
+  const wide c0 = reinterpret_cast<unsigned long long>(c.base), x0 = reinterpret_cast<unsigned long long>(x.base);
+  const wide c_span = 4 * (static_cast<wide>(c.outer - 1) * c.ld + c.inner), x_span = 4 * (static_cast<wide>(x.outer - 1) * x.ld + x.inner);
+  const wide cs = 4 * static_cast<wide>(c.stride), xs = 4 * static_cast<wide>(x.stride), last = batch - 1;
+  const wide c_lo = c0 + (cs < 0 ? last * cs : 0), c_hi = c0 + c_span + (cs > 0 ? last * cs : 0);
+  const wide x_lo = x0 + (xs < 0 ? last * xs : 0), x_hi = x0 + x_span + (xs > 0 ? last * xs : 0);
+  if (c_lo >= x_hi || x_lo >= c_hi) return {false, false};
+  if (c.ld == x.ld && (batch == 1 || (c.stride % c.ld == 0 && x.stride % x.ld == 0))) {
+    // column ranges of the rows of one larger matrix
+    const wide row = 4 * static_cast<wide>(c.ld);
+    wide d = (c0 - x0) % row;
+    if (d < 0) d += row;
+    if (d >= 4 * static_cast<wide>(x.inner) && d + 4 * static_cast<wide>(c.inner) <= row) return {false, false};
+  }
+  if (batch == 1) return {true, false};
+  if (cs != xs) return {true, true};
+  // C_j and X_i, j = i + t: spans meet where -c_span < (c0 - x0) + t * stride < x_span
+  Overlap o{c0 - x0 > -c_span && c0 - x0 < x_span, false};
+  const wide step = cs < 0 ? -cs : cs;
+  if (step == 0) return {o.own, o.own};
+  auto down = [](wide a, wide b) { return a >= 0 ? a / b : -((-a + b - 1) / b); };  // floor, b > 0
+  wide first = down(-c_span - (c0 - x0), step) + 1, past = -down(-(x_span - (c0 - x0)), step);  // first <= t < past
+  if (first < -last) first = -last;
+  if (past > last + 1) past = last + 1;
+  o.across = past - first > 1 || (past - first == 1 && first != 0);
+  return o;
 }
 
 }  // namespace tcec_host

@@ -57,12 +57,13 @@
 //                bound by shared-memory bandwidth, not by issue slots)
 // fp16 policies only; operands must be TMA-addressable (16-byte aligned base, leading
 // dimension and batch stride multiples of 4 elements).  Pointer tables: a small launch before this one
-// (tcec_table_maps_kernel) writes a tensor map per matrix and operand and counts pointers that TMA cannot address; if
-// there are any, this kernel does nothing and the operand-panel kernels, launched behind it, do the work; if there
+// (tcec_table_maps_kernel) writes a tensor map per matrix and operand and counts matrices that cannot be taken (pointers that
+// TMA cannot address, a C over its own operands); if there are any, this kernel does nothing and the operand-panel kernels, launched behind it, do the work; if there
 // are none, they do nothing.
 #pragma once
 #include <cuda.h>
 
+#include "tcec_dispatch.h"
 #include "sm100_ptx.cuh"
 #include "tcec_epilogue.cuh"
 #include "tcec_gemm_panels.cuh"
@@ -84,7 +85,7 @@ struct GemmFusedParams {
   float* c;
   float* const* c_array;
   const CUtensorMap* table_maps;  // pointer tables: maps of A's matrices, then of B's; null: map_a and map_b
-  const unsigned int* table_bad;  // pointer tables: pointers that are not 16-byte aligned
+  const unsigned int* table_bad;  // pointer tables: matrices that this kernel cannot take
   long long ldc, c_batch_stride;
   int c_col_major;
   int* status;
@@ -123,14 +124,29 @@ struct GemmFusedCfg {
   static constexpr int kBoxBarrier0 = 1;    // hardware barriers 1..4: one per converter warp pair
 };
 
-// One thread per matrix: the maps of its two operands and the check of their alignment.  `bad` is zero before.
+// What the matrices of a table look like, to see a result that lies over an operand of its own.
+struct TableShape {
+  float* const* c_array;  // null: nothing to look for (matrices of one tile are read whole before they are written)
+  long long lda, ldb, ldc;
+  int a_inner, a_outer, b_inner, b_outer, c_inner, c_outer;
+};
+
+// One thread per matrix: the maps of its two operands, the check of their alignment, and whether C lies over one of them, which
+// other tiles still read.  `bad` is zero before.
 __global__ void tcec_table_maps_kernel(const float* const* a_array, const float* const* b_array, int batch,
                                        const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                                       CUtensorMap* maps, unsigned int* bad) {
+                                       CUtensorMap* maps, unsigned int* bad, const TableShape t) {
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x) {
     const float* pa = a_array[i];
     const float* pb = b_array[i];
-    if (((reinterpret_cast<uintptr_t>(pa) | reinterpret_cast<uintptr_t>(pb)) & 15) != 0) {
+    const unsigned long long ua = reinterpret_cast<uintptr_t>(pa), ub = reinterpret_cast<uintptr_t>(pb);
+    bool out = ((ua | ub) & 15) != 0;
+    if (t.c_array) {
+      const unsigned long long uc = reinterpret_cast<uintptr_t>(t.c_array[i]);
+      out = out || tcec_host::matrices_may_overlap(uc, t.ldc, t.c_inner, t.c_outer, ua, t.lda, t.a_inner, t.a_outer) ||
+            tcec_host::matrices_may_overlap(uc, t.ldc, t.c_inner, t.c_outer, ub, t.ldb, t.b_inner, t.b_outer);
+    }
+    if (out) {
       atomicAdd(bad, 1u);
       continue;
     }
