@@ -18,7 +18,7 @@ TEST_LIB = os.path.join(ROOT, "tests", "_build", "libtcec_b200_shortwait.so")
 ERR_TIMEOUT = 4
 
 
-def test_a_wait_that_runs_out_is_reported_and_leaves_the_context_usable():
+def _library():
     if not os.path.exists(TEST_LIB):
         pytest.skip("the short-wait test build of the library is missing (run build())")
     lib = ctypes.CDLL(TEST_LIB)
@@ -26,6 +26,11 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_context_usable():
     lib.tcec_sgemm.argtypes = [i, i, i, i, i, i, f, p, ll, p, ll, f, p, ll, i, p]
     lib.tcec_device_status.argtypes = [ctypes.POINTER(i)]
     lib.tcec_set_option.argtypes = [ctypes.c_char_p, i]
+    return lib
+
+
+def test_a_wait_that_runs_out_is_reported_and_leaves_the_context_usable():
+    lib, i = _library(), ctypes.c_int
     rng = np.random.default_rng(3)
     m, n, k = 128, 256, 512  # one tile, 16 K blocks: more than the ring holds
     a = torch.from_numpy(rng.uniform(-1, 1, (m, k)).astype(np.float32)).cuda()
@@ -53,3 +58,40 @@ def test_a_wait_that_runs_out_is_reported_and_leaves_the_context_usable():
     exact = cpu.gemm_f64(a.cpu().numpy(), b.cpu().numpy())
     assert cpu.errors(c.cpu().numpy(), exact)["max_rel"] < 1e-6
     lib.tcec_destroy()
+
+
+@pytest.mark.parametrize("policy", [0, 1, 2, 3])
+@pytest.mark.parametrize("kernel", ["direct", "narrow 32", "narrow 64", "narrow 128"])
+def test_waits_of_the_direct_and_narrow_kernels_run_out_the_same_way(kernel, policy):
+    """Both accumulators exist twice there, and the direct kernel's stages are filled by eight warps (with tf32 two stages
+    at a time), so their ways out are their own."""
+    lib, i = _library(), ctypes.c_int
+    rng = np.random.default_rng(4)
+    m, n, k = 120, 128, 1100  # more K blocks than any ring holds, and a last one that is not whole
+    a = torch.from_numpy(rng.uniform(-1, 1, (m, k)).astype(np.float32)).cuda()
+    b = torch.from_numpy(rng.uniform(-1, 1, (k, n)).astype(np.float32)).cuda()
+    c = torch.zeros((m, n), device="cuda")
+    detail = i(0)
+
+    def run():
+        st = lib.tcec_sgemm(0, 0, 0, m, n, k, 1.0, a.data_ptr(), k, b.data_ptr(), n, 0.0, c.data_ptr(), n, policy, None)
+        return st or lib.tcec_device_status(ctypes.byref(detail))
+
+    options = {b"path": 0, b"direct_kernel": 1 if kernel == "direct" else 0,
+               b"narrow_tiles": -1 if kernel == "direct" else int(kernel.split()[1])}
+    for name, value in options.items():
+        assert lib.tcec_set_option(name, value) == 0
+    try:
+        assert run() == 0
+        want = c.clone()
+        assert lib.tcec_set_option(b"debug_flags", 64) == 0  # one stage is never filled
+        assert run() == ERR_TIMEOUT
+        assert detail.value in (1, 2, 3)
+        assert lib.tcec_set_option(b"debug_flags", 0) == 0
+        c.fill_(float("nan"))
+        assert run() == 0  # the status was cleared, TMEM and barriers are there again
+        assert torch.equal(c, want)
+    finally:
+        for name, value in ((b"debug_flags", 0), (b"direct_kernel", -1), (b"narrow_tiles", -1)):
+            lib.tcec_set_option(name, value)
+        lib.tcec_destroy()

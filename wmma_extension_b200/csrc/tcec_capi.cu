@@ -382,7 +382,7 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
                          (opt.cta_pair == 1 || (opt.cta_pair == -1 && pairs_pay(m, n, k, batch, ec)));
   // Options that ask for one of the wide kernels, or for something only they do, are obeyed there.
   if (!ex.force_one_sm && !ex.row_ready && !ex.sched && opt.cta_pair == -1 && opt.tile_n == 0 && opt.store_turn &&
-      !opt.static_tiles && !opt.debug_flags && opt.narrow_tiles != 0) {
+      !opt.static_tiles && !(opt.debug_flags & ~64) && opt.narrow_tiles != 0) {
     const int width = opt.narrow_tiles > 0 ? opt.narrow_tiles
                                            : panel_choice(m, n, batch, s.nkb, gp.promo, ec, s.tile_n, sms,
                                                           want_pair && s.tile_n == 256 && m > 128).width;
@@ -688,6 +688,7 @@ bool try_direct(int la, int lb, int lc, int m, int n, int k, float alpha, const 
   dp.c_batch_stride = stride_c;
   dp.c_col_major = (lc == TCEC_COL_MAJOR);
   dp.status = st->status;
+  dp.debug_flags = opt.debug_flags;
   const int sms = st->sm_count - opt.reserve_sms > 1 ? st->sm_count - opt.reserve_sms : 1;
   const int grid = dp.ntiles < sms ? dp.ntiles : sms;
   if (policy_tf32(policy)) {

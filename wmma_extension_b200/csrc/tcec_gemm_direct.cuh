@@ -59,6 +59,7 @@ struct GemmDirectParams {
   long long ldc, c_batch_stride;
   int c_col_major;
   int* status;
+  int debug_flags;  // develop builds only: bit 6 = the first stage after the first ring fill is never filled
 };
 
 template <bool kTf32, bool kEc>
@@ -346,8 +347,10 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       }
     };
     uint32_t s = 0, ph = 0;
+    [[maybe_unused]] uint32_t filled = 0;  // stages before the current one
     bool ok = true;
     auto next_stage = [&]() {
+      ++filled;
       if (++s == static_cast<uint32_t>(NST)) {
         s = 0;
         ph ^= 1;
@@ -362,6 +365,9 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
     auto write = [&](const float (&va)[16], const float (&vb)[16], int vec4, int g) {
       if (!stage_free()) return false;
       const uint32_t s0 = s, img0 = smem_base + s * Cfg::STAGE;
+      // injected stall (failure-path test)
+      const bool leave0 = dev_flag(p.debug_flags, 64) && filled == static_cast<uint32_t>(NST);
+      const bool leave1 = dev_flag(p.debug_flags, 64) && filled + 1 == static_cast<uint32_t>(NST);
       uint32_t img1 = img0, s1 = s;
       bool two = false;
       next_stage();
@@ -380,8 +386,8 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       fence_proxy_async_smem();
       __syncwarp();
       if (lane == 0) {
-        mbar_arrive(smem_u32(&bar_full[s0]));
-        if (two) mbar_arrive(smem_u32(&bar_full[s1]));
+        if (!leave0) mbar_arrive(smem_u32(&bar_full[s0]));
+        if (two && !leave1) mbar_arrive(smem_u32(&bar_full[s1]));
       }
       return true;
     };

@@ -80,7 +80,15 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
     // ------------------------------------------------------------ producer
     if (elect_one()) {
       uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0;
+      [[maybe_unused]] uint32_t it = 0;
       bool ok = true;
+      auto next_stage = [&]() {
+        ++it;
+        if (++s == static_cast<uint32_t>(NST)) {
+          s = 0;
+          ph ^= 1;
+        }
+      };
       for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
         const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
         const uint8_t* pa = p.panels_a + tc.b * p.panels_a_batch_stride + static_cast<size_t>(tc.mt) * p.nkb * Cfg::A_BLOCK;
@@ -92,6 +100,11 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 32)) {
             ok = false;
             break;
+          }
+          // injected stall (failure-path test): the first stage after the first ring fill is never filled
+          if (dev_flag(p.debug_flags, 64) && it == static_cast<uint32_t>(NST)) {
+            next_stage();
+            continue;
           }
           const uint32_t full = smem_u32(&bar_full[s]);
           const uint32_t dst = smem_base + s * Cfg::STAGE_BYTES;
@@ -108,10 +121,7 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
           const uint8_t* sb = pb + static_cast<size_t>(kb) * (kPanelBytes * Cfg::NP);
           const uint32_t db = dst + Cfg::KBS * Cfg::A_BLOCK;
           for (int i = 0; i < nblk * Cfg::NP; ++i) bulk_load(db + i * Cfg::B_IMAGE, sb + i * kPanelBytes, Cfg::B_IMAGE, full);
-          if (++s == static_cast<uint32_t>(NST)) {
-            s = 0;
-            ph ^= 1;
-          }
+          next_stage();
         }
       }
       if (!ok) {
