@@ -1,10 +1,13 @@
 """Host-side checks that need no GPU: the C ABI loads, exports what include/tcec.h
 declares, and rejects bad arguments before touching a device."""
 import ctypes
+import importlib.util
 import os
 import re
+import types
 
 import pytest
+import torch
 
 from wmma_extension_b200 import tcec
 
@@ -163,3 +166,21 @@ def test_layout_detection():
         tcec._layout_ld(torch.zeros(6, 8)[:, ::2])
     with pytest.raises(ValueError):
         tcec.sgemm(torch.zeros(2, 2), torch.zeros(2, 2))  # CPU tensors: there is no CPU path
+
+
+def test_binding_without_torchs_private_calls(monkeypatch):
+    """The current device and stream are asked for through calls of torch that are not public: where one is missing, the
+    public way is taken."""
+    for name in ("_cuda_getDevice", "_cuda_getCurrentRawStream"):
+        monkeypatch.delattr(torch._C, name, raising=False)
+    monkeypatch.setattr(torch.cuda, "current_device", lambda: 3)
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda: types.SimpleNamespace(cuda_stream=77))
+    entered = []
+    monkeypatch.setattr(torch.cuda, "device", lambda d: entered.append(d) or "switch")
+    spec = importlib.util.spec_from_file_location("tcec_public", tcec.__file__)
+    public = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(public)
+    assert public._stream_ptr() == 77
+    public._on(torch.device("cuda", 3))
+    assert entered == []
+    assert public._on(torch.device("cuda", 1)) == "switch" and entered == [torch.device("cuda", 1)]
