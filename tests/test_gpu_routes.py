@@ -98,3 +98,29 @@ def test_a_single_product_in_place():
         want = tcec.sgemm(a, w)
         assert torch.equal(tcec.sgemm(a, w, a), want)
     tcec.device_status()
+
+
+def test_tables_captured_behind_a_strided_call():
+    """A strided call of the shape has sized the stream's workspace: the call by tables is then launches only."""
+    gen = torch.Generator(device=DEV).manual_seed(11)
+    batch, m, n, k = 120, 160, 160, 1024
+    a, b = _rand(gen, batch, m, k), _rand(gen, batch, k, n)
+    torch.cuda.synchronize()
+    tcec.destroy()
+    s = torch.cuda.Stream()
+    with torch.cuda.stream(s):
+        tcec.set_option("path", 1)
+        want = tcec.sgemm_strided_batched(a, b)
+        tcec.set_option("path", 0)
+    s.synchronize()
+    c = torch.zeros_like(want)
+    tables = [torch.tensor([x.data_ptr() for x in t], dtype=torch.int64, device=DEV) for t in (a, b, c)]
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=s):
+        st = tcec.load().tcec_sgemm_batched(0, 0, 0, m, n, k, 1.0, tables[0].data_ptr(), k, tables[1].data_ptr(), n, 0.0,
+                                            tables[2].data_ptr(), n, batch, 0, torch.cuda.current_stream().cuda_stream)
+    assert st == tcec.OK
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(c, want)
+    tcec.device_status()

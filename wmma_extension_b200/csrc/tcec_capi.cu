@@ -554,6 +554,9 @@ Overlap operand_overlap(int la, int lb, int lc, int m, int n, int k, const float
   return {with_a.own || with_b.own, with_a.across || with_b.across};
 }
 
+// Two maps per matrix, and a line for the two counters.
+size_t table_map_bytes(int batch) { return 2 * sizeof(CUtensorMap) * static_cast<size_t>(batch) + 128; }
+
 // Launches the FP32-tile kernel if the call qualifies; returns false (nothing launched) otherwise.
 bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const float* a, long long lda,
                long long stride_a, const float* b, long long ldb, long long stride_b, float beta, float* c,
@@ -774,15 +777,17 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
   // Pointer tables: whether TMA can address every matrix is known on the device only, so both ways are launched and one
   // of them does nothing.
   const size_t panel_bytes = (s.a_bytes + s.b_bytes) * batch;
-  const bool table_maps = a_array && b_array && c_array && lda % 4 == 0 && ldb % 4 == 0 &&
-                          fused_wanted(m, n, k, batch, policy, st, opt, FusedStores::kTables);
+  const size_t map_bytes = table_map_bytes(batch);
+  bool table_maps = a_array && b_array && c_array && lda % 4 == 0 && ldb % 4 == 0 &&
+                    fused_wanted(m, n, k, batch, policy, st, opt, FusedStores::kTables);
+  // a capture on a stream whose workspace holds the panels (a strided call's) but not the maps behind them
+  if (table_maps && cannot_grow_workspace(st, stream, panel_bytes + map_bytes)) table_maps = false;
   void* ws = nullptr;
   void* old = nullptr;
   int rc;
   {
     std::lock_guard<std::mutex> lock(g_mu);
-    rc = get_workspace(st, stream, panel_bytes + (table_maps ? 2 * sizeof(CUtensorMap) * static_cast<size_t>(batch) + 128 : 0), &ws,
-                       &old);
+    rc = get_workspace(st, stream, panel_bytes + (table_maps ? map_bytes : 0), &ws, &old);
   }
   const int rel = release_old_workspace(old, stream);
   if (rc != TCEC_OK) return rc;
