@@ -310,7 +310,11 @@ int tcec_get_option(const char* name, int* value);
  */
 int tcec_device_status(int* detail);
 
-/* Bytes of library-owned workspace a call of this shape will use (0 on error). */
+/*
+ * Bytes of library-owned workspace a real call of this shape may use (0 on error): its operand panels and, for
+ * batches that may come as pointer tables, 256 bytes per matrix for tensor maps.  Calls that run on the FP32-tile or
+ * the direct kernel use less or none.
+ */
 size_t tcec_workspace_bytes(int m, int n, int k, int batch, int policy);
 
 /* Frees every cached workspace on every device. */

@@ -149,6 +149,9 @@ def test_workspace_and_packed_sizes():
     assert tcec.packed_bytes(4096, 4096, "tf32_ec") == 4096 * 4096 * 8
     assert tcec.packed_bytes(1, 1, "fp16_ec") == 256 * 32 * 4  # padded to 256 rows x one k block
     assert tcec.workspace_bytes(4096, 4096, 4096) == 2 * 4096 * 4096 * 4
+    # a batch may come as pointer tables: two tensor maps of 128 bytes per matrix, and a line
+    assert tcec.workspace_bytes(512, 512, 512, 256) == 256 * (2 * 512 * 512 * 4 + 256) + 128
+    assert tcec.workspace_bytes(512, 512, 512, 256, "tf32_ec") == 256 * 2 * 512 * 512 * 8
     assert tcec.packed_row_offset(256, 64, "fp16_ec") == tcec.packed_bytes(256, 64, "fp16_ec")
     assert tcec.packed_row_offset(512, 64, "tf32_ec") == 2 * tcec.packed_bytes(256, 64, "tf32_ec")
     assert tcec.packed_row_offset(128, 64, "fp16_ec") == 0  # row blocks are read in pairs: multiples of 256 only

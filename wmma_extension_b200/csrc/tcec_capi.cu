@@ -1180,7 +1180,8 @@ int tcec_device_status(int* detail) {
 size_t tcec_workspace_bytes(int m, int n, int k, int batch, int policy) {
   if (m <= 0 || n <= 0 || k <= 0 || batch <= 0 || policy < 0 || policy > 3) return 0;
   const Shape s = plan(m, n, k, policy, snapshot_options());
-  return (s.a_bytes + s.b_bytes) * batch;
+  const bool maps = batch > 1 && n > 128 && !policy_tf32(policy);  // as a call by pointer tables may take the FP32-tile kernel
+  return (s.a_bytes + s.b_bytes) * batch + (maps ? table_map_bytes(batch) : 0);
 }
 
 int tcec_destroy(void) {
