@@ -81,6 +81,58 @@ __device__ __forceinline__ void store_row_slice(const float (&acc)[NC], int row,
   }
 }
 
+constexpr int kOldValues = 16;  // of C that a lane holds at once
+
+template <int kVec>
+__device__ __forceinline__ void store_updated(const float* src, float* dst, const float (&old)[kVec], const StoreTarget& t) {
+  if constexpr (kVec == 4)
+    *reinterpret_cast<float4*>(dst) = make_float4(axpby(t.alpha, src[0], t.beta, old[0]), axpby(t.alpha, src[1], t.beta, old[1]),
+                                                  axpby(t.alpha, src[2], t.beta, old[2]), axpby(t.alpha, src[3], t.beta, old[3]));
+  else
+    *dst = axpby(t.alpha, src[0], t.beta, old[0]);
+}
+// A lane's part of a 32 x 32 block in the turn buffer: `all` pieces of kVec floats, the first `rows` of which are the matrix's,
+// from `src` on every `src_step` floats to `dst` on every `dst_step`.  Old values of C are read kOldValues at a time, so that
+// they are on their way together.
+template <int kVec>
+__device__ __forceinline__ void store_turned(const float* src, int src_step, float* dst, long long dst_step, int rows, int all,
+                                             const StoreTarget& t) {
+  constexpr int kGroup = kOldValues / kVec;
+  if (rows > all) rows = all;
+  if (t.beta == 0.f) {
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r, src += src_step, dst += dst_step) {
+      if constexpr (kVec == 4)
+        *reinterpret_cast<float4*>(dst) = make_float4(__fmul_rn(t.alpha, src[0]), __fmul_rn(t.alpha, src[1]),
+                                                      __fmul_rn(t.alpha, src[2]), __fmul_rn(t.alpha, src[3]));
+      else
+        *dst = __fmul_rn(t.alpha, src[0]);
+    }
+    return;
+  }
+#pragma unroll 1
+  for (int left = rows; left > 0; left -= kGroup) {
+    float old[kGroup][kVec];
+    const float* q = dst;
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g) {  // beyond the matrix: its last piece again, so that no load needs a predicate
+      if constexpr (kVec == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(q);
+        old[g][0] = v.x;
+        old[g][1] = v.y;
+        old[g][2] = v.z;
+        old[g][3] = v.w;
+      } else {
+        old[g][0] = *q;
+      }
+      q += g + 1 < left ? dst_step : 0;
+    }
+#pragma unroll
+    for (int g = 0; g < kGroup; ++g, src += src_step, dst += dst_step)
+      if (g < left) store_updated<kVec>(src, dst, old[g], t);
+  }
+}
+
 constexpr int kEpiBufFloats = 32 * 33;              // one warp's turn buffer
 constexpr int kEpiBufBytes = kEpiBufFloats * 4;      // 4224
 
@@ -97,7 +149,20 @@ __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row
   // Old values of C a lane holds at once (beta != 0).  Read one before each store, every load waited for the store before it:
   // 1000 x 777 x 1111 with a column-major C and beta 26.6 us, in groups 20.5.  The kernels with fewer registers left
   // (kWide = false) stay with one: groups of 8 cost them 4096 x 128^3 195 -> 230 us without any beta.
-  constexpr int kGroup = 16;
+  constexpr int kGroup = kOldValues;
+  if (kWide && t.vec_ok && t.beta == 0.f && col0 + NC <= t.N && t.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(t.cbase) & 31) == 0) {
+    if (row0 + lane < t.M) {
+      float* dst = t.cbase + static_cast<long long>(row0 + lane) * t.ldc + col0;
+#pragma unroll
+      for (int i = 0; i < NC; i += 8) {
+        float o[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(t.alpha, acc[i + e]);
+        st_global_v8(dst + i, o);
+      }
+    }
+    return;
+  }
   if (t.col_major) {
     // Consecutive lanes hold consecutive addresses; one pointer walks the columns (multiplying and comparing per column
     // cost 256 x 512^3 by pointer tables 342 us instead of 289).
@@ -113,94 +178,63 @@ __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row
     }
     if constexpr (!kWide) {
       store_row_slice(acc, row0 + lane, col0, t);
+    } else if (t.beta == 0.f) {
+      const int left = t.N - col0;
+#pragma unroll
+      for (int i = 0; i < NC; ++i) {
+        if (i < left) *dst = __fmul_rn(t.alpha, acc[i]);
+        dst += t.ldc;
+      }
     } else {
 #pragma unroll
       for (int g = 0; g < NC; g += kGroup) {
         const int left = t.N - col0 - g;
-        float old[kGroup];
-        float* q = dst;
+        if (left > 0) {
+          float old[kGroup];
+          const float* q = dst;
 #pragma unroll
-        for (int i = 0; i < kGroup; ++i) {
-          old[i] = (t.beta != 0.f && i < left) ? *q : 0.f;
-          q += t.ldc;
+          for (int i = 0; i < kGroup; ++i) {  // beyond the matrix: its last column again, so that no load needs a predicate
+            old[i] = *q;
+            q += i + 1 < left ? t.ldc : 0;
+          }
+#pragma unroll
+          for (int i = 0; i < kGroup; ++i) {
+            if (i < left) *dst = axpby(t.alpha, acc[g + i], t.beta, old[i]);
+            dst += t.ldc;
+          }
         }
-#pragma unroll
-        for (int i = 0; i < kGroup; ++i) {
-          if (i < left) *dst = t.beta != 0.f ? axpby(t.alpha, acc[g + i], t.beta, old[i]) : __fmul_rn(t.alpha, acc[g + i]);
-          dst += t.ldc;
-        }
-      }
-    }
-    return;
-  }
-  if (kWide && t.vec_ok && t.beta == 0.f && col0 + NC <= t.N && t.ldc % 8 == 0 && (reinterpret_cast<uintptr_t>(t.cbase) & 31) == 0) {
-    if (row0 + lane < t.M) {
-      float* dst = t.cbase + static_cast<long long>(row0 + lane) * t.ldc + col0;
-#pragma unroll
-      for (int i = 0; i < NC; i += 8) {
-        float o[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(t.alpha, acc[i + e]);
-        st_global_v8(dst + i, o);
       }
     }
     return;
   }
   const int rsub = lane >> 3, cv = (lane & 7) * 4;
+  if constexpr (kWide) {
+    // Short loops, a uniform choice between them, and no predicate per element: with rows, edges and old values unrolled
+    // and predicated together this part kept the warps waiting for instructions (592 x 128 x 200 x 16 on one-SM tiles 90 us,
+    // like this 37; 12000 x 12001 x 1100 1150 and 890; 8192 x 8190 x 2048 830 and 720).
 #pragma unroll
-  for (int cc = 0; cc < NC / 32; ++cc) {
+    for (int cc = 0; cc < NC / 32; ++cc) {
+      const int first = col0 + cc * 32;
+      if (first >= t.N) return;
 #pragma unroll
-    for (int i = 0; i < 32; ++i) wbuf[lane * 33 + i] = acc[cc * 32 + i];
-    __syncwarp();
-    if constexpr (kWide) {
-      // in groups of row slices, so that a group's old values of C (beta != 0) are on their way together
-#pragma unroll
-      for (int part = 0; part < 8; part += kGroup / 4) {
-        const int col = col0 + cc * 32 + cv;
-        const bool vec = t.vec_ok && col + 3 < t.N;
-        float4 old[kGroup / 4];
-#pragma unroll
-        for (int j = 0; j < kGroup / 4; ++j) {
-          old[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-          const int row = row0 + (part + j) * 4 + rsub;
-          if (t.beta != 0.f && row < t.M) {
-            const float* src = t.cbase + static_cast<long long>(row) * t.ldc + col;
-            if (vec) {
-              old[j] = *reinterpret_cast<const float4*>(src);
-            } else {
-              if (col < t.N) old[j].x = src[0];
-              if (col + 1 < t.N) old[j].y = src[1];
-              if (col + 2 < t.N) old[j].z = src[2];
-              if (col + 3 < t.N) old[j].w = src[3];
-            }
-          }
-        }
-#pragma unroll
-        for (int j = 0; j < kGroup / 4; ++j) {
-          const int r = (part + j) * 4 + rsub;
-          const int row = row0 + r;
-          const float* src = wbuf + r * 33 + cv;
-          const float v0 = src[0], v1 = src[1], v2 = src[2], v3 = src[3];
-          if (row < t.M) {
-            float* dst = t.cbase + static_cast<long long>(row) * t.ldc + col;
-            float4 o;
-            if (t.beta != 0.f)
-              o = make_float4(axpby(t.alpha, v0, t.beta, old[j].x), axpby(t.alpha, v1, t.beta, old[j].y),
-                              axpby(t.alpha, v2, t.beta, old[j].z), axpby(t.alpha, v3, t.beta, old[j].w));
-            else
-              o = make_float4(__fmul_rn(t.alpha, v0), __fmul_rn(t.alpha, v1), __fmul_rn(t.alpha, v2), __fmul_rn(t.alpha, v3));
-            if (vec) {
-              *reinterpret_cast<float4*>(dst) = o;
-            } else {
-              if (col < t.N) dst[0] = o.x;
-              if (col + 1 < t.N) dst[1] = o.y;
-              if (col + 2 < t.N) dst[2] = o.z;
-              if (col + 3 < t.N) dst[3] = o.w;
-            }
-          }
-        }
+      for (int i = 0; i < 32; ++i) wbuf[lane * 33 + i] = acc[cc * 32 + i];
+      __syncwarp();
+      if (t.vec_ok && first + 32 <= t.N) {
+        // a row slice of four columns per lane, four rows apart
+        store_turned<4>(wbuf + rsub * 33 + cv, 4 * 33, t.cbase + static_cast<long long>(row0 + rsub) * t.ldc + first + cv, 4 * t.ldc,
+                        (t.M - row0 - rsub + 3) >> 2, 8, t);
+      } else if (first + lane < t.N) {
+        // a column per lane
+        store_turned<1>(wbuf + lane, 33, t.cbase + static_cast<long long>(row0) * t.ldc + first + lane, t.ldc, t.M - row0, 32, t);
       }
-    } else {
+      __syncwarp();
+    }
+  } else {
+#pragma unroll
+    for (int cc = 0; cc < NC / 32; ++cc) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) wbuf[lane * 33 + i] = acc[cc * 32 + i];
+      __syncwarp();
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const int r = j * 4 + rsub;
@@ -230,8 +264,8 @@ __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row
           }
         }
       }
+      __syncwarp();
     }
-    __syncwarp();
   }
 }
 
