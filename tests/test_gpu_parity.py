@@ -204,6 +204,8 @@ def test_direct_store_option_is_bit_identical():
     b = _t(rng.uniform(-1, 1, (200, 700)).astype(np.float32))
     c0 = _t(rng.uniform(-1, 1, (300, 700)).astype(np.float32))
     tcec.set_option("path", 1)
+    tcec.set_option("cta_pair", 0)  # the option is the one-SM kernel's
+    tcec.set_option("narrow_tiles", 0)
     out = {}
     try:
         for turn in (1, 0):
@@ -212,6 +214,7 @@ def test_direct_store_option_is_bit_identical():
             tcec.device_status()
     finally:
         tcec.set_option("store_turn", 1)
+        tcec.set_option("narrow_tiles", -1)
     assert torch.equal(out[0], out[1])
 
 
@@ -222,6 +225,8 @@ def test_tile_order_options_are_bit_identical():
     a = _t(rng.uniform(-1, 1, (2000, 300)).astype(np.float32))
     b = _t(rng.uniform(-1, 1, (300, 5000)).astype(np.float32))  # 16 x 20 = 320 tiles: more than two per SM
     tcec.set_option("path", 1)
+    tcec.set_option("cta_pair", 0)  # the pair and the narrow kernel stride statically
+    tcec.set_option("narrow_tiles", 0)
     try:
         tcec.set_option("static_tiles", 1)
         ref = tcec.sgemm(a, b)
@@ -239,6 +244,7 @@ def test_tile_order_options_are_bit_identical():
     finally:
         tcec.set_option("static_tiles", 0)
         tcec.set_option("reserve_sms", 0)
+        tcec.set_option("narrow_tiles", -1)
     exact = cpu.gemm_f64(a.cpu().numpy()[:64], b.cpu().numpy())
     assert cpu.errors(ref[:64].cpu().numpy(), exact)["max_rel"] < 1e-6
 
@@ -508,20 +514,25 @@ def test_ragged_batch_shapes():
 
 
 def test_more_matrices_than_a_grid_dimension_holds():
-    """70 000 tiny matrices: the batch index of the split kernel is a grid dimension (65 535 at
-    most), so such a batch takes several launches; every matrix must still be right."""
+    """70 000 tiny matrices, more than a grid's y or z dimension holds (65 535): through the direct kernel, which
+    packs them into tiles, and through panels every matrix must be right."""
     if _free_gib() < 12:
         pytest.skip("needs 12 GiB of free device memory")
     g = torch.Generator(device=DEV).manual_seed(44)
     nb = 70000
     a = torch.randn((nb, 16, 16), generator=g, device=DEV)
     b = torch.randn((nb, 16, 16), generator=g, device=DEV)
-    c = tcec.sgemm_strided_batched(a, b)
-    tcec.device_status()
     exact = torch.matmul(a.double(), b.double())
-    err = ((c.double() - exact).abs().amax(dim=(1, 2)) / exact.abs().amax(dim=(1, 2))).max().item()
-    assert err < 1e-6
-    tcec.destroy()  # gives the 4.6 GB workspace back
+    out = []
+    for path in (0, 1):
+        tcec.set_option("path", path)
+        c = tcec.sgemm_strided_batched(a, b)
+        tcec.device_status()
+        err = ((c.double() - exact).abs().amax(dim=(1, 2)) / exact.abs().amax(dim=(1, 2))).max().item()
+        assert err < 1e-6
+        out.append(c)
+    assert torch.equal(out[0], out[1])
+    tcec.destroy()  # gives the panels' 4.6 GB workspace back
 
 
 def test_packed_entry_points_match_plain_call():
@@ -844,12 +855,12 @@ def test_batched_configuration_full_size_properties():
     got = c.double().sum(dim=2)
     scale = want.abs().max().item()
     assert (got - want).abs().max().item() < 1e-4 * scale  # 256 terms of ~1e-7 relative error each
-    # the pointer-array form gives the same bits
+    # the pointer-array form, here from panels, gives the bits that the FP32-tile kernel gave: same split, same products, same
+    # rounding points
     c2 = [torch.empty((n, n), device=DEV) for _ in range(64)]
+    tcec.set_option("path", 1)
     tcec.sgemm_batched(list(a[:64]), list(b[:64]), c2)
     tcec.device_status()
-    # the pointer-array form goes through the panel kernel, the strided form through the FP32-tile
-    # kernel: same split, same products, same rounding points, so not a bit differs
     assert all(torch.equal(x, y) for x, y in zip(c2, c[:64]))
 
 

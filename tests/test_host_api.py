@@ -127,13 +127,18 @@ def test_options_round_trip():
             tcec.set_option("no_such_option", 1)
         for name, default, other in (("cta_pair", -1, 1), ("path", 0, 2), ("store_turn", 1, 0), ("reserve_sms", 0, 8),
                                      ("static_tiles", 0, 1), ("tile_n", 0, 128), ("comm_sms", 8, 16),
-                                     ("comm_panel_rows", 2048, 512), ("comm_helper", 1, 0), ("half_tiles", 1, 0)):
+                                     ("comm_panel_rows", 2048, 512), ("comm_helper", 1, 0), ("half_tiles", 1, 0),
+                                     ("narrow_tiles", -1, 64), ("direct_kernel", -1, 1)):
             assert tcec.get_option(name) == default
             tcec.set_option(name, other)
             assert tcec.get_option(name) == other
             tcec.set_option(name, default)
         with pytest.raises(tcec.TcecError):
             tcec.set_option("store_turn", 2)
+        with pytest.raises(tcec.TcecError):
+            tcec.set_option("narrow_tiles", 48)  # a width that there is no kernel for
+        with pytest.raises(tcec.TcecError):
+            tcec.set_option("direct_kernel", 2)
         with pytest.raises(tcec.TcecError):
             tcec.set_option("comm_panel_rows", 300)  # not a multiple of 256
         with pytest.raises(tcec.TcecError):
