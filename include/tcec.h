@@ -122,7 +122,7 @@ int tcec_sgemm_batched_cublas(int transa, int transb, int m, int n, int k, const
  * make that first call outside any stream capture.  All calls on a device share the one array
  * and it keeps the previous call's panels: two calls whose kernels overlap on the GPU (different
  * streams without an ordering between them) race and give wrong results - order them.  Nothing
- * in the array needs clearing between calls; every byte the GEMM reads is rewritten first.
+ * in the array needs clearing between calls; every byte that reaches C is rewritten first.
  * Bounded-wait expiry is reported by tcec_static_status(), the counterpart of
  * tcec_device_status() for this entry point.
  */
@@ -227,9 +227,9 @@ int tcec_sgemm_packed(int layout_c, int m, int n, int k, float alpha, const void
  * No conjugation.  Built, like the reference's complex fragments, from four real
  * error-corrected products (include/wmma_extension/tcec/complex.hpp:646-727:
  * real = Ar Br + Ai (-Bi), imag = Ai Br + Ar Bi; its test is test/tcec/mma_complex.cu);
- * here each part is one real GEMM over the concatenated K of its two products, so the
- * promotion rule sees K' = 2K.  Scratch (operand panels and two m x n planes) comes from
- * the per-stream workspace.
+ * here all four are one real GEMM of twice the N and K, so the promotion rule sees K' = 2K,
+ * which writes C itself when alpha and beta are real; complex ones take an m x n product in
+ * scratch and a pass that applies them.  Scratch comes from the per-stream workspace.
  */
 int tcec_cgemm(int layout_a, int layout_b, int layout_c, int m, int n, int k, const float* alpha,
                const float* a, long long lda, const float* b, long long ldb, const float* beta, float* c,
@@ -266,7 +266,9 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                slower); 0 = never; 1 = whenever it applies.
  *   "half_tiles" 1 (default) = a call with so few 256 x 256 tiles that they would leave at least half
  *                of the SM pairs idle runs on 256 x 128 half tiles instead (CTA-pair kernel, N = 128
- *                MMAs; 1024^3: 37 -> 27 us); 0 = whole tiles only.  Same results bit for bit.
+ *                MMAs; 1024^3: 37 -> 27 us); 0 = whole tiles only.  Same results bit for bit.  Automatic
+ *                calls of that size run on narrow tiles before they come to this, apart from some of long K
+ *                without error correction.
  *   "reserve_sms" 0..64 (default 0): SMs the GEMM kernels do not occupy.  Their persistent CTAs take
  *                every register of an SM, so a communication kernel launched beside them can only
  *                run where the GEMM has no CTA.
@@ -291,7 +293,7 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                out on the device).  Automatic picks it for batches with k <= 2048 whose matrices are so many, and
  *                so small, that the split would cost more than conversion in every tile.
  *   "narrow_tiles" -1 (default) = a call whose 256-wide tiles are too few to fill the GPU runs in tiles of
- *                128 x 32, 64 or 128 (64 x 4096 x 4096 on packed operands: 82 -> 35 us with the packing of A);
+ *                128 x 32, 64 or 128 (64 x 4096 x 4096 on packed operands: 82 -> 34 us with the packing of A);
  *                0 = never; 32, 64, 128 = that width.  Only while "cta_pair" and "tile_n" are automatic,
  *                "store_turn" is 1 and "static_tiles" 0.  Same results bit for bit.
  *   "direct_kernel" one launch that reads FP32 operands of any layout, alignment and batch form with

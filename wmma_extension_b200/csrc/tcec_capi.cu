@@ -405,7 +405,9 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
     const int max_pairs = sms / 2 > 1 ? sms / 2 : 1;
     // A call with so few tiles that they leave at least half of the pairs idle runs in half-width
     // tiles: twice as many work items, each ~0.6 as long (1024^3: 16 tiles become 32 halves,
-    // 37 -> 27 us).  Halving only the tiles of an underfilled last wave of a larger call does not
+    // 37 -> 27 us).  By default that is what narrow tiles leave over (some calls of long K without error correction):
+    // on 118 calls of this size panel_choice, which prices whole tiles, was at most 10 % from the fastest of half tiles and
+    // the three widths, and more than 3 % on four.  Halving only the tiles of an underfilled last wave of a larger call does not
     // pay: an N = 128 MMA takes nearly as long as an N = 256 one (measured at 4096^3 and 5120^3:
     // 1-2 % slower), so such calls stay on whole tiles.
     const int halved = (opt.half_tiles && 2 * npair_tiles <= max_pairs) ? static_cast<int>(npair_tiles) : 0;
@@ -909,14 +911,12 @@ int cgemm_impl(int la, int lb, int lc, int m, int n, int k, const float* alpha, 
   pa.ld = row ? lda : ldb;
   pa.k_contiguous = row ? la == TCEC_ROW_MAJOR : lb == TCEC_COL_MAJOR;
   pa.rows = outer;
-  pa.row_blocks = s.a_row_blocks;
   pa.panels = panels_a;
   pb.src = row ? b : a;
   pb.ld = row ? ldb : lda;
   pb.k_contiguous = row ? lb == TCEC_COL_MAJOR : la == TCEC_ROW_MAJOR;
   pb.rows = inner;
   pb.doubled = 1;
-  pb.row_blocks = s.b_row_blocks;
   pb.panels = panels_b;
   pa.k = pb.k = k;
   pa.nkb = pb.nkb = s.nkb;

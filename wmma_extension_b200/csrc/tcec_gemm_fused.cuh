@@ -48,10 +48,10 @@
 // is re-balanced at entry with setmaxnreg: the kernel launches with 96 registers per thread, the
 // control warpgroup drops to 32, the converters to 40 and the epilogue rises to 184 (the shares
 // must sum to no more than the launch allocation, or the raise would never be granted).
-//   warp 0       lane 0: TMA producer (own rows of A, own half of B)
-//   warp 1       lane 0: leader: MMA issuer, main products
-//   warp 2       lane 0: leader: MMA issuer, correction products
-//   warp 3       lane 0: relay of "my half of the stage is converted" to the leader
+//   warp 0       one thread: TMA producer (own rows of A, own half of B)
+//   warp 1       one thread: leader: MMA issuer, main products
+//   warp 2       one thread: leader: MMA issuer, correction products
+//   warp 3       one thread: relay of "my half of the stage is converted" to the leader
 //   warps 4-11   epilogue (own 128 rows of the tile)
 //   warps 12-19  converters (sixteen warps were measured no faster than eight: the conversion is
 //                bound by shared-memory bandwidth, not by issue slots)
@@ -112,7 +112,7 @@ struct GemmFusedCfg {
   static_assert(SMEM_BYTES <= 232448 - 512, "dynamic + static shared memory exceed an SM");
   static constexpr int TMEM_COLS = kEc ? 512 : 256;
   static constexpr int THREADS = 128 + 32 * EPI_WARPS + 32 * CONV_WARPS;
-  // setmaxnreg moves registers inside the CTA's launch allocation (896 threads x 72), so the
+  // setmaxnreg moves registers inside the CTA's launch allocation (640 threads x 96), so the
   // three shares must fit in it: a request beyond it would wait forever.
   static constexpr int REGS_LAUNCH = 96, REGS_CONTROL = 32, REGS_CONVERT = 40, REGS_EPILOGUE = 184;
   static_assert(128 * REGS_CONTROL + 32 * CONV_WARPS * REGS_CONVERT + 32 * EPI_WARPS * REGS_EPILOGUE <=
@@ -361,13 +361,13 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
             if (p.a_k_contiguous) {
               tma_load_3d(dst, ma, landed, kb * 32, arow, z);
             } else {
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < 4; ++j) tma_load_3d(dst + j * 4096, ma, landed, arow + 32 * j, kb * 32, z);
             }
             if (p.b_k_contiguous) {
               tma_load_3d(dst + Cfg::STG_A, mb, landed, kb * 32, brow, z);
             } else {
-  #pragma unroll
+#pragma unroll
               for (int j = 0; j < 4; ++j)
                 tma_load_3d(dst + Cfg::STG_A + j * 4096, mb, landed, brow + 32 * j, kb * 32, z);
             }

@@ -1,5 +1,5 @@
-// Roles shared by the three GEMM kernels (operand panels on one SM, operand panels on a CTA
-// pair, FP32 tiles converted in shared memory): the two MMA-issuing threads and the register side
+// Roles shared by the five GEMM kernels (operand panels on one SM, on a CTA pair and on narrow tiles, FP32
+// tiles converted in shared memory, small matrices read directly): the two MMA-issuing threads and the register side
 // of the epilogue.  The kernels differ in how a stage of the ring gets filled and in where the
 // operand images sit inside it; from `full[s]` onward they do the same thing.
 //

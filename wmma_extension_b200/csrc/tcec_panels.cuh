@@ -160,7 +160,6 @@ struct ComplexSplitParams {
   int rows, k;        // complex extents
   int k_contiguous;   // element (r, p) at r*ld + p, else at p*ld + r
   int doubled;
-  int row_blocks;     // of the panels, padded rows / 128
   int nkb;            // K blocks of the panels
   uint8_t* panels;
 };
