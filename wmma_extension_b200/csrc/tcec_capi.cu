@@ -113,8 +113,9 @@ int get_device_state(DeviceState** out) {
     TCEC_CUDA((set_direct_smem_attrs<false, false>()));
     TCEC_CUDA((set_direct_smem_attrs<true, true>()));
     TCEC_CUDA((set_direct_smem_attrs<true, false>()));
-    if (cudaMalloc(&st.status, sizeof(int)) != cudaSuccess) return TCEC_ERR_ALLOC;
-    TCEC_CUDA(cudaMemset(st.status, 0, sizeof(int)));
+    if (cudaMalloc(&st.status, kStatusBytes + kPaceSlots * kPaceSlotBytes) != cudaSuccess) return TCEC_ERR_ALLOC;
+    TCEC_CUDA(cudaMemset(st.status, 0, kStatusBytes + kPaceSlots * kPaceSlotBytes));
+    st.pace = reinterpret_cast<unsigned int*>(st.status) + kStatusBytes / sizeof(unsigned int);
     st.attrs_done = true;
   }
   *out = &st;
@@ -173,6 +174,14 @@ int get_sched(DeviceState* st, cudaStream_t stream, unsigned int** out) {
   }
   *out = p;
   return TCEC_OK;
+}
+
+// The stream's pacing word; null when the slots are used up or there are none (a launch without it is only not paced).  Launches
+// that overlap although they share a word (a captured graph replayed on another stream) pace one another wrongly, no more.
+static unsigned int* get_pace(DeviceState* st, cudaStream_t stream) {
+  if (!st->pace) return nullptr;
+  const int slot = st->pace_slot.emplace(stream, static_cast<int>(st->pace_slot.size())).first->second;
+  return slot < kPaceSlots ? st->pace + slot * (kPaceSlotBytes / sizeof(unsigned int)) : nullptr;
 }
 
 bool policy_tf32(int policy) { return policy == TCEC_POLICY_TF32_EC || policy == TCEC_POLICY_TF32_NO_EC; }
@@ -412,6 +421,8 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
     // 1-2 % slower), so such calls stay on whole tiles.
     const int halved = (opt.half_tiles && 2 * npair_tiles <= max_pairs) ? static_cast<int>(npair_tiles) : 0;
     const int whole = static_cast<int>(npair_tiles) - halved;
+    if (!ex.only_if && pace_pays(gp.tiles_m, gp.tiles_n, batch, s.nkb, s.np, max_pairs) && (gp.pace = get_pace(st, stream)))
+      cudaMemsetAsync(gp.pace, 0, sizeof(unsigned int), stream);
 #define TCEC_PAIR(T, E)                                                                                          \
   do {                                                                                                           \
     if (whole > 0) {                                                                                             \
@@ -1200,6 +1211,8 @@ int tcec_destroy(void) {
     destroy_step_state(&kv.second);
     if (kv.second.status) cudaFree(kv.second.status);
     kv.second.status = nullptr;
+    kv.second.pace = nullptr;
+    kv.second.pace_slot.clear();
     kv.second.attrs_done = false;
   }
   destroy_comm_state();

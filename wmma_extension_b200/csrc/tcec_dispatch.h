@@ -12,12 +12,25 @@ namespace tcec_host {
 
 inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 
-// Whether the wide tiles of the panel GEMM go to CTA pairs.  One product per K block makes the kernel wait on operands from L2,
-// which a pair halves for B: measured 10-15 % faster there.  With three products the pair is faster only while the clocks are
-// high, i.e. for calls too short to reach the board's power cap (2048^3: +8 %, 4096^3: +2 %; 16384^3 back to back: -5 %), so
-// the automatic choice takes it below ~5000^3.
+// Whether the wide tiles of the panel GEMM go to CTA pairs, which bring a third fewer bytes through L2 per product (a half fewer
+// of B).  Long calls run at the board's power limit, where those bytes cost clock: with its pairs kept together along K (below)
+// 16384^3 takes 19.3 ms on pairs and 20.0 on single SMs, 8192^3 2.41 and 2.53, tf32 4.20 and 4.34, 8192^3 without correction 0.91 and
+// 1.0.  Not where the 256 rows of a pair tile are half empty and the call is long: what is lost is one part in the number of
+// 128-row blocks.
 inline bool pairs_pay(int m, int n, int k, int batch, bool ec) {
-  return !ec || 2.0 * m * static_cast<double>(n) * k * batch <= 2.5e11;
+  const long long blocks = ceil_div(m, 128);
+  return !ec || 2.0 * m * static_cast<double>(n) * k * batch <= 2.5e11 || blocks % 2 == 0 || blocks >= 19;
+}
+
+// Pair tiles are taken in groups of kPairGroupM tile rows, column by column.  A launch is paced (tcec_gemm_panels_pair.cuh) if it
+// has more tiles than pairs, so that they get out of step, and the panels that one wave of tiles reads do not stay in L2 (126 MB)
+// all the while.  Unpaced and paced, ms: 16384^3 (290 MB) 21.5, 19.3; 12000 x 4000 x 12000 (212 MB) 2.79, 2.70; 8192^3 (145 MB) 2.46,
+// 2.44; without correction 16384^3 (145 MB) 7.9, 7.3, but 8192^3 (72 MB) 0.912, 0.925.
+constexpr int kPairGroupM = 8;
+inline bool pace_pays(int tiles_m, int tiles_n, int batch, int nkb, int images, int pairs) {
+  if (static_cast<long long>(tiles_m) * tiles_n * batch <= pairs) return false;
+  const long long rows = tiles_m < kPairGroupM ? tiles_m : kPairGroupM, wave = ceil_div(pairs, rows), cols = tiles_n < wave ? tiles_n : wave;
+  return static_cast<double>(rows + cols) * 256 * 64 * images * nkb >= 100e6;
 }
 
 // The panel GEMM of a call: `width` of the narrow tiles if they would finish the call sooner than 256-wide ones, else 0,

@@ -5,9 +5,9 @@
 // (128 of the tile's 256 N rows), and the leader CTA issues every MMA for both SMs
 // (M = 256, N = 256, K = 16): per SM and K block 32 KB instead of 48 KB come through L2 and
 // 48 KB instead of 72 KB of operands are read from shared memory, and the ring holds 6 stages
-// instead of 4.  Measured: a little faster than one SM per tile while the clocks are high
-// (4096^3), but it draws more power per product, so it is slower once the board sits at its
-// power cap (16384^3); the host library chooses by the call's size.
+// instead of 4.  What bounds it at large sizes is the board's power (1000 W): the SM clock settles where the MMAs, the operands'
+// way through L2 and the panels' way from DRAM add up to it.  16384^3 without copies takes 16.4 ms; with them 22.3 as long as the
+// pairs drift apart along K (51.7 GB from DRAM instead of 8) and 19.3 with the pairs kept together (Pace, below).
 //
 // Pair protocol (rank 0 = leader, rank 1 = peer):
 //   full[s]   leader's barrier: its own copies' bytes + one remote arrive by the peer's relay
@@ -27,6 +27,7 @@
 // A launch covers the pair tiles [tile_first, tile_first + tile_count).
 #pragma once
 #include "sm100_ptx.cuh"
+#include "tcec_dispatch.h"
 #include "tcec_gemm_panels.cuh"
 #include "tcec_gemm_roles.cuh"
 
@@ -49,8 +50,52 @@ struct GemmPairCfg {
   // as in the one-SM kernel: the control warpgroup hands registers to the two epilogue warpgroups
   static constexpr int REGS_CONTROL = 40, REGS_EPILOGUE = 232;
   static_assert(128 * REGS_CONTROL + 256 * REGS_EPILOGUE <= THREADS * 168, "register shares");
-  static constexpr int GROUP_M = 8;  // pair tiles are 256 rows tall
+  static constexpr int GROUP_M = tcec_host::kPairGroupM;  // pair tiles are 256 rows tall
 };
+
+// Keeps the pairs of a launch close together along K.  The pairs of a wave share their panels, each row block of A with the other
+// tiles of its row and each of B with those of its column, and a panel comes from DRAM once if all of them read it while it is in
+// L2.  Left alone they drift apart, tile after tile, until most panels are fetched several times.
+// Every kPaceStages stages the leader's producer raises its count.  A thread of its own (the producer has no time for a round
+// trip to L2: 16384^3 without correction 8.0 ms that way, 7.3 this way) adds it to a device-wide sum and holds the producer while
+// its count is more than one above the mean.  A hold is bounded: a pair whose SMs another kernel has taken must not stop the
+// rest, so whoever has held in vain holds no more.
+// 16384^3: 21.4 ms unpaced, 19.3 every 4 or 8 stages, 19.6 every 16; the word is a hint, results do not depend on it.
+constexpr uint32_t kPaceStages = 8;
+constexpr uint32_t kPaceLeft = 1u << 24;  // what a pair adds when it runs out of tiles, so that nobody waits for it
+struct Pace {
+  volatile uint32_t count, hold;  // shared memory; the producer writes `count` (kPaceLeft at its end), the pacing thread `hold`
+};
+__device__ __forceinline__ void pace_producer(Pace& pace, uint32_t count) {
+  pace.count = count;
+  for (int i = 0; i < 512 && pace.hold; ++i) __nanosleep(64);
+}
+__device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* sum, uint32_t pairs, volatile uint32_t* abortp) {
+  uint32_t added = 0;
+  bool may_hold = true;
+  for (uint32_t idle = 0; idle < TCEC_WAIT_LIMIT && !*abortp;) {
+    const uint32_t count = pace.count;
+    if (count == added) {
+      __nanosleep(200);
+      ++idle;
+      continue;
+    }
+    idle = 0;
+    uint32_t seen = atomicAdd(sum, count - added) + (count - added);
+    added = count;
+    if (count >= kPaceLeft) return;
+    const unsigned long long wanted = static_cast<unsigned long long>(count - 1) * pairs;
+    if (!may_hold || seen >= wanted) continue;
+    pace.hold = 1;
+    for (int i = 0; i < 128 && seen < wanted; ++i) {
+      __nanosleep(200);
+      seen = ld_relaxed_gpu(sum);
+    }
+    may_hold = seen >= wanted;
+    pace.hold = 0;
+  }
+  atomicAdd(sum, kPaceLeft);
+}
 
 // p.tiles_m counts 256-row pair tiles here.
 template <bool kTf32, bool kEc, int BN>
@@ -68,6 +113,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   __shared__ uint64_t bar_main_full, bar_main_free, bar_corr_full, bar_corr_free, bar_drain[2];
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_flag;
+  __shared__ Pace pace;
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -89,6 +135,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     mbar_init(smem_u32(&bar_drain[0]), 1);
     mbar_init(smem_u32(&bar_drain[1]), 1);
     abort_flag = 0;
+    pace.count = pace.hold = 0;
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -122,6 +169,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       // ---------------------------------------------------------- producer (each CTA, own panels)
       if (elect_one()) {
         uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0, it = 0;
+        const bool paced = p.pace && leader;  // the peer's ring cannot run ahead of the leader's
         bool ok = true;
         for (int tile = pair; tile < ntiles && ok; tile += npairs) {
           const TileCoord tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
@@ -138,6 +186,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
               ok = false;
               break;
             }
+            if (paced && it % kPaceStages == 0) pace_producer(pace, it / kPaceStages);
             if (dev_flag(p.debug_flags, 1) && it >= static_cast<uint32_t>(NST)) {  // develop builds: no loads
               mbar_arrive(smem_u32(&bar_full[s]));
               if (++s == static_cast<uint32_t>(NST)) {
@@ -174,6 +223,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             }
           }
         }
+        if (paced) pace.count = kPaceLeft;
         if (!ok) {
           raise_abort_pair(&abort_flag);
           atomicCAS(p.status, 0, kErrProducerWait);
@@ -221,6 +271,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[1]);
         }
       }
+    } else if (p.pace && leader && elect_one()) {
+      // ---------------------------------------------------------- leader: pacing
+      pace_launch(pace, p.pace, static_cast<uint32_t>(npairs), abortp);
     }
   } else {
     // ------------------------------------------------------------ epilogue (each CTA, its 128 rows)

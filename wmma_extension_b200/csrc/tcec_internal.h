@@ -41,6 +41,8 @@ struct Options {
 };
 Options snapshot_options();
 
+constexpr int kStatusBytes = 128, kPaceSlots = 63, kPaceSlotBytes = 128;  // what a device's `status` allocation holds
+
 struct Workspace {
   void* ptr = nullptr;
   size_t bytes = 0;
@@ -55,6 +57,8 @@ struct DeviceState {
   bool attrs_done = false;
   std::map<cudaStream_t, Workspace> ws;
   std::map<cudaStream_t, unsigned int*> sched;  // per stream: the panel GEMM's two tile-scheduler counters
+  unsigned int* pace = nullptr;                 // kPaceSlots words, 128 bytes apart, in the allocation of `status`
+  std::map<cudaStream_t, int> pace_slot;        // which of them a stream uses
   unsigned int* sched_fixed = nullptr;          // set instead by the allocation-free entry (a device symbol)
   StepState* step = nullptr;
 };
