@@ -251,6 +251,23 @@ __global__ void split_flat_kernel(const float* __restrict__ in, float* hi, float
   }
 }
 
+// Launches `kernel`, which waits for the kernel before it on the stream by itself (wait_for_launch_before), so that it may be set up
+// while that one ends.
+template <class... Params, class... Args>
+void launch_early(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  cudaLaunchAttribute early{};
+  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  early.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t config{};
+  config.gridDim = dim3(grid);
+  config.blockDim = dim3(threads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  config.attrs = &early;
+  config.numAttrs = 1;
+  cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+
 template <bool T, bool E>
 void launch_split(const SplitParams& sp, int batch, cudaStream_t stream) {
   // the batch index is the grid's z dimension (at most 65535): larger batches go in several launches
@@ -268,14 +285,14 @@ void launch_split(const SplitParams& sp, int batch, cudaStream_t stream) {
 template <int BN, bool T, bool E>
 void launch_gemm(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
   using Cfg = GemmPanelCfg<BN, T, E>;
-  tcec_gemm_panels_kernel<BN, T, E>
-      <<<grid, Cfg::THREADS, gp.store_turn ? Cfg::SMEM_BYTES : Cfg::SMEM_BYTES_NO_TURN, stream>>>(gp);
+  launch_early(tcec_gemm_panels_kernel<BN, T, E>, grid, Cfg::THREADS, gp.store_turn ? Cfg::SMEM_BYTES : Cfg::SMEM_BYTES_NO_TURN,
+         stream, gp);
 }
 
 template <int BN, bool T, bool E>
 void launch_narrow(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
   using Cfg = GemmNarrowCfg<BN, E>;
-  tcec_gemm_panels_narrow_kernel<BN, T, E><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(gp);
+  launch_early(tcec_gemm_panels_narrow_kernel<BN, T, E>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, gp);
 }
 template <bool T, bool E>
 void launch_narrow_as(int width, const GemmPanelParams& gp, int grid, cudaStream_t stream) {
@@ -429,12 +446,12 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
       gp.tile_first = 0;                                                                                         \
       gp.tile_count = whole;                                                                                     \
       const int grid = 2 * (whole < max_pairs ? whole : max_pairs);                                              \
-      tcec_gemm_panels_pair_kernel<T, E, 256><<<grid, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream>>>(gp);         \
+      launch_early(tcec_gemm_panels_pair_kernel<T, E, 256>, grid, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp); \
     }                                                                                                            \
     if (halved > 0) {                                                                                            \
       gp.tile_first = whole;                                                                                     \
       gp.tile_count = halved;                                                                                    \
-      tcec_gemm_panels_pair_kernel<T, E, 128><<<4 * halved, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream>>>(gp);   \
+      launch_early(tcec_gemm_panels_pair_kernel<T, E, 128>, 4 * halved, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp); \
     }                                                                                                            \
   } while (0)
     if (tf32 && ec)
@@ -638,9 +655,9 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
   const int max_pairs = sms / 2;
   const int grid = 2 * static_cast<int>(ntiles < max_pairs ? ntiles : max_pairs);
   if (policy_ec(policy))
-    tcec_gemm_fused_kernel<true><<<grid, GemmFusedCfg<true>::THREADS, GemmFusedCfg<true>::SMEM_BYTES, stream>>>(fp, map_a, map_b, map_c);
+    launch_early(tcec_gemm_fused_kernel<true>, grid, GemmFusedCfg<true>::THREADS, GemmFusedCfg<true>::SMEM_BYTES, stream, fp, map_a, map_b, map_c);
   else
-    tcec_gemm_fused_kernel<false><<<grid, GemmFusedCfg<false>::THREADS, GemmFusedCfg<false>::SMEM_BYTES, stream>>>(fp, map_a, map_b, map_c);
+    launch_early(tcec_gemm_fused_kernel<false>, grid, GemmFusedCfg<false>::THREADS, GemmFusedCfg<false>::SMEM_BYTES, stream, fp, map_a, map_b, map_c);
   return true;
 }
 
@@ -648,8 +665,8 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
 template <bool T, bool E, bool AK, bool BK>
 void launch_direct_as(const GemmDirectParams& dp, int grid, cudaStream_t stream) {
   using Cfg = GemmDirectCfg<T, E>;
-  if (dp.slot == 128) tcec_gemm_direct_kernel<T, E, AK, BK, 64><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(dp);
-  else tcec_gemm_direct_kernel<T, E, AK, BK, 32><<<grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream>>>(dp);
+  if (dp.slot == 128) launch_early(tcec_gemm_direct_kernel<T, E, AK, BK, 64>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, dp);
+  else launch_early(tcec_gemm_direct_kernel<T, E, AK, BK, 32>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, dp);
 }
 template <bool T, bool E>
 void launch_direct(const GemmDirectParams& dp, int grid, cudaStream_t stream) {

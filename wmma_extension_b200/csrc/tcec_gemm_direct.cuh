@@ -115,13 +115,13 @@ __device__ __forceinline__ void loader_setup(LoaderOperand& v, const DirectOpera
       const int u = 2 * w + i, r = (u & 3) * 32 + lane, chunk = u >> 2;
       const int matrix = min(first_matrix + (r >> slot_log2), batch - 1), row = min(row_tile + (r & in_slot), o.rows - 1);
       const float* base = o.array ? o.array[matrix] : o.base + matrix * o.batch_stride;
-      base += static_cast<long long>(chunk * 8) * o.ld + row;
+      base = after_wait(base) + static_cast<long long>(chunk * 8) * o.ld + row;
       if (i == 0) v.p = base;
       else v.p1 = base;
     }
   } else {
     const int r0 = w * 16, matrix = min(first_matrix + (r0 >> slot_log2), batch - 1), row0 = row_tile + (r0 & in_slot);
-    const float* base = o.array ? o.array[matrix] : o.base + matrix * o.batch_stride;
+    const float* base = after_wait(o.array ? o.array[matrix] : o.base + matrix * o.batch_stride);
     v.vec4 = o.ld % 4 == 0 && (reinterpret_cast<uintptr_t>(base) & 15) == 0;
     const int r = min(row0 + (v.vec4 ? lane >> 3 : lane >> 4), o.rows - 1);
     v.rows = o.rows - r;
@@ -316,6 +316,8 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;  // main buffers at +0 and +128, correction buffers at +256 and +384
   volatile uint32_t* abortp = &abort_flag;
+  let_next_launch_start();
+  wait_for_launch_before();
 
   if (warp >= 12) {
     // ------------------------------------------------------------ loaders

@@ -136,6 +136,7 @@ struct TableShape {
 __global__ void tcec_table_maps_kernel(const float* const* a_array, const float* const* b_array, int batch,
                                        const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                        CUtensorMap* maps, unsigned int* bad, const TableShape t) {
+  let_next_launch_start();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x) {
     const float* pa = a_array[i];
     const float* pb = b_array[i];
@@ -220,7 +221,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
                            const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_c) {
   using Cfg = GemmFusedCfg<kEc>;
   constexpr int NST = Cfg::NST, BN = Cfg::BN;
-  if (p.table_bad && *p.table_bad != 0) return;  // every CTA of the launch, before anything is set up
+  if (p.table_bad) {
+    wait_for_launch_before();
+    if (*p.table_bad != 0) return;  // every CTA of the launch, before anything is set up
+  }
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_landed[NST], bar_conv[NST], bar_full[NST], bar_empty[NST];
   __shared__ uint64_t bar_main_full, bar_main_free, bar_corr_full, bar_corr_free, bar_drain[2];
@@ -267,6 +271,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(GemmFusedCfg<kEc>::T
   const uint32_t tmem_main = tmem_base_s;
   const uint32_t tmem_corr = tmem_base_s + BN;
   volatile uint32_t* abortp = &abort_flag;
+  let_next_launch_start();
+  wait_for_launch_before();
 
   if (warp >= 4 + Cfg::EPI_WARPS) {
     // ------------------------------------------------------------ converters

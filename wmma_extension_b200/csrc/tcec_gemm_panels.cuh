@@ -179,7 +179,10 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
     tcec_gemm_panels_kernel(const GemmPanelParams p) {
   using Cfg = GemmPanelCfg<BN, kTf32, kEc>;
   constexpr int NST = Cfg::NST;
-  if (p.only_if && *p.only_if == 0) return;
+  if (p.only_if) {
+    wait_for_launch_before();
+    if (*p.only_if == 0) return;
+  }
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[NST], bar_empty[NST];
   __shared__ uint64_t bar_main_full, bar_main_free, bar_corr_full, bar_corr_free, bar_drain[2];
@@ -221,6 +224,8 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
   const uint32_t tmem_main = tmem_base_s;
   const uint32_t tmem_corr = tmem_base_s + BN;
   volatile uint32_t* abortp = &abort_flag;
+  let_next_launch_start();
+  wait_for_launch_before();
 
   if (warp < 4) {
     if constexpr (Cfg::REBALANCE) setmaxnreg_dec<Cfg::REGS_CONTROL>();

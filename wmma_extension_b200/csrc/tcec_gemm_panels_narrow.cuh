@@ -39,7 +39,10 @@ template <int BN, bool kTf32, bool kEc>
 __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_panels_narrow_kernel(const GemmPanelParams p) {
   using Cfg = GemmNarrowCfg<BN, kEc>;
   constexpr int NST = Cfg::NST;
-  if (p.only_if && *p.only_if == 0) return;
+  if (p.only_if) {
+    wait_for_launch_before();
+    if (*p.only_if == 0) return;
+  }
   extern __shared__ uint8_t smem_raw[];
   __shared__ uint64_t bar_full[NST], bar_empty[NST];
   __shared__ uint64_t bar_main_full[2], bar_main_free[2], bar_corr_full[2], bar_corr_free[2], bar_drain[2];
@@ -75,6 +78,8 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;  // main buffers at +0 and +128, correction buffers at +256 and +384
   volatile uint32_t* abortp = &abort_flag;
+  let_next_launch_start();
+  wait_for_launch_before();
 
   if (warp == 0) {
     // ------------------------------------------------------------ producer

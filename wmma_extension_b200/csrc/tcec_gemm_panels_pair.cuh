@@ -104,7 +104,10 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   static_assert(BN == 256 || BN == 128, "whole or half-width pair tiles");
   using Cfg = GemmPairCfg<kTf32, kEc>;
   constexpr int NST = Cfg::NST;
-  if (p.only_if && *p.only_if == 0) return;
+  if (p.only_if) {
+    wait_for_launch_before();
+    if (*p.only_if == 0) return;
+  }
   constexpr int HALVES = 256 / BN;            // work items per pair tile
   constexpr int NC = BN / 2;                  // columns per epilogue warp
   constexpr int B_PIECE = kPanelBytes / HALVES;  // bytes of one B image (hi or lo) per CTA and K block
@@ -149,6 +152,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   const uint32_t tmem_main = tmem_base_s;
   const uint32_t tmem_corr = tmem_base_s + 256;
   volatile uint32_t* abortp = &abort_flag;
+  let_next_launch_start();
+  wait_for_launch_before();
   // What the leader's two MMA threads need (tcec_gemm_roles.cuh): M = 256 across the pair.
   OperandImage im;
   im.dconst = umma_desc_kmajor_noswizzle(0, 128, 512);

@@ -19,6 +19,8 @@
 
 #include <cstdint>
 
+#include "sm100_ptx.cuh"
+
 namespace tcec_sm100 {
 
 constexpr int kPanelRows = 128;
@@ -204,6 +206,7 @@ __device__ __forceinline__ void split_complex_panel(const ComplexSplitParams& p,
 template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_complex_kernel(const ComplexSplitParams pa, const ComplexSplitParams pb,
                                                                  unsigned int panels_a) {
+  let_next_launch_start();
   const bool second = blockIdx.x >= panels_a;
   const ComplexSplitParams& p = second ? pb : pa;
   const unsigned int i = second ? blockIdx.x - panels_a : blockIdx.x;
@@ -213,6 +216,7 @@ __global__ void __launch_bounds__(256) tcec_split_complex_kernel(const ComplexSp
 // grid = (nkb, row_blocks, batch), 256 threads: one CTA writes one hi(+lo) panel.
 template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_panels_kernel(const SplitParams p) {
+  let_next_launch_start();
   split_one_panel<kTf32, kEc>(p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -233,6 +237,7 @@ __device__ __forceinline__ void split_panel_of_both(const SplitParams& pa, const
 template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_both_kernel(const SplitParams pa, const SplitParams pb,
                                                               unsigned int panels_a) {
+  let_next_launch_start();
   split_panel_of_both<kTf32, kEc>(pa, pb, panels_a, blockIdx.x);
 }
 
@@ -245,6 +250,7 @@ template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_both_gated_kernel(const SplitParams pa, const SplitParams pb,
                                                                     unsigned int panels_a, unsigned int panels,
                                                                     unsigned int* gate) {
+  let_next_launch_start();
   if (*gate == 0) return;
   __shared__ unsigned int next[2];
   int turn = 0;
