@@ -296,6 +296,12 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                128 x 32, 64 or 128 (64 x 4096 x 4096 on packed operands: 82 -> 34 us with the packing of A);
  *                0 = never; 32, 64, 128 = that width.  Only while "cta_pair" and "tile_n" are automatic,
  *                "store_turn" is 1 and "static_tiles" 0.  Same results bit for bit.
+ *   "k_parts"    -1 (default) = a single product of k >= 1200 with more than one 128 x 128 tile, but so few
+ *                that 2, 4 or 8 SMs can share each of them, divides K among these (64 x 4096 x 4096 on packed operands: 27 -> 16 us without the packing).  The parts are
+ *                added in FP32, in the order of K; the error against FP64 is no larger, the last bits are others than those of an
+ *                undivided call.  1 = never (every kernel gives the same bits); 2, 4, 8 = that many where they have
+ *                room.  Only while "narrow_tiles" and "promote_k" are automatic, "reserve_sms" is 0, and under the
+ *                conditions of "narrow_tiles".
  *   "direct_kernel" one launch that reads FP32 operands of any layout, alignment and batch form with
  *                ordinary loads and splits them on the way into shared memory; bit-identical
  *                results.  -1 (default) = for matrices with m, n <= 128, unless they are few and their K long (one

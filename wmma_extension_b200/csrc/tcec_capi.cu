@@ -60,15 +60,40 @@ cudaError_t set_direct_smem_attrs() {
 
 template <bool T, bool E>
 cudaError_t set_narrow_smem_attr() {
-  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<32, T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<32, T, E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        GemmNarrowCfg<32, E>::SMEM_BYTES);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<64, T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<64, T, E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              GemmNarrowCfg<64, E>::SMEM_BYTES);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<128, T, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<128, T, E, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              GemmNarrowCfg<128, E>::SMEM_BYTES);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(tcec_gemm_panels_narrow_kernel<128, T, E, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             GemmNarrowCfg<128, E, true>::SMEM_BYTES);
   return e;
+}
+
+// How many clusters of 2, 4 and 8 CTAs of the divided narrow kernel run at a time; what GPCs of 16 to 20 SMs hold differs from one
+// GPU to the next.  (Every policy's kernel takes a whole SM.)  Allocates nothing.
+void count_cluster_slots(int (&slots)[3]) {
+  using Cfg = GemmNarrowCfg<128, true, true>;
+  for (int i = 0; i < 3; ++i) {
+    cudaLaunchAttribute cluster{};
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = 2u << i;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(2u << i);
+    config.blockDim = dim3(Cfg::THREADS);
+    config.dynamicSmemBytes = Cfg::SMEM_BYTES;
+    config.attrs = &cluster;
+    config.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&slots[i], tcec_gemm_panels_narrow_kernel<128, false, true, true>, &config) != cudaSuccess) {
+      slots[i] = 0;  // K is then never divided that way
+      cudaGetLastError();
+    }
+  }
 }
 
 template <bool T, bool E>
@@ -113,6 +138,7 @@ int get_device_state(DeviceState** out) {
     TCEC_CUDA((set_direct_smem_attrs<false, false>()));
     TCEC_CUDA((set_direct_smem_attrs<true, true>()));
     TCEC_CUDA((set_direct_smem_attrs<true, false>()));
+    count_cluster_slots(st.cluster_slots);
     if (cudaMalloc(&st.status, kStatusBytes + kPaceSlots * kPaceSlotBytes) != cudaSuccess) return TCEC_ERR_ALLOC;
     TCEC_CUDA(cudaMemset(st.status, 0, kStatusBytes + kPaceSlots * kPaceSlotBytes));
     st.pace = reinterpret_cast<unsigned int*>(st.status) + kStatusBytes / sizeof(unsigned int);
@@ -253,19 +279,28 @@ __global__ void split_flat_kernel(const float* __restrict__ in, float* hi, float
 
 // Launches `kernel`, which waits for the kernel before it on the stream by itself (wait_for_launch_before), so that it may be set up
 // while that one ends.
+// cluster > 0: in clusters of so many CTAs.
 template <class... Params, class... Args>
-void launch_early(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
-  cudaLaunchAttribute early{};
-  early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  early.val.programmaticStreamSerializationAllowed = 1;
+void launch_clusters(void (*kernel)(Params...), int cluster, int grid, int threads, size_t smem, cudaStream_t stream,
+                     const Args&... args) {
+  cudaLaunchAttribute attrs[2] = {};
+  attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attrs[0].val.programmaticStreamSerializationAllowed = 1;
+  attrs[1].id = cudaLaunchAttributeClusterDimension;
+  attrs[1].val.clusterDim.x = cluster;
+  attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t config{};
   config.gridDim = dim3(grid);
   config.blockDim = dim3(threads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
-  config.attrs = &early;
-  config.numAttrs = 1;
+  config.attrs = attrs;
+  config.numAttrs = cluster > 0 ? 2 : 1;
   cudaLaunchKernelEx(&config, kernel, Params(args)...);
+}
+template <class... Params, class... Args>
+void launch_early(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+  launch_clusters(kernel, 0, grid, threads, smem, stream, args...);
 }
 
 template <bool T, bool E>
@@ -292,11 +327,14 @@ void launch_gemm(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
 template <int BN, bool T, bool E>
 void launch_narrow(const GemmPanelParams& gp, int grid, cudaStream_t stream) {
   using Cfg = GemmNarrowCfg<BN, E>;
-  launch_early(tcec_gemm_panels_narrow_kernel<BN, T, E>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, gp);
+  launch_early(tcec_gemm_panels_narrow_kernel<BN, T, E, false>, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, gp);
 }
 template <bool T, bool E>
-void launch_narrow_as(int width, const GemmPanelParams& gp, int grid, cudaStream_t stream) {
-  if (width == 32) launch_narrow<32, T, E>(gp, grid, stream);
+void launch_narrow_as(int width, int k_parts, const GemmPanelParams& gp, int grid, cudaStream_t stream) {
+  if (k_parts > 1) {  // a cluster per tile
+    using Cfg = GemmNarrowCfg<128, E, true>;
+    launch_clusters(tcec_gemm_panels_narrow_kernel<128, T, E, true>, k_parts, grid, Cfg::THREADS, Cfg::SMEM_BYTES, stream, gp);
+  } else if (width == 32) launch_narrow<32, T, E>(gp, grid, stream);
   else if (width == 64) launch_narrow<64, T, E>(gp, grid, stream);
   else launch_narrow<128, T, E>(gp, grid, stream);
 }
@@ -409,17 +447,21 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
   // Options that ask for one of the wide kernels, or for something only they do, are obeyed there.
   if (!ex.force_one_sm && !ex.row_ready && !ex.sched && opt.cta_pair == -1 && opt.tile_n == 0 && opt.store_turn &&
       !opt.static_tiles && !(opt.debug_flags & ~64) && opt.narrow_tiles != 0) {
-    const int width = opt.narrow_tiles > 0 ? opt.narrow_tiles
+    const int k_parts = opt.narrow_tiles > 0 || reserve > 0 || opt.promote_k >= 0
+                            ? 1
+                            : divide_k(m, n, k, batch, s.nkb, ec, st->cluster_slots, opt.k_parts);
+    const int width = k_parts > 1             ? 128
+                      : opt.narrow_tiles > 0 ? opt.narrow_tiles
                                            : panel_choice(m, n, batch, s.nkb, gp.promo, ec, s.tile_n, sms,
                                                           want_pair && s.tile_n == 256 && m > 128).width;
     const long long ntiles = static_cast<long long>(s.tiles_m) * ((n + width - 1) / (width ? width : 1)) * batch;
     if (width && ntiles <= 0x3fffffffll) {
       gp.tiles_n = (n + width - 1) / width;
-      const int grid = static_cast<int>(ntiles < sms ? ntiles : sms);
-      if (tf32 && ec) launch_narrow_as<true, true>(width, gp, grid, stream);
-      else if (tf32) launch_narrow_as<true, false>(width, gp, grid, stream);
-      else if (ec) launch_narrow_as<false, true>(width, gp, grid, stream);
-      else launch_narrow_as<false, false>(width, gp, grid, stream);
+      const int grid = k_parts > 1 ? static_cast<int>(ntiles) * k_parts : static_cast<int>(ntiles < sms ? ntiles : sms);
+      if (tf32 && ec) launch_narrow_as<true, true>(width, k_parts, gp, grid, stream);
+      else if (tf32) launch_narrow_as<true, false>(width, k_parts, gp, grid, stream);
+      else if (ec) launch_narrow_as<false, true>(width, k_parts, gp, grid, stream);
+      else launch_narrow_as<false, false>(width, k_parts, gp, grid, stream);
       return TCEC_OK;
     }
   }
@@ -1145,6 +1187,7 @@ struct OptionEntry {
 bool any_value(int) { return true; }
 bool tile_value(int v) { return v == 0 || v == 128 || v == 256; }
 bool narrow_value(int v) { return v <= 0 || v == 32 || v == 64 || v == 128; }
+bool k_parts_value(int v) { return v == -1 || v == 1 || v == 2 || v == 4 || v == 8; }
 bool panel_rows_value(int v) { return v % 256 == 0; }
 const OptionEntry kOptions[] = {
     {"promote_k", &Options::promote_k, -1, 0x7fffffff, any_value},
@@ -1153,6 +1196,7 @@ const OptionEntry kOptions[] = {
     {"half_tiles", &Options::half_tiles, 0, 1, any_value},
     {"path", &Options::path, 0, 2, any_value},
     {"narrow_tiles", &Options::narrow_tiles, -1, 128, narrow_value},
+    {"k_parts", &Options::k_parts, -1, 8, k_parts_value},
     {"direct_kernel", &Options::direct_kernel, -1, 1, any_value},
     {"store_turn", &Options::store_turn, 0, 1, any_value},
     {"reserve_sms", &Options::reserve_sms, 0, 64, any_value},
@@ -1262,6 +1306,7 @@ struct StaticDevice {
   int* status = nullptr;
   unsigned int* sched = nullptr;
   int sm_count = 0;
+  int cluster_slots[3] = {};
 };
 StaticDevice g_static_dev[kMaxStaticDevices];  // fixed table: nothing is allocated on the host either
 
@@ -1301,6 +1346,7 @@ int static_device_state(StaticDevice** out) {
     TCEC_CUDA((set_narrow_smem_attr<true, false>()));
     TCEC_CUDA((set_narrow_smem_attr<true, true>()));
     TCEC_CUDA((set_pair_smem_attr<true, true>()));
+    count_cluster_slots(sd.cluster_slots);
     sd.ready = true;
   }
   *out = &sd;
@@ -1346,6 +1392,7 @@ int tcec_sgemm_static(int layout_a, int layout_b, int layout_c, int m, int n, in
   DeviceState view;  // launch parameters only; owns nothing
   view.status = sd->status;
   view.sm_count = sd->sm_count;
+  memcpy(view.cluster_slots, sd->cluster_slots, sizeof view.cluster_slots);
   view.sched_fixed = sd->sched;
   const int grc = gemm_packed(s, m, n, k, alpha, panels_a, 0, panels_b, 0, beta, c, nullptr, ldc, 0, layout_c, 1,
                               policy, &view, stream, opt);

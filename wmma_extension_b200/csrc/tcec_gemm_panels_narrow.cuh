@@ -1,9 +1,15 @@
 // The panel GEMM on narrow tiles (128 x BN, BN = 32, 64 or 128), one SM per tile, for calls whose 256-wide tiles are
 // too few to fill the GPU.
 //
-// Same panels, products, order and promotion interval as tcec_gemm_panels.cuh, so the same bits; K is not divided,
-// because the correction accumulates over all of it.  With 64 x 4096 x 4096 the wide kernel has 16 tiles for 148
-// SMs, this one 128.
+// Same panels, products, order and promotion interval as tcec_gemm_panels.cuh, so the same bits as long as K is not divided
+// (kSplit = false).  With 64 x 4096 x 4096 the wide kernel has 16 tiles for 148 SMs, this one 128.
+//
+// kSplit: the CTAs of a cluster share one tile and divide its K.  Every CTA walks its part like a tile of that length; the
+// results, main and correction folded, are added in the order of K through the cluster's shared memory, each CTA adding and storing
+// its share of the tile's warp blocks.  Fewer and wider tiles then fill the GPU, and what an SM takes in, which is what
+// bounds this kernel, shrinks: a K block of a 128 x 128 tile is 32 KB for four times the products of a 128 x 32 one's 20 KB.  The
+// correction, which the tensor core accumulates with truncation, covers only a part of K, so the error is no larger; the bits are
+// others than those of the undivided kernels.
 //
 // What bounds it: the copies.  A K block of a 128 x 32 tile brings 16 + 4 KB for 240 tensor cycles (an MMA with N = 32
 // takes 40 cycles, 64: 48, 128: 64), which is more than an SM takes in at 64 bytes per cycle; rows of A's panel that lie
@@ -15,7 +21,7 @@
 
 namespace tcec_sm100 {
 
-template <int BN, bool kEc>
+template <int BN, bool kEc, bool kSplit = false>
 struct GemmNarrowCfg {
   static constexpr int NP = kEc ? 2 : 1;
   static constexpr int KBS = BN == 128 ? 1 : 2;          // K blocks per stage
@@ -23,21 +29,43 @@ struct GemmNarrowCfg {
   static constexpr int B_IMAGE = BN * 64;                 // hi or lo of BN rows
   static constexpr int B_BLOCK = B_IMAGE * NP;
   static constexpr int STAGE_BYTES = KBS * (A_BLOCK + B_BLOCK);
-  static constexpr int NST_RAW = (200 * 1024) / STAGE_BYTES;
-  static constexpr int NST = NST_RAW > 8 ? 8 : NST_RAW;
   static constexpr int EPI_WARPS = BN == 32 ? 4 : 8;
   static constexpr int NC = BN == 128 ? 64 : 32;          // columns per epilogue warp
-  static constexpr int EPI_OFFSET = NST * STAGE_BYTES;
-  static constexpr int SMEM_BYTES = NST * STAGE_BYTES + EPI_WARPS * kEpiBufBytes + 1024;
+  static constexpr int PART_BYTES = 32 * NC * 4;          // divided K: what one CTA adds to one warp block
+  static constexpr int PARTS_BYTES = kSplit ? EPI_WARPS * PART_BYTES : 0;
+  static constexpr int NST_RAW = (200 * 1024 - PARTS_BYTES) / STAGE_BYTES;
+  static constexpr int NST = NST_RAW > 8 ? 8 : NST_RAW;
+  static constexpr int PARTS_OFFSET = NST * STAGE_BYTES;
+  static constexpr int EPI_OFFSET = PARTS_OFFSET + PARTS_BYTES;
+  static constexpr int SMEM_BYTES = EPI_OFFSET + EPI_WARPS * kEpiBufBytes + 1024;
   static_assert(SMEM_BYTES <= 232448 - 512, "dynamic + static shared memory exceed an SM");
   static constexpr int THREADS = 128 + 32 * EPI_WARPS;
   static constexpr int TMEM_COLS = kEc ? 512 : 256;
   static constexpr int GROUP_M = 16;
 };
 
-template <int BN, bool kTf32, bool kEc>
+// Stores one epilogue warp's 32 x NC block of a tile.
+template <class Cfg>
+__device__ __forceinline__ void store_narrow_block(const float (&acc)[Cfg::NC], const GemmPanelParams& p, const TileCoord& tc, int bn,
+                                                   int q, int col_in, uint8_t* smem_gen, int ew, int lane) {
+  StoreTarget st;
+  st.cbase = p.c_array ? p.c_array[tc.b] : p.c + tc.b * p.c_batch_stride;
+  st.ldc = p.ldc;
+  st.M = p.M;
+  st.N = p.N;
+  st.col_major = p.c_col_major;
+  st.vec_ok = !p.c_col_major && (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(st.cbase) & 15) == 0);
+  st.alpha = p.alpha;
+  st.beta = p.beta;
+  const int row0 = tc.mt * 128 + q * 32, col0 = tc.nt * bn + col_in;
+  if (row0 < p.M && col0 < p.N)
+    store_warp_block<true>(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
+}
+
+// Divided K: launched with clusters of 2, 4 or 8 CTAs, one cluster per tile.
+template <int BN, bool kTf32, bool kEc, bool kSplit>
 __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_panels_narrow_kernel(const GemmPanelParams p) {
-  using Cfg = GemmNarrowCfg<BN, kEc>;
+  using Cfg = GemmNarrowCfg<BN, kEc, kSplit>;
   constexpr int NST = Cfg::NST;
   if (p.only_if) {
     wait_for_launch_before();
@@ -53,6 +81,13 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
   uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int ntiles = p.tiles_m * p.tiles_n * p.batch;
+  // this CTA's tiles, and its part of their K in whole stages
+  const int parts = kSplit ? static_cast<int>(cluster_nctarank()) : 1, part = kSplit ? static_cast<int>(cluster_ctarank()) : 0;
+  const int first_tile = blockIdx.x / parts, stride = gridDim.x / parts;
+  const int stages = (p.nkb + Cfg::KBS - 1) / Cfg::KBS;
+  const int kb_first = kSplit ? stages * part / parts * Cfg::KBS : 0;
+  const int kb_end = kSplit ? min(p.nkb, stages * (part + 1) / parts * Cfg::KBS) : p.nkb;
+  const int nkb = kb_end - kb_first;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < NST; ++s) {
@@ -75,6 +110,7 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
   }
   tc_fence_before();
   __syncthreads();
+  if constexpr (kSplit) cluster_sync_all();  // the others' shared memory exists before anything is written to it
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;  // main buffers at +0 and +128, correction buffers at +256 and +384
   volatile uint32_t* abortp = &abort_flag;
@@ -94,14 +130,14 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
           ph ^= 1;
         }
       };
-      for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x) {
+      for (int tile = first_tile; tile < ntiles && ok; tile += stride) {
         const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
         const uint8_t* pa = p.panels_a + tc.b * p.panels_a_batch_stride + static_cast<size_t>(tc.mt) * p.nkb * Cfg::A_BLOCK;
         const int brow = tc.nt * BN;
         const uint8_t* pb = p.panels_b + tc.b * p.panels_b_batch_stride +
                             static_cast<size_t>(brow / 128) * p.nkb * (kPanelBytes * Cfg::NP) + (brow % 128) * 64;
         const int rows = (min(128, p.M - tc.mt * 128) + 7) & ~7;  // of A's panel that the matrix has, in whole groups
-        for (int kb = 0; kb < p.nkb; kb += Cfg::KBS) {
+        for (int kb = kb_first; kb < kb_end; kb += Cfg::KBS) {
           if (!mbar_wait(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 32)) {
             ok = false;
             break;
@@ -113,7 +149,7 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
           }
           const uint32_t full = smem_u32(&bar_full[s]);
           const uint32_t dst = smem_base + s * Cfg::STAGE_BYTES;
-          const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, p.nkb - kb);
+          const int nblk = Cfg::KBS == 1 ? 1 : min(Cfg::KBS, kb_end - kb);
           mbar_arrive_expect_tx(full, nblk * Cfg::NP * (rows * 64 + Cfg::B_IMAGE));
           armed |= 1u << s;
           armed_parity = (armed_parity & ~(1u << s)) | (ph << s);
@@ -150,13 +186,13 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
       im.kstep16 = 16;
       im.a_block16 = Cfg::A_BLOCK >> 4;
       im.b_block16 = Cfg::B_BLOCK >> 4;
-      int tile = static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
+      int tile = first_tile - stride;
       auto next_tile = [&](uint32_t& idesc) {
-        tile += gridDim.x;
+        tile += stride;
         idesc = umma_idesc(kTf32 ? 2u : 0u, 128, BN);
         return tile < ntiles;
       };
-      const KWalk walk{p.nkb, p.promo};
+      const KWalk walk{nkb, p.promo};
       const RingBarriers ring{bar_full, bar_empty};
       const bool ok =
           warp == 1 ? issue_main_double<kTf32, NST, Cfg::KBS>(next_tile, walk, im, tmem, ring, bar_main_full, bar_main_free, abortp)
@@ -168,10 +204,10 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
     // ------------------------------------------------------------ epilogue
     const int ew = warp - 4, q = warp & 3, col_in = (ew >> 2) * Cfg::NC;
     const uint32_t taddr = tmem + (static_cast<uint32_t>(q * 32) << 16) + col_in;
-    const int nchunks = p.promo ? (p.nkb + p.promo - 1) / p.promo : 1;
+    const int nchunks = p.promo ? (nkb + p.promo - 1) / p.promo : 1;
     uint32_t chunk = 0, tcount = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < ntiles && ok; tile += gridDim.x, ++tcount) {
+    for (int tile = first_tile; tile < ntiles && ok; tile += stride, ++tcount) {
       const TileCoord tc = decode_tile(tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
       float acc[Cfg::NC];
       for (int c = 0; c < nchunks; ++c, ++chunk) {
@@ -197,18 +233,15 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
         __syncwarp();
         if (lane == 0) mbar_arrive(smem_u32(&bar_corr_free[tcount & 1]));
       }
-      StoreTarget st;
-      st.cbase = p.c_array ? p.c_array[tc.b] : p.c + tc.b * p.c_batch_stride;
-      st.ldc = p.ldc;
-      st.M = p.M;
-      st.N = p.N;
-      st.col_major = p.c_col_major;
-      st.vec_ok = !p.c_col_major && (p.ldc % 4 == 0) && ((reinterpret_cast<uintptr_t>(st.cbase) & 15) == 0);
-      st.alpha = p.alpha;
-      st.beta = p.beta;
-      const int row0 = tc.mt * 128 + q * 32, col0 = tc.nt * BN + col_in;
-      if (row0 < p.M && col0 < p.N)
-        store_warp_block<true>(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
+      if constexpr (kSplit) {
+        // to the CTA that stores this block; four columns of the 32 rows are 512 consecutive bytes
+        const int per = Cfg::EPI_WARPS / parts;
+        const uint32_t to = map_to_cta(smem_base + Cfg::PARTS_OFFSET + (part * per + ew % per) * Cfg::PART_BYTES + lane * 16, ew / per);
+#pragma unroll
+        for (int i = 0; i < Cfg::NC; i += 4) st_cluster_v4(to + i * 128, acc[i], acc[i + 1], acc[i + 2], acc[i + 3]);
+      } else {
+        store_narrow_block<Cfg>(acc, p, tc, BN, q, col_in, smem_gen, ew, lane);
+      }
     }
     if (!ok) {
       abort_flag = 1;
@@ -219,6 +252,35 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
   tc_fence_before();
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, Cfg::TMEM_COLS);
+  if constexpr (kSplit) {
+    cluster_sync_all();  // every part has arrived
+    const int ew = warp - 4, per = Cfg::EPI_WARPS / parts;
+    if (warp >= 4 && ew / per == part) {
+      const TileCoord tc = decode_tile(first_tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
+      const float4* from = reinterpret_cast<const float4*>(smem_gen + Cfg::PARTS_OFFSET + ew % per * Cfg::PART_BYTES) + lane;
+      float acc[Cfg::NC];
+#pragma unroll
+      for (int i = 0; i < Cfg::NC; i += 4) {
+        const float4 v = from[i * 8];
+        acc[i] = v.x;
+        acc[i + 1] = v.y;
+        acc[i + 2] = v.z;
+        acc[i + 3] = v.w;
+      }
+      for (int r = 1; r < parts; ++r) {
+        from += per * (Cfg::PART_BYTES / 16);
+#pragma unroll
+        for (int i = 0; i < Cfg::NC; i += 4) {
+          const float4 v = from[i * 8];
+          acc[i] += v.x;
+          acc[i + 1] += v.y;
+          acc[i + 2] += v.z;
+          acc[i + 3] += v.w;
+        }
+      }
+      store_narrow_block<Cfg>(acc, p, tc, BN, warp & 3, (ew >> 2) * Cfg::NC, smem_gen, ew, lane);
+    }
+  }
 }
 
 }  // namespace tcec_sm100

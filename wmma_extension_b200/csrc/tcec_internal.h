@@ -32,6 +32,7 @@ struct Options {
   int half_tiles = 1;   // CTA-pair kernel: calls with very few tiles run on 256 x 128 half tiles
   int path = 0;         // 0: chosen per call, 1: always operand panels, 2: FP32-tile kernel whenever it applies
   int narrow_tiles = -1;   // panels: width of the narrow tiles (32, 64, 128) for calls with few tiles; -1: chosen per call; 0: never
+  int k_parts = -1;        // narrow tiles: CTAs that divide the K of a tile (1, 2, 4, 8); -1: chosen per call
   int direct_kernel = -1;  // -1: chosen per call from the sizes; 0: never; 1: whenever the other options allow it
   int comm_sms = 8;     // SMs the column-sharded step leaves to the broadcast (also the broadcast's CTA limit)
   int comm_panel_rows = 2048;  // rows of A per broadcast
@@ -54,6 +55,7 @@ struct StepState;
 struct DeviceState {
   int* status = nullptr;
   int sm_count = 0;
+  int cluster_slots[3] = {};  // clusters of 2, 4, 8 CTAs that run at a time (count_cluster_slots)
   bool attrs_done = false;
   std::map<cudaStream_t, Workspace> ws;
   std::map<cudaStream_t, unsigned int*> sched;  // per stream: the panel GEMM's two tile-scheduler counters
