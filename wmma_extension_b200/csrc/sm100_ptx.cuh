@@ -94,16 +94,16 @@ __device__ __forceinline__ bool mbar_wait_plain(uint32_t bar, uint32_t parity) {
 }
 
 // ---------------------------------------------------------------- programmatic dependent launch
-// The GEMM kernels are launched so that they may be set up while the kernel before them (a split, as a rule) ends: their CTAs take
-// SMs that are done, initialise barriers, allocate TMEM.  None touches global memory before this wait, which returns when the kernel
-// before has ended and what it wrote is visible.  Every thread of every such kernel comes here, whatever it does afterwards: a
-// kernel that left without would let the next one start on the results of the one before.  A short call gains 2 to 4 us: 1024^3
-// 20.3 -> 16.4, 1000 x 777 x 1111 20.5 -> 18.5.
-// The splits are launched plainly.  Their CTAs are small: let in early, all of them crowd on the SMs that the GEMM before them does
-// not use (1500 x 1400 x 300 12.3 us, 14.5 with the split early as well; 1000 x 777 x 1111 18.5, 21.4; only the smallest gain, 512^3
-// 10.3, 9.4).
+// Splits and GEMM kernels are launched so that they may be set up while the kernel before them ends: their CTAs take SMs that are
+// done, initialise barriers, allocate TMEM.  None touches global memory before this wait, which returns when the kernel before has
+// ended and what it wrote is visible.  Every thread of every such kernel comes here, whatever it does afterwards: a kernel that
+// left without would let the next one start on the results of the one before.  Calls in a row, us, plain launches against this:
+// 512^3 12.3, 8.8; 1024^3 20.3, 14.6; 1000 x 777 x 1111 20.5, 16.9; 1500 x 1400 x 300 14.4, 10.8.
 __device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// The next kernel of the stream may be set up as soon as every CTA of this one has come here (or ended).
+// The next kernel of the stream may be set up as soon as every CTA of this one has come here (or ended).  The splits call it: the
+// GEMM behind them takes whole SMs, one by one as they are done.  So do the direct and the FP32-tile kernel, which follow one
+// another.  The panel GEMMs do not: a split follows them, and its small CTAs would all crowd on the SMs that the GEMM leaves
+// idle (1000 x 777 x 1111 21.2 us, 1500 x 1400 x 300 14.1).
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The pointer as a value that the compiler does not know before the wait above: loads through it that are declared read-only
 // (__ldg) are not moved in front of the wait.

@@ -281,7 +281,7 @@ __global__ void split_flat_kernel(const float* __restrict__ in, float* hi, float
 // while that one ends.
 // cluster > 0: in clusters of so many CTAs.
 template <class... Params, class... Args>
-void launch_clusters(void (*kernel)(Params...), int cluster, int grid, int threads, size_t smem, cudaStream_t stream,
+void launch_clusters(void (*kernel)(Params...), int cluster, dim3 grid, int threads, size_t smem, cudaStream_t stream,
                      const Args&... args) {
   cudaLaunchAttribute attrs[2] = {};
   attrs[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -290,7 +290,7 @@ void launch_clusters(void (*kernel)(Params...), int cluster, int grid, int threa
   attrs[1].val.clusterDim.x = cluster;
   attrs[1].val.clusterDim.y = attrs[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t config{};
-  config.gridDim = dim3(grid);
+  config.gridDim = grid;
   config.blockDim = dim3(threads);
   config.dynamicSmemBytes = smem;
   config.stream = stream;
@@ -299,7 +299,7 @@ void launch_clusters(void (*kernel)(Params...), int cluster, int grid, int threa
   cudaLaunchKernelEx(&config, kernel, Params(args)...);
 }
 template <class... Params, class... Args>
-void launch_early(void (*kernel)(Params...), int grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
+void launch_early(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args&... args) {
   launch_clusters(kernel, 0, grid, threads, smem, stream, args...);
 }
 
@@ -313,7 +313,7 @@ void launch_split(const SplitParams& sp, int batch, cudaStream_t stream) {
     else part.src += static_cast<long long>(b0) * part.batch_stride;
     part.panels += static_cast<long long>(b0) * part.panels_batch_stride;
     dim3 grid(part.nkb, part.row_blocks, nb);
-    tcec_split_panels_kernel<T, E><<<grid, 256, 0, stream>>>(part);
+    launch_early(tcec_split_panels_kernel<T, E>, grid, 256, 0, stream, part);
   }
 }
 
@@ -394,14 +394,14 @@ void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a
   if (gate) {  // fp16 policies only
     const unsigned int most = static_cast<unsigned int>(8 * sm_count), claims = (all + kGatedPanels - 1) / kGatedPanels;
     const unsigned int grid = claims < most ? claims : most;
-    if (policy_ec(policy)) tcec_split_both_gated_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, gate);
-    else tcec_split_both_gated_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b, all, gate);
+    if (policy_ec(policy)) launch_early(tcec_split_both_gated_kernel<false, true>, grid, 256, 0, stream, pa, pb, first_b, all, gate);
+    else launch_early(tcec_split_both_gated_kernel<false, false>, grid, 256, 0, stream, pa, pb, first_b, all, gate);
   } else if (policy_tf32(policy)) {
-    if (policy_ec(policy)) tcec_split_both_kernel<true, true><<<all, 256, 0, stream>>>(pa, pb, first_b);
-    else tcec_split_both_kernel<true, false><<<all, 256, 0, stream>>>(pa, pb, first_b);
+    if (policy_ec(policy)) launch_early(tcec_split_both_kernel<true, true>, all, 256, 0, stream, pa, pb, first_b);
+    else launch_early(tcec_split_both_kernel<true, false>, all, 256, 0, stream, pa, pb, first_b);
   } else {
-    if (policy_ec(policy)) tcec_split_both_kernel<false, true><<<all, 256, 0, stream>>>(pa, pb, first_b);
-    else tcec_split_both_kernel<false, false><<<all, 256, 0, stream>>>(pa, pb, first_b);
+    if (policy_ec(policy)) launch_early(tcec_split_both_kernel<false, true>, all, 256, 0, stream, pa, pb, first_b);
+    else launch_early(tcec_split_both_kernel<false, false>, all, 256, 0, stream, pa, pb, first_b);
   }
 }
 
@@ -650,8 +650,8 @@ bool try_fused(int la, int lb, int lc, int m, int n, int k, float alpha, const f
     const bool c_row = lc == TCEC_ROW_MAJOR, more_tiles = m > 256 || n > 256;
     const TableShape shape{more_tiles ? table->c_array : nullptr, lda, ldb, ldc, a_kc ? k : m, a_kc ? m : k, b_kc ? k : n,
                            b_kc ? n : k, c_row ? n : m, c_row ? m : n};
-    tcec_table_maps_kernel<<<(batch + 127) / 128 < st->sm_count ? (batch + 127) / 128 : st->sm_count, 128, 0, stream>>>(
-        table->a_array, table->b_array, batch, map_a, map_b, table->maps, table->bad, shape);
+    launch_early(tcec_table_maps_kernel, (batch + 127) / 128 < st->sm_count ? (batch + 127) / 128 : st->sm_count, 128, 0, stream,
+                 table->a_array, table->b_array, batch, map_a, map_b, table->maps, table->bad, shape);
   } else {
     if (!a || !b || !c) return false;
     if (!tma_addressable(a, lda, stride_a, batch) || !tma_addressable(b, ldb, stride_b, batch)) return false;
@@ -992,11 +992,11 @@ int cgemm_impl(int la, int lb, int lc, int m, int n, int k, const float* alpha, 
   pa.nkb = pb.nkb = s.nkb;
   const unsigned int grid = static_cast<unsigned int>(na + nb), first_b = static_cast<unsigned int>(na);
   if (policy_tf32(policy)) {
-    if (policy_ec(policy)) tcec_split_complex_kernel<true, true><<<grid, 256, 0, stream>>>(pa, pb, first_b);
-    else tcec_split_complex_kernel<true, false><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+    if (policy_ec(policy)) launch_early(tcec_split_complex_kernel<true, true>, grid, 256, 0, stream, pa, pb, first_b);
+    else launch_early(tcec_split_complex_kernel<true, false>, grid, 256, 0, stream, pa, pb, first_b);
   } else {
-    if (policy_ec(policy)) tcec_split_complex_kernel<false, true><<<grid, 256, 0, stream>>>(pa, pb, first_b);
-    else tcec_split_complex_kernel<false, false><<<grid, 256, 0, stream>>>(pa, pb, first_b);
+    if (policy_ec(policy)) launch_early(tcec_split_complex_kernel<false, true>, grid, 256, 0, stream, pa, pb, first_b);
+    else launch_early(tcec_split_complex_kernel<false, false>, grid, 256, 0, stream, pa, pb, first_b);
   }
   {
     std::lock_guard<std::mutex> lock(g_mu);  // the per-stream tile counters may be created here

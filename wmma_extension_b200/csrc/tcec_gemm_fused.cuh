@@ -137,6 +137,7 @@ __global__ void tcec_table_maps_kernel(const float* const* a_array, const float*
                                        const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                                        CUtensorMap* maps, unsigned int* bad, const TableShape t) {
   let_next_launch_start();
+  wait_for_launch_before();
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < batch; i += gridDim.x * blockDim.x) {
     const float* pa = a_array[i];
     const float* pb = b_array[i];

@@ -114,7 +114,6 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
   tc_fence_after();
   const uint32_t tmem = tmem_base_s;  // main buffers at +0 and +128, correction buffers at +256 and +384
   volatile uint32_t* abortp = &abort_flag;
-  let_next_launch_start();
   wait_for_launch_before();
 
   if (warp == 0) {

@@ -152,7 +152,6 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   const uint32_t tmem_main = tmem_base_s;
   const uint32_t tmem_corr = tmem_base_s + 256;
   volatile uint32_t* abortp = &abort_flag;
-  let_next_launch_start();
   wait_for_launch_before();
   // What the leader's two MMA threads need (tcec_gemm_roles.cuh): M = 256 across the pair.
   OperandImage im;

@@ -95,8 +95,7 @@ template <bool kTf32, bool kEc>
 __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, int rb, int b) {
   constexpr int KCH = kTf32 ? 4 : 8;    // fp32 elements per 16-byte operand chunk
   constexpr int KOP = 4 * KCH;          // K extent of one panel
-  const float* __restrict__ src =
-      p.src_array ? p.src_array[b] : p.src + static_cast<long long>(b) * p.batch_stride;
+  const float* src = after_wait(p.src_array ? p.src_array[b] : p.src + static_cast<long long>(b) * p.batch_stride);
   uint8_t* out = p.panels + static_cast<long long>(b) * p.panels_batch_stride +
                  (static_cast<size_t>(rb) * p.nkb + kb) * (kEc ? 2 : 1) * kPanelBytes;
   const int k0 = kb * KOP;
@@ -170,13 +169,14 @@ __device__ __forceinline__ void split_complex_panel(const ComplexSplitParams& p,
   constexpr int PC = kTf32 ? 2 : 4;  // complex elements per 16-byte operand chunk
   uint8_t* out = p.panels + (static_cast<size_t>(rb) * p.nkb + kb) * (kEc ? 2 : 1) * kPanelBytes;
   const int R = p.doubled ? 64 : 128;  // complex rows of this panel
-  const bool pairs = (reinterpret_cast<uintptr_t>(p.src) & 7) == 0;
+  const float* const src = after_wait(p.src);
+  const bool pairs = (reinterpret_cast<uintptr_t>(src) & 7) == 0;
   for (int item = threadIdx.x; item < R * 4; item += 256) {
     const int r = p.k_contiguous ? item >> 2 : item % R, c = p.k_contiguous ? item & 3 : item / R;
     const int row = rb * R + r, k0 = (kb * 4 + c) * PC;
     const long long step = p.k_contiguous ? 1 : p.ld;
     const float* q =
-        p.src + 2 * (p.k_contiguous ? static_cast<long long>(row) * p.ld + k0 : static_cast<long long>(k0) * p.ld + row);
+        src + 2 * (p.k_contiguous ? static_cast<long long>(row) * p.ld + k0 : static_cast<long long>(k0) * p.ld + row);
     float2 z[PC];
 #pragma unroll
     for (int e = 0; e < PC; ++e) {
@@ -207,6 +207,7 @@ template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_complex_kernel(const ComplexSplitParams pa, const ComplexSplitParams pb,
                                                                  unsigned int panels_a) {
   let_next_launch_start();
+  wait_for_launch_before();
   const bool second = blockIdx.x >= panels_a;
   const ComplexSplitParams& p = second ? pb : pa;
   const unsigned int i = second ? blockIdx.x - panels_a : blockIdx.x;
@@ -217,6 +218,7 @@ __global__ void __launch_bounds__(256) tcec_split_complex_kernel(const ComplexSp
 template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_panels_kernel(const SplitParams p) {
   let_next_launch_start();
+  wait_for_launch_before();
   split_one_panel<kTf32, kEc>(p, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
@@ -238,6 +240,7 @@ template <bool kTf32, bool kEc>
 __global__ void __launch_bounds__(256) tcec_split_both_kernel(const SplitParams pa, const SplitParams pb,
                                                               unsigned int panels_a) {
   let_next_launch_start();
+  wait_for_launch_before();
   split_panel_of_both<kTf32, kEc>(pa, pb, panels_a, blockIdx.x);
 }
 
@@ -251,6 +254,7 @@ __global__ void __launch_bounds__(256) tcec_split_both_gated_kernel(const SplitP
                                                                     unsigned int panels_a, unsigned int panels,
                                                                     unsigned int* gate) {
   let_next_launch_start();
+  wait_for_launch_before();
   if (*gate == 0) return;
   __shared__ unsigned int next[2];
   int turn = 0;
