@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       }
     };
     auto stage_free = [&]() {
-      if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 32)) return false;
+      if (!mbar_wait_warp(smem_u32(&bar_empty[s]), ph ^ 1, abortp, 0)) return false;
       mbar_try_wait(smem_u32(&bar_empty[s]), ph ^ 1);  // each lane observes the completed phase itself
       return true;
     };
@@ -470,7 +470,7 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       const DirectTile t = direct_tile(p, tile);
       float acc[NC];
       for (int c = 0; c < nchunks; ++c, ++chunk) {
-        if (!mbar_wait_warp(smem_u32(&bar_main_full[chunk & 1]), (chunk >> 1) & 1, abortp, 32)) {
+        if (!mbar_wait_warp(smem_u32(&bar_main_full[chunk & 1]), (chunk >> 1) & 1, abortp, 0)) {
           ok = false;
           break;
         }
@@ -482,7 +482,7 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       }
       if (!ok) break;
       if constexpr (kEc) {
-        if (!mbar_wait_warp(smem_u32(&bar_corr_full[tcount & 1]), (tcount >> 1) & 1, abortp, 32)) {
+        if (!mbar_wait_warp(smem_u32(&bar_corr_full[tcount & 1]), (tcount >> 1) & 1, abortp, 0)) {
           ok = false;
           break;
         }

@@ -231,7 +231,7 @@ __device__ __forceinline__ bool issue_main_double(NextTile next_tile, const KWal
   while (next_tile(idesc)) {
     int left = 0;  // K blocks still to issue in the current chunk
     for (int kb0 = 0; kb0 < w.nkb; kb0 += kBlocks) {
-      if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 20)) return false;
+      if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 0)) return false;
 #pragma unroll
       for (int i = 0; i < kBlocks; ++i) {
         const int kb = kb0 + i;
@@ -272,7 +272,7 @@ __device__ __forceinline__ bool issue_corr_double(NextTile next_tile, const KWal
     const uint32_t d = tmem_corr + (tcount & 1) * kDoubleCols;
     if (!mbar_wait(smem_u32(&corr_free[tcount & 1]), ((tcount >> 1) & 1) ^ 1, abortp, 0)) return false;
     for (int kb0 = 0; kb0 < w.nkb; kb0 += kBlocks) {
-      if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 20)) return false;
+      if (!mbar_wait(smem_u32(&ring.full[s]), ph, abortp, 0)) return false;
       tc_fence_after();
 #pragma unroll
       for (int i = 0; i < kBlocks; ++i) {
