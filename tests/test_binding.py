@@ -1,0 +1,83 @@
+"""The native binding of the common calls: what it does not take falls through to the Python code, with the same errors; what it
+takes gives the same results."""
+import importlib.util
+
+import pytest
+import torch
+
+from wmma_extension_b200 import tcec
+
+DEV = "cuda:0"
+
+
+def test_it_is_built_and_leaves_other_operands_to_python():
+    assert tcec._binding is not None
+    x = torch.zeros(4, 4)
+    assert tcec._binding.sgemm(x, x, None, 1.0, 0.0, "fp16_ec") is None  # not on a GPU
+    assert tcec._binding.sgemm(x, [1], None, 1.0, 0.0, "fp16_ec") is None
+    assert tcec._binding.sgemm(x) is None
+    assert tcec._binding.strided(x, x, x, 1.0, 0.0, 9) is None
+    assert tcec._binding.pack_a(x, "no_such_policy", None) is None
+    assert tcec._binding.sgemm_packed(x, x, -1, 4, 4, None, 1.0, 0.0, 0) is None
+    with pytest.raises(TypeError):
+        tcec._binding.bind(1)
+    tcec.load()
+    for call in (lambda: tcec.sgemm(x, x), lambda: tcec.sgemm_strided_batched(x[None], x[None]), lambda: tcec.pack_a(x),
+                 lambda: tcec.pack_b(x)):
+        with pytest.raises(ValueError, match="float32 CUDA"):
+            call()
+
+
+@pytest.fixture
+def python_only():
+    """tcec.py once more, without the binding."""
+    spec = importlib.util.spec_from_file_location("tcec_python_only", tcec.__file__, submodule_search_locations=None)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)  # no package: the relative import of the binding fails
+    assert module._binding is None
+    return module
+
+
+@pytest.mark.gpu
+def test_same_results_and_errors_as_the_python_code(python_only):
+    gen = torch.Generator(device=DEV).manual_seed(1)
+    tcec.load()
+
+    def rand(*shape):
+        return torch.rand(shape, generator=gen, device=DEV).mul_(2).sub_(1)
+
+    forms = {
+        "row": lambda r, c: rand(r, c), "col": lambda r, c: rand(c, r).t(), "padded": lambda r, c: rand(r, c + 3)[:, :c],
+        "one row": lambda r, c: rand(1, c).expand(1, c), "offset": lambda r, c: rand(r + 1, c)[1:],
+    }
+    for fa in forms:
+        for fb in forms:
+            a, b = forms[fa](33, 40), forms[fb](40, 17)
+            if a.shape[1] != b.shape[0]:
+                with pytest.raises(ValueError, match="inner"):
+                    tcec.sgemm(a, b)
+                continue
+            for policy in ("fp16_ec", "tf32_ec", 2):
+                assert torch.equal(tcec.sgemm(a, b, policy=policy), python_only.sgemm(a, b, policy=policy))
+            c0 = rand(b.shape[1], a.shape[0]).t()
+            c = [c0.clone(), c0.clone()]
+            got = tcec.sgemm(a, b, c[0], alpha=0.5, beta=-1.0)
+            assert got is c[0] and torch.equal(got, python_only.sgemm(a, b, c[1], alpha=0.5, beta=-1.0))
+            pa, pb = tcec.pack_a(a), tcec.pack_b(b)
+            assert torch.equal(pa, python_only.pack_a(a)) and torch.equal(pb, python_only.pack_b(b))
+            m, n, k = a.shape[0], b.shape[1], a.shape[1]
+            assert torch.equal(tcec.sgemm_packed(pa, pb, m, n, k), python_only.sgemm_packed(pa, pb, m, n, k))
+    x, y = rand(3, 20, 30), rand(3, 9, 30).transpose(1, 2)
+    assert torch.equal(tcec.sgemm_strided_batched(x, y), python_only.sgemm_strided_batched(x, y))
+    assert tcec.sgemm(rand(0, 5), rand(5, 4)).shape == (0, 4) and tcec.sgemm(rand(4, 0), rand(0, 4)).abs().max() == 0
+    for bad in (lambda m: m.sgemm(x[0], x[0]), lambda m: m.sgemm(x[0].double(), y[0]), lambda m: m.sgemm(x[0][:, ::2], y[0][::2]),
+                lambda m: m.sgemm(x[0], y[0], policy="fp8"), lambda m: m.sgemm(x[0], y[0], policy=9),
+                lambda m: m.sgemm(x[0], y[0], torch.zeros(20, 9, dtype=torch.float64, device=DEV)),
+                lambda m: m.sgemm_strided_batched(x, y[:2]), lambda m: m.pack_a(x)):
+        raised = []
+        for module in (tcec, python_only):
+            with pytest.raises(Exception) as e:
+                bad(module)
+            raised.append((type(e.value).__name__, str(e.value)))
+        assert raised[0] == raised[1]
+    tcec.device_status()

@@ -61,6 +61,14 @@ EXPORTED_SYMBOLS = (
 
 _lib = None
 
+# The common calls in native code (csrc/tcec_binding.cpp): one 32 x 32 x 32 product, calls in a row, 10.6 -> 6.6 us, 64 rows packed
+# and multiplied by packed 4096 x 4096 24.6 -> 22.7.  It answers None to whatever is not plain float32 CUDA tensors of the current
+# device, and the code here takes the call.
+try:
+    from . import _binding
+except ImportError:  # not built, or built for another torch: this file does it all
+    _binding = None
+
 
 class TcecError(RuntimeError):
     def __init__(self, status: int, what: str):
@@ -145,6 +153,10 @@ def load() -> ctypes.CDLL:
     lib.tcec_version.argtypes = []
     lib.tcec_version.restype = ctypes.c_char_p
     _lib = lib
+    if _binding is not None:
+        _binding.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (
+            lib.tcec_sgemm, lib.tcec_sgemm_strided_batched, lib.tcec_pack_a, lib.tcec_pack_b, lib.tcec_sgemm_packed,
+            lib.tcec_packed_bytes)))
     return lib
 
 
@@ -155,6 +167,13 @@ def status_string(status: int) -> str:
 def _check(status: int, what: str) -> None:
     if status != OK:
         raise TcecError(status, what)
+
+
+def _answer(done, what: str) -> torch.Tensor:
+    """What _binding returned: the result, or a status."""
+    if done.__class__ is int:
+        raise TcecError(done, what)
+    return done
 
 
 def _policy(policy) -> int:
@@ -221,6 +240,10 @@ def device_status() -> int:
 def sgemm(a: torch.Tensor, b: torch.Tensor, c: Optional[torch.Tensor] = None, *, alpha: float = 1.0,
           beta: float = 0.0, policy="fp16_ec") -> torch.Tensor:
     """C = alpha * A @ B + beta * C for 2-D float32 CUDA tensors (row- or column-major views)."""
+    if _binding is not None and _lib is not None:
+        done = _binding.sgemm(a, b, c, alpha, beta, policy)
+        if done is not None:
+            return _answer(done, "tcec_sgemm")
     _require_cuda_f32(a, b)
     m, k = a.shape
     k2, n = b.shape
@@ -299,6 +322,10 @@ def static_status() -> int:
 def sgemm_strided_batched(a: torch.Tensor, b: torch.Tensor, c: Optional[torch.Tensor] = None, *,
                           alpha: float = 1.0, beta: float = 0.0, policy="fp16_ec") -> torch.Tensor:
     """Batched product of 3-D tensors [batch, m, k] x [batch, k, n] with a uniform batch stride."""
+    if _binding is not None and _lib is not None:
+        done = _binding.strided(a, b, c, alpha, beta, policy)
+        if done is not None:
+            return _answer(done, "tcec_sgemm_strided_batched")
     _require_cuda_f32(a, b)
     batch, m, k = a.shape
     _, k2, n = b.shape
@@ -356,6 +383,10 @@ def packed_row_offset(row: int, k: int, policy="fp16_ec") -> int:
 
 def pack_a(a: torch.Tensor, policy="fp16_ec", out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Split A (m x k) once into operand panels; returns the uint8 panel buffer."""
+    if _binding is not None and _lib is not None:
+        done = _binding.pack_a(a, policy, out)
+        if done is not None:
+            return _answer(done, "tcec_pack_a")
     _require_cuda_f32(a)
     m, k = a.shape
     la, lda = _layout_ld(a)
@@ -369,6 +400,10 @@ def pack_a(a: torch.Tensor, policy="fp16_ec", out: Optional[torch.Tensor] = None
 
 def pack_b(b: torch.Tensor, policy="fp16_ec", out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Split B (k x n) once into operand panels; returns the uint8 panel buffer."""
+    if _binding is not None and _lib is not None:
+        done = _binding.pack_b(b, policy, out)
+        if done is not None:
+            return _answer(done, "tcec_pack_b")
     _require_cuda_f32(b)
     k, n = b.shape
     lb, ldb = _layout_ld(b)
@@ -384,6 +419,10 @@ def sgemm_packed(a_packed: torch.Tensor, b_packed: torch.Tensor, m: int, n: int,
                  c: Optional[torch.Tensor] = None, *, alpha: float = 1.0, beta: float = 0.0,
                  policy="fp16_ec") -> torch.Tensor:
     """C = alpha * A @ B + beta * C on operands packed by pack_a / pack_b."""
+    if _binding is not None and _lib is not None:
+        done = _binding.sgemm_packed(a_packed, b_packed, m, n, k, c, alpha, beta, policy)
+        if done is not None:
+            return _answer(done, "tcec_sgemm_packed")
     if c is None:
         c = torch.empty((m, n), dtype=torch.float32, device=a_packed.device)
     _require_cuda_f32(c)
