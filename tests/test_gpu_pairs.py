@@ -26,10 +26,10 @@ def _one_sm(a, b, policy):
     return want
 
 
-# 80 and more tiles on at most 74 pairs, panels of a wave just above 100 MB; ragged sizes; K that is no multiple of what a count covers
+# four rounds of tiles and more on 74 pairs, panels of a wave just above 100 MB; ragged sizes; K that is no multiple of what a count covers
 @pytest.mark.parametrize("m,n,k,policy", [
-    (2048, 2560, 5472, "fp16_ec"), (2000, 2390, 5999, "fp16_ec"), (5000, 4700, 5441, "fp16_ec"), (2048, 2560, 2800, "tf32_ec"),
-    (2048, 2560, 11000, "fp16_no_ec"),
+    (5120, 4096, 5472, "fp16_ec"), (5000, 4090, 5999, "fp16_ec"), (9000, 2390, 5541, "fp16_ec"), (5120, 4096, 2800, "tf32_ec"),
+    (5120, 4096, 11000, "fp16_no_ec"),
 ])
 def test_paced_pairs_have_the_bits_of_single_sms(m, n, k, policy):
     a, b = _operands(m, n, k, m + k)
@@ -41,7 +41,7 @@ def test_paced_pairs_have_the_bits_of_single_sms(m, n, k, policy):
 
 def test_paced_launches_overlap_on_streams_and_in_a_replayed_graph():
     """A graph replayed beside calls on the stream it was captured on shares that stream's word; a 64th stream has none."""
-    a, b = _operands(2048, 2560, 5472, 7)
+    a, b = _operands(5120, 4096, 5472, 7)
     want = _one_sm(a, b, "fp16_ec")
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in range(4)]

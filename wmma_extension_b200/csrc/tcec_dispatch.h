@@ -23,12 +23,13 @@ inline bool pairs_pay(int m, int n, int k, int batch, bool ec) {
 }
 
 // Pair tiles are taken in groups of kPairGroupM tile rows, column by column.  A launch is paced (tcec_gemm_panels_pair.cuh) if it
-// has more tiles than pairs, so that they get out of step, and the panels that one wave of tiles reads do not stay in L2 (126 MB)
-// all the while.  Unpaced and paced, ms: 16384^3 (290 MB) 21.5, 19.3; 12000 x 4000 x 12000 (212 MB) 2.79, 2.70; 8192^3 (145 MB) 2.46,
-// 2.44; without correction 16384^3 (145 MB) 7.9, 7.3, but 8192^3 (72 MB) 0.912, 0.925.
+// has several rounds of tiles, over which they get out of step, and the panels that one wave of tiles reads do not stay in L2 (126
+// MB) all the while.  Unpaced and paced, ms: 16384^3 (290 MB) 21.5, 19.3; 12000 x 4000 x 12000 (212 MB) 2.79, 2.70; 8192^3 (145 MB) 2.46,
+// 2.44; without correction 16384^3 (145 MB) 7.9, 7.3, but 8192^3 (72 MB) 0.912, 0.925.  Two
+// rounds do not earn the clearing of the word between split and GEMM (tf32 534 x 8189 x 1828, 105 MB: 147.6, 148.7 us).
 constexpr int kPairGroupM = 8;
 inline bool pace_pays(int tiles_m, int tiles_n, int batch, int nkb, int images, int pairs) {
-  if (static_cast<long long>(tiles_m) * tiles_n * batch <= pairs) return false;
+  if (static_cast<long long>(tiles_m) * tiles_n * batch < 4 * pairs) return false;
   const long long rows = tiles_m < kPairGroupM ? tiles_m : kPairGroupM, wave = ceil_div(pairs, rows), cols = tiles_n < wave ? tiles_n : wave;
   return static_cast<double>(rows + cols) * 256 * 64 * images * nkb >= 100e6;
 }
