@@ -11,6 +11,8 @@
 #pragma once
 #include <cstdint>
 
+#include "sm100_ptx.cuh"
+
 namespace tcec_sm100 {
 
 struct StoreTarget {
@@ -133,6 +135,58 @@ __device__ __forceinline__ void store_turned(const float* src, int src_step, flo
   }
 }
 
+// The two ways below are the direct kernel's.  Its warps share the SM's instruction cache with loaders and MMA issuers and waited for
+// instructions more than for anything else: they are short loops, with 32-bit shared addresses, and rows of C that are 16-byte
+// aligned go through the buffer in 128-bit pieces.  us, unrolled with a predicate per element and like this: 16384 x 64^3 182, 171;
+// 16384 x 32^3 72, 55; 4096 x 128^3 200, 183; 3000 x 127^3 217, 163; 2000 x 100^3 117, 94; one 32^3 6.4, 4.7.  The FP32-tile
+// kernel, whose C leaves by TMA or column-major, gains nothing; the panel kernels, whose code would hold both ways four times,
+// lose (300 x 201^3 87.2, 89.8).
+// A lane's column of a 32 x 32 block in the turn buffer, row pitch 33 floats: `rows` rows of the matrix (at most 32), from `src`, to
+// `dst` on every `ldc`.
+__device__ __forceinline__ void store_column(uint32_t src, float* dst, int rows, const StoreTarget& t) {
+  if (rows > 32) rows = 32;
+  if (t.beta == 0.f) {
+#pragma unroll 4
+    for (int r = 0; r < rows; ++r, src += 132, dst += t.ldc) *dst = __fmul_rn(t.alpha, ld_shared_f32(src));
+  } else {
+#pragma unroll 1
+    for (int r = 0; r < rows; ++r, src += 132, dst += t.ldc) *dst = axpby(t.alpha, ld_shared_f32(src), t.beta, *dst);
+  }
+}
+
+// A whole 32-column block, `v` this lane's row of it, to `dst` (row 0, column 0 of the block), of which the matrix has `rows` rows.
+// Eight 128-bit accesses of the buffer each way instead of 32 of 32 bits.
+__device__ __forceinline__ void store_whole_block(const float* v, float* dst, int rows, const StoreTarget& t, uint32_t wbuf, int lane) {
+  const uint32_t row = wbuf + lane * 128, turn = (lane & 7) << 4;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) st_shared_v4(row + ((j << 4) ^ turn), v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+  __syncwarp();
+  int r = lane >> 3;  // row r's piece p is at 128 r + 16 (p ^ r % 8); this lane's rows are r, r + 4, ...
+  const int piece = lane & 7;
+  dst += static_cast<long long>(r) * t.ldc + 4 * piece;
+  const long long step = 4 * t.ldc;
+  if (t.beta == 0.f) {
+#pragma unroll 4
+    for (int i = 0; i < 8; ++i, r += 4, dst += step) {
+      const float4 x = ld_shared_v4(wbuf + r * 128 + ((piece ^ (r & 7)) << 4));
+      if (r < rows)
+        *reinterpret_cast<float4*>(dst) =
+            make_float4(__fmul_rn(t.alpha, x.x), __fmul_rn(t.alpha, x.y), __fmul_rn(t.alpha, x.z), __fmul_rn(t.alpha, x.w));
+    }
+  } else {
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i, r += 4, dst += step) {
+      const float4 x = ld_shared_v4(wbuf + r * 128 + ((piece ^ (r & 7)) << 4));
+      if (r < rows) {
+        const float4 old = *reinterpret_cast<const float4*>(dst);
+        *reinterpret_cast<float4*>(dst) = make_float4(axpby(t.alpha, x.x, t.beta, old.x), axpby(t.alpha, x.y, t.beta, old.y),
+                                                      axpby(t.alpha, x.z, t.beta, old.z), axpby(t.alpha, x.w, t.beta, old.w));
+      }
+    }
+  }
+  __syncwarp();
+}
+
 constexpr int kEpiBufFloats = 32 * 33;              // one warp's turn buffer
 constexpr int kEpiBufBytes = kEpiBufFloats * 4;      // 4224
 
@@ -143,7 +197,8 @@ constexpr int kEpiBufBytes = kEpiBufFloats * 4;      // 4224
 // directly, a whole 32-byte sector per store, and leaves shared memory to the MMAs' operand reads.  Panel kernels
 // (64 x 4096 x 4096 packed 34.8 -> 32.9 us, 2048^3 complex 216 -> 212, no other case slower); not the direct kernel, whose
 // loads and stores share the path (16384 x 64^3 194 -> 204), nor the FP32-tile kernel, which stores through TMA.
-template <bool kWide, int NC>
+// kPieces: the direct kernel's stores of a row-major C (above).
+template <bool kWide, bool kPieces = false, int NC>
 __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row0, int col0, const StoreTarget& t,
                                                  float* wbuf, int lane) {
   // Old values of C a lane holds at once (beta != 0).  Read one before each store, every load waited for the store before it:
@@ -203,6 +258,25 @@ __device__ __forceinline__ void store_warp_block(const float (&acc)[NC], int row
             dst += t.ldc;
           }
         }
+      }
+    }
+    return;
+  }
+  if constexpr (kPieces) {
+    const uint32_t turn = smem_u32(wbuf);
+#pragma unroll
+    for (int cc = 0; cc < NC / 32; ++cc) {
+      const int first = col0 + cc * 32;
+      if (first >= t.N) return;
+      float* const dst = t.cbase + static_cast<long long>(row0) * t.ldc + first;
+      if (t.vec_ok && first + 32 <= t.N) {
+        store_whole_block(&acc[cc * 32], dst, t.M - row0, t, turn, lane);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i) st_shared_f32(turn + lane * 132 + i * 4, acc[cc * 32 + i]);
+        __syncwarp();
+        if (first + lane < t.N) store_column(turn + lane * 4, dst + lane, t.M - row0, t);
+        __syncwarp();
       }
     }
     return;

@@ -505,7 +505,7 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       st.beta = p.beta;
       const int row0 = t.mt * 128 + row_in, col0 = t.nt * 128 + col_in;
       if (row0 < p.M && col0 < p.N)
-        store_warp_block<false>(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
+        store_warp_block<false, true>(acc, row0, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
     }
     if (!ok) {
       abort_flag = 1;
