@@ -332,6 +332,27 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       loader_setup<kAk>(oa, p.a, t.matrix, p.batch, p.slot_log2, t.mt * 128, w, lane);
       loader_setup<kBk>(ob, p.b, t.matrix, p.batch, p.slot_log2, t.nt * 128, w, lane);
     };
+    // From a tile to the CTA's next one a lane's pointers move by one and the same step in a strided batch of matrices of one tile,
+    // as long as the tile is full and 16-byte loads stay aligned: six instructions instead of a hundred per tile, in a kernel whose
+    // warps wait for instructions.  16384 x 64^3 172 -> 165 us, 10000 x 50 x 40 x 100 190 -> 179, 4096 x 128^3 176 -> 171.  (A third
+    // granule in flight, i.e. half as much loader code again, cost 16384 x 64^3 170 -> 198.)
+    const int members = 128 >> p.slot_log2, full_tiles = p.batch >> (7 - p.slot_log2);
+    const bool steady = p.tiles_m * p.tiles_n == 1 && !p.a.array && !p.b.array &&
+                        (!kAk || p.a.ld % 4 != 0 || p.a.batch_stride % 4 == 0) && (!kBk || p.b.ld % 4 != 0 || p.b.batch_stride % 4 == 0);
+    const long long step_a = static_cast<long long>(gridDim.x) * members * p.a.batch_stride;
+    const long long step_b = static_cast<long long>(gridDim.x) * members * p.b.batch_stride;
+    auto next_tile = [&]() {
+      rtile += gridDim.x;
+      if (rtile >= p.ntiles) return;
+      if (steady && rtile < full_tiles) {
+        oa.p += step_a;
+        ob.p += step_b;
+        if constexpr (!kAk) oa.p1 += step_a;
+        if constexpr (!kBk) ob.p1 += step_b;
+      } else {
+        setup();
+      }
+    };
     auto read = [&](float (&va)[16], float (&vb)[16], int& vec4) {
       if (rtile >= p.ntiles) return;
       if (rg * 32 + 32 <= p.K) {
@@ -344,8 +365,7 @@ __global__ void __launch_bounds__(GemmDirectCfg<kTf32, kEc>::THREADS, 1) tcec_ge
       vec4 = (kAk && oa.vec4 ? 1 : 0) | (kBk && ob.vec4 ? 2 : 0);
       if (++rg == ngran) {
         rg = 0;
-        rtile += gridDim.x;
-        if (rtile < p.ntiles) setup();
+        next_tile();
       }
     };
     uint32_t s = 0, ph = 0;
