@@ -385,10 +385,10 @@ def batched_extra(torch, tcec, sharded, peaks, args, rank, world, device, dist_o
             "kernel": "tcec_gemm_fused_kernel<ec> (CTA pairs)"}
 
 
-# DRAM traffic of one launch of tcec_gemm_panels_kernel<256,fp16,ec> on M = N = K = size, from ncu captures
-# (dram__bytes_read.sum + dram__bytes_write.sum; profiles/): C is written once, A's panels are read about
-# once per pass, and B's panels once per group of 2048 rows of A, because neither operand fits the L2.
-TRAFFIC_POINTS = {6144: 1.130e9, 8192: 2.535e9, 16384: 37.2e9}
+# DRAM traffic of one launch of tcec_gemm_panels_pair_kernel<fp16,ec> on M = N = K = size, from ncu captures
+# (dram__bytes_read.sum + dram__bytes_write.sum; profiles/): C is written once, and every wave of tiles reads its
+# panels about once, because neither operand fits the L2.
+TRAFFIC_POINTS = {6144: 1.129e9, 8192: 2.535e9, 16384: 20.29e9}
 
 
 def panel_gemm_traffic(size):
@@ -516,7 +516,7 @@ def run_single(args, torch, np, tcec, sharded, peaks, device):
         "frac_of_sustained_peak": achieved / (peaks["bf16_sustained"] / 3.0),
         "sustained_is": "the same with the sustained dense figure: this kernel runs ~20 ms per launch, back to back, at "
                         "the board's power cap",
-        "kernel": "tcec_gemm_panels_kernel<256,fp16,ec>", "kernel_ms": ms_k / args.steps,
+        "kernel": "tcec_gemm_panels_pair_kernel<fp16,ec,256>", "kernel_ms": ms_k / args.steps,
         "kernel_timed": "an event pair around each GEMM launch of full steps (split A, split B, GEMM) run back to back, "
                         "in a short loop (two steps) directly before and a loop directly after the timed region; the mean of the two",
         "kernel_ms_before": ms_k_before, "kernel_ms_after": ms_k_after}

@@ -257,13 +257,12 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                the reference's mma_rn_sync uses 16 or 8 (:640-706).
  *   "tile_n"     0 = automatic, 128 or 256.
  *   "cta_pair"   256-wide tiles on pairs of SMs (tcgen05 cta_group::2: 256 x 256 tiles, each SM
- *                loads its rows of A and half of B; bit-identical results).  -1 (default) = for
- *                the policies without error correction, where one product per K block leaves the
- *                kernel waiting on operands from L2 and the pair is 10-15 % faster (16384^3
- *                fp16: 812 vs 677-735 TFLOP/s), and with error correction for calls below about
- *                5000^3, which are over before the board reaches its power cap (2048^3: +8 %,
- *                4096^3: +2 %; at the cap the pair draws more power per product and is 5 %
- *                slower); 0 = never; 1 = whenever it applies.
+ *                loads its rows of A and half of B; bit-identical results).  -1 (default) = whenever it
+ *                applies, except for long calls (more than about 5000^3) with error correction whose
+ *                last 256 rows are half empty and one of few.  Long calls run at the board's power cap;
+ *                with the pairs kept together along K, which large ones are, a pair's fewer bytes
+ *                through L2 count (16384^3: 19.3 ms, 20.0 on single SMs; 8192^3: 2.41, 2.53).  0 = never;
+ *                1 = whenever it applies.
  *   "half_tiles" 1 (default) = a call with so few 256 x 256 tiles that they would leave at least half
  *                of the SM pairs idle runs on 256 x 128 half tiles instead (CTA-pair kernel, N = 128
  *                MMAs; 1024^3: 37 -> 27 us); 0 = whole tiles only.  Same results bit for bit.  Automatic

@@ -159,3 +159,40 @@ def test_no_overlap_goes_unseen(rules):
 ], ids=lambda v: v if isinstance(v, str) else "")
 def test_usual_forms_are_told_apart(rules, what, c, x, batch, want):
     assert rules.batch_overlap_c(ctypes.byref(c), ctypes.byref(x), batch) == want
+
+
+SLOTS = (ctypes.c_int * 3)(74, 33, 15)  # clusters of 2, 4, 8 CTAs that run at a time
+
+# m, n, k, K per block, with error correction, the number of parts that was measured fastest
+PARTS = [
+    (64, 4096, 4096, 32, 1, 4), (33, 206, 11446, 32, 1, 8), (110, 1161, 3881, 32, 1, 8), (813, 1122, 3183, 32, 1, 2),
+    (16, 8182, 3244, 32, 1, 2), (344, 402, 2524, 32, 0, 8), (632, 538, 5451, 16, 1, 4), (187, 1155, 9382, 32, 0, 4),
+    (77, 6331, 1115, 32, 1, 1), (1747, 274, 1502, 32, 0, 1), (35, 3250, 795, 32, 1, 1), (4096, 4096, 4096, 32, 1, 1),
+]
+
+
+@pytest.mark.parametrize("case", PARTS, ids=lambda c: "x".join(map(str, c[:3])))
+def test_k_is_divided_as_was_measured_fastest(rules, case):
+    m, n, k, kop, ec, parts = case
+    nkb = -(-k // kop)
+    assert rules.divide_k_c(m, n, k, 1, nkb, ec, SLOTS, -1) == parts
+    assert rules.divide_k_c(m, n, k, 1, nkb, ec, SLOTS, 1) == 1
+    assert rules.divide_k_c(m, n, k, 2, nkb, ec, SLOTS, -1) == 1  # batches stay whole
+    assert rules.divide_k_c(m, n, k, 1, nkb, ec, (ctypes.c_int * 3)(), -1) == 1  # nowhere to divide
+
+
+def test_a_part_has_a_k_block_and_a_cluster_has_room(rules):
+    for forced in (2, 4, 8):
+        assert rules.divide_k_c(200, 200, 96, 1, forced - 1, 1, SLOTS, forced) == 1
+        assert rules.divide_k_c(200, 200, 96, 1, forced, 1, SLOTS, forced) == forced
+    assert rules.divide_k_c(128, 128 * 16, 4000, 1, 125, 1, SLOTS, 8) == 1  # 16 tiles, 15 clusters of 8
+    assert rules.divide_k_c(100, 128, 4000, 1, 125, 1, SLOTS, 8) == 1  # one tile
+
+
+def test_pairs_and_pacing(rules):
+    for m, n, k, ec, pays in ((16384, 16384, 16384, 1, 1), (8192, 8192, 8192, 1, 1), (1000, 1000, 1000, 1, 1), (300, 16384, 65536, 0, 1),
+                              (300, 16384, 65536, 1, 0), (128 * 19, 16384, 16384, 1, 1)):
+        assert rules.pairs_pay_c(m, n, k, 1, ec) == pays, (m, n, k, ec)
+    for m, n, k, images, paced in ((16384, 16384, 16384, 2, 1), (8192, 8192, 8192, 2, 1), (12000, 4000, 12000, 2, 1), (4096, 4096, 4096, 2, 0),
+                                   (16384, 16384, 16384, 1, 1), (8192, 8192, 8192, 1, 0), (534, 8189, 3656, 2, 0)):
+        assert rules.pace_pays_c(m, n, 1, -(-k // 32), images, 74) == paced, (m, n, k, images)

@@ -7,7 +7,8 @@
 // 48 KB instead of 72 KB of operands are read from shared memory, and the ring holds 6 stages
 // instead of 4.  What bounds it at large sizes is the board's power (1000 W): the SM clock settles where the MMAs, the operands'
 // way through L2 and the panels' way from DRAM add up to it.  16384^3 without copies takes 16.4 ms; with them 22.3 as long as the
-// pairs drift apart along K (51.7 GB from DRAM instead of 8) and 19.3 with the pairs kept together (Pace, below).
+// pairs drift apart along K (51.7 GB read from DRAM) and 19.3 with the pairs kept together (Pace, below: 19.2 GB, 16 if every wave
+// read each of its panels once).
 //
 // Pair protocol (rank 0 = leader, rank 1 = peer):
 //   full[s]   leader's barrier: its own copies' bytes + one remote arrive by the peer's relay
