@@ -66,22 +66,24 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 //
 // A try_wait suspends its thread in hardware for a while, so a loop of them polls seldom; sleeping between polls on top of that
 // only delays the hand-offs (2048^3 62.4 -> 62.1 us, complex 203.3 -> 200.1, 16384^3 19.45 -> 19.36 ms without).  Only waits that go
-// on sleep, `ns` a poll (0: never), so that the limit is long in time: operands may be on their way from another GPU.
+// on for `awake` polls sleep, `ns` a poll (0: never), so that the limit is long in time: operands may be on their way from another
+// GPU.  Without correction and with a long K the epilogue sleeps at once (awake = 0): it waits for a tile's whole K, and the MMAs'
+// operand reads need the shared-memory cycles (8192^3 1070 -> 1043 us; but 8 x 2048^3 186 -> 191).
 constexpr uint32_t kPollsAwake = 512;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
-                                          uint32_t ns = 64) {
+                                          uint32_t ns = 64, uint32_t awake = kPollsAwake) {
   for (uint32_t i = 0; i < TCEC_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (ns && i >= kPollsAwake) __nanosleep(ns);
+    if (ns && i >= awake) __nanosleep(ns);
     if ((i & 0x3ff) == 0x3ff && *abort_flag) return false;
   }
   return false;
 }
 // Warp-collective form: lane 0 polls, the result is broadcast.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
-                                               uint32_t ns = 128) {
+                                               uint32_t ns = 128, uint32_t awake = kPollsAwake) {
   bool ok = true;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, ns);
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, ns, awake);
   return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
 }
 

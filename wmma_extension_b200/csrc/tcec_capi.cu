@@ -98,10 +98,13 @@ void count_cluster_slots(int (&slots)[3]) {
 
 template <bool T, bool E>
 cudaError_t set_pair_smem_attr() {
-  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256>,
+  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256, E>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, GemmPairCfg<T, E>::SMEM_BYTES);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             GemmPairCfg<T, E>::SMEM_BYTES);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 128, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               GemmPairCfg<T, E>::SMEM_BYTES);
 }
 
@@ -488,12 +491,14 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
       gp.tile_first = 0;                                                                                         \
       gp.tile_count = whole;                                                                                     \
       const int grid = 2 * (whole < max_pairs ? whole : max_pairs);                                              \
-      launch_early(tcec_gemm_panels_pair_kernel<T, E, 256>, grid, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp); \
+      launch_early(E || gp.pace ? tcec_gemm_panels_pair_kernel<T, E, 256, true>                                  \
+                                : tcec_gemm_panels_pair_kernel<T, E, 256, E>,                                    \
+                   grid, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp);                                        \
     }                                                                                                            \
     if (halved > 0) {                                                                                            \
       gp.tile_first = whole;                                                                                     \
       gp.tile_count = halved;                                                                                    \
-      launch_early(tcec_gemm_panels_pair_kernel<T, E, 128>, 4 * halved, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp); \
+      launch_early(tcec_gemm_panels_pair_kernel<T, E, 128, E>, 4 * halved, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp); \
     }                                                                                                            \
   } while (0)
     if (tf32 && ec)

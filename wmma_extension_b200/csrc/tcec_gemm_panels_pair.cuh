@@ -98,8 +98,10 @@ __device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* sum, uint3
   atomicAdd(sum, kPaceLeft);
 }
 
-// p.tiles_m counts 256-row pair tiles here.
-template <bool kTf32, bool kEc, int BN>
+// p.tiles_m counts 256-row pair tiles here.  kPaced: a launch may be paced (p.pace).  Without correction launches that are not paced
+// have a kernel without it: the mere test in the producer's loop costs them 2 % (5000 x 6000 x 7000 460 us, 447).  With correction
+// there is one kernel: apart, 4096^3 took 388.4 us instead of 385.7, complex 2048^3 207.2 instead of 204.7.
+template <bool kTf32, bool kEc, int BN, bool kPaced>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     tcec_gemm_panels_pair_kernel(const GemmPanelParams p) {
   static_assert(BN == 256 || BN == 128, "whole or half-width pair tiles");
@@ -174,7 +176,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       // ---------------------------------------------------------- producer (each CTA, own panels)
       if (elect_one()) {
         uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0, it = 0;
-        const bool paced = p.pace && leader;  // the peer's ring cannot run ahead of the leader's
+        const bool paced = kPaced && p.pace && leader;  // the peer's ring cannot run ahead of the leader's
         bool ok = true;
         for (int tile = pair; tile < ntiles && ok; tile += npairs) {
           const TileCoord tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
@@ -276,7 +278,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[1]);
         }
       }
-    } else if (p.pace && leader && elect_one()) {
+    } else if (kPaced && p.pace && leader && elect_one()) {
       // ---------------------------------------------------------- leader: pacing
       pace_launch(pace, p.pace, static_cast<uint32_t>(npairs), abortp);
     }
@@ -298,7 +300,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       const int nchunks = p.promo ? (p.nkb + p.promo - 1) / p.promo : 1;
       float acc[NC];
       for (int c = 0; c < nchunks; ++c, ++chunk) {
-        if (!mbar_wait_warp(smem_u32(&bar_main_full), chunk & 1, abortp)) {
+        if (!mbar_wait_warp(smem_u32(&bar_main_full), chunk & 1, abortp, 128, kEc || p.nkb <= 128 ? kPollsAwake : 0)) {
           ok = false;
           break;
         }
