@@ -1,6 +1,10 @@
 """The native binding of the common calls: what it does not take falls through to the Python code, with the same errors; what it
 takes gives the same results."""
 import importlib.util
+import os
+import shutil
+import subprocess
+import sys
 
 import pytest
 import torch
@@ -26,6 +30,39 @@ def test_it_is_built_and_leaves_other_operands_to_python():
                  lambda: tcec.pack_b(x)):
         with pytest.raises(ValueError, match="float32 CUDA"):
             call()
+
+
+def test_the_library_is_published_after_the_binding_has_it(monkeypatch):
+    """Another thread that sees the library goes straight into the binding, which then has to know the library's addresses."""
+    seen = []
+
+    class Binding:
+        @staticmethod
+        def bind(*addresses):
+            seen.append((tcec._lib, all(addresses)))
+
+    monkeypatch.setattr(tcec, "_lib", None)
+    monkeypatch.setattr(tcec, "_binding", Binding)
+    lib = tcec.load()
+    assert seen == [(None, True)] and tcec._lib is lib
+
+
+@pytest.mark.gpu
+def test_nothing_is_called_before_bind(tmp_path):
+    """A copy of the extension that nobody has bound, in a process of its own: every call is left to the Python code."""
+    copy = shutil.copy(tcec._binding.__file__, tmp_path / "_binding.so")
+    code = f"""
+import importlib.util, torch
+spec = importlib.util.spec_from_file_location("_binding", {str(copy)!r})
+binding = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(binding)
+x = torch.zeros(4, 4, device="cuda:0")
+p = torch.zeros(1 << 16, dtype=torch.uint8, device="cuda:0")
+got = [binding.sgemm(x, x, None, 1.0, 0.0, 0), binding.strided(x[None], x[None], None, 1.0, 0.0, 0), binding.pack_a(x, 0, None),
+       binding.pack_b(x, 0, p), binding.sgemm_packed(p, p, 4, 4, 4, None, 1.0, 0.0, 0)]
+assert got == [None] * 5, got
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=120, cwd=os.path.dirname(os.path.dirname(tcec.__file__)))
 
 
 @pytest.fixture

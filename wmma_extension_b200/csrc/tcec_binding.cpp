@@ -1,7 +1,7 @@
 // The common calls of wmma_extension_b200/tcec.py without their interpreter time: one product, a strided batch, packing, and a
 // product of packed operands on plain float32 CUDA tensors of the current device.  Anything else (and everything that has to raise)
-// returns None, and tcec.py's own code, which accepts and checks it all, takes the call.  A status other than TCEC_OK comes back
-// as an int.
+// returns None, and tcec.py's own code, which accepts and checks it all, takes the call; so does every call before bind().  A status
+// other than TCEC_OK comes back as an int.
 //
 // Calls in a row, us, interpreted and native: 32 x 32 x 32 10.6, 6.7 (the kernel: 6.5); pack_a of 64 x 4096 and the product with a packed
 // 4096 x 4096 24.6, 22.7.
@@ -26,6 +26,7 @@ StridedFn g_strided = nullptr;
 PackFn g_pack[2] = {nullptr, nullptr};
 PackedFn g_packed = nullptr;
 PackedBytesFn g_packed_bytes = nullptr;
+bool g_bound = false;  // read and written with the GIL held
 
 const at::Tensor* plain_tensor(PyObject* o) { return THPVariable_CheckExact(o) ? &THPVariable_Unpack(o) : nullptr; }
 bool cuda_f32(const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat; }
@@ -95,7 +96,7 @@ PyObject* guarded(Body body) {
 template <int kDims>
 PyObject* product(PyObject* const* args, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
-    if (n_args != 6) Py_RETURN_NONE;
+    if (n_args != 6 || !g_bound) Py_RETURN_NONE;
     const at::Tensor *a = plain_tensor(args[0]), *b = plain_tensor(args[1]), *c = args[2] == Py_None ? nullptr : plain_tensor(args[2]);
     float alpha, beta;
     int policy;
@@ -134,7 +135,7 @@ PyObject* strided(PyObject*, PyObject* const* args, Py_ssize_t n) { return produ
 template <int kB>
 PyObject* pack(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
-    if (n_args != 3) Py_RETURN_NONE;
+    if (n_args != 3 || !g_bound) Py_RETURN_NONE;
     const at::Tensor *x = plain_tensor(args[0]), *given = args[2] == Py_None ? nullptr : plain_tensor(args[2]);
     int policy;
     Layout l;
@@ -159,7 +160,7 @@ PyObject* pack(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
 // sgemm_packed(a_packed, b_packed, m, n, k, c, alpha, beta, policy)
 PyObject* sgemm_packed(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   return guarded([&]() -> PyObject* {
-    if (n_args != 9) Py_RETURN_NONE;
+    if (n_args != 9 || !g_bound) Py_RETURN_NONE;
     const at::Tensor *a = plain_tensor(args[0]), *b = plain_tensor(args[1]), *c = args[5] == Py_None ? nullptr : plain_tensor(args[5]);
     int m, n, k, policy;
     float alpha, beta;
@@ -200,6 +201,7 @@ PyObject* bind(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
   g_pack[1] = reinterpret_cast<PackFn>(p[3]);
   g_packed = reinterpret_cast<PackedFn>(p[4]);
   g_packed_bytes = reinterpret_cast<PackedBytesFn>(p[5]);
+  g_bound = true;
   Py_RETURN_NONE;
 }
 

@@ -152,11 +152,11 @@ def load() -> ctypes.CDLL:
     lib.tcec_status_string.restype = ctypes.c_char_p
     lib.tcec_version.argtypes = []
     lib.tcec_version.restype = ctypes.c_char_p
-    _lib = lib
     if _binding is not None:
         _binding.bind(*(ctypes.cast(f, ctypes.c_void_p).value for f in (
             lib.tcec_sgemm, lib.tcec_sgemm_strided_batched, lib.tcec_pack_a, lib.tcec_pack_b, lib.tcec_sgemm_packed,
             lib.tcec_packed_bytes)))
+    _lib = lib  # last: other threads go into the binding as soon as they see it
     return lib
 
 
