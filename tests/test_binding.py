@@ -8,6 +8,7 @@ import sys
 
 import pytest
 import torch
+from torch._subclasses.fake_tensor import FakeTensorMode
 
 from wmma_extension_b200 import tcec
 
@@ -63,6 +64,83 @@ got = [binding.sgemm(x, x, None, 1.0, 0.0, 0), binding.strided(x[None], x[None],
 assert got == [None] * 5, got
 """
     subprocess.run([sys.executable, "-c", code], check=True, timeout=120, cwd=os.path.dirname(os.path.dirname(tcec.__file__)))
+
+
+def _calls_without_room(dev):
+    """Calls whose result, packed operands or second operand are not where or as large as the kernels would take them to be."""
+    def f(*shape, device=dev):
+        return torch.empty(shape, device=device)
+
+    def u8(n, device=dev):
+        return torch.empty(n, dtype=torch.uint8, device=device)
+
+    need = 256 * 64 * 4  # 100 or 60 rows are two blocks of 128, 50 of K two of 32
+    a, b, a3, b3 = f(100, 50), f(50, 60), f(4, 100, 50), f(4, 50, 60)
+    return {
+        "too few rows": lambda m: m.sgemm(a, b, f(10, 60)),
+        "too few columns": lambda m: m.sgemm(a, b, f(100, 59)),
+        "too few rows, column-major": lambda m: m.sgemm(a, b, f(60, 99).t()),
+        "transposed result": lambda m: m.sgemm(a, b, f(60, 100)),
+        "result of no matrices": lambda m: m.sgemm(a, b, f(0, 100, 60)),
+        "complex result": lambda m: m.cgemm(*(torch.empty(s, dtype=torch.complex64, device=dev) for s in ((100, 50), (50, 60), (99, 60)))),
+        "too few matrices": lambda m: m.sgemm_strided_batched(a3, b3, f(3, 100, 60)),
+        "too few rows in a batch": lambda m: m.sgemm_strided_batched(a3, b3, f(4, 99, 60)),
+        "one matrix for a batch": lambda m: m.sgemm_strided_batched(a3, b3, f(100, 60)),
+        "no room to pack A": lambda m: m.pack_a(a, "fp16_ec", u8(need - 1)),
+        "no room to pack B": lambda m: m.pack_b(b, "fp16_ec", u8(need - 1)),
+        "room with holes": lambda m: m.pack_a(a, "fp16_ec", u8(2 * need)[::2]),
+        "packed A too short": lambda m: m.sgemm_packed(u8(need - 1), u8(need), 100, 60, 50),
+        "packed B too short": lambda m: m.sgemm_packed(u8(need), u8(need - 1), 100, 60, 50),
+        "packed for another policy": lambda m: m.sgemm_packed(u8(need // 2), u8(need // 2), 100, 60, 50),
+        "packed result too small": lambda m: m.sgemm_packed(u8(need), u8(need), 100, 60, 50, f(99, 60)),
+        "packed operand on the host": lambda m: m.sgemm_packed(u8(need, "cpu"), u8(need), 100, 60, 50, f(100, 60)),
+        "room on the host": lambda m: m.pack_a(a, "fp16_ec", u8(need, "cpu")),
+        "B on the host": lambda m: m.sgemm(a, f(50, 60, device="cpu")),
+    }
+
+
+def _refused_before_anything_is_launched(module, call):
+    with pytest.raises(ValueError, match="the result needs|consecutive bytes|one device|float32 CUDA"):
+        call(module)
+
+
+def test_calls_without_room_are_refused_in_python(monkeypatch):
+    """Without a GPU, on stand-in tensors."""
+    tcec.load()
+    monkeypatch.setattr(torch.cuda, "is_available", lambda: False)  # the stand-ins' devices need not exist
+    with FakeTensorMode():
+        for name, call in _calls_without_room(DEV).items():
+            try:
+                _refused_before_anything_is_launched(tcec, call)
+            except BaseException as e:
+                raise AssertionError(name) from e
+        a, b = torch.empty(100, 50, device=DEV), torch.empty(50, 60, device=DEV)
+        packed = torch.empty(1 << 16, dtype=torch.uint8, device=DEV)
+        for call in (lambda: tcec.sgemm(a, torch.empty(50, 60, device="cuda:1")),
+                     lambda: tcec.sgemm(a, b, torch.empty(100, 60, device="cuda:1")),
+                     lambda: tcec.pack_a(a, "fp16_ec", torch.empty(1 << 16, dtype=torch.uint8, device="cuda:1")),
+                     lambda: tcec.sgemm_packed(packed, packed, 100, 60, 50, torch.empty(100, 60, device="cuda:1"))):
+            with pytest.raises(ValueError, match="one device"):
+                call()
+
+
+@pytest.mark.gpu
+def test_calls_without_room_are_refused(python_only):
+    tcec.load()
+    for call in _calls_without_room(DEV).values():
+        _refused_before_anything_is_launched(tcec, call)
+        _refused_before_anything_is_launched(python_only, call)
+    # a result that is larger than the product takes it in its first rows and columns
+    gen = torch.Generator(device=DEV).manual_seed(2)
+    a, b = torch.rand((100, 50), generator=gen, device=DEV), torch.rand((50, 60), generator=gen, device=DEV)
+    want = tcec.sgemm(a, b)
+    for module in (tcec, python_only):
+        for c in (torch.full((103, 64), 7.0, device=DEV), torch.full((64, 103), 7.0, device=DEV).t(), torch.full((1, 100, 60), 7.0, device=DEV)):
+            assert module.sgemm(a, b, c) is c
+            rest = c.clone()
+            rest[..., :100, :60] = 7.0
+            assert torch.equal(c[..., :100, :60].reshape(100, 60), want) and bool((rest == 7.0).all())
+    tcec.device_status()
 
 
 @pytest.fixture

@@ -61,6 +61,10 @@ def test_invalid_arguments_are_rejected_without_a_device():
     assert lib.tcec_cgemm(0, 0, 0, 0, 4, 4, one, z, 4, z, 4, one, z, 4, 0, z) == tcec.OK
     assert lib.tcec_pack_a(0, 4, 4, z, 4, z, 0, z) == tcec.ERR_INVALID_ARGUMENT
     assert lib.tcec_sgemm_packed(0, 4, 4, 4, 1.0, z, z, 0.0, z, 4, 0, z) == tcec.ERR_INVALID_ARGUMENT
+    # packed operands that bulk copies cannot start at
+    even, odd = ((p.value + 15) // 16 * 16 + offset for offset in (0, 8))
+    assert lib.tcec_sgemm_packed(0, 4, 4, 4, 1.0, odd, even, 0.0, p, 4, 0, z) == tcec.ERR_INVALID_ARGUMENT
+    assert lib.tcec_sgemm_packed(0, 4, 4, 4, 1.0, even, odd, 0.0, p, 4, 0, z) == tcec.ERR_INVALID_ARGUMENT
 
 
 def test_new_entry_points_reject_bad_arguments_without_a_device():

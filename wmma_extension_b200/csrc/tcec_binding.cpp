@@ -32,6 +32,8 @@ const at::Tensor* plain_tensor(PyObject* o) { return THPVariable_CheckExact(o) ?
 bool cuda_f32(const at::Tensor& t) { return t.is_cuda() && t.scalar_type() == at::kFloat; }
 // Of the current device; other devices need a switch.
 bool here(const at::Tensor& t) { return t.is_cuda() && t.device().index() == c10::cuda::current_device(); }
+// A packed operand or room for one: `bytes` consecutive bytes on the current device, as _require_packed in tcec.py.
+bool packed_here(const at::Tensor& t, size_t bytes) { return here(t) && t.is_contiguous() && t.nbytes() >= bytes; }
 
 // Layout and leading dimension of the last two dimensions, as _layout_ld in tcec.py; false: neither.
 struct Layout {
@@ -103,13 +105,14 @@ PyObject* product(PyObject* const* args, Py_ssize_t n_args) {
     if (!a || !b || (!c && args[2] != Py_None) || !scalar(args[3], alpha) || !scalar(args[4], beta) || !policy_of(args[5], policy))
       Py_RETURN_NONE;
     if (a->dim() != kDims || b->dim() != kDims || (c && c->dim() != kDims) || !cuda_f32(*a) || !cuda_f32(*b) || (c && !cuda_f32(*c)) ||
-        !here(*a))
+        !here(*a) || !here(*b) || (c && !here(*c)))
       Py_RETURN_NONE;
     const int64_t batch = kDims == 3 ? a->size(0) : 1, m = a->size(kDims - 2), k = a->size(kDims - 1), n = b->size(kDims - 1);
     Layout la, lb, lc;
     if (b->size(kDims - 2) != k || (kDims == 3 && b->size(0) != batch) || !fits(m) || !fits(n) || !fits(k) || !fits(batch) ||
         !layout_of(*a, la) || !layout_of(*b, lb))
       Py_RETURN_NONE;
+    if (c && (c->size(kDims - 2) < m || c->size(kDims - 1) < n || (kDims == 3 && c->size(0) < batch))) Py_RETURN_NONE;
     std::optional<at::Tensor> made;
     if (!c) made = kDims == 3 ? at::empty({batch, m, n}, a->options()) : at::empty({m, n}, a->options());
     const at::Tensor& out = c ? *c : *made;
@@ -144,9 +147,9 @@ PyObject* pack(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
       Py_RETURN_NONE;
     const int first = x->size(0), second = x->size(1);
     std::optional<at::Tensor> made;
-    if (!given)
-      made = at::empty({static_cast<int64_t>(kB ? g_packed_bytes(second, first, policy) : g_packed_bytes(first, second, policy))},
-                       x->options().dtype(at::kByte));
+    const size_t bytes = kB ? g_packed_bytes(second, first, policy) : g_packed_bytes(first, second, policy);
+    if (given && !packed_here(*given, bytes)) Py_RETURN_NONE;
+    if (!given) made = at::empty({static_cast<int64_t>(bytes)}, x->options().dtype(at::kByte));
     const float* src = static_cast<const float*>(x->data_ptr());
     void *dst = (given ? *given : *made).data_ptr(), *stream = stream_here();
     int status;
@@ -167,7 +170,8 @@ PyObject* sgemm_packed(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     if (!a || !b || (!c && args[5] != Py_None) || !extent(args[2], m) || !extent(args[3], n) || !extent(args[4], k) ||
         !scalar(args[6], alpha) || !scalar(args[7], beta) || !policy_of(args[8], policy))
       Py_RETURN_NONE;
-    if (c ? c->dim() != 2 || !cuda_f32(*c) || !here(*c) : !here(*a)) Py_RETURN_NONE;
+    if (!packed_here(*a, g_packed_bytes(m, k, policy)) || !packed_here(*b, g_packed_bytes(n, k, policy))) Py_RETURN_NONE;
+    if (c && (c->dim() != 2 || !cuda_f32(*c) || !here(*c) || c->size(0) < m || c->size(1) < n)) Py_RETURN_NONE;
     std::optional<at::Tensor> made;
     if (!c) made = at::empty({m, n}, a->options().dtype(at::kFloat));
     const at::Tensor& out = c ? *c : *made;

@@ -1099,6 +1099,9 @@ int tcec_sgemm_packed(int layout_c, int m, int n, int k, float alpha, const void
   if (m == 0 || n == 0) return TCEC_OK;
   if (!c || ldc < (layout_c == TCEC_ROW_MAJOR ? n : m)) return TCEC_ERR_INVALID_ARGUMENT;
   if (k > 0 && (!a_packed || !b_packed)) return TCEC_ERR_INVALID_ARGUMENT;
+  // bulk copies start on 16-byte boundaries
+  if (k > 0 && alpha != 0.f && ((reinterpret_cast<uintptr_t>(a_packed) | reinterpret_cast<uintptr_t>(b_packed)) & 15) != 0)
+    return TCEC_ERR_INVALID_ARGUMENT;
   std::lock_guard<std::mutex> lock(g_mu);
   DeviceState* st = nullptr;
   const int rc = get_device_state(&st);

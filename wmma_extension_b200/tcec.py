@@ -199,6 +199,24 @@ def _require_cuda_f32(*ts: torch.Tensor) -> None:
             raise ValueError("operands must be float32 CUDA tensors")
 
 
+def _require_room(c: torch.Tensor, shape, *operands: torch.Tensor) -> None:
+    """`c` holds a result of this shape (a larger one takes it in its first rows and columns), on the operands' device."""
+    if c.dim() < len(shape) or any(have < want for have, want in zip(c.shape[-len(shape):], shape)) or 0 in c.shape[:-len(shape)]:
+        raise ValueError(f"the result needs {tuple(shape)}, c is {tuple(c.shape)}")
+    _require_one_device(c, *operands)
+
+
+def _require_one_device(first: torch.Tensor, *others: torch.Tensor) -> None:
+    if any(t.device != first.device for t in others):
+        raise ValueError("operands must be on one device")
+
+
+def _require_packed(t: torch.Tensor, rows: int, k: int, policy) -> None:
+    """`t` is a packed operand of this size, or room for one."""
+    if not t.is_cuda or not t.is_contiguous() or t.numel() * t.element_size() < packed_bytes(rows, k, policy):
+        raise ValueError(f"a packed operand of {rows} rows and k = {k} takes {packed_bytes(rows, k, policy)} consecutive bytes on a GPU")
+
+
 # torch's own short ways to the current device and to a device's current stream as a number: a Stream object costs 3 us and a
 # device switch 1.5 us of a 12 us call.  They are not public; without them the public ones serve.
 _current_device = getattr(torch._C, "_cuda_getDevice", None) or torch.cuda.current_device
@@ -252,6 +270,7 @@ def sgemm(a: torch.Tensor, b: torch.Tensor, c: Optional[torch.Tensor] = None, *,
     if c is None:
         c = a.new_empty((m, n))
     _require_cuda_f32(c)
+    _require_room(c, (m, n), a, b)
     la, lda = _layout_ld(a)
     lb, ldb = _layout_ld(b)
     lc, ldc = _layout_ld(c)
@@ -274,6 +293,7 @@ def cgemm(a: torch.Tensor, b: torch.Tensor, c: Optional[torch.Tensor] = None, *,
         raise ValueError("inner dimensions differ")
     if c is None:
         c = a.new_empty((m, n))
+    _require_room(c, (m, n), a, b)
     la, lda = _layout_ld(a)
     lb, ldb = _layout_ld(b)
     lc, ldc = _layout_ld(c)
@@ -334,6 +354,7 @@ def sgemm_strided_batched(a: torch.Tensor, b: torch.Tensor, c: Optional[torch.Te
     if c is None:
         c = a.new_empty((batch, m, n))
     _require_cuda_f32(c)
+    _require_room(c, (batch, m, n), a, b)
     la, lda = _layout_ld(a)
     lb, ldb = _layout_ld(b)
     lc, ldc = _layout_ld(c)
@@ -392,6 +413,8 @@ def pack_a(a: torch.Tensor, policy="fp16_ec", out: Optional[torch.Tensor] = None
     la, lda = _layout_ld(a)
     if out is None:
         out = a.new_empty(packed_bytes(m, k, policy), dtype=torch.uint8)
+    _require_packed(out, m, k, policy)
+    _require_one_device(a, out)
     with _on(a.device):
         st = load().tcec_pack_a(la, m, k, a.data_ptr(), lda, out.data_ptr(), _policy(policy), _stream_ptr())
     _check(st, "tcec_pack_a")
@@ -409,6 +432,8 @@ def pack_b(b: torch.Tensor, policy="fp16_ec", out: Optional[torch.Tensor] = None
     lb, ldb = _layout_ld(b)
     if out is None:
         out = b.new_empty(packed_bytes(n, k, policy), dtype=torch.uint8)
+    _require_packed(out, n, k, policy)
+    _require_one_device(b, out)
     with _on(b.device):
         st = load().tcec_pack_b(lb, k, n, b.data_ptr(), ldb, out.data_ptr(), _policy(policy), _stream_ptr())
     _check(st, "tcec_pack_b")
@@ -426,6 +451,9 @@ def sgemm_packed(a_packed: torch.Tensor, b_packed: torch.Tensor, m: int, n: int,
     if c is None:
         c = torch.empty((m, n), dtype=torch.float32, device=a_packed.device)
     _require_cuda_f32(c)
+    _require_packed(a_packed, m, k, policy)
+    _require_packed(b_packed, n, k, policy)
+    _require_room(c, (m, n), a_packed, b_packed)
     lc, ldc = _layout_ld(c)
     with _on(c.device):
         st = load().tcec_sgemm_packed(lc, m, n, k, alpha, a_packed.data_ptr(), b_packed.data_ptr(), beta,
