@@ -33,6 +33,28 @@ def test_it_is_built_and_leaves_other_operands_to_python():
             call()
 
 
+def _another_tcec(name):
+    spec = importlib.util.spec_from_file_location(f"wmma_extension_b200.{name}", tcec.__file__)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    return module
+
+
+def test_a_binding_of_another_torch_is_neither_used_nor_kept(monkeypatch, tmp_path):
+    import __graft_entry__ as build
+
+    assert _another_tcec("again")._binding is tcec._binding
+    tag = build._binding_tag()
+    assert tcec._binding.built_for == tag
+    so, source = tmp_path / "binding.so", tmp_path / "source"
+    source.write_text("")
+    shutil.copyfile(tcec._binding.__file__, so)
+    assert build._binding_current(str(so), [str(source)], tag)
+    monkeypatch.setattr(torch, "__version__", torch.__version__ + "x")
+    assert not build._binding_current(str(so), [str(source)], build._binding_tag())
+    assert _another_tcec("elsewhere")._binding is None
+
+
 def test_the_library_is_published_after_the_binding_has_it(monkeypatch):
     """Another thread that sees the library goes straight into the binding, which then has to know the library's addresses."""
     seen = []

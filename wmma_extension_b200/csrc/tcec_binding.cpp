@@ -11,16 +11,19 @@
 #include <torch/csrc/autograd/python_variable.h>
 
 #include <optional>
+#include <type_traits>
+
+#include "../../include/tcec.h"
 
 namespace {
 
-typedef int (*SgemmFn)(int, int, int, int, int, int, float, const float*, long long, const float*, long long, float, float*, long long,
-                       int, void*);
-typedef int (*StridedFn)(int, int, int, int, int, int, float, const float*, long long, long long, const float*, long long, long long,
-                         float, float*, long long, long long, int, int, void*);
-typedef int (*PackFn)(int, int, int, const float*, long long, void*, int, void*);
-typedef int (*PackedFn)(int, int, int, int, float, const void*, const void*, float, float*, long long, int, void*);
-typedef size_t (*PackedBytesFn)(int, int, int);
+// The types of the calls are those of the header that the library was built from.
+typedef decltype(&tcec_sgemm) SgemmFn;
+typedef decltype(&tcec_sgemm_strided_batched) StridedFn;
+typedef decltype(&tcec_pack_a) PackFn;
+static_assert(std::is_same<PackFn, decltype(&tcec_pack_b)>::value, "one type packs A and B");
+typedef decltype(&tcec_sgemm_packed) PackedFn;
+typedef decltype(&tcec_packed_bytes) PackedBytesFn;
 SgemmFn g_sgemm = nullptr;
 StridedFn g_strided = nullptr;
 PackFn g_pack[2] = {nullptr, nullptr};
@@ -222,4 +225,12 @@ PyModuleDef kModule = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, kMethods,
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__binding() { return PyModule_Create(&kModule); }
+PyMODINIT_FUNC PyInit__binding() {
+  PyObject* module = PyModule_Create(&kModule);
+  // What this was compiled against: tcec.py does not use it with another torch or another header.
+  if (module && (PyModule_AddStringConstant(module, "built_for", TCEC_BINDING_BUILT_FOR) != 0)) {
+    Py_DECREF(module);
+    return nullptr;
+  }
+  return module;
+}

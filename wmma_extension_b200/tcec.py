@@ -13,6 +13,7 @@ from __future__ import annotations
 import contextlib
 import ctypes
 import os
+import sys
 from typing import Optional, Sequence
 
 import torch
@@ -66,7 +67,10 @@ _lib = None
 # device, and the code here takes the call.
 try:
     from . import _binding
-except ImportError:  # not built, or built for another torch: this file does it all
+
+    if _binding.built_for != f"torch {torch.__version__}, Python {sys.version_info[0]}.{sys.version_info[1]}":
+        _binding = None  # tensors may be laid out in another way there
+except (ImportError, AttributeError):  # not built, or it does not load here: this file does it all
     _binding = None
 
 
