@@ -95,3 +95,37 @@ def test_waits_of_the_direct_and_narrow_kernels_run_out_the_same_way(kernel, pol
         for name, value in ((b"debug_flags", 0), (b"direct_kernel", -1), (b"narrow_tiles", -1)):
             lib.tcec_set_option(name, value)
         lib.tcec_destroy()
+
+
+@pytest.mark.parametrize("policy", [0, 1, 2, 3])
+@pytest.mark.parametrize("parts", [2, 4, 8])
+def test_a_tile_of_which_one_part_is_missing_is_not_stored(parts, policy):
+    """Of the CTAs that share a tile's K one gives up; the others have their parts, and still none of the tile is written."""
+    lib, i = _library(), ctypes.c_int
+    rng = np.random.default_rng(5)
+    m, n, k = 130, 250, 8 * 32 * 11  # a part has more K blocks than the ring, whatever the policy
+    a = torch.from_numpy(rng.uniform(-1, 1, (m, k)).astype(np.float32)).cuda()
+    b = torch.from_numpy(rng.uniform(-1, 1, (k, n)).astype(np.float32)).cuda()
+    c = torch.full((m, n), 5.0, device="cuda")
+    detail = i(0)
+
+    def run():
+        st = lib.tcec_sgemm(0, 0, 0, m, n, k, 1.0, a.data_ptr(), k, b.data_ptr(), n, 0.0, c.data_ptr(), n, policy, None)
+        return st or lib.tcec_device_status(ctypes.byref(detail))
+
+    assert lib.tcec_set_option(b"k_parts", parts) == 0
+    try:
+        assert run() == 0
+        want = c.clone()
+        assert not bool((want == 5.0).any())
+        assert lib.tcec_set_option(b"debug_flags", 64) == 0  # one stage of one part is never filled
+        c.fill_(5.0)
+        assert run() == ERR_TIMEOUT
+        assert detail.value in (1, 2, 3)
+        assert bool((c == 5.0).all())
+        assert lib.tcec_set_option(b"debug_flags", 0) == 0
+        assert run() == 0 and torch.equal(c, want)
+    finally:
+        for name, value in ((b"debug_flags", 0), (b"k_parts", -1)):
+            lib.tcec_set_option(name, value)
+        lib.tcec_destroy()

@@ -141,8 +141,8 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
             ok = false;
             break;
           }
-          // injected stall (failure-path test): the first stage after the first ring fill is never filled
-          if (dev_flag(p.debug_flags, 64) && it == static_cast<uint32_t>(NST)) {
+          // injected stall (failure-path test): the first stage after the first ring fill is never filled, of a cluster's CTAs in one
+          if (dev_flag(p.debug_flags, 64) && it == static_cast<uint32_t>(NST) && part == parts / 2) {
             next_stage();
             continue;
           }
@@ -252,9 +252,12 @@ __global__ void __launch_bounds__(GemmNarrowCfg<BN, kEc>::THREADS, 1) tcec_gemm_
   __syncthreads();
   if (warp == 1) tmem_dealloc(tmem, Cfg::TMEM_COLS);
   if constexpr (kSplit) {
-    cluster_sync_all();  // every part has arrived
+    // A CTA whose wait ran out has no part: it tells the others, and none of them stores its share of the tile.
+    if (static_cast<int>(threadIdx.x) < parts && *abortp) raise_abort_in(&abort_flag, threadIdx.x);
+    __syncwarp();
+    cluster_sync_all();  // every part, or word that one is missing, has arrived
     const int ew = warp - 4, per = Cfg::EPI_WARPS / parts;
-    if (warp >= 4 && ew / per == part) {
+    if (warp >= 4 && ew / per == part && !*abortp) {
       const TileCoord tc = decode_tile(first_tile, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
       const float4* from = reinterpret_cast<const float4*>(smem_gen + Cfg::PARTS_OFFSET + ew % per * Cfg::PART_BYTES) + lane;
       float acc[Cfg::NC];
