@@ -257,7 +257,7 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                the reference's mma_rn_sync uses 16 or 8 (:640-706).
  *   "tile_n"     0 = automatic, 128 or 256.
  *   "cta_pair"   256-wide tiles on pairs of SMs (tcgen05 cta_group::2: 256 x 256 tiles, each SM
- *                loads its rows of A and half of B; bit-identical results).  -1 (default) = whenever it
+ *                loads its rows of A and half of B; the bits of every undivided call, see "k_parts").  -1 (default) = whenever it
  *                applies, except for long calls (more than about 5000^3) with error correction whose
  *                last 256 rows are half empty and one of few.  Long calls run at the board's power cap;
  *                with the pairs kept together along K, which large ones are, a pair's fewer bytes
@@ -265,7 +265,7 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                1 = whenever it applies.
  *   "half_tiles" 1 (default) = a call with so few 256 x 256 tiles that they would leave at least half
  *                of the SM pairs idle runs on 256 x 128 half tiles instead (CTA-pair kernel, N = 128
- *                MMAs; 1024^3: 37 -> 27 us); 0 = whole tiles only.  Same results bit for bit.  Automatic
+ *                MMAs; 1024^3: 37 -> 27 us); 0 = whole tiles only.  The bits of every undivided call.  Automatic
  *                calls of that size run on narrow tiles before they come to this, apart from some of long K
  *                without error correction.
  *   "reserve_sms" 0..64 (default 0): SMs the GEMM kernels do not occupy.  Their persistent CTAs take
@@ -280,7 +280,7 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *   "static_tiles" 0 (default) = after the first wave the panel GEMM's CTAs draw their tiles from a
  *                device-wide counter, so a CTA that gets its SM late (another kernel was running
  *                there) processes fewer tiles instead of delaying the launch; 1 = static striding
- *                (CTA i takes tiles i, i + grid, ...).  Same results bit for bit.
+ *                (CTA i takes tiles i, i + grid, ...).  The bits of every undivided call.
  *   "store_turn" 1 (default) = the panel kernel turns its C stores through shared memory into full
  *                128-byte lines and uses all 227 KB of the SM; 0 = direct stores and ~30 KB of
  *                shared memory per SM left free.
@@ -294,13 +294,20 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *   "narrow_tiles" -1 (default) = a call whose 256-wide tiles are too few to fill the GPU runs in tiles of
  *                128 x 32, 64 or 128 (64 x 4096 x 4096 on packed operands: 82 -> 34 us with the packing of A);
  *                0 = never; 32, 64, 128 = that width.  Only while "cta_pair" and "tile_n" are automatic,
- *                "store_turn" is 1 and "static_tiles" 0.  Same results bit for bit.
+ *                "store_turn" is 1 and "static_tiles" 0.  The bits of every undivided call.
  *   "k_parts"    -1 (default) = a single product of k >= 1200 with more than one 128 x 128 tile, but so few
- *                that 2, 4 or 8 SMs can share each of them, divides K among these (64 x 4096 x 4096 on packed operands: 27 -> 16 us without the packing).  The parts are
- *                added in FP32, in the order of K; the error against FP64 is no larger, the last bits are others than those of an
- *                undivided call.  1 = never (every kernel gives the same bits); 2, 4, 8 = that many where they have
- *                room.  Only while "narrow_tiles" and "promote_k" are automatic, "reserve_sms" is 0, and under the
- *                conditions of "narrow_tiles".
+ *                that 2, 4 or 8 SMs can share each of them, divides K among these (64 x 4096 x 4096 on packed
+ *                operands: 27 -> 16 us without the packing).  Sizes and policy alone say into how many parts (8 up to
+ *                15 tiles, 4 up to 33, 2 up to 74); only a GPU that cannot run clusters of so many CTAs takes fewer.
+ *                The parts are added in FP32, in the order of K: the error against FP64 is no larger, but the last
+ *                bits are others than those of the undivided product, on which all other kernels agree.
+ *                  Divided: tcec_sgemm, tcec_sgemm_cublas, tcec_sgemm_packed, tcec_sgemm_static, the real product in
+ *                tcec_cgemm, and tcec_sgemm_host just as tcec_sgemm.
+ *                  Undivided: batches, of one matrix too, and the column-sharded calls, on any number of GPUs; calls
+ *                with "cta_pair", "tile_n", "narrow_tiles", "promote_k", "store_turn", "static_tiles" or "reserve_sms"
+ *                other than automatic; the FP32-tile and the direct kernel.
+ *                So a divided product may differ in its last bits from the same rows or columns of a larger product, and
+ *                from the undivided ones above.  1 = never, and they all agree; 2, 4, 8 = that many where they have room.
  *   "direct_kernel" one launch that reads FP32 operands of any layout, alignment and batch form with
  *                ordinary loads and splits them on the way into shared memory; bit-identical
  *                results.  -1 (default) = for matrices with m, n <= 128, unless they are few and their K long (one

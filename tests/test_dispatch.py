@@ -181,6 +181,20 @@ def test_k_is_divided_as_was_measured_fastest(rules, case):
     assert rules.divide_k_c(m, n, k, 1, nkb, ec, (ctypes.c_int * 3)(), -1) == 1  # nowhere to divide
 
 
+def test_parts_follow_from_sizes_alone(rules):
+    """GPUs differ in how many clusters they run at a time (a GPC may lack SMs); results do not."""
+    rng = random.Random(11)
+    gpus = [(ctypes.c_int * 3)(*s) for s in ((74, 37, 18), (74, 35, 16), (74, 33, 15), (70, 30, 12), (1, 1, 1))]
+    seen = set()
+    for _ in range(3000):
+        m, n, k, ec = rng.randrange(1, 3000), rng.randrange(1, 3000), rng.randrange(1000, 9000), rng.randrange(2)
+        for forced in (-1, 2, 4, 8):
+            parts = {rules.divide_k_c(m, n, k, 1, -(-k // 32), ec, s, forced) for s in gpus}
+            assert len(parts) == 1, (m, n, k, forced)
+            seen |= parts
+    assert seen == {1, 2, 4, 8}
+
+
 def test_a_part_has_a_k_block_and_a_cluster_has_room(rules):
     for forced in (2, 4, 8):
         assert rules.divide_k_c(200, 200, 96, 1, forced - 1, 1, SLOTS, forced) == 1

@@ -107,3 +107,71 @@ def test_non_finite_operands_stay_in_their_rows_and_columns():
     want[3, :] = True
     want[:, 150] = True
     assert torch.equal(bad, want)
+
+
+def _undivided(call):
+    tcec.set_option("k_parts", 1)
+    out = call()
+    tcec.set_option("k_parts", -1)
+    return out
+
+
+@pytest.mark.parametrize("policy", ["fp16_ec", "tf32_ec", "fp16_no_ec"])
+@pytest.mark.parametrize("m,n,k", [(900, 520, 3200), (300, 260, 5000)])
+def test_host_operands_divide_as_one_device_call_does(m, n, k, policy):
+    """Row panels have fewer tiles than the whole product, which alone decides."""
+    gen = torch.Generator(device=DEV).manual_seed(8)
+    a, b = _rand(gen, m, k), _rand(gen, k, n)
+    want = tcec.sgemm(a, b, policy=policy)
+    assert not torch.equal(want, _undivided(lambda: tcec.sgemm(a, b, policy=policy)))  # divided, that is
+    ah, bh, ch = a.cpu().pin_memory(), b.cpu().pin_memory(), torch.empty((m, n)).pin_memory()
+    for rows in (256, 512, 0):
+        ch.fill_(float("nan"))
+        tcec.sgemm_host(ah, bh, ch, policy=policy, panel_rows=rows)
+        torch.cuda.current_stream().synchronize()
+        assert torch.equal(ch, want.cpu()), rows
+    tcec.device_status()
+
+
+def test_a_batch_of_one_matrix_has_the_bits_of_a_larger_one():
+    gen = torch.Generator(device=DEV).manual_seed(9)
+    a, b = _rand(gen, 3, 200, 3000), _rand(gen, 3, 3000, 300)
+    batch = tcec.sgemm_strided_batched(a, b)
+    assert not torch.equal(batch[1], tcec.sgemm(a[1], b[1]))
+    assert torch.equal(batch[1:2], tcec.sgemm_strided_batched(a[1:2], b[1:2]))
+    c = [torch.zeros(200, 300, device=DEV)]
+    tcec.sgemm_batched([a[1]], [b[1]], c)
+    assert torch.equal(batch[1], c[0])
+    assert torch.equal(batch[1], _undivided(lambda: tcec.sgemm(a[1], b[1])))
+
+
+@pytest.mark.parametrize("policy", ["fp16_ec", "tf32_ec", "fp16_no_ec"])
+def test_undivided_calls_agree_at_long_k(policy):
+    """What the options say of each other's bits, where K is long enough to be divided: forced kernels, a row range and a column
+    range of packed operands, and the column-sharded calls."""
+    gen = torch.Generator(device=DEV).manual_seed(10)
+    m, n, k = 600, 520, 3000  # 25 tiles: four parts
+    a, b = _rand(gen, m, k), _rand(gen, k, n)
+    want = _undivided(lambda: tcec.sgemm(a, b, policy=policy))
+    assert not torch.equal(want, tcec.sgemm(a, b, policy=policy))
+    for name, values, default in (("cta_pair", (0, 1), -1), ("static_tiles", (1,), 0), ("narrow_tiles", (0, 32, 64, 128), -1),
+                                  ("reserve_sms", (20,), 0), ("store_turn", (0,), 1), ("half_tiles", (0,), 1)):
+        for value in values:
+            tcec.set_option(name, value)
+            try:
+                got = tcec.sgemm(a, b, policy=policy) if name != "half_tiles" else _undivided(lambda: tcec.sgemm(a, b, policy=policy))
+            finally:
+                tcec.set_option(name, default)
+            assert torch.equal(got, want), (name, value)
+    ap, bp = tcec.pack_a(a, policy), tcec.pack_b(b, policy)
+    oa, ob = tcec.packed_row_offset(512, k, policy), tcec.packed_row_offset(256, k, policy)
+    part = _undivided(lambda: tcec.sgemm_packed(ap[oa:], bp[ob:], m - 512, n - 256, k, policy=policy))
+    assert torch.equal(part, want[512:, 256:])
+    shard = torch.empty(m, n, device=DEV)
+    tcec.sgemm_column_shard(a, b, shard, m, k, policy=policy)
+    assert torch.equal(shard, want)
+    bh, ch = b.cpu().pin_memory(), torch.empty(m, n).pin_memory()
+    tcec.sgemm_column_shard_host(a.cpu().pin_memory(), bh, ch, m, k, policy=policy, panel_rows=256)
+    torch.cuda.current_stream().synchronize()
+    assert torch.equal(ch, want.cpu())
+    tcec.device_status()

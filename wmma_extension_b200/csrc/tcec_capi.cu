@@ -74,8 +74,7 @@ cudaError_t set_narrow_smem_attr() {
   return e;
 }
 
-// How many clusters of 2, 4 and 8 CTAs of the divided narrow kernel run at a time; what GPCs of 16 to 20 SMs hold differs from one
-// GPU to the next.  (Every policy's kernel takes a whole SM.)  Allocates nothing.
+// How many clusters of 2, 4 and 8 CTAs of the divided narrow kernel run at a time: whether it can be launched that way.  (Every policy's kernel takes a whole SM.)  Allocates nothing.
 void count_cluster_slots(int (&slots)[3]) {
   using Cfg = GemmNarrowCfg<128, true, true>;
   for (int i = 0; i < 3; ++i) {
@@ -408,6 +407,11 @@ void pack_both(bool a_k_contiguous, int m, const float* a, const float* const* a
   }
 }
 
+int k_parts_of(const Shape& s, int m, int n, int k, int batch, int policy, int reserve_sms, const DeviceState* st, const Options& opt) {
+  if (opt.narrow_tiles > 0 || reserve_sms > 0 || opt.promote_k >= 0) return 1;
+  return divide_k(m, n, k, batch, s.nkb, policy_ec(policy), st->cluster_slots, opt.k_parts);
+}
+
 int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t* panels_a, size_t a_stride,
                 const uint8_t* panels_b, size_t b_stride, float beta, float* c, float* const* c_array, long long ldc,
                 long long stride_c, int lc, int batch, int policy, DeviceState* st, cudaStream_t stream,
@@ -450,9 +454,7 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
   // Options that ask for one of the wide kernels, or for something only they do, are obeyed there.
   if (!ex.force_one_sm && !ex.row_ready && !ex.sched && opt.cta_pair == -1 && opt.tile_n == 0 && opt.store_turn &&
       !opt.static_tiles && !(opt.debug_flags & ~64) && opt.narrow_tiles != 0) {
-    const int k_parts = opt.narrow_tiles > 0 || reserve > 0 || opt.promote_k >= 0
-                            ? 1
-                            : divide_k(m, n, k, batch, s.nkb, ec, st->cluster_slots, opt.k_parts);
+    const int k_parts = ex.k_parts > 0 ? ex.k_parts : k_parts_of(s, m, n, k, batch, policy, reserve, st, opt);
     const int width = k_parts > 1             ? 128
                       : opt.narrow_tiles > 0 ? opt.narrow_tiles
                                            : panel_choice(m, n, batch, s.nkb, gp.promo, ec, s.tile_n, sms,
@@ -800,7 +802,7 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
               const float* const* a_array, long long lda, long long stride_a, const float* b,
               const float* const* b_array, long long ldb, long long stride_b, float beta, float* c,
               float* const* c_array, long long ldc, long long stride_c, int batch, int policy,
-              void* stream_v) {
+              void* stream_v, bool may_divide) {
   if (bad_layout(la) || bad_layout(lb) || bad_layout(lc)) return TCEC_ERR_INVALID_ARGUMENT;
   if (m < 0 || n < 0 || k < 0 || batch < 0) return TCEC_ERR_INVALID_ARGUMENT;
   if (policy < 0 || policy > 3) return TCEC_ERR_INVALID_ARGUMENT;
@@ -872,6 +874,7 @@ int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const fl
   uint8_t* panels_a = static_cast<uint8_t*>(ws);
   uint8_t* panels_b = panels_a + s.a_bytes * batch;
   LaunchExtras gate;
+  if (!may_divide) gate.k_parts = 1;
   unsigned int* gated = nullptr;
   if (table_maps) {
     TableMaps table;
@@ -1030,7 +1033,7 @@ int tcec_sgemm(int layout_a, int layout_b, int layout_c, int m, int n, int k, fl
                const float* a, long long lda, const float* b, long long ldb, float beta, float* c,
                long long ldc, int policy, void* stream) {
   return gemm_impl(layout_a, layout_b, layout_c, m, n, k, alpha, a, nullptr, lda, 0, b, nullptr,
-                   ldb, 0, beta, c, nullptr, ldc, 0, 1, policy, stream);
+                   ldb, 0, beta, c, nullptr, ldc, 0, 1, policy, stream, true);
 }
 
 int tcec_sgemm_batched(int layout_a, int layout_b, int layout_c, int m, int n, int k, float alpha,
@@ -1134,7 +1137,7 @@ int tcec_sgemm_cublas(int transa, int transb, int m, int n, int k, const float* 
   if (!alpha || !beta || cublas_layout(transa, &la) != TCEC_OK || cublas_layout(transb, &lb) != TCEC_OK)
     return TCEC_ERR_INVALID_ARGUMENT;
   return gemm_impl(la, lb, TCEC_COL_MAJOR, m, n, k, *alpha, a, nullptr, lda, 0, b, nullptr, ldb, 0, *beta, c,
-                   nullptr, ldc, 0, 1, policy, stream);
+                   nullptr, ldc, 0, 1, policy, stream, true);
 }
 
 int tcec_sgemm_batched_cublas(int transa, int transb, int m, int n, int k, const float* alpha,

@@ -87,8 +87,11 @@ inline PanelChoice panel_choice(int m, int n, int batch, int nkb, int promo, boo
   return c;
 }
 
-// How many CTAs share the K of a 128 x 128 tile (1: undivided, and then other widths are open).  As many as have room at a time:
-// slots[i] clusters of 2 << i.  Undivided against 2, 4, 8 parts, us, GEMM alone on packed operands:
+// How many CTAs share the K of a 128 x 128 tile (1: undivided, and then other widths are open): as many as have room at a time.  The
+// B200s seen run 74 clusters of two, 33 of four and 15 of eight; GPUs differ in which SMs of their GPCs are there, so the rule has these
+// numbers and does not ask the device: a call has the same bits on every GPU.  (A GPU with room for 16 clusters of eight gives up
+// what 15 tiles, 128 x 1920 x 4096, gain from it: 14.8 us in four parts, 12.0 in eight.)  Only one that runs no such cluster at all,
+// runs[i] = 0, does without.  Undivided against 2, 4, 8 parts, us, GEMM alone on packed operands:
 //   64 x 4096 x 4096 (32 tiles) 27.3, 24.0, 15.8    300 x 500 x 4100 (12, with split) 33.9, 28.9, 22.5, 18.8
 //   33 x 206 x 11446 (2) 67.6, 48.0, 28.4, 18.8    110 x 1161 x 3881 (10) 26.2, 22.3, 15.7, 13.3    813 x 1122 x 3183 (63) 24.0, 21.1
 //   344 x 402 x 2524 no correction (12) 15.8, 15.5, 11.7, 10.8    128 x 512 x 8192 tf32 (4, with split) 51, 47, 31, 24
@@ -97,12 +100,13 @@ inline PanelChoice panel_choice(int m, int n, int batch, int nkb, int promo, boo
 // stay undivided and keep the bits of the other kernels.  So do batches and matrices of one tile, which have another kernel to
 // go to where no workspace can be allocated (a first call that is captured): its bits would differ.
 // `forced`: -1 = by this rule, else that many wherever they have room.
-inline int divide_k(int m, int n, int k, int batch, int nkb, bool ec, const int (&slots)[3], int forced) {
+constexpr int kClusterRoom[3] = {74, 33, 15};  // clusters of 2, 4, 8 CTAs
+inline int divide_k(int m, int n, int k, int batch, int nkb, bool ec, const int (&runs)[3], int forced) {
   const long long tiles = ceil_div(m, 128) * ceil_div(n, 128);
   if (batch > 1 || tiles == 1) return 1;
   for (int i = 2; i >= 0; --i) {
     const int parts = 2 << i;
-    if (tiles > slots[i] || nkb < parts) continue;
+    if (tiles > kClusterRoom[i] || runs[i] < 1 || nkb < parts) continue;
     if (forced == parts || (forced == -1 && k >= 1200 && (parts > 2 || nkb >= (ec ? 64 : 96)))) return parts;
   }
   return 1;

@@ -55,7 +55,7 @@ struct StepState;
 struct DeviceState {
   int* status = nullptr;
   int sm_count = 0;
-  int cluster_slots[3] = {};  // clusters of 2, 4, 8 CTAs that run at a time (count_cluster_slots)
+  int cluster_slots[3] = {};  // clusters of 2, 4, 8 CTAs that run at a time (count_cluster_slots); only whether any do counts
   bool attrs_done = false;
   std::map<cudaStream_t, Workspace> ws;
   std::map<cudaStream_t, unsigned int*> sched;  // per stream: the panel GEMM's two tile-scheduler counters
@@ -101,16 +101,20 @@ struct LaunchExtras {
   int all_from_counter = 0;                // with `sched`: this launch's CTAs draw even their first tile
   const unsigned int* only_if = nullptr;   // device word: zero = the launch does nothing
   int force_one_sm = 0;                    // never the CTA-pair kernel (it knows neither flags nor shared counters)
+  int k_parts = 0;                         // > 0: so many CTAs share the K of a tile, instead of what the sizes say
 };
+// How many CTAs share the K of a tile of this product.
+int k_parts_of(const Shape& s, int m, int n, int k, int batch, int policy, int reserve_sms, const DeviceState* st, const Options& opt);
 int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t* panels_a, size_t a_stride,
                 const uint8_t* panels_b, size_t b_stride, float beta, float* c, float* const* c_array, long long ldc,
                 long long stride_c, int lc, int batch, int policy, DeviceState* st, cudaStream_t stream,
                 const Options& opt, const LaunchExtras* extras = nullptr);
-// The whole single-GPU call (argument checks included): tcec_sgemm and its batched forms.
+// The whole single-GPU call (argument checks included): tcec_sgemm and its batched forms.  may_divide: single products; a batch
+// stays undivided, one matrix or many, so that every slice of it has the same bits.
 int gemm_impl(int la, int lb, int lc, int m, int n, int k, float alpha, const float* a, const float* const* a_array,
               long long lda, long long stride_a, const float* b, const float* const* b_array, long long ldb,
               long long stride_b, float beta, float* c, float* const* c_array, long long ldc, long long stride_c,
-              int batch, int policy, void* stream_v);
+              int batch, int policy, void* stream_v, bool may_divide = false);
 int scale_only(float beta, float* c, float* const* c_array, long long ldc, long long stride_c, int m, int n, int lc,
                int batch, cudaStream_t stream);
 

@@ -392,9 +392,10 @@ int column_step_device(std::vector<Lane>& lanes, int nranks, int root, int la, i
 // Host operands (pinned memory for real overlap): every lane's B block is copied in and split
 // once; A travels from the root's host memory in row panels (copy-in, split, broadcast); each
 // panel's GEMM runs as its own launch into one of two device buffers and is copied out while the
-// next panel is multiplied.  Copy-in, broadcast, GEMM and copy-out run on four streams.
+// next panel is multiplied.  Copy-in, broadcast, GEMM and copy-out run on four streams.  k_parts: CTAs that share the K of a tile,
+// the same in every panel.
 int column_step_host(std::vector<Lane>& lanes, int nranks, int root, int la, int lb, int lc, int m, int k, float alpha,
-                     float beta, int policy, int panel_rows, const Options& opt) {
+                     float beta, int policy, int panel_rows, int k_parts, const Options& opt) {
   // Automatic panel height: on one GPU the pipeline is bound by the copy-in of A and B, and what
   // counts is a short tail behind the last copy (16384^3: 43.8 ms with 512 rows, 46.2 with 2048,
   // 49.7 with 4096; the two copies alone take 38.7 ms); with a broadcast per panel, 2048.
@@ -524,6 +525,7 @@ int column_step_host(std::vector<Lane>& lanes, int nranks, int root, int la, int
         const Shape s = plan(pn.rows, ln.n_local, k, policy, opt);
         LaunchExtras ex;
         if (nranks > 1) ex.reserve_sms = opt.comm_sms;
+        ex.k_parts = k_parts;
         std::lock_guard<std::mutex> lock(state_mutex());  // the per-stream tile counters may be created here
         rc = gemm_packed(s, pn.rows, ln.n_local, k, alpha, static_cast<const uint8_t*>(ln.ss->packed_a.ptr) + pn.offset, 0,
                          static_cast<const uint8_t*>(ln.ss->packed_b.ptr), 0, beta, lb_.c32[slot], nullptr, ldc_dev, 0, lc,
@@ -644,7 +646,9 @@ int tcec_sgemm_host(int layout_a, int layout_b, int layout_c, int m, int n, int 
   ln.c = c_host;
   ln.ldc = ldc;
   ln.n_local = n;
-  return column_step_host(lanes, 1, 0, layout_a, layout_b, layout_c, m, k, alpha, beta, policy, panel_rows, opt);
+  // K divided as tcec_sgemm divides that of the whole product, so that panels have its bits
+  const int k_parts = k > 0 ? k_parts_of(plan(m, n, k, policy, opt), m, n, k, 1, policy, opt.reserve_sms, ln.st, opt) : 1;
+  return column_step_host(lanes, 1, 0, layout_a, layout_b, layout_c, m, k, alpha, beta, policy, panel_rows, k_parts, opt);
 }
 
 int tcec_comm_set_library(const char* path) {
@@ -733,7 +737,8 @@ static int column_shard_entry(bool host, int root, int layout_a, int layout_b, i
   ln.ldc = ldc;
   ln.n_local = n_local;
   if (host)
-    return column_step_host(lanes, nranks, root, layout_a, layout_b, layout_c, m, k, alpha, beta, policy, panel_rows, opt);
+    return column_step_host(lanes, nranks, root, layout_a, layout_b, layout_c, m, k, alpha, beta, policy, panel_rows, 1,
+                            opt);  // undivided, so that the bits do not depend on how many ranks there are
   return column_step_device(lanes, nranks, root, layout_a, layout_b, layout_c, m, k, alpha, beta, policy, opt);
 }
 
