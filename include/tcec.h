@@ -277,10 +277,11 @@ int tcec_split(const float* in, float* hi, float* lo, size_t count, int policy, 
  *                of 256).
  *   "comm_helper" 1 (default) = once the broadcast is over, a second GEMM launch that shares the
  *                first one's tile counter takes the SMs it had; 0 = they stay idle.
- *   "static_tiles" 0 (default) = after the first wave the panel GEMM's CTAs draw their tiles from a
- *                device-wide counter, so a CTA that gets its SM late (another kernel was running
- *                there) processes fewer tiles instead of delaying the launch; 1 = static striding
- *                (CTA i takes tiles i, i + grid, ...).  The bits of every undivided call.
+ *   "static_tiles" 0 (default) = the panel GEMM on single SMs after its first wave, and on CTA pairs in calls with error
+ *                correction of more than 2.5e11 flop, draws its tiles from a device-wide counter, so a CTA or pair that
+ *                gets its SMs late (another kernel was running there) processes fewer tiles instead of delaying the
+ *                launch; other calls on pairs, and captured ones there, stride, as do all with 1 (CTA i takes tiles i,
+ *                i + grid, ...).  The bits of every undivided call.
  *   "store_turn" 1 (default) = the panel kernel turns its C stores through shared memory into full
  *                128-byte lines and uses all 227 KB of the SM; 0 = direct stores and ~30 KB of
  *                shared memory per SM left free.

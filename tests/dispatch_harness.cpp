@@ -15,6 +15,9 @@ int pairs_pay_c(int m, int n, int k, int batch, int ec) { return pairs_pay(m, n,
 int pace_pays_c(int m, int n, int batch, int nkb, int images, int pairs) {
   return pace_pays(static_cast<int>(ceil_div(m, 256)), static_cast<int>(ceil_div(n, 256)), batch, nkb, images, pairs);
 }
+int draws_pay_c(int m, int n, int k, int ec, int pairs) {
+  return draws_pay(m, n, k, 1, ec != 0, ceil_div(m, 256) * ceil_div(n, 256), pairs);
+}
 int divide_k_c(int m, int n, int k, int batch, int nkb, int ec, const int* slots, int forced) {
   const int s[3] = {slots[0], slots[1], slots[2]};
   return divide_k(m, n, k, batch, nkb, ec != 0, s, forced);

@@ -210,3 +210,9 @@ def test_pairs_and_pacing(rules):
     for m, n, k, images, paced in ((16384, 16384, 16384, 2, 1), (8192, 8192, 8192, 2, 1), (12000, 4000, 12000, 2, 1), (4096, 4096, 4096, 2, 0),
                                    (16384, 16384, 16384, 1, 1), (8192, 8192, 8192, 1, 0), (534, 8189, 3656, 2, 0)):
         assert rules.pace_pays_c(m, n, 1, -(-k // 32), images, 74) == paced, (m, n, k, images)
+
+
+def test_long_calls_with_correction_draw_their_tiles(rules):
+    for m, n, k, ec, draws in ((16384, 16384, 16384, 1, 1), (8192, 8192, 4096, 1, 1), (40000, 50000, 64, 1, 1), (4096, 4096, 4096, 1, 0),
+                               (2048, 2048, 60000, 1, 0), (8192, 8192, 8192, 0, 0)):
+        assert rules.draws_pay_c(m, n, k, ec, 74) == draws, (m, n, k, ec)

@@ -129,3 +129,38 @@ def test_a_tile_of_which_one_part_is_missing_is_not_stored(parts, policy):
         for name, value in ((b"debug_flags", 0), (b"k_parts", -1)):
             lib.tcec_set_option(name, value)
         lib.tcec_destroy()
+
+
+@pytest.mark.parametrize("policy", [0, 1, 2, 3])
+@pytest.mark.parametrize("long", [False, True])
+def test_waits_of_the_pair_kernel_run_out_the_same_way(long, policy):
+    """Both CTAs of a pair leave; with correction a long call draws its tiles, and the counter is back at zero for the next one."""
+    lib, i = _library(), ctypes.c_int
+    m, n, k = (5000, 5000, 5200) if long else (300, 600, 1100)
+    gen = torch.Generator(device="cuda").manual_seed(6)
+    a, b = torch.rand((m, k), generator=gen, device="cuda"), torch.rand((k, n), generator=gen, device="cuda")
+    c = torch.zeros((m, n), device="cuda")
+    detail = i(0)
+
+    def run():
+        st = lib.tcec_sgemm(0, 0, 0, m, n, k, 1.0, a.data_ptr(), k, b.data_ptr(), n, 0.0, c.data_ptr(), n, policy, None)
+        return st or lib.tcec_device_status(ctypes.byref(detail))
+
+    for name, value in ((b"cta_pair", 1), (b"half_tiles", 0)):
+        assert lib.tcec_set_option(name, value) == 0
+    try:
+        # the short limit of this build is no longer than a long call's waits, so it may run out by itself there
+        healthy = run()
+        assert healthy in ((0, ERR_TIMEOUT) if long else (0,))
+        want = c.clone()
+        assert lib.tcec_set_option(b"debug_flags", 32) == 0  # one stage of every CTA is never filled
+        assert run() == ERR_TIMEOUT
+        assert detail.value in (1, 2, 3)
+        assert lib.tcec_set_option(b"debug_flags", 0) == 0
+        again = run()
+        assert again in ((0, ERR_TIMEOUT) if long else (0,))
+        assert torch.equal(c, want) or healthy or again
+    finally:
+        for name, value in ((b"debug_flags", 0), (b"cta_pair", -1), (b"half_tiles", 1)):
+            lib.tcec_set_option(name, value)
+        lib.tcec_destroy()

@@ -1,4 +1,6 @@
-"""The CTA-pair kernel where its launch is paced: the bits of the one-SM kernel, whatever else uses the pacing words."""
+"""The CTA-pair kernel where its launch is paced or draws its tiles: the bits of the one-SM kernel, whatever else runs."""
+import time
+
 import pytest
 import torch
 
@@ -37,6 +39,77 @@ def test_paced_pairs_have_the_bits_of_single_sms(m, n, k, policy):
     tcec.device_status()
     want = _one_sm(a, b, policy)
     assert torch.equal(got[0], want) and torch.equal(got[1], want)
+
+
+# long enough to draw tiles, paced or not: K of one, two and 43 K blocks, tiles that are cut on both sides, one tile row, a round and a bit
+@pytest.mark.parametrize("m,n,k,policy", [
+    (40000, 50000, 64, "fp16_ec"), (45000, 45001, 64, "tf32_ec"), (60001, 70001, 31, "fp16_ec"), (10000, 9500, 1350, "fp16_ec"),
+    (256, 40000, 12500, "fp16_ec"), (2500, 2100, 24000, "fp16_ec"), (2500, 2100, 24000, "tf32_ec"),
+])
+def test_drawn_tiles_have_the_bits_of_single_sms(m, n, k, policy):
+    a, b = _operands(m, n, k, m + k)
+    got = [tcec.sgemm(a, b, policy=policy) for _ in range(2)]
+    tcec.device_status()
+    want = _one_sm(a, b, policy)
+    assert torch.equal(got[0], want) and torch.equal(got[1], want)
+    tcec.set_option("static_tiles", 1)
+    tcec.set_option("cta_pair", 1)
+    try:
+        assert torch.equal(tcec.sgemm(a, b, policy=policy), want)
+    finally:
+        tcec.set_option("static_tiles", 0)
+
+
+@pytest.mark.parametrize("policy", ["fp16_ec", "tf32_ec"])
+def test_a_long_call_waits_for_no_sms_that_another_kernel_holds(policy):
+    """Four CTAs of another stream's product hold four SMs for longer than the call takes.  The pairs that have none of them do it all
+    (70 of 74: 1.06 times as long); with a share of its own for every pair it took 1.61 to 1.88 times as long."""
+    held = torch.rand(128, 1 << 20, device=DEV)
+    a, b = _operands(8192, 8192, 4096, 3)
+    c = torch.empty(8192, 8192, device=DEV)
+    side = torch.cuda.Stream()
+
+    def timed():
+        start, end = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+        start.record()
+        tcec.sgemm(a, b, c, policy=policy)
+        end.record()
+        return start, end
+
+    def hold():
+        tcec.set_option("direct_kernel", 1)  # one CTA a matrix
+        try:
+            with torch.cuda.stream(side):
+                tcec.sgemm_strided_batched(held.expand(4, 128, 1 << 20), held.t().expand(4, 1 << 20, 128))
+        finally:
+            tcec.set_option("direct_kernel", -1)
+        event = torch.cuda.Event()
+        event.record(side)
+        return event
+
+    hold()
+    for _ in range(3):
+        timed()
+    torch.cuda.synchronize()
+    alone, beside = [], []
+    for _ in range(5):
+        start, end = timed()
+        end.synchronize()
+        alone.append(start.elapsed_time(end))
+    want = c.clone()
+    for _ in range(5):
+        c.fill_(float("nan"))
+        torch.cuda.synchronize()
+        holder = hold()
+        time.sleep(0.003)
+        start, end = timed()
+        end.synchronize()
+        assert not holder.query()  # it was there all the while
+        torch.cuda.synchronize()
+        beside.append(start.elapsed_time(end))
+        assert torch.equal(c, want)
+    tcec.device_status()
+    assert sorted(beside)[2] < 1.35 * sorted(alone)[2], (alone, beside)
 
 
 def test_paced_launches_overlap_on_streams_and_in_a_replayed_graph():

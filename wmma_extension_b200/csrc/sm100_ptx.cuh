@@ -351,6 +351,16 @@ __device__ __forceinline__ void raise_abort_pair(uint32_t* abort_flag) {
   *abort_flag = 1;
   raise_abort_in(abort_flag, cluster_ctarank() ^ 1u);
 }
+// One word that says all there is to say, between the CTAs of a cluster: relaxed, so that it waits for nothing else under way (a
+// release at cluster scope beside bulk copies takes 1300 cycles).
+__device__ __forceinline__ void st_relaxed_cluster(uint32_t cluster_addr, uint32_t v) {
+  asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ uint32_t ld_relaxed_cluster_own(uint32_t addr) {
+  uint32_t v;
+  asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

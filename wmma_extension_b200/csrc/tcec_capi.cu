@@ -97,13 +97,14 @@ void count_cluster_slots(int (&slots)[3]) {
 
 template <bool T, bool E>
 cudaError_t set_pair_smem_attr() {
-  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256, E>,
+  constexpr int kPlain = E ? kStridedPaced : kStrided, kOther = E ? kDrawn : kStridedPaced;
+  cudaError_t e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256, kPlain>,
                                        cudaFuncAttributeMaxDynamicSharedMemorySize, GemmPairCfg<T, E>::SMEM_BYTES);
   if (e == cudaSuccess)
-    e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    e = cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 256, kOther>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              GemmPairCfg<T, E>::SMEM_BYTES);
   if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 128, E>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+  return cudaFuncSetAttribute(tcec_gemm_panels_pair_kernel<T, E, 128, kPlain>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                               GemmPairCfg<T, E>::SMEM_BYTES);
 }
 
@@ -141,9 +142,9 @@ int get_device_state(DeviceState** out) {
     TCEC_CUDA((set_direct_smem_attrs<true, true>()));
     TCEC_CUDA((set_direct_smem_attrs<true, false>()));
     count_cluster_slots(st.cluster_slots);
-    if (cudaMalloc(&st.status, kStatusBytes + kPaceSlots * kPaceSlotBytes) != cudaSuccess) return TCEC_ERR_ALLOC;
-    TCEC_CUDA(cudaMemset(st.status, 0, kStatusBytes + kPaceSlots * kPaceSlotBytes));
-    st.pace = reinterpret_cast<unsigned int*>(st.status) + kStatusBytes / sizeof(unsigned int);
+    if (cudaMalloc(&st.status, kStatusBytes + kPairLines * kPairLineBytes) != cudaSuccess) return TCEC_ERR_ALLOC;
+    TCEC_CUDA(cudaMemset(st.status, 0, kStatusBytes + kPairLines * kPairLineBytes));
+    st.pair_lines = reinterpret_cast<uint8_t*>(st.status) + kStatusBytes;
     st.attrs_done = true;
   }
   *out = &st;
@@ -204,12 +205,24 @@ int get_sched(DeviceState* st, cudaStream_t stream, unsigned int** out) {
   return TCEC_OK;
 }
 
-// The stream's pacing word; null when the slots are used up or there are none (a launch without it is only not paced).  Launches
-// that overlap although they share a word (a captured graph replayed on another stream) pace one another wrongly, no more.
-static unsigned int* get_pace(DeviceState* st, cudaStream_t stream) {
-  if (!st->pace) return nullptr;
-  const int slot = st->pace_slot.emplace(stream, static_cast<int>(st->pace_slot.size())).first->second;
-  return slot < kPaceSlots ? st->pace + slot * (kPaceSlotBytes / sizeof(unsigned int)) : nullptr;
+// The stream's line; null when they are used up or there are none.
+static PairLine* get_pair_line(DeviceState* st, cudaStream_t stream) {
+  if (!st->pair_lines) return nullptr;
+  const int i = st->pair_line.emplace(stream, static_cast<int>(st->pair_line.size())).first->second;
+  return i < kPairLines ? reinterpret_cast<PairLine*>(st->pair_lines + i * kPairLineBytes) : nullptr;
+}
+// Counters from which a pair launch on this stream may draw its tiles; null: it strides.  Launches that share counters must not
+// overlap: a captured one may be replayed beside anything, and cudaStreamPerThread is another stream in every thread.
+static int pair_counters(DeviceState* st, cudaStream_t stream, PairLine* line, unsigned int** out) {
+  *out = nullptr;
+  cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+  if (stream == cudaStreamPerThread || cudaStreamIsCapturing(stream, &status) != cudaSuccess || status != cudaStreamCaptureStatusNone)
+    return TCEC_OK;
+  if (line) {
+    *out = line->sched;
+    return TCEC_OK;
+  }
+  return get_sched(st, stream, out);
 }
 
 bool policy_tf32(int policy) { return policy == TCEC_POLICY_TF32_EC || policy == TCEC_POLICY_TF32_NO_EC; }
@@ -485,22 +498,37 @@ int gemm_packed(const Shape& s, int m, int n, int k, float alpha, const uint8_t*
     // 1-2 % slower), so such calls stay on whole tiles.
     const int halved = (opt.half_tiles && 2 * npair_tiles <= max_pairs) ? static_cast<int>(npair_tiles) : 0;
     const int whole = static_cast<int>(npair_tiles) - halved;
-    if (!ex.only_if && pace_pays(gp.tiles_m, gp.tiles_n, batch, s.nkb, s.np, max_pairs) && (gp.pace = get_pace(st, stream)))
-      cudaMemsetAsync(gp.pace, 0, sizeof(unsigned int), stream);
+    const bool paced = !ex.only_if && pace_pays(gp.tiles_m, gp.tiles_n, batch, s.nkb, s.np, max_pairs);
+    const bool draws = !opt.static_tiles && draws_pay(m, n, k, batch, ec, whole, max_pairs);
+    if (paced || draws) {
+      // Paced launches that overlap although they share a line (a captured graph of packed calls replayed beside its stream) pace one
+      // another wrongly, no more.  Without a line a launch is not paced.
+      PairLine* const line = get_pair_line(st, stream);
+      if (paced && line) {
+        gp.pace = line->pace;
+        TCEC_CUDA(cudaMemsetAsync(gp.pace, 0, sizeof line->pace, stream));
+      }
+      if (draws) {
+        const int rc = pair_counters(st, stream, line, &gp.sched);
+        if (rc != TCEC_OK) return rc;
+      }
+    }
 #define TCEC_PAIR(T, E)                                                                                          \
   do {                                                                                                           \
     if (whole > 0) {                                                                                             \
       gp.tile_first = 0;                                                                                         \
       gp.tile_count = whole;                                                                                     \
       const int grid = 2 * (whole < max_pairs ? whole : max_pairs);                                              \
-      launch_early(E || gp.pace ? tcec_gemm_panels_pair_kernel<T, E, 256, true>                                  \
-                                : tcec_gemm_panels_pair_kernel<T, E, 256, E>,                                    \
+      launch_early(gp.sched       ? tcec_gemm_panels_pair_kernel<T, E, 256, E ? kDrawn : kStridedPaced>          \
+                   : E || gp.pace ? tcec_gemm_panels_pair_kernel<T, E, 256, kStridedPaced>                       \
+                                  : tcec_gemm_panels_pair_kernel<T, E, 256, E ? kStridedPaced : kStrided>,       \
                    grid, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp);                                        \
     }                                                                                                            \
     if (halved > 0) {                                                                                            \
       gp.tile_first = whole;                                                                                     \
       gp.tile_count = halved;                                                                                    \
-      launch_early(tcec_gemm_panels_pair_kernel<T, E, 128, E>, 4 * halved, 384, GemmPairCfg<T, E>::SMEM_BYTES, stream, gp); \
+      launch_early(tcec_gemm_panels_pair_kernel<T, E, 128, E ? kStridedPaced : kStrided>, 4 * halved, 384,       \
+                   GemmPairCfg<T, E>::SMEM_BYTES, stream, gp);                                                   \
     }                                                                                                            \
   } while (0)
     if (tf32 && ec)
@@ -1283,8 +1311,8 @@ int tcec_destroy(void) {
     destroy_step_state(&kv.second);
     if (kv.second.status) cudaFree(kv.second.status);
     kv.second.status = nullptr;
-    kv.second.pace = nullptr;
-    kv.second.pace_slot.clear();
+    kv.second.pair_lines = nullptr;
+    kv.second.pair_line.clear();
     kv.second.attrs_done = false;
   }
   destroy_comm_state();

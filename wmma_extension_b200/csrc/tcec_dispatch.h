@@ -17,9 +17,10 @@ inline long long ceil_div(long long a, long long b) { return (a + b - 1) / b; }
 // 16384^3 takes 19.3 ms on pairs and 20.0 on single SMs, 8192^3 2.41 and 2.53, tf32 4.20 and 4.34, 8192^3 without correction 0.91 and
 // 1.0.  Not where the 256 rows of a pair tile are half empty and the call is long: what is lost is one part in the number of
 // 128-row blocks.
+constexpr double kLongCall = 2.5e11;  // flop
 inline bool pairs_pay(int m, int n, int k, int batch, bool ec) {
   const long long blocks = ceil_div(m, 128);
-  return !ec || 2.0 * m * static_cast<double>(n) * k * batch <= 2.5e11 || blocks % 2 == 0 || blocks >= 19;
+  return !ec || 2.0 * m * static_cast<double>(n) * k * batch <= kLongCall || blocks % 2 == 0 || blocks >= 19;
 }
 
 // Pair tiles are taken in groups of kPairGroupM tile rows, column by column.  A launch is paced (tcec_gemm_panels_pair.cuh) if it
@@ -32,6 +33,12 @@ inline bool pace_pays(int tiles_m, int tiles_n, int batch, int nkb, int images, 
   if (static_cast<long long>(tiles_m) * tiles_n * batch < 4 * pairs) return false;
   const long long rows = tiles_m < kPairGroupM ? tiles_m : kPairGroupM, wave = ceil_div(pairs, rows), cols = tiles_n < wave ? tiles_n : wave;
   return static_cast<double>(rows + cols) * 256 * 64 * images * nkb >= 100e6;
+}
+
+// Whether the tiles of a pair launch are drawn from a counter: calls with correction above the size up to which pairs were always
+// taken.  Longer ones ran on single SMs, which draw theirs, and have to do as well as those beside another stream's kernel.
+inline bool draws_pay(int m, int n, int k, int batch, bool ec, long long tiles, int pairs) {
+  return ec && tiles > pairs && 2.0 * m * static_cast<double>(n) * k * batch > kLongCall;
 }
 
 // The panel GEMM of a call: `width` of the narrow tiles if they would finish the call sooner than 256-wide ones, else 0,

@@ -56,7 +56,7 @@ struct GemmPanelParams {
   int ready_rows;                 // operands only once the word of the tile's rows equals `ready_epoch` (A is
   unsigned int ready_epoch;       // arriving from another GPU while the kernel runs); the wait is bounded
   const unsigned int* only_if; // optional device word: zero = this launch does nothing (another kernel did the work)
-  unsigned int* pace;          // CTA-pair kernel only, optional: a word, zero before the launch, that keeps the pairs together along K
+  unsigned int* pace;          // CTA-pair kernel only, optional: two words, zero before the launch, that keep the pairs together along K
   int tile_first, tile_count;  // CTA-pair kernel only: the pair tiles this launch covers
   int store_turn;          // 1: stores go through the per-warp shared-memory buffers (launched with
                            // SMEM_BYTES); 0: direct stores, launched with SMEM_BYTES_NO_TURN

@@ -54,16 +54,64 @@ struct GemmPairCfg {
   static constexpr int GROUP_M = tcec_host::kPairGroupM;  // pair tiles are 256 rows tall
 };
 
+// How the pairs of a launch share its tiles.  Strided: pair, pair + npairs, ...; with code for pacing (below) or without.  Drawn
+// (and perhaps paced): from a device-wide counter, so that a pair that got its SMs late (another stream's kernel was there) takes
+// fewer tiles instead of starting its whole share when the others are done: 8192 x 8192 x 4096 beside a kernel that holds four SMs
+// 1884 us strided, 1226 drawn; alone 1179 and 1172.
+enum PairTileMode : int { kStrided, kStridedPaced, kDrawn };
+
+// Drawn tiles.  The leader's producer claims the next tile late in the one before, early enough for the counter's answer, and
+// writes it, the end mark too, into a ring in either CTA, from which the other roles read.  An entry is one word, the tile and a bit
+// that changes from round to round, so that nothing else has to be ordered with it; it is written again when all who read it, in
+// either CTA, have arrived on its barrier in the leader.  Claimed only when it is needed, it
+// kept the tensor pipe waiting for the counter (8192 x 8192 x 4096 2 % slower); claimed a whole tile ahead by a thread of its own, the pairs that
+// start first took two tiles of the first wave, whose panels are then shared less (6000^3 10 % slower).
+constexpr uint32_t kNoTile = 0x7fffffff;  // the end mark; tiles are below 2^31 - 1
+struct DrawnTiles {
+  const uint32_t* ring;   // this CTA's
+  const uint64_t* empty;  // the barriers, of which the leader's are used
+  uint32_t count = 0;
+  // The index-th tile of this pair.  Whole warps read the entry in every lane: handed from one lane to the others it made every
+  // promotion of the epilogue slower (10000 x 9500 x 1350 810 us, 717 so, 726 strided), by what ptxas then does with its registers.
+  template <bool kWarp>
+  __device__ __forceinline__ int at(uint32_t index, volatile uint32_t* abortp) const {
+    const uint32_t slot = index % kTileRing, round = ~(index / kTileRing) & 1u;
+    for (uint32_t i = 0; i < TCEC_WAIT_LIMIT; ++i) {
+      const uint32_t v = ld_relaxed_cluster_own(smem_u32(ring + slot));
+      const bool there = v >> 31 == round;
+      if (kWarp ? __all_sync(0xffffffffu, there) : there) {
+        if (!kWarp || (threadIdx.x & 31) == 0) mbar_arrive_cluster(map_to_cta(smem_u32(empty + slot), 0));
+        return (v & kNoTile) == kNoTile ? static_cast<int>(kNoMoreTiles) : static_cast<int>(v & kNoTile);
+      }
+      __nanosleep(64);
+      if ((i & 0xff) == 0xff && (kWarp ? __any_sync(0xffffffffu, *abortp != 0) : *abortp != 0)) break;
+    }
+    return kTileWaitFailed;
+  }
+  __device__ __forceinline__ int next(volatile uint32_t* abortp) { return at<false>(count++, abortp); }
+  // The leader's producer: what it drew, to everybody.
+  __device__ __forceinline__ int publish(unsigned int drawn, int ntiles, volatile uint32_t* abortp) {
+    const bool more = drawn < static_cast<unsigned int>(ntiles);
+    const uint32_t slot = count % kTileRing, round = ~(count / kTileRing) & 1u;
+    if (!mbar_wait(smem_u32(empty + slot), round, abortp, 64)) return kTileWaitFailed;
+    const uint32_t word = (more ? drawn : kNoTile) | round << 31;
+    st_relaxed_cluster(map_to_cta(smem_u32(ring + slot), 1), word);
+    st_relaxed_cluster(map_to_cta(smem_u32(ring + slot), 0), word);
+    ++count;
+    return more ? static_cast<int>(drawn) : static_cast<int>(kNoMoreTiles);
+  }
+};
+
 // Keeps the pairs of a launch close together along K.  The pairs of a wave share their panels, each row block of A with the other
 // tiles of its row and each of B with those of its column, and a panel comes from DRAM once if all of them read it while it is in
 // L2.  Left alone they drift apart, tile after tile, until most panels are fetched several times.
 // Every kPaceStages stages the leader's producer raises its count.  A thread of its own (the producer has no time for a round
 // trip to L2: 16384^3 without correction 8.0 ms that way, 7.3 this way) adds it to a device-wide sum and holds the producer while
-// its count is more than one above the mean.  A hold is bounded: a pair whose SMs another kernel has taken must not stop the
-// rest, so whoever has held in vain holds no more.
-// 16384^3: 21.4 ms unpaced, 19.3 every 4 or 8 stages, 19.6 every 16; the word is a hint, results do not depend on it.
+// its count is more than one above the mean of the pairs that run.  One that starts when the others are well under way counts from
+// where they are.  A hold is bounded, and whoever has held in vain holds no more.
+// 16384^3: 21.4 ms unpaced, 19.3 every 4 or 8 stages, 19.6 every 16; the words are a hint, results do not depend on them.
 constexpr uint32_t kPaceStages = 8;
-constexpr uint32_t kPaceLeft = 1u << 24;  // what a pair adds when it runs out of tiles, so that nobody waits for it
+constexpr uint32_t kPaceLeft = 1u << 25;  // what a pair adds when it runs out of tiles, so that nobody waits for it
 struct Pace {
   volatile uint32_t count, hold;  // shared memory; the producer writes `count` (kPaceLeft at its end), the pacing thread `hold`
 };
@@ -71,9 +119,10 @@ __device__ __forceinline__ void pace_producer(Pace& pace, uint32_t count) {
   pace.count = count;
   for (int i = 0; i < 512 && pace.hold; ++i) __nanosleep(64);
 }
-__device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* sum, uint32_t pairs, volatile uint32_t* abortp) {
-  uint32_t added = 0;
-  bool may_hold = true;
+// words[0]: the sum of the counts; words[1]: the pairs in it.
+__device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* words, volatile uint32_t* abortp) {
+  uint32_t added = 0, base = 0;
+  bool may_hold = true, joined = false;
   for (uint32_t idle = 0; idle < TCEC_WAIT_LIMIT && !*abortp;) {
     const uint32_t count = pace.count;
     if (count == added) {
@@ -82,28 +131,38 @@ __device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* sum, uint3
       continue;
     }
     idle = 0;
-    uint32_t seen = atomicAdd(sum, count - added) + (count - added);
+    if (!joined) {
+      joined = true;
+      const uint32_t others = ld_relaxed_gpu(words + 1), mean = others ? ld_relaxed_gpu(words) / others : 0;
+      if (mean >= kPaceLeft / 128) return;  // some have left
+      if (mean > 4) base = mean;            // pairs that start together differ by less
+      atomicAdd(words + 1, 1u);
+    }
+    const uint32_t more = count - added + (added == 0 ? base : 0);
+    uint32_t seen = atomicAdd(words, more) + more;
     added = count;
     if (count >= kPaceLeft) return;
-    const unsigned long long wanted = static_cast<unsigned long long>(count - 1) * pairs;
+    const unsigned long long wanted = static_cast<unsigned long long>(base + count - 1) * ld_relaxed_gpu(words + 1);
     if (!may_hold || seen >= wanted) continue;
     pace.hold = 1;
     for (int i = 0; i < 128 && seen < wanted; ++i) {
       __nanosleep(200);
-      seen = ld_relaxed_gpu(sum);
+      seen = ld_relaxed_gpu(words);
     }
     may_hold = seen >= wanted;
     pace.hold = 0;
   }
-  atomicAdd(sum, kPaceLeft);
+  atomicAdd(words, kPaceLeft);
 }
 
-// p.tiles_m counts 256-row pair tiles here.  kPaced: a launch may be paced (p.pace).  Without correction launches that are not paced
-// have a kernel without it: the mere test in the producer's loop costs them 2 % (5000 x 6000 x 7000 460 us, 447).  With correction
-// there is one kernel: apart, 4096^3 took 388.4 us instead of 385.7, complex 2048^3 207.2 instead of 204.7.
-template <bool kTf32, bool kEc, int BN, bool kPaced>
+// p.tiles_m counts 256-row pair tiles here.  Without correction launches that are not paced have a kernel without it: the mere test in
+// the producer's loop costs them 2 % (5000 x 6000 x 7000 460 us, 447).  With correction strided launches have one kernel, paced or
+// not: apart, 4096^3 took 388.4 us instead of 385.7, complex 2048^3 207.2 instead of 204.7.  Drawing has a kernel of its own: as a
+// choice at run time it cost the strided launches 4 % (4096^3 390, 407).
+template <bool kTf32, bool kEc, int BN, int kMode>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     tcec_gemm_panels_pair_kernel(const GemmPanelParams p) {
+  constexpr bool kTilesDrawn = kMode == kDrawn;
   static_assert(BN == 256 || BN == 128, "whole or half-width pair tiles");
   using Cfg = GemmPairCfg<kTf32, kEc>;
   constexpr int NST = Cfg::NST;
@@ -120,6 +179,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   __shared__ uint32_t tmem_base_s;
   __shared__ uint32_t abort_flag;
   __shared__ Pace pace;
+  __shared__ uint64_t bar_tile_empty[kTileRing];  // used in the leader only
+  __shared__ uint32_t tile_ring[kTileRing];
 
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* const smem_gen = smem_raw + (smem_base - smem_u32(smem_raw));
@@ -142,6 +203,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     mbar_init(smem_u32(&bar_drain[1]), 1);
     abort_flag = 0;
     pace.count = pace.hold = 0;
+    if constexpr (kTilesDrawn)
+      for (int i = 0; i < kTileRing; ++i) {
+        mbar_init(smem_u32(&bar_tile_empty[i]), (kEc ? 2 : 1) + 8 + 10);  // MMA threads and epilogue; the peer's producer, relay, epilogue
+        tile_ring[i] = 0;
+      }
     fence_mbar_init();
   }
   if (warp == 1) {
@@ -166,7 +232,11 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   im.b_lo16 = (Cfg::A_BYTES + kPanelBytes) >> 4;
   im.idesc = umma_idesc(kTf32 ? 2u : 0u, 256, BN);
   im.a_block16 = im.b_block16 = Cfg::BLOCK >> 4;
-  const StridedTiles tiles{pair, npairs, ntiles};
+  auto tiles = [&] {
+    if constexpr (kTilesDrawn) return DrawnTiles{tile_ring, bar_tile_empty};
+    else return StridedTiles{pair, npairs, ntiles};
+  }();
+  auto more = [&](int tile) { return kTilesDrawn ? tile >= 0 : tile < ntiles; };  // a failed wait for a drawn tile is no tile either
   const KWalk walk{p.nkb, p.promo};
   const RingBarriers ring{bar_full, bar_empty};
 
@@ -176,9 +246,16 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       // ---------------------------------------------------------- producer (each CTA, own panels)
       if (elect_one()) {
         uint32_t s = 0, ph = 0, armed = 0, armed_parity = 0, it = 0;
-        const bool paced = kPaced && p.pace && leader;  // the peer's ring cannot run ahead of the leader's
+        const bool paced = kMode != kStrided && p.pace && leader;  // the peer's ring cannot run ahead of the leader's
         bool ok = true;
-        for (int tile = pair; tile < ntiles && ok; tile += npairs) {
+        [[maybe_unused]] unsigned int drawn = kTilesDrawn && leader ? atomicAdd(&p.sched[0], 1u) : 0;
+        [[maybe_unused]] const int claim_kb = p.nkb > 2 * NST * Cfg::KBS ? (p.nkb / Cfg::KBS - 2 * NST) * Cfg::KBS : 0;
+        auto drawn_tile = [&] {
+          if constexpr (kTilesDrawn) return leader ? tiles.publish(drawn, ntiles, abortp) : tiles.next(abortp);
+          else return 0;
+        };
+        int tile = kTilesDrawn ? drawn_tile() : pair;
+        for (; more(tile) && ok; tile = kTilesDrawn ? drawn_tile() : tile + npairs) {
           const TileCoord tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
           const uint8_t* pa = p.panels_a + tc.b * p.panels_a_batch_stride +
                               static_cast<size_t>(tc.mt * 2 + rank) * p.nkb * Cfg::BLOCK;
@@ -194,8 +271,17 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
               break;
             }
             if (paced && it % kPaceStages == 0) pace_producer(pace, it / kPaceStages);
+            if (kTilesDrawn && kb == claim_kb && leader) drawn = atomicAdd(&p.sched[0], 1u);
             if (dev_flag(p.debug_flags, 1) && it >= static_cast<uint32_t>(NST)) {  // develop builds: no loads
               mbar_arrive(smem_u32(&bar_full[s]));
+              if (++s == static_cast<uint32_t>(NST)) {
+                s = 0;
+                ph ^= 1;
+              }
+              continue;
+            }
+            // injected stall (failure-path test): the first stage after the first ring fill is never filled
+            if (dev_flag(p.debug_flags, 32) && it == static_cast<uint32_t>(NST)) {
               if (++s == static_cast<uint32_t>(NST)) {
                 s = 0;
                 ph ^= 1;
@@ -231,6 +317,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
           }
         }
         if (paced) pace.count = kPaceLeft;
+        if (kTilesDrawn && tile == kTileWaitFailed) ok = false;
         if (!ok) {
           raise_abort_pair(&abort_flag);
           atomicCAS(p.status, 0, kErrProducerWait);
@@ -244,7 +331,8 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
           // -------------------------------------------------------- peer: relay "my stage landed"
           uint32_t s = 0, ph = 0, it = 0;
           bool ok = true;
-          for (int tile = pair; tile < ntiles && ok; tile += npairs) {
+          int tile = kTilesDrawn ? tiles.next(abortp) : pair;
+          for (; more(tile) && ok; tile = kTilesDrawn ? tiles.next(abortp) : tile + npairs) {
             for (int kb = 0; kb < p.nkb; kb += Cfg::KBS, ++it) {
               if (!mbar_wait(smem_u32(&bar_full[s]), ph, abortp, 32)) {
                 ok = false;
@@ -257,6 +345,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
               }
             }
           }
+          if (kTilesDrawn && tile == kTileWaitFailed) ok = false;
           if (!ok) {
             raise_abort_pair(&abort_flag);
             atomicCAS(p.status, 0, kErrMmaWait);
@@ -278,9 +367,9 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
             mma_thread_gave_up<true>(&abort_flag, p.status, kErrMmaWait, &bar_drain[1]);
         }
       }
-    } else if (kPaced && p.pace && leader && elect_one()) {
+    } else if (kMode != kStrided && p.pace && leader && elect_one()) {
       // ---------------------------------------------------------- leader: pacing
-      pace_launch(pace, p.pace, static_cast<uint32_t>(npairs), abortp);
+      pace_launch(pace, p.pace, abortp);
     }
   } else {
     // ------------------------------------------------------------ epilogue (each CTA, its 128 rows)
@@ -295,8 +384,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
     const uint32_t corr_free_leader = map_to_cta(smem_u32(&bar_corr_free), 0);
     uint32_t chunk = 0, tcount = 0;
     bool ok = true;
-    for (int tile = pair; tile < ntiles && ok; tile += npairs, ++tcount) {
-      const TileCoord tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
+    int tile = pair;
+    for (; (kTilesDrawn || tile < ntiles) && ok; tile += kTilesDrawn ? 0 : npairs, ++tcount) {
+      TileCoord tc{};
+      if constexpr (kTilesDrawn) {
+        tile = tiles.template at<true>(tcount, abortp);
+        if (tile < 0) break;
+      } else {
+        tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
+      }
       const int nchunks = p.promo ? (p.nkb + p.promo - 1) / p.promo : 1;
       float acc[NC];
       for (int c = 0; c < nchunks; ++c, ++chunk) {
@@ -321,6 +417,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
         }
         tc_fence_after();
       }
+      if constexpr (kTilesDrawn) tc = decode_tile(p.tile_first + tile / HALVES, p.tiles_m, p.tiles_n, Cfg::GROUP_M);
       float* cbase = p.c_array ? p.c_array[tc.b] : p.c + tc.b * p.c_batch_stride;
       const int col0 = tc.nt * 256 + (tile % HALVES) * BN + colbase;
       const bool vec_ok = vec_store && ((reinterpret_cast<uintptr_t>(cbase) & 15) == 0);
@@ -341,6 +438,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       st.beta = p.beta;
       store_warp_block<true>(acc, tc.mt * 256 + static_cast<int>(rank) * 128 + q * 32, col0, st, reinterpret_cast<float*>(smem_gen + Cfg::EPI_OFFSET) + ew * kEpiBufFloats, lane);
     }
+    if (kTilesDrawn && tile == kTileWaitFailed) ok = false;
     if (!ok) {
       raise_abort_pair(&abort_flag);
       if (lane == 0) atomicCAS(p.status, 0, kErrEpilogueWait);
@@ -351,6 +449,15 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
   __syncthreads();
   cluster_sync_all();  // neither CTA leaves while the other may still signal it or read its operands
   if (warp == 1) tmem_dealloc_pair(tmem_base_s, Cfg::TMEM_COLS);
+  if (kTilesDrawn && leader && threadIdx.x == 0) {
+    // Every pair has drawn its end mark by now; the last one out leaves the counters at zero.
+    __threadfence();
+    if (atomicAdd(&p.sched[1], 1u) == static_cast<unsigned int>(npairs) - 1) {
+      p.sched[0] = 0;
+      p.sched[1] = 0;
+      __threadfence();
+    }
+  }
 }
 
 }  // namespace tcec_sm100

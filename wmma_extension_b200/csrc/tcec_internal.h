@@ -42,7 +42,12 @@ struct Options {
 };
 Options snapshot_options();
 
-constexpr int kStatusBytes = 128, kPaceSlots = 63, kPaceSlotBytes = 128;  // what a device's `status` allocation holds
+// What a device's `status` allocation holds: the status word, and 63 lines for the pair launches of as many streams, each two pacing
+// words and two tile counters.
+constexpr int kStatusBytes = 128, kPairLines = 63, kPairLineBytes = 128;
+struct PairLine {
+  unsigned int pace[2], sched[2];
+};
 
 struct Workspace {
   void* ptr = nullptr;
@@ -59,8 +64,8 @@ struct DeviceState {
   bool attrs_done = false;
   std::map<cudaStream_t, Workspace> ws;
   std::map<cudaStream_t, unsigned int*> sched;  // per stream: the panel GEMM's two tile-scheduler counters
-  unsigned int* pace = nullptr;                 // kPaceSlots words, 128 bytes apart, in the allocation of `status`
-  std::map<cudaStream_t, int> pace_slot;        // which of them a stream uses
+  uint8_t* pair_lines = nullptr;                // kPairLines lines in the allocation of `status`
+  std::map<cudaStream_t, int> pair_line;        // which of them a stream uses
   unsigned int* sched_fixed = nullptr;          // set instead by the allocation-free entry (a device symbol)
   StepState* step = nullptr;
 };
