@@ -107,12 +107,30 @@ __device__ __forceinline__ void wait_for_launch_before() { asm volatile("griddep
 // another.  The panel GEMMs do not: a split follows them, and its small CTAs would all crowd on the SMs that the GEMM leaves
 // idle (1000 x 777 x 1111 21.2 us, 1500 x 1400 x 300 14.1).
 __device__ __forceinline__ void let_next_launch_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-// The pointer as a value that the compiler does not know before the wait above: loads through it that are declared read-only
-// (__ldg) are not moved in front of the wait.
+// The pointer as a value that the compiler does not know before the wait above: loads through it are not moved in front of the wait.
 template <class T>
 __device__ __forceinline__ T* after_wait(T* p) {
   asm volatile("" : "+l"(p) : : "memory");
   return p;
+}
+// Operand loads of the kernels that start early.  The compiler may order them freely among stores, as it may __ldg, but they are
+// ordinary coherent loads: __ldg's path is for data that nobody writes while the kernel is there, and an early kernel is there,
+// perhaps on the same SM, while the one before still writes its operands.  They cost nothing (16384 x 64^3 182.6 us with __ldg, 180.7;
+// 8192^3 without correction and its split 1045, 1061 with runs 2.6 % apart).
+__device__ __forceinline__ float ld_operand(const float* p) {
+  float v;
+  asm("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 ld_operand(const float2* p) {
+  float2 v;
+  asm("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float4 ld_operand(const float4* p) {
+  float4 v;
+  asm("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+  return v;
 }
 
 // ---------------------------------------------------------------- fences

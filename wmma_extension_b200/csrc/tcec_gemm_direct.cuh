@@ -140,7 +140,7 @@ __device__ __forceinline__ void loader_read(float (&v)[16], const LoaderOperand&
       const float* q = (i == 0 ? o.p : o.p1) + static_cast<long long>(k0) * ld;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        v[8 * i + e] = (kFull || e < kleft) ? __ldg(q) : 0.f;
+        v[8 * i + e] = (kFull || e < kleft) ? ld_operand(q) : 0.f;
         q += ld;
       }
     }
@@ -152,11 +152,11 @@ __device__ __forceinline__ void loader_read(float (&v)[16], const LoaderOperand&
       float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
       if (i == 0 || 4 * i < o.rows) {
         if (kFull || kleft >= 4) {
-          t = __ldg(reinterpret_cast<const float4*>(q));
+          t = ld_operand(reinterpret_cast<const float4*>(q));
         } else {
-          if (kleft > 0) t.x = __ldg(q);
-          if (kleft > 1) t.y = __ldg(q + 1);
-          if (kleft > 2) t.z = __ldg(q + 2);
+          if (kleft > 0) t.x = ld_operand(q);
+          if (kleft > 1) t.y = ld_operand(q + 1);
+          if (kleft > 2) t.z = ld_operand(q + 2);
         }
       }
       v[4 * i] = t.x;
@@ -171,8 +171,8 @@ __device__ __forceinline__ void loader_read(float (&v)[16], const LoaderOperand&
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const bool row = i == 0 || 2 * i < o.rows;
-      v[2 * i] = (row && (kFull || kleft > 0)) ? __ldg(q) : 0.f;
-      v[2 * i + 1] = (row && (kFull || kleft > 1)) ? __ldg(q + 1) : 0.f;
+      v[2 * i] = (row && (kFull || kleft > 0)) ? ld_operand(q) : 0.f;
+      v[2 * i + 1] = (row && (kFull || kleft > 1)) ? ld_operand(q + 1) : 0.f;
       q += 2 * ld;
     }
   }

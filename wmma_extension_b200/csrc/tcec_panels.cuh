@@ -120,7 +120,7 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
       if (row < p.rows && kk + KCH <= p.k && vec_ok) {
 #pragma unroll
         for (int q = 0; q < KCH / 4; ++q) {
-          const float4 t = __ldg(reinterpret_cast<const float4*>(s) + q);
+          const float4 t = ld_operand(reinterpret_cast<const float4*>(s) + q);
           v[4 * q + 0] = t.x;
           v[4 * q + 1] = t.y;
           v[4 * q + 2] = t.z;
@@ -128,13 +128,13 @@ __device__ __forceinline__ void split_one_panel(const SplitParams& p, int kb, in
         }
       } else {
 #pragma unroll
-        for (int q = 0; q < KCH; ++q) v[q] = (row < p.rows && kk + q < p.k) ? __ldg(s + q) : 0.f;
+        for (int q = 0; q < KCH; ++q) v[q] = (row < p.rows && kk + q < p.k) ? ld_operand(s + q) : 0.f;
       }
     } else {
 #pragma unroll
       for (int q = 0; q < KCH; ++q)
         v[q] = (row < p.rows && kk + q < p.k)
-                   ? __ldg(src + static_cast<long long>(kk + q) * p.ld + row)
+                   ? ld_operand(src + static_cast<long long>(kk + q) * p.ld + row)
                    : 0.f;
     }
     uint4 hi, lo;
@@ -182,7 +182,7 @@ __device__ __forceinline__ void split_complex_panel(const ComplexSplitParams& p,
     for (int e = 0; e < PC; ++e) {
       const float* x = q + 2 * e * step;
       z[e] = make_float2(0.f, 0.f);
-      if (row < p.rows && k0 + e < p.k) z[e] = pairs ? __ldg(reinterpret_cast<const float2*>(x)) : make_float2(__ldg(x), __ldg(x + 1));
+      if (row < p.rows && k0 + e < p.k) z[e] = pairs ? ld_operand(reinterpret_cast<const float2*>(x)) : make_float2(ld_operand(x), ld_operand(x + 1));
     }
     const int halves = p.doubled ? 2 : 1;
     for (int h = 0; h < halves; ++h) {
