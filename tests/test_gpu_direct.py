@@ -63,6 +63,50 @@ def test_same_bits_as_the_panel_path(m, n, k, batch, policy):
             cbuf.copy_(before)
 
 
+def _strided(gen, batch, rows, cols, k_contiguous, pad, stride_pad, is_b):
+    """Operand of which K is contiguous or not, `pad` elements after each row of memory, `stride_pad` after each matrix; stride_pad None: one
+    matrix for all."""
+    r, c = (rows, cols) if k_contiguous != is_b else (cols, rows)
+    ld = c + pad
+    stride = 0 if stride_pad is None else r * ld + stride_pad
+    buf = torch.rand(((batch - 1) * stride + r * ld,), generator=gen, device=DEV).mul_(2).sub_(1)
+    v = buf.as_strided((batch, r, c), (stride, ld, 1))
+    return v if k_contiguous != is_b else v.transpose(1, 2)
+
+
+# Three or more tiles a CTA, so that a lane's pointers are carried from tile to tile, and a last tile that is not full.
+@pytest.mark.parametrize("m,n,k,per_tile", [
+    (32, 32, 32, 4), (20, 31, 40, 4), (31, 32, 33, 4), (64, 64, 64, 2), (50, 40, 100, 2), (33, 64, 31, 2), (128, 128, 64, 1), (100, 127, 36, 1),
+    (65, 128, 97, 1),
+])
+@pytest.mark.parametrize("policy", ["fp16_ec", "tf32_ec"])
+def test_pointers_carried_over_many_tiles(m, n, k, per_tile, policy):
+    gen = torch.Generator(device=DEV).manual_seed(m + n + k)
+    batch = per_tile * 148 * 3 + (per_tile + 1) // 2  # the last tile holds half of what it could
+    # pad to a leading dimension that is a multiple of 4 or not, and to a stride that is or not; for A and B alike and crossed
+    def pads(ka, kb):
+        ca, cb = (k if ka else m), (k if kb else n)
+        for ld4_a, s4_a, ld4_b, s4_b in ((1, 1, 1, 1), (1, 0, 1, 1), (1, 1, 1, 0), (0, 0, 1, 1), (1, 1, 0, 0), (0, 1, 0, 1), (1, None, 1, 1),
+                                         (1, 1, 1, None), (0, None, 0, None)):
+            def pad(cols, ld4):
+                return -cols % 4 if ld4 else (1 if (cols + 1) % 4 else 2)
+            def extra(s4):
+                return None if s4 is None else 4 if s4 else 1
+            yield pad(ca, ld4_a), extra(s4_a), pad(cb, ld4_b), extra(s4_b)
+
+    for ka in (True, False):
+        for kb in (True, False):
+            for pa, sa, pb, sb in pads(ka, kb):
+                a = _strided(gen, batch, m, k, ka, pa, sa, False)
+                b = _strided(gen, batch, k, n, kb, pb, sb, True)
+                c = torch.full((batch, m, n), float("nan"), device=DEV)
+                _run(False, a, b, c, 1.0, 0.0, policy, False)
+                want = c.clone()
+                c.fill_(float("nan"))
+                _run(True, a, b, c, 1.0, 0.0, policy, False)
+                assert torch.equal(c, want), (ka, kb, pa, sa, pb, sb)
+
+
 def test_non_finite_operands_stay_in_their_rows_and_columns():
     gen = torch.Generator(device=DEV).manual_seed(3)
     for m, n, batch in ((40, 40, 6), (20, 30, 9), (100, 90, 2)):

@@ -37,13 +37,17 @@ def test_divided_k_is_no_further_from_fp64_than_undivided(m, n, k, policy):
             # Errors relative to what the elements of C are expected to be (products of elements of variance 1/3), not to what they
             # are: a single element may lie close to zero.
             size = abs(alpha) * (m * n * k) ** 0.5 / 3
-            out = {}
+            out, bits = {}, {}
             for parts in (1, 2, 4, 8):
                 tcec.set_option("k_parts", parts)
                 c = torch.full_like(c0, float("nan")) if beta == 0.0 else c0.clone()
                 tcec.sgemm(a, b, c, alpha=alpha, beta=beta, policy=policy)
                 tcec.device_status()
                 out[parts] = (c.double() - exact).norm().item() / size
+                bits[parts] = c
+            # the option does divide: added in parts, some sums of a hundred and more round in another way
+            if policy.endswith("_ec") and not policy.endswith("no_ec"):
+                assert not any(torch.equal(bits[p], bits[q]) for p in bits for q in bits if p < q), (layouts, alpha)
             # On few elements the undivided error may be small by chance.  Adding the parts rounds once per part, by at most 2^-24
             # of sums that are seldom larger than three times the expected size.
             for parts in (2, 4, 8):

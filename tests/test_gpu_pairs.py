@@ -1,4 +1,5 @@
 """The CTA-pair kernel where its launch is paced or draws its tiles: the bits of the one-SM kernel, whatever else runs."""
+import ctypes
 import time
 
 import pytest
@@ -113,23 +114,64 @@ def test_a_long_call_waits_for_no_sms_that_another_kernel_holds(policy):
 
 
 def test_paced_launches_overlap_on_streams_and_in_a_replayed_graph():
-    """A graph replayed beside calls on the stream it was captured on shares that stream's word; a 64th stream has none."""
-    a, b = _operands(5120, 4096, 5472, 7)
+    """Products of packed operands, which share nothing else.  A graph replayed beside calls on the stream that it was captured on shares
+    that stream's pacing words."""
+    m, n, k = 5120, 4096, 5472
+    a, b = _operands(m, n, k, 7)
     want = _one_sm(a, b, "fp16_ec")
+    ap, bp = tcec.pack_a(a), tcec.pack_b(b)
     torch.cuda.synchronize()
     streams = [torch.cuda.Stream() for _ in range(4)]
-    outs = []
-    for s in streams:
+    outs = [torch.zeros_like(want) for _ in range(16)]
+    captured = torch.zeros_like(want)
+    torch.cuda.synchronize()
+    for s, out in zip(streams, outs):
         with torch.cuda.stream(s):
-            outs.append(tcec.sgemm(a, b))
+            tcec.sgemm_packed(ap, bp, m, n, k, out)
     torch.cuda.synchronize()
-    graph, captured = torch.cuda.CUDAGraph(), torch.zeros_like(want)
+    graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph, stream=streams[0]):
-        tcec.sgemm(a, b, captured)
-    for _ in range(3):
-        graph.replay()
+        tcec.sgemm_packed(ap, bp, m, n, k, captured)
+    for i in range(3):
+        captured.zero_()
+        torch.cuda.synchronize()
         with torch.cuda.stream(streams[1]):
-            outs.append(tcec.sgemm(a, b))
-    torch.cuda.synchronize()
-    assert torch.equal(captured, want) and all(torch.equal(o, want) for o in outs)
+            for _ in range(4):
+                graph.replay()
+        with torch.cuda.stream(streams[0]):
+            for j in range(4):
+                tcec.sgemm_packed(ap, bp, m, n, k, outs[4 + 4 * i + j])
+        torch.cuda.synchronize()
+        assert torch.equal(captured, want)
+    assert all(torch.equal(o, want) for o in outs)
     tcec.device_status()
+
+
+def test_more_streams_than_there_are_lines():
+    """Every stream beyond the 63rd draws its tiles from counters of its own and is not paced."""
+    cudart = torch.cuda.cudart()
+    handles = []
+    for _ in range(70):  # torch's own streams are fewer
+        handle = ctypes.c_void_p(0)
+        assert int(cudart.cudaStreamCreate(ctypes.addressof(handle))) == 0
+        handles.append(handle.value)
+    try:
+        for m, n, k in ((5120, 4096, 5472), (4900, 5000, 5300)):  # paced; paced and drawn
+            a, b = _operands(m, n, k, 8)
+            want = _one_sm(a, b, "fp16_ec")
+            ap, bp = tcec.pack_a(a), tcec.pack_b(b)
+            outs = [torch.zeros_like(want) for _ in handles]
+            torch.cuda.synchronize()
+            for _ in range(2):
+                for h, out in zip(handles, outs):
+                    with torch.cuda.stream(torch.cuda.ExternalStream(h)):
+                        tcec.sgemm_packed(ap, bp, m, n, k, out)
+            torch.cuda.synchronize()
+            assert all(torch.equal(o, want) for o in outs)
+            del outs
+        tcec.device_status()
+    finally:
+        torch.cuda.synchronize()
+        tcec.destroy()  # the lines are free again
+        for h in handles:
+            cudart.cudaStreamDestroy(h)
