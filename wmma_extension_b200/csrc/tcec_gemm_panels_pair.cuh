@@ -57,7 +57,7 @@ struct GemmPairCfg {
 // How the pairs of a launch share its tiles.  Strided: pair, pair + npairs, ...; with code for pacing (below) or without.  Drawn
 // (and perhaps paced): from a device-wide counter, so that a pair that got its SMs late (another stream's kernel was there) takes
 // fewer tiles instead of starting its whole share when the others are done: 8192 x 8192 x 4096 beside a kernel that holds four SMs
-// 1884 us strided, 1226 drawn; alone 1179 and 1172.
+// 1890 us strided, 1200 drawn; alone 1210 and 1180.
 enum PairTileMode : int { kStrided, kStridedPaced, kDrawn };
 
 // Drawn tiles.  The leader's producer claims the next tile late in the one before, early enough for the counter's answer, and
@@ -107,8 +107,9 @@ struct DrawnTiles {
 // L2.  Left alone they drift apart, tile after tile, until most panels are fetched several times.
 // Every kPaceStages stages the leader's producer raises its count.  A thread of its own (the producer has no time for a round
 // trip to L2: 16384^3 without correction 8.0 ms that way, 7.3 this way) adds it to a device-wide sum and holds the producer while
-// its count is more than one above the mean of the pairs that run.  One that starts when the others are well under way counts from
-// where they are.  A hold is bounded, and whoever has held in vain holds no more.
+// its count is more than one above the mean of the pairs that have started: one whose SMs another kernel has taken must not stop the
+// rest, and one that starts when the others are well under way counts from where they are.  A hold is bounded, and whoever has held
+// in vain holds no more.
 // 16384^3: 21.4 ms unpaced, 19.3 every 4 or 8 stages, 19.6 every 16; the words are a hint, results do not depend on them.
 constexpr uint32_t kPaceStages = 8;
 constexpr uint32_t kPaceLeft = 1u << 25;  // what a pair adds when it runs out of tiles, so that nobody waits for it
@@ -119,10 +120,16 @@ __device__ __forceinline__ void pace_producer(Pace& pace, uint32_t count) {
   pace.count = count;
   for (int i = 0; i < 512 && pace.hold; ++i) __nanosleep(64);
 }
-// words[0]: the sum of the counts; words[1]: the pairs in it.
-__device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* words, volatile uint32_t* abortp) {
-  uint32_t added = 0, base = 0;
-  bool may_hold = true, joined = false;
+// words[0]: the sum of the counts; words[1]: the pairs in it, each from its start on: from its first count on, those that start some
+// microseconds before others did not wait for them (16384^3 without correction with the GPU hot 7.6 ms, 7.9 that way).
+__device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* words, uint32_t pairs, volatile uint32_t* abortp) {
+  const uint32_t others = ld_relaxed_gpu(words + 1), mean = others ? ld_relaxed_gpu(words) / others : 0;
+  if (mean >= kPaceLeft / 128) return;        // some have left
+  const uint32_t base = mean > 16 ? mean : 0;  // pairs that the launch has SMs for start closer together
+  atomicAdd(words + 1, 1u);
+  if (base) atomicAdd(words, base);
+  uint32_t added = 0;
+  bool may_hold = true;
   for (uint32_t idle = 0; idle < TCEC_WAIT_LIMIT && !*abortp;) {
     const uint32_t count = pace.count;
     if (count == added) {
@@ -131,20 +138,13 @@ __device__ __forceinline__ void pace_launch(Pace& pace, unsigned int* words, vol
       continue;
     }
     idle = 0;
-    if (!joined) {
-      joined = true;
-      const uint32_t others = ld_relaxed_gpu(words + 1), mean = others ? ld_relaxed_gpu(words) / others : 0;
-      if (mean >= kPaceLeft / 128) return;  // some have left
-      if (mean > 4) base = mean;            // pairs that start together differ by less
-      atomicAdd(words + 1, 1u);
-    }
-    const uint32_t more = count - added + (added == 0 ? base : 0);
-    uint32_t seen = atomicAdd(words, more) + more;
+    uint32_t seen = atomicAdd(words, count - added) + (count - added);
     added = count;
     if (count >= kPaceLeft) return;
-    const unsigned long long wanted = static_cast<unsigned long long>(base + count - 1) * ld_relaxed_gpu(words + 1);
-    if (!may_hold || seen >= wanted) continue;
+    const unsigned long long wanted_of_one = base + count - 1;
+    if (!may_hold || seen >= wanted_of_one * pairs) continue;
     pace.hold = 1;
+    const unsigned long long wanted = wanted_of_one * ld_relaxed_gpu(words + 1);  // all pairs, or fewer
     for (int i = 0; i < 128 && seen < wanted; ++i) {
       __nanosleep(200);
       seen = ld_relaxed_gpu(words);
@@ -369,7 +369,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       }
     } else if (kMode != kStrided && p.pace && leader && elect_one()) {
       // ---------------------------------------------------------- leader: pacing
-      pace_launch(pace, p.pace, abortp);
+      pace_launch(pace, p.pace, static_cast<uint32_t>(npairs), abortp);
     }
   } else {
     // ------------------------------------------------------------ epilogue (each CTA, its 128 rows)
