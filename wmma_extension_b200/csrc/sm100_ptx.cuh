@@ -64,26 +64,25 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // Bounded waits.  `abort_flag` is a CTA-shared word any role may raise; a waiter that sees
 // it raised, or that runs out of polls, returns false.
 //
-// A try_wait suspends its thread in hardware for a while, so a loop of them polls seldom; sleeping between polls on top of that
-// only delays the hand-offs (2048^3 62.4 -> 62.1 us, complex 203.3 -> 200.1, 16384^3 19.45 -> 19.36 ms without).  Only waits that go
-// on for `awake` polls sleep, `ns` a poll (0: never), so that the limit is long in time: operands may be on their way from another
-// GPU.  Without correction and with a long K the epilogue sleeps at once (awake = 0): it waits for a tile's whole K, and the MMAs'
-// operand reads need the shared-memory cycles (8192^3 1070 -> 1043 us; but 8 x 2048^3 186 -> 191).
+// A try_wait suspends its thread in hardware for a while, so a loop of them polls seldom, and the MMAs' operand reads do not notice it:
+// sleeping between polls on top of that measures the same, for the epilogue of a tile of long K too (8192^3 without correction 889 us
+// with its waits asleep, 886 awake; 8 x 2048^3 209, 205; 16384^3 6.72 ms, 6.75; runs 1 % apart).  Only waits that go on for kPollsAwake
+// polls sleep, `ns` a poll (0: never), so that the limit is long in time: operands may be on their way from another GPU.
 constexpr uint32_t kPollsAwake = 512;
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
-                                          uint32_t ns = 64, uint32_t awake = kPollsAwake) {
+                                          uint32_t ns = 64) {
   for (uint32_t i = 0; i < TCEC_WAIT_LIMIT; ++i) {
     if (mbar_try_wait(bar, parity)) return true;
-    if (ns && i >= awake) __nanosleep(ns);
+    if (ns && i >= kPollsAwake) __nanosleep(ns);
     if ((i & 0x3ff) == 0x3ff && *abort_flag) return false;
   }
   return false;
 }
 // Warp-collective form: lane 0 polls, the result is broadcast.
 __device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag,
-                                               uint32_t ns = 128, uint32_t awake = kPollsAwake) {
+                                               uint32_t ns = 128) {
   bool ok = true;
-  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, ns, awake);
+  if ((threadIdx.x & 31) == 0) ok = mbar_wait(bar, parity, abort_flag, ns);
   return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
 }
 

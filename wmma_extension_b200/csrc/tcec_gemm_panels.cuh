@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(GemmPanelCfg<BN, kTf32, kEc>::THREADS, 1)
       const int nchunks = p.promo ? (p.nkb + p.promo - 1) / p.promo : 1;
       float acc[128];
       for (int c = 0; c < nchunks; ++c, ++chunk) {
-        if (!mbar_wait_warp(smem_u32(&bar_main_full), chunk & 1, abortp, 128, kEc || p.nkb <= 128 ? kPollsAwake : 0)) {
+        if (!mbar_wait_warp(smem_u32(&bar_main_full), chunk & 1, abortp)) {
           ok = false;
           break;
         }

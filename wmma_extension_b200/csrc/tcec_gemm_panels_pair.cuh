@@ -396,7 +396,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(384, 1)
       const int nchunks = p.promo ? (p.nkb + p.promo - 1) / p.promo : 1;
       float acc[NC];
       for (int c = 0; c < nchunks; ++c, ++chunk) {
-        if (!mbar_wait_warp(smem_u32(&bar_main_full), chunk & 1, abortp, 128, kEc || p.nkb <= 128 ? kPollsAwake : 0)) {
+        if (!mbar_wait_warp(smem_u32(&bar_main_full), chunk & 1, abortp)) {
           ok = false;
           break;
         }
