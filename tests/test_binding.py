@@ -88,6 +88,37 @@ assert got == [None] * 5, got
     subprocess.run([sys.executable, "-c", code], check=True, timeout=120, cwd=os.path.dirname(os.path.dirname(tcec.__file__)))
 
 
+@pytest.mark.gpu
+def test_an_exception_out_of_the_library_leaves_the_call_to_python(tmp_path):
+    """A library whose calls throw (as on a host that is out of memory), in a process of its own: the interpreter goes on, and every call
+    is left to the Python code."""
+    source, library = tmp_path / "throws.cpp", tmp_path / "throws.so"
+    source.write_text('#include <new>\n#include <cstddef>\nextern "C" { int call(...) { throw std::bad_alloc(); } size_t bytes(int, int, int) { return 16; } }\n')
+    subprocess.run(["g++", "-shared", "-fPIC", "-o", str(library), str(source)], check=True)
+    copy = shutil.copy(tcec._binding.__file__, tmp_path / "_binding.so")
+    code = f"""
+import ctypes, importlib.util, threading, torch
+lib = ctypes.CDLL({str(library)!r})
+spec = importlib.util.spec_from_file_location("_binding", {str(copy)!r})
+binding = importlib.util.module_from_spec(spec)
+spec.loader.exec_module(binding)
+call, bytes_ = (ctypes.cast(f, ctypes.c_void_p).value for f in (lib.call, lib.bytes))
+binding.bind(call, call, call, call, call, bytes_)
+x = torch.zeros(4, 4, device="cuda:0")
+p = torch.zeros(16, dtype=torch.uint8, device="cuda:0")
+def run():
+    for _ in range(200):
+        got = [binding.sgemm(x, x, None, 1.0, 0.0, 0), binding.strided(x[None], x[None], None, 1.0, 0.0, 0), binding.pack_a(x, 0, None),
+               binding.pack_b(x, 0, p), binding.sgemm_packed(p, p, 4, 4, 4, None, 1.0, 0.0, 0)]
+        assert got == [None] * 5, got
+threads = [threading.Thread(target=run) for _ in range(4)]
+[t.start() for t in threads]
+[t.join() for t in threads]
+run()
+"""
+    subprocess.run([sys.executable, "-c", code], check=True, timeout=120, cwd=os.path.dirname(os.path.dirname(tcec.__file__)))
+
+
 def _calls_without_room(dev):
     """Calls whose result, packed operands or second operand are not where or as large as the kernels would take them to be."""
     def f(*shape, device=dev):

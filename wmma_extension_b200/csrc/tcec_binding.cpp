@@ -87,6 +87,18 @@ PyObject* answer(int status, PyObject* given, std::optional<at::Tensor>& made) {
   return given;
 }
 
+// Other threads run while the library is called; back in, an exception on its way too.
+class OthersRun {
+ public:
+  OthersRun() : state_(PyEval_SaveThread()) {}
+  ~OthersRun() { PyEval_RestoreThread(state_); }
+  OthersRun(const OthersRun&) = delete;
+  OthersRun& operator=(const OthersRun&) = delete;
+
+ private:
+  PyThreadState* state_;
+};
+
 template <class Body>
 PyObject* guarded(Body body) {
   try {
@@ -124,13 +136,14 @@ PyObject* product(PyObject* const* args, Py_ssize_t n_args) {
     float* pc = static_cast<float*>(out.data_ptr());
     void* stream = stream_here();
     int status;
-    Py_BEGIN_ALLOW_THREADS;
-    if constexpr (kDims == 3)
-      status = g_strided(la.order, lb.order, lc.order, m, n, k, alpha, pa, la.ld, a->stride(0), pb, lb.ld, b->stride(0), beta, pc, lc.ld,
-                         out.stride(0), batch, policy, stream);
-    else
-      status = g_sgemm(la.order, lb.order, lc.order, m, n, k, alpha, pa, la.ld, pb, lb.ld, beta, pc, lc.ld, policy, stream);
-    Py_END_ALLOW_THREADS;
+    {
+      const OthersRun others_run;
+      if constexpr (kDims == 3)
+        status = g_strided(la.order, lb.order, lc.order, m, n, k, alpha, pa, la.ld, a->stride(0), pb, lb.ld, b->stride(0), beta, pc, lc.ld,
+                           out.stride(0), batch, policy, stream);
+      else
+        status = g_sgemm(la.order, lb.order, lc.order, m, n, k, alpha, pa, la.ld, pb, lb.ld, beta, pc, lc.ld, policy, stream);
+    }
     return answer(status, args[2], made);
   });
 }
@@ -156,9 +169,10 @@ PyObject* pack(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     const float* src = static_cast<const float*>(x->data_ptr());
     void *dst = (given ? *given : *made).data_ptr(), *stream = stream_here();
     int status;
-    Py_BEGIN_ALLOW_THREADS;
-    status = g_pack[kB](l.order, first, second, src, l.ld, dst, policy, stream);
-    Py_END_ALLOW_THREADS;
+    {
+      const OthersRun others_run;
+      status = g_pack[kB](l.order, first, second, src, l.ld, dst, policy, stream);
+    }
     return answer(status, args[2], made);
   });
 }
@@ -184,9 +198,10 @@ PyObject* sgemm_packed(PyObject*, PyObject* const* args, Py_ssize_t n_args) {
     float* pc = static_cast<float*>(out.data_ptr());
     void* stream = stream_here();
     int status;
-    Py_BEGIN_ALLOW_THREADS;
-    status = g_packed(l.order, m, n, k, alpha, pa, pb, beta, pc, l.ld, policy, stream);
-    Py_END_ALLOW_THREADS;
+    {
+      const OthersRun others_run;
+      status = g_packed(l.order, m, n, k, alpha, pa, pb, beta, pc, l.ld, policy, stream);
+    }
     return answer(status, args[5], made);
   });
 }
