@@ -26,9 +26,9 @@ struct Options {
   int promote_k = -1;   // -1: chosen per call from K and the policy
   int tile_n = 0;
   int store_turn = 1;   // 0: the panel kernel stores directly and leaves ~30 KB of shared memory per SM free
-  int static_tiles = 0; // 0: tiles beyond the first wave are drawn from a device-wide counter; 1: static striding
+  int static_tiles = 0; // 0: single SMs, and pairs in long calls with correction, draw tiles from a device-wide counter; 1: static striding
   int reserve_sms = 0;  // SMs the GEMM kernels leave idle (for a caller's communication kernels)
-  int cta_pair = -1;    // -1: CTA-pair kernel for the policies without error correction; 0: never; 1: whenever it applies
+  int cta_pair = -1;    // -1: chosen per call (pairs_pay); 0: never; 1: whenever it applies
   int half_tiles = 1;   // CTA-pair kernel: calls with very few tiles run on 256 x 128 half tiles
   int path = 0;         // 0: chosen per call, 1: always operand panels, 2: FP32-tile kernel whenever it applies
   int narrow_tiles = -1;   // panels: width of the narrow tiles (32, 64, 128) for calls with few tiles; -1: chosen per call; 0: never
